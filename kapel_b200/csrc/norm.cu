@@ -132,11 +132,13 @@ __global__ void add_rmsnorm_reg_kernel(float* __restrict__ residual, const Src<T
 
 // bfloat16 branch, weights and output with a width that is a multiple of eight: a thread keeps up
 // to CPT chunks of eight components in registers and moves them with 16-byte loads and stores.
-template <int CPT>
-__global__ void add_rmsnorm_bf16x8_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ branch,
+// CENTER: either norm may take the row's mean off first (`center_post`, `center_next`), in a sum of its own ahead of the
+// squares' as the row is in registers anyway.
+template <int CPT, bool CENTER = false>
+__global__ void __launch_bounds__(1024) add_rmsnorm_bf16x8_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ branch,
                                           const __nv_bfloat16* __restrict__ w_post, float eps_post, float off_post,
                                           const __nv_bfloat16* __restrict__ w_next, float eps_next, float off_next,
-                                          __nv_bfloat16* __restrict__ h, int width) {
+                                          __nv_bfloat16* __restrict__ h, int width, int center_post, int center_next) {
     __shared__ float scratch[32];
     const size_t base = (size_t)blockIdx.x * width;
     const int chunks = width >> 3;
@@ -164,6 +166,24 @@ __global__ void add_rmsnorm_bf16x8_kernel(float* __restrict__ residual, const __
         }
     }
     float inv = 1.f;
+    if (CENTER && center_post && w_post != nullptr) {
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            if (threadIdx.x + c * blockDim.x < chunks)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) sum += b[c][j];
+        const float mean = block_sum(sum, scratch) / (float)width;
+        ss = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            if (threadIdx.x + c * blockDim.x < chunks)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    b[c][j] -= mean;
+                    ss += b[c][j] * b[c][j];
+                }
+    }
     if (w_post != nullptr) {
         ss = block_sum(ss, scratch);
         inv = 1.f / sqrtf(ss / (float)width + eps_post);
@@ -208,6 +228,24 @@ __global__ void add_rmsnorm_bf16x8_kernel(float* __restrict__ residual, const __
         }
         return;
     }
+    if (CENTER && center_next) {
+        float sum = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            if (threadIdx.x + c * blockDim.x < chunks)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) sum += r[c][j];
+        const float mean = block_sum(sum, scratch) / (float)width;
+        ss2 = 0.f;
+#pragma unroll
+        for (int c = 0; c < CPT; ++c)
+            if (threadIdx.x + c * blockDim.x < chunks)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    r[c][j] -= mean;
+                    ss2 += r[c][j] * r[c][j];
+                }
+    }
     ss2 = block_sum(ss2, scratch);
     const float inv2 = 1.f / sqrtf(ss2 / (float)width + eps_next);
 #pragma unroll
@@ -228,15 +266,33 @@ __global__ void add_rmsnorm_bf16x8_kernel(float* __restrict__ residual, const __
     }
 }
 
+// The mean over the row off every value of this thread's groups of four; the thread's share of the squares' sum.
+template <int CPT>
+__device__ __forceinline__ float center_groups(float4 (&v)[CPT], int chunks, int width, float* scratch) {
+    float sum = 0.f;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+        if (threadIdx.x + c * blockDim.x < chunks) sum += v[c].x + v[c].y + v[c].z + v[c].w;
+    const float mean = block_sum(sum, scratch) / (float)width;
+    float ss = 0.f;
+#pragma unroll
+    for (int c = 0; c < CPT; ++c)
+        if (threadIdx.x + c * blockDim.x < chunks) {
+            v[c].x -= mean; v[c].y -= mean; v[c].z -= mean; v[c].w -= mean;
+            ss += v[c].x * v[c].x + v[c].y * v[c].y + v[c].z * v[c].z + v[c].w * v[c].w;
+        }
+    return ss;
+}
+
 // Float32 partial sums of a product split over K (few rows: a decode step), bfloat16 weights and
 // output, a width that is a multiple of four: a thread owns up to CPT groups of four components,
 // reads each slice's four with one 16-byte load, eight slices in flight, and adds them in slice
 // order. The rest is the register-resident kernel's.
-template <int CPT>
-__global__ void add_rmsnorm_splits_kernel(float* __restrict__ residual, const float* __restrict__ parts, int splits, size_t stride,
+template <int CPT, bool CENTER = false>
+__global__ void __launch_bounds__(1024) add_rmsnorm_splits_kernel(float* __restrict__ residual, const float* __restrict__ parts, int splits, size_t stride,
                                           const __nv_bfloat16* __restrict__ w_post, float eps_post, float off_post,
                                           const __nv_bfloat16* __restrict__ w_next, float eps_next, float off_next,
-                                          __nv_bfloat16* __restrict__ h, int width KB_TL_PARAM) {
+                                          __nv_bfloat16* __restrict__ h, int width, int center_post, int center_next KB_TL_PARAM) {
     __shared__ float scratch[32];
     KB_TL_ENTER(norm, blockIdx.x == 0, 2, splits, w_next != nullptr);
     const size_t base = (size_t)blockIdx.x * width;
@@ -288,6 +344,7 @@ __global__ void add_rmsnorm_splits_kernel(float* __restrict__ residual, const fl
         }
     }
     float inv = 1.f;
+    if (CENTER && center_post && w_post != nullptr) ss = center_groups<CPT>(b, chunks, width, scratch);
     KB_TL_MARK(norm, 3, threadIdx.x == 0 && blockIdx.x == 0);          // the slices and the residual are here
     if (w_post != nullptr) {
         ss = block_sum(ss, scratch);
@@ -331,6 +388,7 @@ __global__ void add_rmsnorm_splits_kernel(float* __restrict__ residual, const fl
         KB_TL_LEAVE(norm, blockIdx.x == 0, 0);
         return;
     }
+    if (CENTER && center_next) ss2 = center_groups<CPT>(r, chunks, width, scratch);
     ss2 = block_sum(ss2, scratch);
     KB_TL_MARK(norm, 4, threadIdx.x == 0 && blockIdx.x == 0);          // both sums are known
     const float inv2 = 1.f / sqrtf(ss2 / (float)width + eps_next);
@@ -372,11 +430,11 @@ __device__ __forceinline__ bool nb_wait(uint64_t* bar, uint32_t parity) {
     }
 }
 
-template <int CPT>
-__global__ void add_rmsnorm_splits_bulk_kernel(float* __restrict__ residual, const float* __restrict__ parts, int splits, size_t stride,
+template <int CPT, bool CENTER = false>
+__global__ void __launch_bounds__(1024) add_rmsnorm_splits_bulk_kernel(float* __restrict__ residual, const float* __restrict__ parts, int splits, size_t stride,
                                                const __nv_bfloat16* __restrict__ w_post, float eps_post, float off_post,
                                                const __nv_bfloat16* __restrict__ w_next, float eps_next, float off_next,
-                                               __nv_bfloat16* __restrict__ h, int width, int room KB_TL_PARAM) {
+                                               __nv_bfloat16* __restrict__ h, int width, int room, int center_post, int center_next KB_TL_PARAM) {
     extern __shared__ __align__(128) unsigned char nb_smem[];
     __shared__ float scratch[32];
     __shared__ __align__(8) uint64_t landed;
@@ -440,6 +498,7 @@ __global__ void add_rmsnorm_splits_bulk_kernel(float* __restrict__ residual, con
     for (int c = 0; c < CPT; ++c) ss += b[c].x * b[c].x + b[c].y * b[c].y + b[c].z * b[c].z + b[c].w * b[c].w;
     KB_TL_MARK(norm, 3, threadIdx.x == 0 && blockIdx.x == 0);
     float inv = 1.f;
+    if (CENTER && center_post && w_post != nullptr) ss = center_groups<CPT>(b, chunks, width, scratch);
     if (w_post != nullptr) {
         ss = block_sum(ss, scratch);
         inv = 1.f / sqrtf(ss / (float)width + eps_post);
@@ -482,6 +541,7 @@ __global__ void add_rmsnorm_splits_bulk_kernel(float* __restrict__ residual, con
         KB_TL_LEAVE(norm, blockIdx.x == 0, 0);
         return;
     }
+    if (CENTER && center_next) ss2 = center_groups<CPT>(r, chunks, width, scratch);
     ss2 = block_sum(ss2, scratch);
     KB_TL_MARK(norm, 4, threadIdx.x == 0 && blockIdx.x == 0);
     const float inv2 = 1.f / sqrtf(ss2 / (float)width + eps_next);
@@ -647,6 +707,62 @@ extern "C" int kb_rmsnorm(void* y, int y_dt, const void* x, int x_dt, const void
     return check_launch("rmsnorm");
 }
 
+// The vector kernels, where they take the types, the width and the alignment (bfloat16 weights and output, a branch in bfloat16 or
+// in 32-bit slices): what the launch gave, or -1 where they do not. With 2,048 rows of 2,048 and both norms centered a row in
+// registers takes 11 us where the row in shared memory, a value at a time, takes 45; a decoding step's row over slices 6.1 against 8.3.
+template <bool CENTER>
+static int launch_vectors(float* residual, const void* branch, int splits, long long split_stride, const void* w_post, float eps_post,
+                          float off_post, int center_post, const void* w_next, float eps_next, float off_next, int center_next, void* h,
+                          int code, int rows, int width, cudaStream_t s) {
+    const bool aligned = (((uintptr_t)residual | (uintptr_t)branch | (uintptr_t)w_post | (uintptr_t)w_next | (uintptr_t)h) & 15) == 0;
+    if (code == 7 && splits == 1 && width % 8 == 0 && width <= 4 * 8 * 1024 && aligned) {
+        const int chunks = width / 8;
+        const int cpt = chunks <= 1024 ? 1 : (chunks <= 2048 ? 2 : 4);
+        const int tv = min(1024, ((chunks + cpt - 1) / cpt + 31) / 32 * 32);
+        const bf16 *b = (const bf16*)branch, *wp = (const bf16*)w_post, *wn = (const bf16*)w_next;
+        bf16* out = (bf16*)h;
+        if (cpt == 1) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<1, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next);
+        else if (cpt == 2) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<2, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next);
+        else launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<4, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next);
+        return check_launch("add_rmsnorm");
+    }
+    // float32 partial sums of a product split over K (a decode step, or a prompt portion of a few hundred rows): a block a row
+    if (code == KB_DT_F32 * 4 + KB_DT_BF16 * 2 + KB_DT_BF16 && rows <= 65535 && width % 4 == 0 && width <= 4 * 4 * 1024 &&
+        (split_stride % 4) == 0 && (((uintptr_t)residual | (uintptr_t)branch | (uintptr_t)h) & 15) == 0 &&
+        (((uintptr_t)w_post | (uintptr_t)w_next) & 7) == 0) {
+        const int chunks = width / 4;
+        const int cpt = chunks <= 1024 ? 1 : (chunks <= 2048 ? 2 : 4);
+        const int tv = min(1024, ((chunks + cpt - 1) / cpt + 31) / 32 * 32);
+        const float* b = (const float*)branch;
+        const bf16 *wp = (const bf16*)w_post, *wn = (const bf16*)w_next;
+        const size_t stride = (size_t)split_stride;
+        bf16* out = (bf16*)h;
+        // A decode step's rows: the slices come into shared memory by bulk copies (see the kernel). Up to 192 KB of
+        // it, so sixteen slices of 2,304 or eleven of 4,608 values land in one round.
+        const int room = (int)std::min<size_t>((size_t)splits, (size_t)(192 * 1024) / ((size_t)width * 4));
+        if (rows <= DEPENDENT_ROWS && splits > 1 && room >= 1) {
+            static bool attr_set = false;
+            if (!attr_set) {
+                const cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<1, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
+                const cudaError_t e2 = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<2, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
+                const cudaError_t e4 = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<4, CENTER>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
+                if (e != cudaSuccess || e2 != cudaSuccess || e4 != cudaSuccess) return fail("add_rmsnorm: cannot have 192 KB of shared memory");
+                attr_set = true;
+            }
+            const size_t bytes = (size_t)room * width * 4;
+            if (cpt == 1) launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<1, CENTER>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+            else if (cpt == 2) launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<2, CENTER>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+            else launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<4, CENTER>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+            return check_launch("add_rmsnorm");
+        }
+        if (cpt == 1) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<1, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+        else if (cpt == 2) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<2, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+        else launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<4, CENTER>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, center_post, center_next KB_TL_SLOT(norm, 2, splits, wn != nullptr));
+        return check_launch("add_rmsnorm");
+    }
+    return -1;
+}
+
 // residual: f32 in and out. branch: `branch_dt`, as `splits` slices `split_stride` elements apart
 // that are added up on the way in (1 slice: the branch itself). h: `h_dt`. Both weights: `w_dt`.
 extern "C" int kb_add_rmsnorm(float* residual, const void* branch, int branch_dt, int splits, long long split_stride,
@@ -669,52 +785,9 @@ extern "C" int kb_add_rmsnorm(float* residual, const void* branch, int branch_dt
                                                               (const TW*)w_next, eps_next, off_next, (TH*)h, width); \
     } while (0)
     const int code = branch_dt * 4 + w_dt * 2 + h_dt;
-    const bool aligned = (((uintptr_t)residual | (uintptr_t)branch | (uintptr_t)w_post | (uintptr_t)w_next | (uintptr_t)h) & 15) == 0;
-    if (code == 7 && splits == 1 && width % 8 == 0 && width <= 4 * 8 * 1024 && aligned) {
-        const int chunks = width / 8;
-        const int cpt = chunks <= 1024 ? 1 : (chunks <= 2048 ? 2 : 4);
-        const int tv = min(1024, ((chunks + cpt - 1) / cpt + 31) / 32 * 32);
-        const bf16 *b = (const bf16*)branch, *wp = (const bf16*)w_post, *wn = (const bf16*)w_next;
-        bf16* out = (bf16*)h;
-        if (cpt == 1) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<1>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width);
-        else if (cpt == 2) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<2>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width);
-        else launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_bf16x8_kernel<4>, dim3(rows), dim3(tv), 0, s, residual, b, wp, eps_post, off_post, wn, eps_next, off_next, out, width);
-        return check_launch("add_rmsnorm");
-    }
-    // float32 partial sums of a product split over K (a decode step, or a prompt portion of a few hundred rows): a block a row
-    if (branch_dt == KB_DT_F32 && w_dt == KB_DT_BF16 && h_dt == KB_DT_BF16 && rows <= 65535 && width % 4 == 0 && width <= 4 * 4 * 1024 &&
-        (split_stride % 4) == 0 && (((uintptr_t)residual | (uintptr_t)branch | (uintptr_t)h) & 15) == 0 &&
-        (((uintptr_t)w_post | (uintptr_t)w_next) & 7) == 0) {
-        const int chunks = width / 4;
-        const int cpt = chunks <= 1024 ? 1 : (chunks <= 2048 ? 2 : 4);
-        const int tv = min(1024, ((chunks + cpt - 1) / cpt + 31) / 32 * 32);
-        const float* b = (const float*)branch;
-        const bf16 *wp = (const bf16*)w_post, *wn = (const bf16*)w_next;
-        const size_t stride = (size_t)split_stride;
-        bf16* out = (bf16*)h;
-        // A decode step's rows: the slices come into shared memory by bulk copies (see the kernel). Up to 192 KB of
-        // it, so sixteen slices of 2,304 or eleven of 4,608 values land in one round.
-        const int room = (int)std::min<size_t>((size_t)splits, (size_t)(192 * 1024) / ((size_t)width * 4));
-        if (rows <= DEPENDENT_ROWS && splits > 1 && room >= 1) {
-            static bool attr_set = false;
-            if (!attr_set) {
-                const cudaError_t e = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
-                const cudaError_t e2 = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
-                const cudaError_t e4 = cudaFuncSetAttribute(add_rmsnorm_splits_bulk_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 192 * 1024);
-                if (e != cudaSuccess || e2 != cudaSuccess || e4 != cudaSuccess) return fail("add_rmsnorm: cannot have 192 KB of shared memory");
-                attr_set = true;
-            }
-            const size_t bytes = (size_t)room * width * 4;
-            if (cpt == 1) launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<1>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-            else if (cpt == 2) launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<2>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-            else launch_dependent_if(true, add_rmsnorm_splits_bulk_kernel<4>, dim3(rows), dim3(tv), bytes, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width, room KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-            return check_launch("add_rmsnorm");
-        }
-        if (cpt == 1) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<1>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-        else if (cpt == 2) launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<2>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-        else launch_dependent_if(rows <= DEPENDENT_ROWS, add_rmsnorm_splits_kernel<4>, dim3(rows), dim3(tv), 0, s, residual, b, splits, stride, wp, eps_post, off_post, wn, eps_next, off_next, out, width KB_TL_SLOT(norm, 2, splits, wn != nullptr));
-        return check_launch("add_rmsnorm");
-    }
+    const int taken = launch_vectors<false>(residual, branch, splits, split_stride, w_post, eps_post, off_post, 0, w_next, eps_next, off_next, 0, h,
+                                            code, rows, width, s);
+    if (taken >= 0) return taken;
     switch (code) {
         case 0: KB_ADDNORM(float, float, float); break;
         case 1: KB_ADDNORM(float, float, bf16); break;
@@ -772,6 +845,10 @@ extern "C" int kb_add_norm(float* residual, const void* branch, int branch_dt, i
     KB_REQUIRE(smem <= 200 * 1024, "add_norm: a row of %d values does not fit the shared memory of a block", width);
     if (rows == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
+    const int code = branch_dt * 4 + w_dt * 2 + h_dt;
+    const int taken = launch_vectors<true>(residual, branch, splits, split_stride, w_post, eps_post, off_post, center_post, w_next, eps_next,
+                                           off_next, center_next, h, code, rows, width, s);
+    if (taken >= 0) return taken;
     // few rows (a decode step): latency counts, so a row is spread over as many threads as it has pairs of values
     const int t = rows <= DEPENDENT_ROWS ? std::min(1024, std::max(128, ((width + 1) / 2 + 31) / 32 * 32)) : threads_for(width);
 #define KB_ADDLN(TB, TW, TH)                                                                                              \
@@ -781,7 +858,6 @@ extern "C" int kb_add_norm(float* residual, const void* branch, int branch_dt, i
                                                                  (const TW*)w_post, eps_post, off_post, center_post,        \
                                                                  (const TW*)w_next, eps_next, off_next, center_next, (TH*)h, width); \
     } while (0)
-    const int code = branch_dt * 4 + w_dt * 2 + h_dt;
     switch (code) {
         case 0: KB_ADDLN(float, float, float); break;
         case 1: KB_ADDLN(float, float, bf16); break;
