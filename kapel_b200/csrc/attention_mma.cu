@@ -1318,15 +1318,15 @@ extern "C" long long kb_attention_mma_scratch_floats(int rows, int hq, int d, in
 }
 
 // Merges the partial sums [rows, hq, slots, d + 2] that a prompt kernel left in `scratch`; rows whose
-// keys all lie in one slot were finished by that slot's block and are left alone.
+// keys all lie in one slot were finished by that slot's block and are left alone. `sinks` [hq] or null.
 extern "C" int kb_attention_mma_combine(void* out, const int* row_count, const float* scratch, int rows, int hq, int d,
-                                        int window, int split, int slots, void* stream) {
+                                        int window, int split, int slots, const float* sinks, void* stream) {
     KB_REQUIRE(rows >= 0 && hq > 0 && d > 0 && d % 2 == 0, "attention combine: rows %d, heads %d, head_dim %d", rows, hq, d);
     KB_REQUIRE(split > 0 && slots > 1 && scratch != nullptr, "attention combine: split %d, %d slots", split, slots);
     if (rows == 0) return 0;
     AttMmaParams p = {};
     p.row_count = row_count; p.out = (bf16*)out; p.partial = const_cast<float*>(scratch);
-    p.rows = rows; p.hq = hq; p.d = d; p.window = window; p.split = split; p.slots = slots; p.direct = 1;
+    p.rows = rows; p.hq = hq; p.d = d; p.window = window; p.split = split; p.slots = slots; p.direct = 1; p.sinks = sinks;
     const unsigned blocks = (unsigned)(((long long)rows * hq + AC_WARPS - 1) / AC_WARPS);
     if (int e = combine_smem(slots)) return e;
     attention_mma_combine_warp_kernel<<<blocks, AC_WARPS * 32, (size_t)AC_WARPS * slots * sizeof(float), (cudaStream_t)stream>>>(p);

@@ -56,6 +56,12 @@ def decode_split(pairs: int, longest: int, sms: int, window: Optional[int] = Non
     return split, max(1, -(-(span if relative else longest) // split))
 
 
+# Latent attention: a request's rows from which its keys and values are made for every head: that costs about 6 ns a position (16 heads of
+# 128 / 128 from 512 components), and then a pair of a row and a key costs 0.02 ns instead of the 0.4 that it costs over the cached
+# lines, so a portion of some twenty rows pays for it; 64 leaves room for the launches. And the most positions laid out so in a pass (9 KB each at 16 heads; the partial sums that the kernel over shared lines would write for them are more).
+LATENT_PROMPT_ROWS = 64
+LATENT_PROMPT_POSITIONS = 131072
+
 # What a block costs beyond its 64-key steps, what the merge of partial sums costs beyond its traffic
 # (both in steps), microseconds a step, and how many multiprocessors a block takes, by prompt kernel;
 # from sweeps of the split at Gemma 2 2B head sizes with 2,048 tokens behind 4,096 to 129,024 (a block
@@ -63,7 +69,7 @@ def decode_split(pairs: int, longest: int, sms: int, window: Optional[int] = Non
 # what it costs in a launch of its own). The tcgen05 kernels' steps are short, so their fixed costs
 # weigh more and they are cut into slots only when a few tiles face a long history; "tcgen05_pair" is
 # the kernel on pairs of blocks (a tile of 256 rows on two multiprocessors, half the time a step).
-PROMPT_KERNEL_COSTS = {"mma": (0.5, 1.0, 4.5, 1), "tcgen05": (18.0, 15.0, 1.2, 1), "tcgen05_pair": (32.0, 18.0, 0.85, 2)}
+PROMPT_KERNEL_COSTS = {"mma": (0.5, 1.0, 4.5, 1), "flash": (18.0, 15.0, 0.6, 1), "tcgen05": (18.0, 15.0, 1.2, 1), "tcgen05_pair": (32.0, 18.0, 0.85, 2)}
 
 
 def prompt_costs_of(prompt_kernel: str, head_dim: int, pairs: Optional[int] = None) -> str:
@@ -284,6 +290,32 @@ class StepBatch:
                 self.memo[key] = (dev[:n], dev[n : 2 * n], dev[2 * n :], host)
         tiles = self.memo[key]
         return tiles[:3] if tiles is not None else None
+
+    def latent_tiles(self):
+        """How the prompt path of latent attention cuts this step, or None where no request brings enough rows for it: (rows before
+        the first such request's, requests before it, the most rows one of those brings, (tile_entry, tile_row0, tile_nq), entry_base,
+        entry_length, positions, longest): tiles of 128 rows, counted from the first such request's; where each request's positions begin
+        among those laid out densely, and how many it has there (none where it brings few rows)."""
+        key = "latent_tiles"
+        if key not in self.memo:
+            plan = self.plan
+            q_len = np.asarray(plan.q_len, np.int64)
+            many = q_len >= LATENT_PROMPT_ROWS
+            first = int(np.argmax(many)) if many.any() else 0
+            lengths = np.where(many, plan.row_count[np.asarray(plan.q_start, np.int64) + np.maximum(q_len, 1) - 1], 0) if q_len.size else q_len
+            positions = int(lengths.sum())
+            # Requests with few rows have to lie before the others (as the scheduler orders a pass).
+            if not many.any() or not many[first:].all() or positions > LATENT_PROMPT_POSITIONS or not self.ids.is_cuda:
+                self.memo[key] = None
+            else:
+                base = np.cumsum(lengths) - lengths
+                tiles = cut_tiles(plan.q_start[first:], plan.q_len[first:], 128)
+                arrays = [tiles[0] + first, tiles[1] - int(plan.q_start[first]), tiles[2], base.astype(np.int32), lengths.astype(np.int32)]
+                host = torch.from_numpy(np.concatenate([a.astype(np.int32) for a in arrays])).pin_memory()
+                views = host.to(self.ids.device, non_blocking=True).split([a.size for a in arrays])
+                self.memo[key] = (int(plan.q_start[first]), first, int(q_len[:first].max()) if first else 0, tuple(v.contiguous() for v in views[:3]), views[3].contiguous(), views[4].contiguous(),
+                                  positions, int(lengths.max()), host)
+        return self.memo[key][:8] if self.memo[key] is not None else None
 
     def longest_count(self) -> int:
         """The most positions any row of this step has seen (its own included)."""

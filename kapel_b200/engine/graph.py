@@ -71,6 +71,12 @@ class StaticBatch:
     def longest_portion(self) -> int:
         return 1                                             # every request brings one token
 
+    def shortest_portion(self) -> int:
+        return 1
+
+    def latent_tiles(self):
+        return None
+
     def pooled_slices(self, window: Optional[int], pool: int):
         """(slices, keys a slice) for the longest request this recording's block tables can hold."""
         from .. import kernels as K

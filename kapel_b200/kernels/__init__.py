@@ -85,6 +85,8 @@ def check_async_errors() -> None:
         bad.append("tcgen05 product (a TMA load or an MMA commit never arrived)")
     if lib.kb_attention_tc_error() != 0:
         bad.append("tcgen05 attention (a TMA load, an MMA commit or a softmax warp never arrived)")
+    if lib.kb_attention_flash_error() != 0:
+        bad.append("tcgen05 attention without a soft cap (a TMA load, an MMA commit or a softmax warp never arrived)")
     if lib.kb_rope_error() != 0:
         bad.append("rotate and append (a bulk copy of partial sums into shared memory never completed)")
     if lib.kb_norm_error() != 0:
@@ -710,6 +712,66 @@ def latent_attention_mma(q, table, block_table, row_count, ranges, entries: int,
     return out
 
 
+def latent_prompt_takes(dtype, hq: int, d: int, rot: int, dv: int, kv_rank: int, scale: float) -> bool:
+    """Whether `latent_prompt` takes these sizes."""
+    return dtype == torch.bfloat16 and kv_rank % 64 == 0 and bool(library().kb_attention_flash_latent_takes(int(hq), int(d), int(rot), int(dv), _f(scale)))
+
+
+def latent_query(q, heads: int, d: int, rot: int, cos_sin) -> torch.Tensor:
+    """[rows, heads, d + rot] bfloat16 from the queries' product (a tensor or a SplitSum): the last `rot` components of
+    every head turned in pairs (i, i + rot/2) by `cos_sin` [rows, rot/2, 2]."""
+    src, dt, splits, stride, rows, width = _stacked(q, "latent_query input")
+    if width != heads * (d + rot):
+        raise KernelError(f"latent_query: rows of {width} for {heads} heads of {d} + {rot}")
+    _need(cos_sin, "latent_query cos_sin", torch.float32, (rows, rot // 2, 2))
+    out = _fresh((rows, heads, d + rot), torch.bfloat16, src.device)
+    _check(library().kb_latent_query(_ptr(out), _ptr(src), dt, splits, ctypes.c_longlong(stride), _ptr(cos_sin), rows, int(heads), int(d), int(rot), _stream()))
+    return out
+
+
+def latent_gather(table, block_table, entry_base, entry_length, positions: int, longest: int, page_size: int, kv_rank: int, rot: int):
+    """(c [positions, kv_rank], rotated keys [positions, rot]) of the cached lines of whole requests: position p of request e at row
+    entry_base[e] + p, for p below entry_length[e]."""
+    _need(table, "latent_gather table", torch.bfloat16)
+    if table.dim() != 4 or table.shape[1] != 1 or table.shape[2] != page_size or table.shape[3] != kv_rank + rot:
+        raise KernelError(f"latent_gather: a table of {tuple(table.shape)} for lines of {kv_rank} + {rot}, pages of {page_size}")
+    _need(block_table, "latent_gather block table", torch.int32)
+    entries = entry_base.numel()
+    _need(entry_base, "latent_gather entry bases", torch.int32)
+    _need(entry_length, "latent_gather entry lengths", torch.int32, (entries,))
+    if block_table.shape[0] < entries:
+        raise KernelError(f"latent_gather: block tables for {block_table.shape[0]} of {entries} requests")
+    c = _fresh((positions, kv_rank), torch.bfloat16, table.device)
+    rot_keys = _fresh((positions, rot), torch.bfloat16, table.device)
+    _check(library().kb_latent_gather(_ptr(c), _ptr(rot_keys), _ptr(table), _ptr(block_table), int(block_table.shape[1]), int(table.shape[0]),
+                                      int(page_size), _ptr(entry_base), _ptr(entry_length), entries, int(longest), int(kv_rank), int(rot), _stream()))
+    return c, rot_keys
+
+
+def latent_prompt(q, kv, rot_keys, entry_base, row_count, tiles, scale: float, sinks, d: int, dv: int) -> torch.Tensor:
+    """Attention of prompt portions over every head's own keys and values: q [rows, hq, d + rot] bfloat16, `kv` [positions,
+    hq d + hq dv] (all heads' plain keys, then their values), `rot_keys` [positions, rot]; `tiles` of 128 rows; [rows, hq, dv] float32.
+    Rows that no tile names are left as they are."""
+    rows, hq, width = q.shape
+    rot = width - d
+    positions = kv.shape[0]
+    _need(q, "latent_prompt q", torch.bfloat16)
+    _need(kv, "latent_prompt keys and values", torch.bfloat16, (positions, hq * (d + dv)))
+    _need(rot_keys, "latent_prompt rotated keys", torch.bfloat16, (positions, rot))
+    _need(entry_base, "latent_prompt entry bases", torch.int32)
+    _need(row_count, "latent_prompt row_count", torch.int32, (rows,))
+    if sinks is not None:
+        _need(sinks, "latent_prompt sinks", torch.float32, (hq,))
+    n_tiles = tiles[0].numel()
+    for t in tiles:
+        _need(t, "latent_prompt tiles", torch.int32, (n_tiles,))
+    out = _fresh((rows, hq, dv), torch.float32, q.device)
+    _check(library().kb_attention_flash_latent(_ptr(out), _ptr(q), _ptr(kv), _ptr(rot_keys), _ptr(entry_base), int(positions), _ptr(row_count),
+                                               _ptr(tiles[0]), _ptr(tiles[1]), _ptr(tiles[2]), n_tiles, rows, hq, int(d), int(rot), int(dv),
+                                               _f(scale), _ptr(sinks), _stream()))
+    return out
+
+
 def attention_keep_slots(window: Optional[int], keep_first: int) -> int:
     """Chunk slots the row-wise kernel spends on the kept first keys of a windowed layer."""
     return -(-int(keep_first) // attention_chunk()) if (window and keep_first) else 0
@@ -734,6 +796,8 @@ def prompt_pairs(rows: int, longest: int) -> int:
 def attention_tile_rows(decode: bool, prompt_kernel: str = "mma", d: int = 0, pairs: Optional[int] = None) -> int:
     """Rows a tile holds for the kernel that will run: the decode kernel's, the mma.sync prompt
     kernel's, or the tcgen05 prompt kernel's (twice as many where pairs of blocks run it)."""
+    if not decode and prompt_kernel == "flash":
+        return 128
     if not decode and prompt_kernel == "tcgen05":
         return int(library().kb_attention_tc_rows(int(d), int(ATTENTION_PAIRS if pairs is None else pairs)))
     return attention_mma_rows(decode)
@@ -744,9 +808,14 @@ def attention_mma_takes(dtype, d: int, heads_per_kv: int) -> bool:
     return dtype == torch.bfloat16 and d % 16 == 0 and d <= 256 and heads_per_kv <= 16
 
 
-def attention_prompt_kernel(hq: int, hkv: int, d: int, page_size: int, softcap: Optional[float]) -> str:
-    """Which kernel `paged_attention_mma` runs for prompt portions of these sizes: "tcgen05" or "mma"."""
-    if ATTENTION_PROMPT == "tcgen05" and library().kb_attention_tc_takes(int(hq), int(hkv), int(d), int(page_size), _f(softcap or 0.0)):
+def attention_prompt_kernel(hq: int, hkv: int, d: int, page_size: int, softcap: Optional[float], scale: Optional[float] = None,
+                            plain: bool = True) -> str:
+    """Which kernel `paged_attention_mma` runs for prompt portions of these sizes: "tcgen05" (a soft cap bounds the
+    scores), "flash" (no soft cap; a window, a sink) or "mma". With `plain` False the layer has a sink, kept first keys or a block mask,
+    which the kernel for soft caps does not know; `scale` None names a layer that the kernel without a cap cannot take."""
+    if not softcap and scale is not None and ATTENTION_PROMPT == "tcgen05" and library().kb_attention_flash_takes(int(hq), int(hkv), int(d), int(page_size), _f(scale)):
+        return "flash"
+    if plain and ATTENTION_PROMPT == "tcgen05" and library().kb_attention_tc_takes(int(hq), int(hkv), int(d), int(page_size), _f(softcap or 0.0)):
         return "tcgen05"
     return "mma"
 
@@ -812,7 +881,7 @@ def paged_attention_decode_fused(qkv: "SplitSum", cos_sin, lines, k_table, v_tab
 def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page_size: int, window: Optional[int],
                         scale: float, softcap: Optional[float], decode: int, split: int, slots: int,
                         relative: bool = False, pairs: Optional[int] = None, keep_first: int = 0, block: int = 0,
-                        sinks: Optional[torch.Tensor] = None) -> torch.Tensor:
+                        sinks: Optional[torch.Tensor] = None, prompt_kernel: Optional[str] = None) -> torch.Tensor:
     """Attention over the paged cache on tensor cores (bfloat16). `tiles` = (tile_entry, tile_row0,
     tile_nq) int32 device tensors: each tile is up to `attention_mma_rows(decode) // group` tokens of
     one request at consecutive positions. `decode` is 0 for prompt portions, else the most rows
@@ -822,7 +891,8 @@ def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page
     visible key, so a windowed row needs ceil(window / split) slots however long its history. With a
     window, `keep_first` keys from position 0 stay visible below it (prompt portions in one slot only).
     With `block` > 0 a row at position i sees only the keys from floor(i / block) * block on (prompt portions
-    in one slot only). With `sinks` [hq] float32 e^sink joins each row's denominator."""
+    in one slot only). With `sinks` [hq] float32 e^sink joins each row's denominator.
+    `prompt_kernel` "flash" (whose tiles the caller then gives) runs prompt portions on the tcgen05 kernel for scores without a bound."""
     rows, hq, d = q.shape
     if sinks is not None:
         _need(sinks, "attention sinks", torch.float32, (hq,))
@@ -842,6 +912,17 @@ def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page
     lib = library()
     need = lib.kb_attention_mma_scratch_floats(rows, hq, d, int(slots))
     scratch = _fresh((need,), torch.float32, q.device) if need else None
+    if not decode and not keep_first and not block and prompt_kernel == "flash":
+        _check(
+            lib.kb_attention_flash(_ptr(out), _ptr(q), _ptr(k_table), _ptr(v_table), _ptr(block_table), _ptr(row_count),
+                                   _ptr(tile_entry), _ptr(tile_row0), _ptr(tile_nq), n_tiles, rows, hq, hkv, d, int(page_size),
+                                   int(block_table.shape[1]), int(n_pages), int(window or 0), int(split), int(slots), _f(scale),
+                                   _ptr(scratch), _ptr(sinks), _stream())
+        )
+        if slots > 1:
+            _check(lib.kb_attention_mma_combine(_ptr(out), _ptr(row_count), _ptr(scratch), rows, hq, d, int(window or 0), int(split),
+                                                int(slots), _ptr(sinks), _stream()))
+        return out
     if not decode and not keep_first and not block and sinks is None and attention_prompt_kernel(hq, hkv, d, page_size, softcap) == "tcgen05":
         _check(
             lib.kb_attention_tc(_ptr(out), _ptr(q), _ptr(k_table), _ptr(v_table), _ptr(block_table), _ptr(row_count),
@@ -851,7 +932,7 @@ def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page
         )
         if slots > 1:
             _check(lib.kb_attention_mma_combine(_ptr(out), _ptr(row_count), _ptr(scratch), rows, hq, d, int(window or 0), int(split),
-                                                int(slots), _stream()))
+                                                int(slots), None, _stream()))
         return out
     _check(
         lib.kb_attention_mma_masked(_ptr(out), _ptr(q), _ptr(k_table), _ptr(v_table), _ptr(block_table), _ptr(row_count),

@@ -305,13 +305,13 @@ class Attention(Part):
         if dv == s.head_dim and K.attention_mma_takes(q.dtype, s.head_dim, heads_per_kv):
             # with kept first keys only prompt portions go to the tensor-core kernel; a pass of single tokens stays with
             # the row-wise kernel below
-            prompt = "mma" if keep or self.sinks is not None else K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim,
-                                                                                            self.ctx.page_size, s.softcap)
+            prompt = "mma" if keep else K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap,
+                                                                  s.scale, self.sinks is None)
             decode, tiles, split, slots, relative = batch.attention_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt, keep_first=keep)
             if not (decode and keep):
                 y = K.paged_attention_mma(q, k_table, v_table, group.block_table, batch.row_count, tiles, self.ctx.page_size,
                                           s.window, s.scale, s.softcap, decode, split, slots, relative, pairs=getattr(batch, "pairs", None),
-                                          keep_first=keep, sinks=self.sinks)
+                                          keep_first=keep, sinks=self.sinks, prompt_kernel=prompt)
         if y is None:
             y = K.paged_attention_rows(
                 q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count, self.ctx.page_size, s.window, s.scale,
@@ -345,10 +345,10 @@ class Attention(Part):
                                     s.num_heads, s.num_kv_heads, s.head_dim, dv, cache.owns, self.ctx.dtype)
         heads_per_kv = s.num_heads // s.num_kv_heads
         if dv == s.head_dim and s.head_dim % 16 == 0 and K.attention_mma_takes(q.dtype, s.head_dim, heads_per_kv):
-            prompt = "mma" if self.sinks is not None else K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap)
+            prompt = K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap, s.scale, self.sinks is None)
             decode, tiles, split, slots, relative = batch.attention_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt)
             y = K.paged_attention_mma(q, k_table, v_table, group.block_table, batch.row_count, tiles, self.ctx.page_size, s.window,
-                                      s.scale, s.softcap, decode, split, slots, relative, pairs=getattr(batch, "pairs", None), sinks=self.sinks)
+                                      s.scale, s.softcap, decode, split, slots, relative, pairs=getattr(batch, "pairs", None), sinks=self.sinks, prompt_kernel=prompt)
         else:
             y = K.paged_attention_rows(q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count, self.ctx.page_size,
                                        s.window, s.scale, s.softcap, batch.attention_slots(s.window), sinks=self.sinks)
@@ -391,13 +391,12 @@ class Attention(Part):
             out_dtype=self.ctx.dtype,
         )
         if K.attention_mma_takes(q.dtype, s.head_dim, heads_per_kv):
-            decode, tiles, split, slots, relative = batch.attention_tiles(
-                heads_per_kv, s.num_kv_heads, s.window, s.head_dim,
-                K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap))
+            prompt = K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap, s.scale)
+            decode, tiles, split, slots, relative = batch.attention_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt)
             y = K.paged_attention_mma(
                 q, k_table, v_table, group.block_table, batch.row_count, tiles,
                 self.ctx.page_size, s.window, s.scale, s.softcap, decode, split, slots, relative,
-                pairs=getattr(batch, "pairs", None),
+                pairs=getattr(batch, "pairs", None), prompt_kernel=prompt,
             )
         else:                   # the 32-bit path, and sizes the tensor-core kernel does not take
             y = K.paged_attention_rows(

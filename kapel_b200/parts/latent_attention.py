@@ -81,6 +81,10 @@ class LatentAttention(Part):
         self.turned = not ctx.is_f32
         self.m_uk = (uk.transpose(1, 2) if self.turned else uk).contiguous()
         self.m_uv = (uv if self.turned else uv.transpose(1, 2)).contiguous()
+        # prompts: every head's keys and values as one product of a line's latent
+        self.expands = K.latent_prompt_takes(ctx.dtype, H, s.head_dim, s.rot_dim, s.v_head_dim, s.kv_rank, s.scale) if not ctx.is_f32 else False
+        if self.expands:
+            self.w_ukv = torch.cat([uk.reshape(-1, s.kv_rank), uv.reshape(-1, s.kv_rank)]).contiguous()
         norm = lambda n: (tensors[n].to(dev).float() if ctx.is_f32 else tensors[n].to(dev).contiguous())
         self.norm_q, self.norm_kv = norm(w["dq_norm"]), norm(w["dkv_norm"])
         if self.norm_q.dtype != self.norm_kv.dtype:
@@ -94,22 +98,49 @@ class LatentAttention(Part):
     def forward(self, h, batch, cache):
         s, ctx = self.spec, self.ctx
         H, d, r = s.num_heads, s.head_dim, s.rot_dim
-        stacked = linear(ctx, h, self.w_down, out_dtype=torch.float32, keep_split=True)
+        cut = batch.latent_tiles() if self.expands else None
+        few = cut[0] if cut is not None else 0               # rows of requests that bring few, ahead of the others
+        stacked = linear(ctx, h, self.w_down, out_dtype=torch.float32, keep_split=few == 0)
         k_table, _ = cache.tables()
         group = batch.groups[cache.group]
         cos_sin = self.position.tables(batch)
         c_q = K.latent_append(stacked, 0, s.q_rank, s.q_rank, s.kv_rank, r, self.norm_q, self.norm_kv, s.eps,
                               cos_sin, group.lines, k_table, cache.owns, ctx.dtype, pad_to=self.w_uq.shape[1])
-        q = linear(ctx, c_q, self.w_uq, out_dtype=torch.float32, keep_split=True)
+        q = linear(ctx, c_q, self.w_uq, out_dtype=torch.float32, keep_split=few == 0)
+        if cut is not None:
+            o = self._expanded(q[few:] if few else q, cos_sin[few:] if few else cos_sin, stacked[few:] if few else stacked, batch, group, k_table, cut)
+            if few:
+                o = torch.cat([self._over_lines(q[:few], cos_sin[:few], stacked[:few], batch, group, k_table, batch.row_count[:few], cut[1], cut[2]), o])
+        else:
+            o = self._over_lines(q, cos_sin, stacked, batch, group, k_table, batch.row_count, batch.entries, batch.longest_portion())
+        return linear(ctx, o, self.w_o, keep_split=True)
+
+    def _expanded(self, q, cos_sin, stacked, batch, group, k_table, cut):
+        """Prompt portions: the lines of the whole requests are laid out densely, one product makes every head's own keys and
+        values of them, and attention runs at the heads' own sizes. Per pair of a row and a key that is a third of the
+        multiply-adds of attention over the lines, which a portion of LATENT_PROMPT_ROWS rows pays back."""
+        s, ctx = self.spec, self.ctx
+        few, _, _, tiles, entry_base, entry_length, positions, longest = cut
+        c, rot_keys = K.latent_gather(k_table, group.block_table, entry_base, entry_length, positions, longest, ctx.page_size, s.kv_rank, s.rot_dim)
+        kv = linear(ctx, c, self.w_ukv)
+        heads = K.latent_query(q, s.num_heads, s.head_dim, s.rot_dim, cos_sin)
+        y = K.latent_prompt(heads, kv, rot_keys, entry_base, batch.row_count[few:], tiles, s.scale, self.sinks,
+                            s.head_dim, s.v_head_dim)
+        return K.head_gate(y, stacked, s.q_rank + s.kv_rank + s.rot_dim if s.gated else 0, None, False, 0.0, ctx.dtype,
+                           pad_to=product_width(ctx, s.num_heads * s.v_head_dim), gate_act="sigmoid" if s.gated else "none")
+
+    def _over_lines(self, q, cos_sin, stacked, batch, group, k_table, row_count, entries, longest):
+        """Single tokens and short portions: all heads over the cached lines themselves."""
+        s, ctx = self.spec, self.ctx
+        H, d, r = s.num_heads, s.head_dim, s.rot_dim
         q_lat = K.head_linear(q, H, d + r, 0, self.m_uk, y_head=s.kv_rank + r, tail_off=d, tail=r, cos_sin=cos_sin, transposed=self.turned)
         if K.latent_attention_mma_takes(q_lat.dtype, s.kv_rank + r, s.kv_rank):
-            y = K.latent_attention_mma(q_lat.view(-1, H, s.kv_rank + r), k_table, group.block_table, batch.row_count, batch.entry_ranges(),
-                                       batch.entries, batch.longest_portion(), ctx.page_size, s.scale, batch.attention_slots(None),
+            y = K.latent_attention_mma(q_lat.view(-1, H, s.kv_rank + r), k_table, group.block_table, row_count, batch.entry_ranges(),
+                                       entries, longest, ctx.page_size, s.scale, batch.attention_slots(None),
                                        self.sinks, s.kv_rank)
         else:                   # the 32-bit path, and sizes the tensor-core kernel does not take
             y = K.paged_attention_rows(q_lat.view(-1, H, s.kv_rank + r), k_table, k_table, group.block_table, batch.row_entry,
-                                       batch.row_count, ctx.page_size, None, s.scale, None, batch.attention_slots(None),
+                                       row_count, ctx.page_size, None, s.scale, None, batch.attention_slots(None),
                                        sinks=self.sinks, value_dim=s.kv_rank)
-        o = K.head_linear(y.view(-1, H * s.kv_rank), H, s.kv_rank, 0, self.m_uv, gate=stacked if s.gated else None,
+        return K.head_linear(y.view(-1, H * s.kv_rank), H, s.kv_rank, 0, self.m_uv, gate=stacked if s.gated else None,
                           g_off=s.q_rank + s.kv_rank + r, pad_to=product_width(ctx, H * s.v_head_dim), transposed=self.turned)
-        return linear(ctx, o, self.w_o, keep_split=True)
