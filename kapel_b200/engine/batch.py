@@ -325,6 +325,10 @@ class StepBatch:
         """The most rows any request brings in this step (what sizes a launch of a block a run of a request's rows)."""
         return int(self.plan.q_len.max()) if len(self.plan.q_len) else 0
 
+    def shortest_portion(self) -> int:
+        """The fewest rows any request brings in this step."""
+        return int(self.plan.q_len.min()) if len(self.plan.q_len) else 0
+
     def entry_ranges(self):
         """(start, end) on the device: rows [start[e], end[e]) are request e's. Made once a step."""
         if "entry_ranges" not in self.memo:

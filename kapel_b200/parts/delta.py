@@ -79,7 +79,7 @@ class Delta(Part):
         after = base + 2 * kd + 2 * he
         o = K.delta_scan(stacked, base, base + kd, base + 2 * kd, after, after + s.num_heads, self.conv, self.a_log, self.dt_bias,
                          cache.state(), batch.row_entry, batch.entry_ranges(), batch.slots, batch.entries, s.num_heads, s.num_kv_heads,
-                         s.head_dim, s.v_head_dim, s.conv, s.head_dim ** -0.5, s.unit_eps)
+                         s.head_dim, s.v_head_dim, s.conv, s.head_dim ** -0.5, s.unit_eps, batch.longest_portion(), batch.shortest_portion())
         return K.head_gate(o, stacked, base + 2 * kd + he, self.norm_weight, True, s.eps, self.ctx.dtype, gate_act="silu", scale=scale, out=out,
                            column=column, pad_to=product_width(self.ctx, he) if pad_to is None else pad_to)
 

@@ -1,0 +1,56 @@
+"""The gated delta rule by chunks of rows against 64-bit and against the scan: portions of every remainder, behind a memory and a history,
+beside short portions, with decays of 0; rows of no request."""
+import numpy as np
+import pytest
+import torch
+
+import plain_kofutar as PK
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("H,G,d,e,taps", [(4, 2, 32, 16, 4), (2, 1, 128, 48, 4), (3, 3, 64, 16, 3), (4, 1, 96, 32, 4)])
+def test_against_64_bit_and_the_scan(H, G, d, e, taps):
+    from kapel_b200 import kernels as K
+
+    dev = lambda x, dtype=torch.float32: torch.tensor(np.asarray(x), dtype=dtype, device="cuda")
+    rng = np.random.default_rng(d + e)
+    n, nv = G * d, H * e
+    width = 2 * n + nv + 2 * H
+    conv, a_log, dt_bias = rng.standard_normal((2 * n + nv, taps)) * 0.6, rng.standard_normal(H) * 0.5, rng.standard_normal(H)
+    data, want = {}, {}
+    for name, T in {"a": 300, "b": 161, "c": 33}.items():
+        x = rng.standard_normal((T, width))
+        x[:, -2 * H :] *= 3.0                                # decays and step sizes that swing
+        x[T // 2, -H:] = 400.0                               # a decay that is 0 in 32-bit: everything is forgotten
+        x = x.astype(np.float32).astype(np.float64)
+        data[name] = x
+        q, k, v, g, beta = PK.delta_inputs(x, conv.astype(np.float32).astype(np.float64), a_log.astype(np.float32).astype(np.float64),
+                                           dt_bias.astype(np.float32).astype(np.float64), H, G, d, e)
+        want[name] = np.stack([PK.delta_recurrence(q[:, h // (H // G)], k[:, h // (H // G)], v[:, h], g[:, h], beta[:, h]) for h in range(H)], axis=1)
+    steps = [[("a", 1, 0, 64), ("b", 2, 0, 3)], [("b", 2, 3, 100), ("a", 1, 64, 65)], [("c", 3, 0, 33), ("a", 1, 65, 194)], [("a", 1, 194, 300), ("b", 2, 100, 161)]]
+    per = K.delta_state_floats(H, G, d, e, taps)
+
+    def run(chunked):
+        state, worst = torch.zeros((4, per), dtype=torch.float32, device="cuda"), 0.0
+        for step in steps:
+            sizes = [b - a for _, _, a, b in step]
+            entry = dev(np.repeat(np.arange(len(step)), sizes), torch.int32)
+            out = K.delta_scan(dev(np.concatenate([data[m][a:b] for m, _, a, b in step])), 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, dev(conv), dev(a_log),
+                               dev(dt_bias), state, entry, K.entry_ranges(entry, len(step)), dev([s for _, s, _, _ in step], torch.int32), len(step),
+                               H, G, d, e, taps, d ** -0.5, 1e-6, max(sizes) if chunked else 0, min(sizes)).cpu().numpy()
+            at = 0
+            for (m, _, a, b), size in zip(step, sizes):
+                worst = max(worst, float(np.abs(out[at : at + size] - want[m][a:b]).max() / np.abs(want[m]).max()))
+                at += size
+        return worst, state
+
+    (scan, by_scan), (chunks, by_chunks) = run(False), run(True)
+    print(f"scan {scan:.2e}, chunks {chunks:.2e}")
+    assert chunks < 5e-5 and chunks < 2.0 * scan + 1e-6      # the same recurrence in 32-bit, summed in another order
+    assert (by_scan - by_chunks).abs().max() <= 5e-5 * by_scan.abs().max()
+    before = by_chunks.clone()
+    entry = dev(np.zeros(70), torch.int32)
+    out = K.delta_scan(dev(data["a"][:70]), 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, dev(conv), dev(a_log), dev(dt_bias), by_chunks, entry,
+                       K.entry_ranges(entry, 1), dev([0], torch.int32), 1, H, G, d, e, taps, d ** -0.5, 1e-6, 70, 70)
+    assert float(out.abs().max()) == 0.0 and torch.equal(before, by_chunks)
