@@ -500,7 +500,7 @@ extern "C" int kb_moe_route(int* experts, float* weights, const void* h, int h_d
 extern "C" int kb_moe_sort(const int* experts, int pairs, int n_experts, int* offsets, int* order, int* tile_expert,
                            int* tile_first, int* tile_rows, int* n_tiles, int tile_cap, int rows_a_tile, void* stream) {
     KB_REQUIRE(pairs >= 0 && n_experts > 0 && tile_cap >= 0, "moe_sort: %d pairs, %d experts", pairs, n_experts);
-    KB_REQUIRE(rows_a_tile == GM || rows_a_tile == GM_LARGE, "moe_sort: tiles of %d rows (%d or %d)", rows_a_tile, GM, GM_LARGE);
+    KB_REQUIRE(rows_a_tile == GM || rows_a_tile == GM_LARGE || rows_a_tile == 128, "moe_sort: tiles of %d rows (%d, %d or 128)", rows_a_tile, GM, GM_LARGE);
     const size_t smem = (size_t)2 * n_experts * sizeof(int);
     KB_REQUIRE(smem <= 48 * 1024, "moe_sort: %d experts are too many", n_experts);
     moe_sort_kernel<<<1, SORT_THREADS, smem, (cudaStream_t)stream>>>(experts, pairs, n_experts, offsets, order, tile_expert, tile_first,

@@ -1735,7 +1735,45 @@ class ExpertLists:
     __slots__ = ("order", "offsets", "tiles", "tile_cap", "tile_rows", "pairs", "top")
 
 
-def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.float32) -> ExpertLists:
+# Rows an expert gets on average from which its products run on tcgen05 tiles of 128 rows: 272 rows an expert
+# took 77 + 52 us where the 64-row tiles of mma.sync took 145 + 145 and 23 for the unit between them; at 48 a tile is filled to three
+# eighths, which the five times faster products still pay for. Below, the tiles of 32 and 64 rows.
+MOE_TCGEN05_ROWS = 48
+
+
+def moe_tcgen05_takes(dtype: torch.dtype, rows: int, top: int, n_experts: int, widths, act: str, gated: bool) -> bool:
+    """Whether a pass of `rows` tokens runs its experts' products on tcgen05: bfloat16, gated units (or no activation between a
+    plain product and its reader), inner sizes of whole 16-byte pieces, rows enough an expert."""
+    return (dtype == torch.bfloat16 and gated and act in GLU_EPILOGUES and GEMM_LARGE in ("tcgen05", "pair") and rows * top >= MOE_TCGEN05_ROWS * n_experts
+            and all(w % 8 == 0 for w in widths))
+
+
+def moe_gather(a: torch.Tensor, lists: "ExpertLists") -> torch.Tensor:
+    """[pairs, k]: the rows of a [tokens, k] in the lists' order (what lies behind the listed pairs is left as it is)."""
+    _need(a, "moe_gather input", torch.bfloat16)
+    out = _fresh((lists.pairs, a.shape[1]), a.dtype, a.device)
+    _check(library().kb_moe_gather(_ptr(out), _ptr(a), _ptr(lists.order), _ptr(lists.offsets[-1:]), lists.pairs, int(a.shape[1]), int(lists.top), _stream()))
+    return out
+
+
+def moe_tcgen05(a: torch.Tensor, w: torch.Tensor, lists: "ExpertLists", act: Optional[str], out_by_pair: bool, out_dtype: torch.dtype,
+                limit: float = 0.0, alpha: float = 0.0) -> torch.Tensor:
+    """The grouped product on tcgen05: a [pairs, k] in the lists' order, w [experts, n, k] or, with a gated unit `act` in the
+    epilogue, [experts, 2 n, k] (gates, then ups); lists with tiles of 128 rows."""
+    _need(a, "moe_tcgen05 input", torch.bfloat16)
+    _need(w, "moe_tcgen05 weights", torch.bfloat16)
+    if w.dim() != 3 or w.shape[2] != a.shape[1] or a.shape[0] != lists.pairs or lists.tile_rows != 128:
+        raise KernelError(f"moe_tcgen05: weights {tuple(w.shape)} against {tuple(a.shape)}, tiles of {lists.tile_rows} rows")
+    n, k = int(w.shape[1]) // (2 if act is not None else 1), int(w.shape[2])
+    out = _fresh((lists.pairs, n), out_dtype, a.device)
+    t = lists.tiles
+    _check(library().kb_moe_tcgen05(_ptr(out), _CODES[out_dtype], _ptr(a), _ptr(w), int(w.shape[0]), _ptr(t[0]), _ptr(t[1]), _ptr(t[2]), _ptr(t[3]),
+                                    int(lists.tile_cap), _ptr(lists.order) if out_by_pair else None, lists.pairs, n, k,
+                                    2 + GLU_EPILOGUES[act] if act is not None else 0, _f(limit), _f(alpha), _stream()))
+    return out
+
+
+def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.float32, tile_rows: Optional[int] = None) -> ExpertLists:
     """Lists the pairs of `experts` [rows, top] by expert, those from number `n_experts` on (experts without weights) left out; `dtype` is the grouped products' (it and the
     rows an expert gets on average decide how many rows a tile of those products has)."""
     _need(experts, "moe_sort experts", torch.int32)
@@ -1743,7 +1781,7 @@ def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.f
     pairs = rows * top
     lists = ExpertLists()
     lists.pairs, lists.top = pairs, top
-    lists.tile_rows = int(library().kb_moe_tile_rows(_CODES[dtype], ctypes.c_longlong(pairs // max(n_experts, 1))))
+    lists.tile_rows = tile_rows or int(library().kb_moe_tile_rows(_CODES[dtype], ctypes.c_longlong(pairs // max(n_experts, 1))))
     # every expert's list ends with at most one tile that is not full
     lists.tile_cap = pairs // lists.tile_rows + min(n_experts, pairs)
     buf = _fresh((n_experts + 1 + pairs + 3 * max(lists.tile_cap, 1) + 1,), torch.int32, experts.device)

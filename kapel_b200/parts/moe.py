@@ -80,10 +80,15 @@ class MoE(Part):
         experts, weights = K.moe_route(h, self.router, self.correction, s.top, s.groups, s.keep_groups, s.group_top, s.scoring,
                                        s.renormalize, s.route_scale)
         own = h if s.identity else None
-        lists = K.moe_sort(experts, s.experts, self.w_up.dtype)
+        tiled = K.moe_tcgen05_takes(self.w_up.dtype, h.shape[0], s.top, s.experts, (s.hidden, s.intermediate), s.activation, s.gated)
+        lists = K.moe_sort(experts, s.experts, self.w_up.dtype, 128 if tiled else None)
         if h.dtype != self.w_up.dtype:
             h = K.cast(h, self.w_up.dtype)
         also = self.shared.forward(h) if self.shared is not None else None
+        if tiled:                      # a prompt: the gated unit is the first product's epilogue
+            inner = K.moe_tcgen05(K.moe_gather(h, lists), self.w_up, lists, s.activation, False, self.w_up.dtype, s.limit or 0.0, s.swish_alpha)
+            y = K.moe_tcgen05(inner, self.w_down, lists, None, True, torch.float32)
+            return K.moe_combine(y, weights, torch.float32, also=also, experts=experts if s.identity else None, real=s.experts, own=own)
         if s.gated:
             both = K.moe_grouped(h, self.w_up, lists, "none", True, False, torch.float32)
             if self.clamped:

@@ -1,0 +1,44 @@
+"""The experts' products of prompts on tcgen05 tiles of 128 rows: lists with empty experts, full and nearly full tiles and identity
+pairs, inner sizes that fill no tile, every gated unit, rows placed by list and by pair, each against 64-bit."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def units(gate, up, act, limit, alpha):
+    if act == "clamped_swish":
+        g, u = gate.clamp(max=limit), up.clamp(-limit, limit)
+        return g * torch.sigmoid(alpha * g) * (u + 1.0)
+    return torch.nn.functional.gelu(gate, approximate="tanh") * up if act.startswith("gelu") else gate * torch.sigmoid(gate) * up
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", "clamped_swish"])
+@pytest.mark.parametrize("counts,identity", [([0, 128, 129, 1], 40), ([300], 0), ([7, 0, 0, 255, 256, 3], 9)])
+@pytest.mark.parametrize("width,inner", [(72, 40), (128, 264), (520, 128)])
+def test_against_64_bit(act, counts, identity, width, inner):
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(width + len(counts))
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    n = len(counts)
+    chosen = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)] + [torch.full((identity,), n + 1)])
+    top = 1 if len(chosen) % 2 else 2
+    chosen = chosen[torch.randperm(len(chosen), generator=torch.Generator().manual_seed(2))].to(torch.int32).view(-1, top).cuda()
+    tokens = chosen.shape[0]
+    h = make(tokens, width).bfloat16()
+    w_up, w_down = (make(n, 2 * inner, width) * width ** -0.5 * 2).bfloat16(), (make(n, width, inner) * inner ** -0.5).bfloat16()
+    lists = K.moe_sort(chosen, n, torch.bfloat16, 128)
+    got = K.moe_tcgen05(K.moe_gather(h, lists), w_up, lists, act, False, torch.bfloat16, 1.5, 1.702)
+    y = K.moe_tcgen05(got, w_down, lists, None, True, torch.float32)
+    listed = int(lists.offsets[-1])
+    assert listed == sum(counts)
+    order = lists.order[:listed].long()
+    expert = chosen.view(-1)[order].long()
+    both = torch.einsum("pk,pnk->pn", h[order // top].double(), w_up[expert].double())
+    want = units(both[:, :inner], both[:, inner:], act, 1.5, 1.702)
+    # rounded to bfloat16 (2^-8 of the value at most) from 32-bit sums
+    assert ((got[:listed].double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-5 * want.abs().max()).all()
+    back = torch.einsum("pk,pnk->pn", got[:listed].double(), w_down[expert].double())
+    assert (y[order].double() - back).abs().max() <= 1e-5 * back.abs().max()
+    K.check_async_errors()
