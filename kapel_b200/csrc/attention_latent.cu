@@ -38,6 +38,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
 __global__ void __launch_bounds__(LM_THREADS, 1)
 latent_mma_kernel(const AttParams p, const int* __restrict__ entry_start, const int* __restrict__ entry_end, int tokens_per_tile,
                   int heads_per_tile, int head_slices) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ __align__(16) unsigned char lm_smem[];
     const int d = p.d, dv = p.dv, H = p.hq;
     const int ld = d + 8;                                       // elements between rows in shared memory: 16-byte rows, banks spread
@@ -277,6 +279,194 @@ latent_mma_kernel(const AttParams p, const int* __restrict__ entry_start, const 
     }
 }
 
+// Single tokens: one block = one token's slice of 16 heads x one chunk of LD_KEYS keys, all fetched at once. A tile of one token has 16 rows
+// of the 64 above, so there the row groups would have one group's work between them; here the four groups of warps take a quarter of
+// the keys each, and meet once, through shared memory. Slots, partial sums and merge are the other kernel's. 8 requests
+// of 1,024 to 3,072 positions, 16 heads, in a decoding step of a four-layer model: 413 us the step with the kernel above in chunks of 128
+// keys (430 in chunks of 256), 375 with this one.
+constexpr int LD_KEYS = 128, LD_HEADS = 16;
+__host__ __device__ inline size_t latent_decode_smem(int d, int dv) {
+    const size_t in = ((size_t)LD_HEADS + LD_KEYS) * (d + 8) * sizeof(bf16);
+    const size_t merge = (size_t)4 * LD_HEADS * (dv + 4) * sizeof(float);        // takes the keys' place
+    return (in > merge ? in : merge) + (4 * LD_HEADS * 2) * sizeof(float) + LD_KEYS * sizeof(int);
+}
+__global__ void __launch_bounds__(LM_THREADS, 1)
+latent_decode_kernel(const AttParams p, const int* __restrict__ entry_start, const int* __restrict__ entry_end, int head_slices) {
+    extern __shared__ __align__(16) unsigned char lm_smem[];
+    const int d = p.d, dv = p.dv, H = p.hq;
+    const int ld = d + 8, lo_dv = dv + 4;
+    bf16* sq = reinterpret_cast<bf16*>(lm_smem);                // [LD_HEADS][ld]
+    bf16* sk = sq + (size_t)LD_HEADS * ld;                      // [LD_KEYS][ld]
+    float* so = reinterpret_cast<float*>(lm_smem);              // [4][LD_HEADS][dv + 4], once queries and keys are done with
+    float* sml = reinterpret_cast<float*>(lm_smem + latent_decode_smem(d, dv) - (4 * LD_HEADS * 2) * sizeof(float) - LD_KEYS * sizeof(int));     // [4][LD_HEADS][2]
+    int* sline = reinterpret_cast<int*>(sml + 4 * LD_HEADS * 2);
+    const int entry = blockIdx.y / head_slices, h0 = (blockIdx.y % head_slices) * LD_HEADS, z = blockIdx.x;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int gid = lane >> 2, t4 = lane & 3, group = warp & 3, half = warp >> 2;
+    const int nheads = min(LD_HEADS, H - h0);
+    const int nvec = d >> 3, half_cols = dv >> 1, ntiles = half_cols >> 3, col0 = half * half_cols;
+    dependent_wait();                                           // returns at once after a plain launch
+    dependent_trigger();
+    const int r = entry_start[entry];
+    if (r >= entry_end[entry]) return;
+    const int count = p.row_count[r];
+    bf16* out = static_cast<bf16*>(p.out);
+    if (count <= 0) {                                           // a row that sees nothing at all: zeros, from the first chunk's block
+        if (z == 0)
+            for (int i = tid; i < nheads * dv; i += LM_THREADS) out[((size_t)r * H + h0) * dv + i] = __float2bfloat16_rn(0.f);
+        return;
+    }
+    const int lo = z * LD_KEYS, hi = min(count, lo + LD_KEYS);
+    if (lo >= hi) return;
+    if (tid < LD_KEYS) {
+        const int pos = lo + tid, lp = pos / p.page_size;
+        int line = -1;
+        if (pos < hi) {
+            const int page = lp < p.table_width ? p.block_table[(size_t)entry * p.table_width + lp] : -1;
+            if (page >= 0 && page < p.n_pages) line = page * p.page_size + pos % p.page_size;
+        }
+        sline[tid] = line;
+    }
+    const bf16* qg = static_cast<const bf16*>(p.q) + ((size_t)r * H + h0) * d;
+    for (int i = tid; i < LD_HEADS * nvec; i += LM_THREADS) {
+        const int hh = i / nvec, v = i - hh * nvec;
+        *reinterpret_cast<uint4*>(sq + (size_t)hh * ld + v * 8) = hh < nheads ? *reinterpret_cast<const uint4*>(qg + (size_t)hh * d + v * 8) : make_uint4(0u, 0u, 0u, 0u);
+    }
+    __syncthreads();
+    const bf16* kt = static_cast<const bf16*>(p.k_table);
+    for (int key = warp; key < LD_KEYS; key += LM_THREADS / 32) {       // a warp a line
+        const int line = sline[key];
+        bf16* to = sk + (size_t)key * ld;
+        if (line >= 0) {
+            const bf16* from = kt + kv_row(line, 0, 1, p.page_size) * d;
+            for (int v = lane; v < nvec; v += 32)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(to + v * 8)), "l"(from + v * 8) : "memory");
+        } else {
+            for (int v = lane; v < nvec; v += 32) *reinterpret_cast<uint4*>(to + v * 8) = make_uint4(0u, 0u, 0u, 0u);
+        }
+    }
+    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+
+    const int key0 = group * 32;                                // this group's keys of the chunk
+    float s[4][4], s2[4][4];
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt) s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = s2[nt][0] = s2[nt][1] = s2[nt][2] = s2[nt][3] = 0.f;
+    const uint32_t qaddr = (uint32_t)__cvta_generic_to_shared(sq + (size_t)(lane & 15) * ld + (lane >> 4) * 8);
+    const uint32_t kaddr = (uint32_t)__cvta_generic_to_shared(sk + (size_t)(key0 + (lane >> 4) * 8 + (lane & 7)) * ld + ((lane >> 3) & 1) * 8);
+#pragma unroll 2
+    for (int kk = 0; kk < d; kk += 32) {                        // two sets of sums taking the 16-component steps in turn
+        uint32_t a[4], b[4], c[4];
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(qaddr + kk * 2));
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(kaddr + kk * 2));
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(kaddr + (16 * ld + kk) * 2));
+        mma_bf16(s[0], a, b[0], b[1]);
+        mma_bf16(s[1], a, b[2], b[3]);
+        mma_bf16(s[2], a, c[0], c[1]);
+        mma_bf16(s[3], a, c[2], c[3]);
+        if (kk + 16 < d) {
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3]) : "r"(qaddr + (kk + 16) * 2));
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(b[0]), "=r"(b[1]), "=r"(b[2]), "=r"(b[3]) : "r"(kaddr + (kk + 16) * 2));
+            asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3]) : "r"(kaddr + (16 * ld + kk + 16) * 2));
+            mma_bf16(s2[0], a, b[0], b[1]);
+            mma_bf16(s2[1], a, b[2], b[3]);
+            mma_bf16(s2[2], a, c[0], c[1]);
+            mma_bf16(s2[3], a, c[2], c[3]);
+        }
+    }
+    float top_a = -INFINITY, top_b = -INFINITY;                 // rows gid and gid + 8 of the 16
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const int key = key0 + nt * 8 + 2 * t4 + (c & 1);
+            s[nt][c] = sline[key] >= 0 ? (s[nt][c] + s2[nt][c]) * p.scale : -INFINITY;
+            if (c & 2) top_b = fmaxf(top_b, s[nt][c]);
+            else top_a = fmaxf(top_a, s[nt][c]);
+        }
+    top_a = fmaxf(top_a, __shfl_xor_sync(0xffffffffu, top_a, 1));
+    top_a = fmaxf(top_a, __shfl_xor_sync(0xffffffffu, top_a, 2));
+    top_b = fmaxf(top_b, __shfl_xor_sync(0xffffffffu, top_b, 1));
+    top_b = fmaxf(top_b, __shfl_xor_sync(0xffffffffu, top_b, 2));
+    float l_a = 0.f, l_b = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < 4; ++nt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            const float w = s[nt][c] == -INFINITY ? 0.f : __expf(s[nt][c] - ((c & 2) ? top_b : top_a));
+            s[nt][c] = w;
+            if (c & 2) l_b += w;
+            else l_a += w;
+        }
+    l_a += __shfl_xor_sync(0xffffffffu, l_a, 1);
+    l_a += __shfl_xor_sync(0xffffffffu, l_a, 2);
+    l_b += __shfl_xor_sync(0xffffffffu, l_b, 1);
+    l_b += __shfl_xor_sync(0xffffffffu, l_b, 2);
+    float o[LM_MAX_NT][4];
+#pragma unroll
+    for (int j = 0; j < LM_MAX_NT; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+        uint32_t a[4];
+        a[0] = pack_bf16(s[2 * ks][0], s[2 * ks][1]);
+        a[1] = pack_bf16(s[2 * ks][2], s[2 * ks][3]);
+        a[2] = pack_bf16(s[2 * ks + 1][0], s[2 * ks + 1][1]);
+        a[3] = pack_bf16(s[2 * ks + 1][2], s[2 * ks + 1][3]);
+        const uint32_t row_addr = (uint32_t)__cvta_generic_to_shared(sk + (size_t)(key0 + ks * 16 + (lane & 15)) * ld + col0);
+#pragma unroll
+        for (int j = 0; j < LM_MAX_NT; ++j)
+            if (j < ntiles) {
+                uint32_t b0, b1;
+                asm volatile("ldmatrix.sync.aligned.m8n8.x2.trans.shared.b16 {%0,%1}, [%2];" : "=r"(b0), "=r"(b1) : "r"(row_addr + j * 16));
+                mma_bf16(o[j], a, b0, b1);
+            }
+    }
+    __syncthreads();                                            // the keys are done with: the groups' sums take their place
+    float* mine = so + (size_t)group * LD_HEADS * lo_dv + col0;
+#pragma unroll
+    for (int j = 0; j < LM_MAX_NT; ++j)
+        if (j < ntiles) {
+            *reinterpret_cast<float2*>(mine + (size_t)gid * lo_dv + j * 8 + 2 * t4) = make_float2(o[j][0], o[j][1]);
+            *reinterpret_cast<float2*>(mine + (size_t)(gid + 8) * lo_dv + j * 8 + 2 * t4) = make_float2(o[j][2], o[j][3]);
+        }
+    if (half == 0 && t4 == 0) {
+        sml[(group * LD_HEADS + gid) * 2] = top_a, sml[(group * LD_HEADS + gid) * 2 + 1] = l_a;
+        sml[(group * LD_HEADS + gid + 8) * 2] = top_b, sml[(group * LD_HEADS + gid + 8) * 2 + 1] = l_b;
+    }
+    __syncthreads();
+    for (int i = tid; i < nheads * (dv >> 1); i += LM_THREADS) {        // two columns of one head at a time
+        const int hh = i / (dv >> 1), c = (i - hh * (dv >> 1)) * 2, h = h0 + hh;
+        float m = -INFINITY, w[4], l = 0.f;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) m = fmaxf(m, sml[(g * LD_HEADS + hh) * 2]);
+        float x = 0.f, y = 0.f;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const float mg = sml[(g * LD_HEADS + hh) * 2];
+            w[g] = mg == -INFINITY ? 0.f : __expf(mg - m);
+            l = fmaf(w[g], sml[(g * LD_HEADS + hh) * 2 + 1], l);
+            const float2 v = *reinterpret_cast<const float2*>(so + ((size_t)g * LD_HEADS + hh) * lo_dv + c);
+            x = fmaf(w[g], v.x, x);
+            y = fmaf(w[g], v.y, y);
+        }
+        if (p.slots == 1) {
+            float inv = l > 0.f ? 1.f / l : 0.f;
+            if (p.sinks != nullptr) {
+                const float sink = p.sinks[h], top = fmaxf(m, sink), wk = m == -INFINITY ? 0.f : __expf(m - top);
+                inv = wk / (l * wk + __expf(sink - top));
+            }
+            *reinterpret_cast<uint32_t*>(out + ((size_t)r * H + h) * dv + c) = pack_bf16(x * inv, y * inv);
+        } else {
+            float* dst = p.partial + (((size_t)r * H + h) * p.slots + z) * (dv + 2);
+            *reinterpret_cast<float2*>(dst + c) = make_float2(x, y);
+            if (c == 0) {
+                dst[dv] = m;
+                dst[dv + 1] = l;
+            }
+        }
+    }
+}
+
 }  // namespace kb
 
 using namespace kb;
@@ -293,6 +483,7 @@ extern "C" int kb_latent_attention_mma_takes(int d, int dv) {
 // entry_start / entry_end [entries]: the rows of each request; `longest`: the most rows any request brings.
 // `chunk`: keys a slot holds, `slots` >= ceil(longest count / chunk).
 // scratch: kb_paged_attention_scratch_floats(rows, hq, dv, slots) floats when slots > 1.
+extern "C" int kb_latent_decode_keys() { return LD_KEYS; }
 extern "C" int kb_latent_attention_mma(void* out, const void* q, const void* table, const int* block_table, const int* row_count,
                                        const int* entry_start, const int* entry_end, int entries, int longest, int rows, int hq,
                                        int d, int dv, int page_size, int table_width, int n_pages, int slots, int chunk, float scale,
@@ -323,10 +514,27 @@ extern "C" int kb_latent_attention_mma(void* out, const void* q, const void* tab
         attr_set = true;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    latent_mma_kernel<<<dim3((unsigned)tiles, entries, slots), LM_THREADS, smem, s>>>(p, entry_start, entry_end, tokens_per_tile, heads_per_tile, head_slices);
+    if (longest == 1 && chunk == LD_KEYS && latent_decode_smem(d, dv) <= 227 * 1024) {
+        const int slices = (hq + LD_HEADS - 1) / LD_HEADS;
+        KB_REQUIRE((long long)entries * slices <= 65535, "latent_attention_mma: too many requests for one launch");
+        static bool decode_attr_set = false;
+        if (!decode_attr_set) {
+            if (cudaFuncSetAttribute(latent_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess)
+                return fail("latent_attention_mma: cannot have 227 KB of shared memory");
+            decode_attr_set = true;
+        }
+        launch_dependent_if(rows <= DEPENDENT_ROWS, latent_decode_kernel, dim3(slots, entries * slices), dim3(LM_THREADS), latent_decode_smem(d, dv), s, p, entry_start, entry_end, slices);
+        if (int e = check_launch("latent_attention_mma decode")) return e;
+        if (slots > 1) {
+            launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(128), 0, s, p);
+            return check_launch("latent_attention_mma combine");
+        }
+        return 0;
+    }
+    launch_dependent_if(rows <= DEPENDENT_ROWS, latent_mma_kernel, dim3((unsigned)tiles, entries, slots), dim3(LM_THREADS), smem, s, p, entry_start, entry_end, tokens_per_tile, heads_per_tile, head_slices);
     if (int e = check_launch("latent_attention_mma")) return e;
     if (slots > 1) {
-        combine_kernel<bf16><<<dim3(rows, hq), 128, 0, s>>>(p);
+        launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(128), 0, s, p);
         return check_launch("latent_attention_mma combine");
     }
     return 0;

@@ -63,6 +63,8 @@ __global__ void proj_rope_append_kernel(const Src<TS> src, int row_width, int q_
                                         const int* __restrict__ lines, TO* __restrict__ q_out, TO* __restrict__ k_table,
                                         TO* __restrict__ v_table, int hq, int hkv, int d, int dv, long long table_lines,
                                         int page_size) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ float row[];                          // q [hq d] | k [hkv d]
     __shared__ float scratch[32];
     const int r = blockIdx.x;
@@ -528,7 +530,7 @@ extern "C" int kb_proj_rope_append(const void* src, int src_dt, int splits, long
 #define KB_PRA(TS, TW, TO)                                                                                                      \
     do {                                                                                                                        \
         if (smem > 48 * 1024) cudaFuncSetAttribute(proj_rope_append_kernel<TS, TW, TO>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        proj_rope_append_kernel<TS, TW, TO><<<rows, threads, smem, s>>>(                                                        \
+        launch_dependent_if(rows <= DEPENDENT_ROWS, proj_rope_append_kernel<TS, TW, TO>, dim3(rows), dim3(threads), smem, s,                                                         \
             Src<TS>{(const TS*)src, splits, (size_t)split_stride}, row_width, q_off, k_off, v_off, (const TW*)bq, (const TW*)bk,   \
             (const TW*)bv, (const TW*)wq, eps_q, off_q, (const TW*)wk, eps_k, off_k, (const float2*)cos_sin, rotary, neighbours, \
             v_other, (const TW*)lambda, v_keep, lines, (TO*)q_out, write_kv ? (TO*)k_table : nullptr, write_kv ? (TO*)v_table : nullptr, \

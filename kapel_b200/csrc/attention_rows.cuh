@@ -292,6 +292,8 @@ rows_kernel(const AttParams p) {
 constexpr int COMBINE_SLOTS = 1024;    // slots whose weights fit shared memory; beyond that they are computed again a component
 template <typename T>
 __global__ void combine_kernel(const AttParams p) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     __shared__ float scratch[32];
     __shared__ float weight[COMBINE_SLOTS];
     const int r = blockIdx.x, h = blockIdx.y;

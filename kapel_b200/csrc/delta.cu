@@ -62,6 +62,8 @@ __device__ __forceinline__ float delta_silu(float x) { return x / (1.f + expf(-x
 template <typename TS>
 __global__ void __launch_bounds__(1024)
 delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ float act[];                              // [channels]
     const int r = blockIdx.x;
     const int nq = p.kv_heads * p.d, nv = p.heads * p.e;
@@ -215,6 +217,8 @@ delta_prep_rows_kernel(const Src<TS> src, const DeltaParams p) {
 // history <- the last taps - 1 inputs of (history, this step's rows), per channel of a request.
 template <typename TS>
 __global__ void delta_history_kernel(const Src<TS> src, const DeltaParams p) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const int entry = blockIdx.y;
     const int nq = p.kv_heads * p.d, nv = p.heads * p.e;
     const int channels = 2 * nq + nv;
@@ -260,6 +264,8 @@ __device__ __forceinline__ void delta_copy16(float* dst, const float* src) {
 template <int R, int CH, int DW>
 __global__ void __launch_bounds__(DC * 32)
 delta_scan_kernel(const DeltaParams p) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     constexpr int DCOLS = DC * DW;                              // columns a block
     constexpr int SHIFT = DW == 4 ? 2 : (DW == 2 ? 3 : 4);     // the sum of column c ends in lane c << SHIFT (M.k) and 16 + (c << SHIFT) (M.q)
     extern __shared__ __align__(16) float staged[];             // [2][CH][rowf]
@@ -500,11 +506,11 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
             kernel<<<(rows + DPR - 1) / DPR, 256, DPR * smem, s>>>(Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); \
         } else {                                                                                                           \
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        delta_prep_kernel<TS><<<rows, rows <= DEPENDENT_ROWS ? 1024 : 256, smem, s>>>(Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \
+        launch_dependent_if(rows <= DEPENDENT_ROWS, delta_prep_kernel<TS>, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 256), smem, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \
         }                                                                                                                  \
         if (int err = check_launch("delta prep")) return err;                                                              \
         if (taps > 1) {                                                                                                    \
-            delta_history_kernel<TS><<<dim3((unsigned)((channels + 127) / 128), entries), 128, 0, s>>>(                     \
+            launch_dependent_if(rows <= DEPENDENT_ROWS, delta_history_kernel<TS>, dim3((unsigned)((channels + 127) / 128), entries), dim3(128), 0, s,                      \
                 Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p);                                                 \
             if (int err = check_launch("delta history")) return err;                                                       \
         }                                                                                                                  \
@@ -538,7 +544,7 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     KB_REQUIRE((e + DC * dw - 1) / (DC * dw) <= 65535, "delta: too many value components for one launch");
     dim3 grid(entries, heads, (e + DC * dw - 1) / (DC * dw));
     const int need = (d + 31) / 32;
-#define KB_DELTA_SCAN(R, CH, W) delta_scan_kernel<R, CH, W><<<grid, DC * 32, (size_t)2 * CH * (2 * R * 32 + DC * W + 8) * sizeof(float), s>>>(p)
+#define KB_DELTA_SCAN(R, CH, W) launch_dependent_if(rows <= DEPENDENT_ROWS, delta_scan_kernel<R, CH, W>, grid, dim3(DC * 32), ((size_t)2 * CH * (2 * R * 32 + DC * W + 8) * sizeof(float)), s, p)
 #define KB_DELTA_SCAN_W(R, CH)            \
     do {                                  \
         if (dw == 4) KB_DELTA_SCAN(R, CH, 4);      \

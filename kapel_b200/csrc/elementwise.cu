@@ -274,6 +274,8 @@ __global__ void rope_append_bf16x8_kernel(const __nv_bfloat16* __restrict__ qkv,
 // out[r, i] = act(x[r, i]) * x[r, n + i]: the gated unit after a stacked gate|up product.
 template <typename TI, typename T>
 __global__ void glu_kernel(T* __restrict__ out, const Src<TI> x, long long rows, int n, int act) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * n) return;
     const long long r = idx / n;
@@ -310,6 +312,8 @@ __global__ void glu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bf
 // the gated unit with both halves bounded and the linear half shifted by one.
 template <typename TI, typename T>
 __global__ void glu_clamped_kernel(T* __restrict__ out, const Src<TI> x, long long rows, int n, float limit, float alpha) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= rows * n) return;
     const long long r = idx / n;
@@ -328,6 +332,8 @@ __global__ void cast_kernel(TO* __restrict__ out, const TI* __restrict__ in, lon
 // rows wanted: out[i, :] = x[rows[i], :]
 __global__ void gather_rows_f32_kernel(float* __restrict__ out, const float* __restrict__ x,
                                        const int* __restrict__ rows, int n, int width, int src_rows) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const int i = blockIdx.x;
     if (i >= n) return;
     const int r = rows[i];
@@ -504,7 +510,7 @@ extern "C" int kb_glu(void* out, int out_dt, const void* x, int in_dt, int split
     const unsigned blocks = (unsigned)((total + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
 #define KB_GLU(TI, T) \
-    glu_kernel<TI, T><<<blocks, 256, 0, s>>>((T*)out, Src<TI>{(const TI*)x, splits, (size_t)split_stride}, rows, n, act)
+    launch_dependent_if(rows <= DEPENDENT_ROWS, glu_kernel<TI, T>, dim3(blocks), dim3(256), 0, s, (T*)out, Src<TI>{(const TI*)x, splits, (size_t)split_stride}, rows, n, act)
     if (in_dt == KB_DT_BF16 && out_dt == KB_DT_BF16 && splits == 1 && n % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0) {
         const long long vec = rows * (n / 8);
         glu_bf16x8_kernel<<<(unsigned)((vec + 255) / 256), 256, 0, s>>>((bf16*)out, (const bf16*)x, rows, n, act);
@@ -567,6 +573,8 @@ extern "C" int kb_take_cols(void* out, int out_dt, const void* x, int in_dt, int
 // out[r, :] = (a[r, :], b[r, :]) side by side, float32 in, `out_dt` out.
 template <typename TO>
 __global__ void concat2_kernel(TO* __restrict__ out, const float* __restrict__ a, const float* __restrict__ b, long long rows, int width) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * 2 * width) return;
     const long long r = i / (2 * width);
@@ -580,8 +588,8 @@ extern "C" int kb_concat2(void* out, int out_dt, const float* a, const float* b,
     KB_REQUIRE((n + 255) / 256 <= 0x7fffffffll, "concat2: too many values for one launch");
     const unsigned blocks = (unsigned)((n + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
-    if (out_dt == KB_DT_F32) concat2_kernel<float><<<blocks, 256, 0, s>>>((float*)out, a, b, rows, width);
-    else if (out_dt == KB_DT_BF16) concat2_kernel<bf16><<<blocks, 256, 0, s>>>((bf16*)out, a, b, rows, width);
+    if (out_dt == KB_DT_F32) launch_dependent_if(rows <= DEPENDENT_ROWS, concat2_kernel<float>, dim3(blocks), dim3(256), 0, s, (float*)out, a, b, rows, width);
+    else if (out_dt == KB_DT_BF16) launch_dependent_if(rows <= DEPENDENT_ROWS, concat2_kernel<bf16>, dim3(blocks), dim3(256), 0, s, (bf16*)out, a, b, rows, width);
     else return fail("concat2: dtype code %d is not known", out_dt);
     return check_launch("concat2");
 }
@@ -608,7 +616,7 @@ extern "C" int kb_gather_rows_f32(float* out, const float* x, const int* rows, i
                                   void* stream) {
     KB_REQUIRE(n >= 0 && width > 0, "gather_rows: n %d, width %d", n, width);
     if (n == 0) return 0;
-    gather_rows_f32_kernel<<<n, 256, 0, (cudaStream_t)stream>>>(out, x, rows, n, width, src_rows);
+    launch_dependent_if(src_rows <= DEPENDENT_ROWS, gather_rows_f32_kernel, dim3(n), dim3(256), 0, (cudaStream_t)stream, out, x, rows, n, width, src_rows);
     return check_launch("gather_rows");
 }
 
@@ -621,7 +629,7 @@ extern "C" int kb_glu_clamped(void* out, int out_dt, const void* x, int in_dt, i
     const unsigned blocks = (unsigned)((rows * n + 255) / 256);
     cudaStream_t s = (cudaStream_t)stream;
 #define KB_GLUC(TI, T) \
-    glu_clamped_kernel<TI, T><<<blocks, 256, 0, s>>>((T*)out, Src<TI>{(const TI*)x, splits, (size_t)split_stride}, rows, n, limit, alpha)
+    launch_dependent_if(rows <= DEPENDENT_ROWS, glu_clamped_kernel<TI, T>, dim3(blocks), dim3(256), 0, s, (T*)out, Src<TI>{(const TI*)x, splits, (size_t)split_stride}, rows, n, limit, alpha)
     if (in_dt == KB_DT_F32 && out_dt == KB_DT_F32) KB_GLUC(float, float);
     else if (in_dt == KB_DT_F32 && out_dt == KB_DT_BF16) KB_GLUC(float, bf16);
     else if (in_dt == KB_DT_BF16 && out_dt == KB_DT_BF16) KB_GLUC(bf16, bf16);

@@ -83,6 +83,8 @@ template <typename TY, typename TS, typename TW, typename TO>
 __global__ void head_gate_kernel(TO* __restrict__ out, const TY* __restrict__ y, const Src<TS> gate, int row_width,
                                  int g_off, const TW* __restrict__ w, int unit, float eps, long long pairs, int heads, int e,
                                  int out_stride, int fill_to, int act, int by_head, float scale) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (pair >= pairs) return;
     const int lane = threadIdx.x & 31;
@@ -123,6 +125,8 @@ template <typename TY, typename TS, typename TW, typename TO>
 __global__ void __launch_bounds__(1024)
 head_gate_wide_kernel(TO* __restrict__ out, const TY* __restrict__ y, const Src<TS> gate, int row_width, int g_off, const TW* __restrict__ w,
                       int unit, float eps, int heads, int e, int out_stride, int fill_to, int act, int by_head, float scale) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     __shared__ float scratch[32];
     const long long pair = blockIdx.x;
     const long long r = pair / heads;
@@ -166,6 +170,8 @@ __global__ void head_norm_rope_append_kernel(const Src<TS> src, int row_width, i
                                              const int* __restrict__ lines, TO* __restrict__ q_out, TO* __restrict__ k_table,
                                              TO* __restrict__ v_table, int hq, int hkv, int d, int dv, long long table_lines,
                                              int page_size) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ float vecs[];                             // [warps][d]
     const int r = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -221,6 +227,8 @@ __global__ void latent_append_kernel(const Src<TS> src, int row_width, int q_off
                                      const float2* __restrict__ cos_sin, const int* __restrict__ lines,
                                      TO* __restrict__ cq_out, int cq_stride, TO* __restrict__ k_table, long long table_lines,
                                      int page_size) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     __shared__ float scratch[32];
     const int r = blockIdx.x;
     const size_t base = (size_t)r * row_width;
@@ -431,19 +439,24 @@ constexpr int HF_WARPS = 8;
 template <typename TX>
 __global__ void __launch_bounds__(HF_WARPS * 32)
 head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX> x, int x_row, int x_head, int x_off,
-                       const bf16* __restrict__ mt, int n_in, int n_out, int rows, int heads,
+                       const bf16* __restrict__ mt, int n_in, int n_out, int columns, int rows, int heads,
                        int tail_off, int tail, const float2* __restrict__ cos_sin,
                        const Src<float> gate, int g_row, int g_off) {
     extern __shared__ float xf[];                               // [rows][n_in]
     const int h = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int c0 = (blockIdx.y * HF_WARPS + warp) * columns;
+    // the matrix is nobody's output: its columns set out for L2 ahead of the wait on the kernel before
+    for (int i = lane * 64; i < columns * n_in && c0 + i / n_in < n_out; i += 32 * 64)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(mt + ((size_t)h * n_out + c0) * n_in + i));
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     for (int idx = tid; idx < rows * n_in; idx += HF_WARPS * 32) {
         const int t = idx / n_in, i = idx - t * n_in;
         xf[idx] = x.at((size_t)t * x_row + (size_t)h * x_head + x_off + i);
     }
     __syncthreads();
-    const int c = blockIdx.y * HF_WARPS + warp;
-    if (c < n_out) {
+    for (int c = c0; c < min(c0 + columns, n_out); ++c) {
         float acc[HF_ROWS];
 #pragma unroll
         for (int t = 0; t < HF_ROWS; ++t) acc[t] = 0.f;
@@ -454,17 +467,19 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
             for (int t = 0; t < HF_ROWS; ++t)
                 if (t < rows) acc[t] = fmaf(xf[t * n_in + i], w, acc[t]);
         }
+        float v = 0.f;                                          // lane t ends up with row t
 #pragma unroll
         for (int t = 0; t < HF_ROWS; ++t) {
             if (t >= rows) continue;
-            float v = warp_sum(acc[t]);
-            if (lane == 0) {
-                if (gate.p != nullptr) {
-                    const float z = gate.at((size_t)t * g_row + g_off + (size_t)h * n_out + c);
-                    v *= 1.f / (1.f + expf(-z));
-                }
-                y[(size_t)t * y_row + (size_t)h * y_head + c] = __float2bfloat16_rn(v);
+            const float total = warp_sum(acc[t]);
+            if (lane == t) v = total;
+        }
+        if (lane < rows) {
+            if (gate.p != nullptr) {
+                const float z = gate.at((size_t)lane * g_row + g_off + (size_t)h * n_out + c);
+                v *= 1.f / (1.f + expf(-z));
             }
+            y[(size_t)lane * y_row + (size_t)h * y_head + c] = __float2bfloat16_rn(v);
         }
     }
     if (blockIdx.y != 0) return;
@@ -574,11 +589,11 @@ extern "C" int kb_head_gate(void* out, int out_dt, const void* y, int y_dt, cons
     const int wide = e >= 512 ? (rows <= DEPENDENT_ROWS ? (e >= 1024 ? 1024 : 512) : 256) : 0;      // threads of a block a head; 0: a warp a head
 #define KB_HG(TY, TS, TW, TO)                                                                                       \
     if (wide)                                                                                                       \
-        head_gate_wide_kernel<TY, TS, TW, TO><<<(unsigned)pairs, wide, 0, s>>>((TO*)out, (const TY*)y,                   \
+        launch_dependent_if(rows <= DEPENDENT_ROWS, head_gate_wide_kernel<TY, TS, TW, TO>, dim3((unsigned)pairs), dim3(wide), 0, s, (TO*)out, (const TY*)y,                   \
                                                                              Src<TS>{(const TS*)gate, splits, (size_t)split_stride}, \
                                                                              row_width, g_off, (const TW*)w, unit, eps, heads, e, out_stride, fill_to, act, by_head, scale); \
     else                                                                                                            \
-    head_gate_kernel<TY, TS, TW, TO><<<(unsigned)blocks, warps * 32, 0, s>>>((TO*)out, (const TY*)y,                    \
+    launch_dependent_if(rows <= DEPENDENT_ROWS, head_gate_kernel<TY, TS, TW, TO>, dim3((unsigned)blocks), dim3(warps * 32), 0, s, (TO*)out, (const TY*)y,                    \
                                                                              Src<TS>{(const TS*)gate, splits, (size_t)split_stride}, \
                                                                              row_width, g_off, (const TW*)w, unit, eps, pairs, heads, e, out_stride, fill_to, act, by_head, scale)
     const int code = y_dt * 8 + g_dt * 4 + w_dt * 2 + out_dt;
@@ -625,7 +640,7 @@ extern "C" int kb_head_norm_rope_append(const void* src, int in_dt, int splits, 
     const int warps = rows <= DEPENDENT_ROWS ? 16 : 4;          // few rows: a head vector a warp side by side
     const size_t smem = (size_t)warps * d * sizeof(float);
 #define KB_HNRA(TS, TW, TO)                                                                                              \
-    head_norm_rope_append_kernel<TS, TW, TO><<<rows, warps * 32, smem, s>>>(                                                 \
+    launch_dependent_if(rows <= DEPENDENT_ROWS, head_norm_rope_append_kernel<TS, TW, TO>, dim3(rows), dim3(warps * 32), smem, s,                                                  \
         Src<TS>{(const TS*)src, splits, (size_t)split_stride}, row_width, q_off, k_off, v_off, (const TW*)wq, eps_q, off_q,  \
         (const TW*)wk, eps_k, off_k, (const float2*)cos_sin, rotary, lines, (TO*)q_out, (TO*)kt, (TO*)v_table, hq, hkv, d, dv, \
         table_lines, page_size)
@@ -660,7 +675,7 @@ extern "C" int kb_latent_append(const void* src, int in_dt, int splits, long lon
     cudaStream_t s = (cudaStream_t)stream;
     void* kt = write_kv ? k_table : nullptr;
 #define KB_LA(TS, TW, TO)                                                                                                  \
-    latent_append_kernel<TS, TW, TO><<<rows, rows <= DEPENDENT_ROWS ? 1024 : 128, 0, s>>>(Src<TS>{(const TS*)src, splits, (size_t)split_stride}, row_width, q_off, \
+    launch_dependent_if(rows <= DEPENDENT_ROWS, latent_append_kernel<TS, TW, TO>, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 128), 0, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, row_width, q_off, \
                                                           kv_off, q_rank, kv_rank, rot, (const TW*)wq, (const TW*)wkv, eps,     \
                                                           (const float2*)cos_sin, lines, (TO*)cq_out, cq_stride, (TO*)kt,       \
                                                           table_lines, page_size)
@@ -736,13 +751,16 @@ extern "C" int kb_head_linear_mma(void* y, int y_row, int y_head, const void* x,
     const Src<float> g{gate, gate ? g_splits : 1, (size_t)g_split_stride};
     const size_t few_smem = (size_t)rows * n_in * sizeof(float);
     if (rows <= HF_ROWS && few_smem <= 48 * 1024 && (n_out + HF_WARPS - 1) / HF_WARPS <= 65535) {     // a decode step: a warp a column
-        dim3 few(heads, (n_out + HF_WARPS - 1) / HF_WARPS);
+        // columns a warp: every block adds up the rows' inputs of its head again, so several where the blocks still fill the GPU
+        int columns = 1;
+        while (columns < 8 && (long long)heads * (n_out / (2 * columns * HF_WARPS)) >= 148) columns *= 2;
+        dim3 few(heads, (n_out + HF_WARPS * columns - 1) / (HF_WARPS * columns));
         if (x_dt == KB_DT_F32)
-            head_linear_few_kernel<float><<<few, HF_WARPS * 32, few_smem, s>>>((bf16*)y, y_row, y_head, Src<float>{(const float*)x, x_splits, (size_t)x_split_stride}, x_row,
-                                                                             x_head, x_off, (const bf16*)mt, n_in, n_out, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
+            launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<float>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, Src<float>{(const float*)x, x_splits, (size_t)x_split_stride}, x_row,
+                                                                             x_head, x_off, (const bf16*)mt, n_in, n_out, columns, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
         else if (x_dt == KB_DT_BF16)
-            head_linear_few_kernel<bf16><<<few, HF_WARPS * 32, few_smem, s>>>((bf16*)y, y_row, y_head, Src<bf16>{(const bf16*)x, x_splits, (size_t)x_split_stride}, x_row,
-                                                                            x_head, x_off, (const bf16*)mt, n_in, n_out, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
+            launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<bf16>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, Src<bf16>{(const bf16*)x, x_splits, (size_t)x_split_stride}, x_row,
+                                                                            x_head, x_off, (const bf16*)mt, n_in, n_out, columns, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
         else return fail("head_linear_mma: dtype code %d is not known", x_dt);
         return check_launch("head_linear_few");
     }

@@ -73,11 +73,23 @@ __device__ __forceinline__ void route_by_warp(float* score, float* choice, const
         }
 }
 
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x, v[1] = x.y, v[2] = x.z, v[3] = x.w;
+}
+__device__ __forceinline__ void load4(const bf16* p, float (&v)[4]) {
+    const uint2 x = *reinterpret_cast<const uint2*>(p);
+    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.x)), b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&x.y));
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
 template <typename TH>
 __global__ void __launch_bounds__(ROUTE_THREADS_FEW)
 moe_route_kernel(const TH* __restrict__ h, const float* __restrict__ router, const float* __restrict__ correction,
                  int* __restrict__ experts_out, float* __restrict__ weights_out, int width, int n_experts, int top, int groups,
                  int keep_groups, int group_top, int softmax, int renormalize, float scale) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ float sm[];
     float* score = sm;                         // [E] s
     float* choice = sm + n_experts;            // [E] s + correction
@@ -88,18 +100,41 @@ moe_route_kernel(const TH* __restrict__ h, const float* __restrict__ router, con
     const TH* hr = h + (size_t)r * width;
     for (int x = warp; x < n_experts; x += blockDim.x / 32) {
         const float* w = router + (size_t)x * width;
-        // eight loads of each operand ahead of their eight additions, which keep the order of i
         float acc = 0.f;
-        for (int i0 = lane; i0 < width; i0 += 32 * 8) {
-            float hv[8], wv[8];
+        if (width % 4 == 0 && (((uintptr_t)h | (uintptr_t)router) & 15) == 0) {
+            // four neighbouring values a load and eight loads of each operand ahead of their sums: 2,048 values are two trips to memory
+            float part[4] = {0.f, 0.f, 0.f, 0.f};
+            for (int i0 = lane * 4; i0 < width; i0 += 32 * 4 * 8) {
+                float hv[8][4];
+                float4 wv[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                const int i = i0 + 32 * u;
-                hv[u] = i < width ? Elem<TH>::load(hr + i) : 0.f;
-                wv[u] = i < width ? w[i] : 0.f;
+                for (int u = 0; u < 8; ++u) {
+                    const int i = i0 + 128 * u;
+                    wv[u] = i < width ? *reinterpret_cast<const float4*>(w + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    load4(hr + (i < width ? i : 0), hv[u]);
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    part[0] = fmaf(hv[u][0], wv[u].x, part[0]);
+                    part[1] = fmaf(hv[u][1], wv[u].y, part[1]);
+                    part[2] = fmaf(hv[u][2], wv[u].z, part[2]);
+                    part[3] = fmaf(hv[u][3], wv[u].w, part[3]);
+                }
             }
+            acc = (part[0] + part[1]) + (part[2] + part[3]);
+        } else {
+            // eight loads of each operand ahead of their eight additions, which keep the order of i
+            for (int i0 = lane; i0 < width; i0 += 32 * 8) {
+                float hv[8], wv[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) acc = fmaf(hv[u], wv[u], acc);
+                for (int u = 0; u < 8; ++u) {
+                    const int i = i0 + 32 * u;
+                    hv[u] = i < width ? Elem<TH>::load(hr + i) : 0.f;
+                    wv[u] = i < width ? w[i] : 0.f;
+                }
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc = fmaf(hv[u], wv[u], acc);
+            }
         }
         acc = warp_sum(acc);
         if (lane == 0) score[x] = acc;
@@ -205,6 +240,8 @@ __global__ void __launch_bounds__(SORT_THREADS)
 moe_sort_kernel(const int* __restrict__ experts, int pairs, int n_experts, int* __restrict__ offsets, int* __restrict__ order,
                 int* __restrict__ tile_expert, int* __restrict__ tile_first, int* __restrict__ tile_rows, int* __restrict__ n_tiles,
                 int tile_cap, int rows_a_tile) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     extern __shared__ int si[];
     int* count = si;                 // [E]
     int* cursor = si + n_experts;    // [E]
@@ -326,7 +363,7 @@ moe_grouped_f32_kernel(const GroupedParams p) {
 // step) keeps loads in flight instead of waiting for each tile; rows of k that are no multiple of
 // 8 are loaded value by value. Two shapes: 32 x 64 (few rows an expert) and 64 x 128 (prompts); 128 x 128 was
 // built and measured no faster (the products run at about 215 TFLOP/s either way).
-constexpr int BSTAGES = 3;
+constexpr int BSTAGES = 3;              // four measured no faster (a decoding step's 31 us a launch is not the ring's depth)
 
 __device__ __forceinline__ void moe_copy16(void* dst, const void* src, bool valid) {
     const uint32_t d32 = (uint32_t)__cvta_generic_to_shared(dst);
@@ -342,6 +379,8 @@ __device__ __forceinline__ void moe_ldmatrix4(uint32_t (&r)[4], const void* at) 
 template <typename TO, int TM, int TN, int WM, int WN, int TK>
 __global__ void __launch_bounds__(WM * WN * 32)
 moe_grouped_bf16_kernel(const GroupedParams p) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     static_assert((TN / WN / 8) % 2 == 0, "a warp's n8 tiles come in pairs");
     constexpr int THREADS = WM * WN * 32;
     constexpr int MT = TM / WM / 16, NT = TN / WN / 8;       // m16 and n8 tiles a warp
@@ -449,6 +488,8 @@ template <typename TO, typename TA>
 __global__ void moe_combine_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights,
                                    long long rows, int width, int top, const Src<TA> also, const int* __restrict__ experts, int real,
                                    const void* __restrict__ self, int self_dt) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * width) return;
     const long long r = i / width;
@@ -488,22 +529,22 @@ extern "C" int kb_moe_route(int* experts, float* weights, const void* h, int h_d
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = rows <= DEPENDENT_ROWS ? ROUTE_THREADS_FEW : ROUTE_THREADS;
     if (h_dt == KB_DT_F32)
-        moe_route_kernel<float><<<rows, threads, smem, s>>>((const float*)h, router, correction, experts, weights, width, n_experts, top,
+        launch_dependent_if(rows <= DEPENDENT_ROWS, moe_route_kernel<float>, dim3(rows), dim3(threads), smem, s, (const float*)h, router, correction, experts, weights, width, n_experts, top,
                                                                   groups, keep_groups, group_top, softmax, renormalize, scale);
     else if (h_dt == KB_DT_BF16)
-        moe_route_kernel<bf16><<<rows, threads, smem, s>>>((const bf16*)h, router, correction, experts, weights, width, n_experts, top,
+        launch_dependent_if(rows <= DEPENDENT_ROWS, moe_route_kernel<bf16>, dim3(rows), dim3(threads), smem, s, (const bf16*)h, router, correction, experts, weights, width, n_experts, top,
                                                                  groups, keep_groups, group_top, softmax, renormalize, scale);
     else return fail("moe_route: dtype code %d is not known", h_dt);
     return check_launch("moe_route");
 }
 
 extern "C" int kb_moe_sort(const int* experts, int pairs, int n_experts, int* offsets, int* order, int* tile_expert,
-                           int* tile_first, int* tile_rows, int* n_tiles, int tile_cap, int rows_a_tile, void* stream) {
+                           int* tile_first, int* tile_rows, int* n_tiles, int tile_cap, int rows_a_tile, int rows, void* stream) {
     KB_REQUIRE(pairs >= 0 && n_experts > 0 && tile_cap >= 0, "moe_sort: %d pairs, %d experts", pairs, n_experts);
     KB_REQUIRE(rows_a_tile == GM || rows_a_tile == GM_LARGE || rows_a_tile == 128, "moe_sort: tiles of %d rows (%d, %d or 128)", rows_a_tile, GM, GM_LARGE);
     const size_t smem = (size_t)2 * n_experts * sizeof(int);
     KB_REQUIRE(smem <= 48 * 1024, "moe_sort: %d experts are too many", n_experts);
-    moe_sort_kernel<<<1, SORT_THREADS, smem, (cudaStream_t)stream>>>(experts, pairs, n_experts, offsets, order, tile_expert, tile_first,
+    launch_dependent_if(rows <= DEPENDENT_ROWS, moe_sort_kernel, dim3(1), dim3(SORT_THREADS), smem, (cudaStream_t)stream, experts, pairs, n_experts, offsets, order, tile_expert, tile_first,
                                                                     tile_rows, n_tiles, tile_cap, rows_a_tile);
     return check_launch("moe_sort");
 }
@@ -511,7 +552,7 @@ extern "C" int kb_moe_sort(const int* experts, int pairs, int n_experts, int* of
 // act: 0 none, 1 relu squared, 2 gelu_tanh, 3 silu.
 extern "C" int kb_moe_grouped(void* out, int out_dt, const void* a, const void* w, int dt, const int* order, const int* tile_expert,
                               const int* tile_first, const int* tile_rows, const int* n_tiles, int tile_cap, int rows_a_tile, int n,
-                              int k, int top, int act, int a_by_token, int out_by_pair, void* stream) {
+                              int k, int top, int act, int a_by_token, int out_by_pair, int rows, void* stream) {
     KB_REQUIRE(n > 0 && k > 0 && top > 0 && tile_cap >= 0, "moe_grouped: n %d, k %d, top %d", n, k, top);
     KB_REQUIRE(rows_a_tile == GM || (rows_a_tile == GM_LARGE && dt == KB_DT_BF16), "moe_grouped: tiles of %d rows", rows_a_tile);
     KB_REQUIRE(act >= 0 && act <= 3, "moe_grouped: activation code %d is not known", act);
@@ -541,7 +582,7 @@ extern "C" int kb_moe_grouped(void* out, int out_dt, const void* a, const void* 
                 set = true;                                                                                                \
             }                                                                                                              \
         }                                                                                                                  \
-        moe_grouped_bf16_kernel<TO, TM, TN, WM, WN, TK><<<grid, WM * WN * 32, bytes, s>>>(p);                                \
+        launch_dependent_if(rows <= DEPENDENT_ROWS, moe_grouped_bf16_kernel<TO, TM, TN, WM, WN, TK>, grid, dim3(WM * WN * 32), bytes, s, p);                                \
     } while (0)
         if (rows_a_tile == GM_LARGE) {
             if (out_dt == KB_DT_F32) KB_MOE_TILE(float, GM_LARGE, 128, 2, 4, 32);
@@ -567,7 +608,7 @@ extern "C" int kb_moe_combine(void* out, int out_dt, const float* y, const float
     KB_REQUIRE(blocks <= 0x7fffffffll, "moe_combine: too many rows for one launch");
     cudaStream_t s = (cudaStream_t)stream;
 #define KB_COMBINE(TO, TA) \
-    moe_combine_kernel<TO, TA><<<(unsigned)blocks, 256, 0, s>>>((TO*)out, y, weights, rows, width, top, Src<TA>{(const TA*)also, also ? also_splits : 1, (size_t)also_stride}, experts, real, self, self_dt)
+    launch_dependent_if(rows <= DEPENDENT_ROWS, moe_combine_kernel<TO, TA>, dim3((unsigned)blocks), dim3(256), 0, s, (TO*)out, y, weights, rows, width, top, Src<TA>{(const TA*)also, also ? also_splits : 1, (size_t)also_stride}, experts, real, self, self_dt)
     const bool narrow = also != nullptr && also_dt == KB_DT_BF16;
     KB_REQUIRE(also == nullptr || also_dt == KB_DT_F32 || also_dt == KB_DT_BF16, "moe_combine: addend dtype code %d is not known", also_dt);
     if (out_dt == KB_DT_F32) { if (narrow) KB_COMBINE(float, bf16); else KB_COMBINE(float, float); }

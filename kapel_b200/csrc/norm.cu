@@ -17,6 +17,8 @@ KB_TIMELINE_ARRAY(norm)        // slots: kind 2 add-and-norm over split sums (sl
 template <typename TX, typename TW, typename TY>
 __global__ void rmsnorm_kernel(TY* __restrict__ y, const TX* __restrict__ x, const TW* __restrict__ w, int width,
                                float eps, float offset) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     __shared__ float scratch[32];
     const size_t base = (size_t)blockIdx.x * width;
     float ss = 0.f;
@@ -569,6 +571,8 @@ __global__ void __launch_bounds__(1024) add_rmsnorm_splits_bulk_kernel(float* __
 template <typename TX, typename TW, typename TY>
 __global__ void centered_norm_kernel(TY* __restrict__ y, const TX* __restrict__ x, const TW* __restrict__ w, const TW* __restrict__ bias,
                                      int width, float eps, float offset) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     __shared__ float scratch[32];
     const size_t base = (size_t)blockIdx.x * width;
     float sum = 0.f;
@@ -690,7 +694,7 @@ extern "C" int kb_rmsnorm(void* y, int y_dt, const void* x, int x_dt, const void
     cudaStream_t s = (cudaStream_t)stream;
     const int t = threads_for(width);
 #define KB_NORM(TX, TW, TY) \
-    rmsnorm_kernel<TX, TW, TY><<<rows, t, 0, s>>>((TY*)y, (const TX*)x, (const TW*)w, width, eps, offset)
+    launch_dependent_if(rows <= DEPENDENT_ROWS, rmsnorm_kernel<TX, TW, TY>, dim3(rows), dim3(t), 0, s, (TY*)y, (const TX*)x, (const TW*)w, width, eps, offset)
     const int code = x_dt * 4 + w_dt * 2 + y_dt;
     switch (code) {
         case 0: KB_NORM(float, float, float); break;
@@ -813,7 +817,7 @@ extern "C" int kb_layernorm(void* y, int y_dt, const void* x, int x_dt, const vo
     cudaStream_t s = (cudaStream_t)stream;
     const int t = threads_for(width);
 #define KB_LNORM(TX, TW, TY) \
-    centered_norm_kernel<TX, TW, TY><<<rows, t, 0, s>>>((TY*)y, (const TX*)x, (const TW*)w, (const TW*)bias, width, eps, offset)
+    launch_dependent_if(rows <= DEPENDENT_ROWS, centered_norm_kernel<TX, TW, TY>, dim3(rows), dim3(t), 0, s, (TY*)y, (const TX*)x, (const TW*)w, (const TW*)bias, width, eps, offset)
     const int code = x_dt * 4 + w_dt * 2 + y_dt;
     switch (code) {
         case 0: KB_LNORM(float, float, float); break;

@@ -427,6 +427,8 @@ struct RetentionParams {
 template <typename TS>
 __global__ void __launch_bounds__(1024)
 retention_prep_kernel(const Src<TS> src, const RetentionParams p, const ScanInputs s) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const int r = blockIdx.x;
     const size_t base = (size_t)r * p.row_width;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -986,8 +988,8 @@ extern "C" int kb_retention_scan(float* out, float* scratch, const void* src, in
     in.nv = 2;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = rows <= DEPENDENT_ROWS ? 1024 : 256;      // few rows: latency counts
-    if (in_dt == KB_DT_F32) retention_prep_kernel<float><<<rows, threads, 0, s>>>(Src<float>{(const float*)src, splits, (size_t)split_stride}, g, in);
-    else if (in_dt == KB_DT_BF16) retention_prep_kernel<bf16><<<rows, threads, 0, s>>>(Src<bf16>{(const bf16*)src, splits, (size_t)split_stride}, g, in);
+    if (in_dt == KB_DT_F32) launch_dependent_if(rows <= DEPENDENT_ROWS, retention_prep_kernel<float>, dim3(rows), dim3(threads), 0, s, Src<float>{(const float*)src, splits, (size_t)split_stride}, g, in);
+    else if (in_dt == KB_DT_BF16) launch_dependent_if(rows <= DEPENDENT_ROWS, retention_prep_kernel<bf16>, dim3(rows), dim3(threads), 0, s, Src<bf16>{(const bf16*)src, splits, (size_t)split_stride}, g, in);
     else return fail("retention: dtype code %d is not known", in_dt);
     if (int err = check_launch("retention prep")) return err;
     if (by_chunks(longest))

@@ -228,6 +228,8 @@ stream_step_kernel(const StreamParams p, const Src<TB> a, const Src<TB> b, TH* _
 
 __global__ void stream_sum_kernel(float* __restrict__ out, const float* __restrict__ x, const int* __restrict__ rows, int width, int streams,
                                   int src_rows) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
     const int i = blockIdx.y, c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= width) return;
     const int r = rows[i];
@@ -304,6 +306,6 @@ extern "C" int kb_stream_sum(float* out, const float* x, const int* rows, int n,
     KB_REQUIRE(n >= 0 && width > 0 && streams >= 1, "stream_sum: n %d, width %d, %d streams", n, width, streams);
     KB_REQUIRE(n <= 65535, "stream_sum: %d rows are too many for one launch", n);
     if (n == 0) return 0;
-    stream_sum_kernel<<<dim3((unsigned)((width + 255) / 256), n), 256, 0, (cudaStream_t)stream>>>(out, x, rows, width, streams, src_rows);
+    launch_dependent_if(src_rows <= DEPENDENT_ROWS, stream_sum_kernel, dim3((unsigned)((width + 255) / 256), n), dim3(256), 0, (cudaStream_t)stream, out, x, rows, width, streams, src_rows);
     return check_launch("stream_sum");
 }

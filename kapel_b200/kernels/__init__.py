@@ -702,6 +702,10 @@ def latent_attention_mma(q, table, block_table, row_count, ranges, entries: int,
     out = _fresh((rows, hq, dv), torch.bfloat16, q.device)
     lib = library()
     chunk = attention_chunk()
+    if longest == 1:        # single tokens: a block a chunk of 128 keys, while the launch stays within four waves of blocks
+        finer = -(-int(slots) * chunk // int(lib.kb_latent_decode_keys()))
+        if rows * (-(-hq // 16)) * finer <= 4 * 148:
+            chunk, slots = int(lib.kb_latent_decode_keys()), finer
     if longest > 1:         # measured at 2,048 tokens, 16 heads, lines of 576: 4.91, 4.68, 4.52, 4.43 ms a four-layer prefill with 1, 2, 4, 8
         chunk, slots = chunk * LATENT_PROMPT_CHUNKS, -(-int(slots) // LATENT_PROMPT_CHUNKS)
     need = lib.kb_paged_attention_scratch_floats(rows, hq, dv, int(slots))
@@ -1792,7 +1796,7 @@ def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.f
     lists.tiles = (buf[at : at + cap], buf[at + cap : at + 2 * cap], buf[at + 2 * cap : at + 3 * cap], buf[at + 3 * cap :])
     _check(library().kb_moe_sort(_ptr(experts), pairs, int(n_experts), _ptr(lists.offsets), _ptr(lists.order), _ptr(lists.tiles[0]),
                                  _ptr(lists.tiles[1]), _ptr(lists.tiles[2]), _ptr(lists.tiles[3]), int(lists.tile_cap),
-                                 int(lists.tile_rows), _stream()))
+                                 int(lists.tile_rows), rows, _stream()))
     return lists
 
 
@@ -1812,7 +1816,7 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, lists: ExpertLists, act: str, 
     t = lists.tiles
     _check(library().kb_moe_grouped(_ptr(out), _CODES[out_dtype], _ptr(a), _ptr(w), _dt(a, "moe_grouped input"), _ptr(lists.order),
                                     _ptr(t[0]), _ptr(t[1]), _ptr(t[2]), _ptr(t[3]), int(lists.tile_cap), int(lists.tile_rows), n, k, int(lists.top),
-                                    MOE_ACT_CODES[act], int(bool(a_by_token)), int(bool(out_by_pair)), _stream()))
+                                    MOE_ACT_CODES[act], int(bool(a_by_token)), int(bool(out_by_pair)), lists.pairs // lists.top, _stream()))
     return out
 
 
