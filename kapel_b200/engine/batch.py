@@ -62,6 +62,11 @@ def decode_split(pairs: int, longest: int, sms: int, window: Optional[int] = Non
 LATENT_PROMPT_ROWS = 64
 LATENT_PROMPT_POSITIONS = 131072
 
+# The 32-bit attention by tiles: rows a tile, and the fewest tokens a request may bring (a tile takes 17 us a 64 keys however few its rows,
+# the row-wise kernel a twentieth of that a row and chunk side by side).
+ROW_TILE = 32
+ROW_TILE_TOKENS = 16
+
 # What a block costs beyond its 64-key steps, what the merge of partial sums costs beyond its traffic
 # (both in steps), microseconds a step, and how many multiprocessors a block takes, by prompt kernel;
 # from sweeps of the split at Gemma 2 2B head sizes with 2,048 tokens behind 4,096 to 129,024 (a block
@@ -284,6 +289,23 @@ class StepBatch:
                 self.memo[key] = None
             else:
                 arrays = cut_tiles(plan.q_start, plan.q_len, K.pooled_attention_tile_rows())
+                n = arrays[0].size
+                host = torch.from_numpy(np.concatenate(arrays)).pin_memory()
+                dev = host.to(self.ids.device, non_blocking=True)
+                self.memo[key] = (dev[:n], dev[n : 2 * n], dev[2 * n :], host)
+        tiles = self.memo[key]
+        return tiles[:3] if tiles is not None else None
+
+    def row_tiles(self, heads_per_kv: int):
+        """(tile_entry, tile_row0, tile_nq) on the device for the 32-bit attention by tiles of ROW_TILE rows (tokens x query heads of a kv
+        head), or None where some request brings fewer than ROW_TILE_TOKENS tokens (its tile would hold a few rows and walk all its keys alone)."""
+        key = ("row_tiles", heads_per_kv)
+        if key not in self.memo:
+            plan = self.plan
+            if not len(plan.q_len) or self.shortest_portion() < ROW_TILE_TOKENS or heads_per_kv > ROW_TILE or not self.ids.is_cuda:
+                self.memo[key] = None
+            else:
+                arrays = cut_tiles(plan.q_start, plan.q_len, ROW_TILE // heads_per_kv)
                 n = arrays[0].size
                 host = torch.from_numpy(np.concatenate(arrays)).pin_memory()
                 dev = host.to(self.ids.device, non_blocking=True)

@@ -74,6 +74,9 @@ class StaticBatch:
     def shortest_portion(self) -> int:
         return 1
 
+    def row_tiles(self, heads_per_kv: int):
+        return None
+
     def latent_tiles(self):
         return None
 

@@ -630,14 +630,15 @@ def attention_chunk() -> int:
 
 def paged_attention_rows(q, k_table, v_table, block_table, row_entry, row_count, page_size: int, window: Optional[int],
                          scale: float, softcap: Optional[float], slots: int, keep_first: int = 0,
-                         sinks: Optional[torch.Tensor] = None, value_dim: Optional[int] = None, block: int = 0) -> torch.Tensor:
+                         sinks: Optional[torch.Tensor] = None, value_dim: Optional[int] = None, block: int = 0, tiles=None) -> torch.Tensor:
     """Attention of each query row over its sequence's pages; with `block` > 0 a row at position i sees
     only the keys from floor(i / block) * block on (`slots` as for a window of `block` positions); `slots` is the largest number of
     key chunks (of `attention_chunk()` positions, cut at absolute multiples) any row touches, plus,
     with a window and `keep_first` > 0, the chunks of the first `keep_first` keys, which stay
     visible below the window (`attention_keep_slots`). The values' size is the v table's last, or
     `value_dim`: the first that many components of each of the v table's lines (the v table may then be
-    the k table itself). `sinks` [hq] float32: e^sink joins each row's denominator (no key, no value)."""
+    the k table itself). `sinks` [hq] float32: e^sink joins each row's denominator (no key, no value). With `tiles`
+    (`StepBatch.row_tiles`) float32 prompt portions run by tiles of rows where that kernel takes the sizes."""
     rows, hq, d = q.shape
     _need(q, "attention q")
     _need(k_table, "attention k table", q.dtype)
@@ -655,6 +656,14 @@ def paged_attention_rows(q, k_table, v_table, block_table, row_entry, row_count,
     _need(row_count, "attention row_count", torch.int32, (rows,))
     out = _fresh((rows, hq, dv), q.dtype, q.device)
     lib = library()
+    if tiles is not None and q.dtype == torch.float32 and dv == d == v_stride and not keep_first and not block and lib.kb_attention_f32_tiles_takes(hq, hkv, d):
+        n_tiles = tiles[0].numel()
+        for t in tiles:
+            _need(t, "attention tiles", torch.int32, (n_tiles,))
+        _check(lib.kb_attention_f32_tiles(_ptr(out), _ptr(q), _ptr(k_table), _ptr(v_table), _ptr(block_table), _ptr(row_count), _ptr(tiles[0]), _ptr(tiles[1]),
+                                          _ptr(tiles[2]), n_tiles, rows, hq, hkv, d, int(page_size), int(block_table.shape[1]), int(n_pages), int(window or 0),
+                                          _f(scale), _f(softcap or 0.0), _ptr(sinks), _stream()))
+        return out
     need = lib.kb_paged_attention_scratch_floats(rows, hq, dv, int(slots))
     scratch = _fresh((need,), torch.float32, q.device) if need else None
     _check(

@@ -1,0 +1,53 @@
+"""The 32-bit attention by tiles of rows against 64-bit and against the row-wise kernel: windows, soft caps, sinks, several requests, keys at
+the borders of tiles and pages."""
+import pytest
+import torch
+
+from test_gpu_flash import cut
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("portions", [[(0, 16), (0, 65)], [(0, 63), (64, 17)], [(129, 40), (0, 130), (500, 16)]])
+@pytest.mark.parametrize("hq,hkv,d,window,cap", [(2, 2, 128, None, None), (8, 4, 256, None, 50.0), (8, 2, 128, 70, None), (3, 1, 256, 64, 5.0)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_against_64_bit_and_by_rows(portions, hq, hkv, d, window, cap, sink):
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    longest = max(b + n for b, n in portions)
+    width = -(-longest // 16)
+    order = torch.randperm(width * len(portions) + 2, generator=torch.Generator().manual_seed(1))
+    k_table, v_table = (torch.full((len(order), hkv, 16, d), float("nan"), device="cuda") for _ in range(2))
+    table = torch.full((len(portions), width + 1), -1, dtype=torch.int32)
+    rows = sum(n for _, n in portions)
+    q, sinks = make(rows, hq, d) * 2, (make(hq) * 2 if sink else None)
+    counts, want, entries, at = [], [], [], 0
+    for e, (before, n) in enumerate(portions):
+        T = before + n
+        k, v = make(T, hkv, d), make(T, hkv, d)
+        k[T // 2] *= 4.0
+        for pg in range(-(-T // 16)):
+            where = int(order[e * width + pg])
+            table[e, pg] = where
+            m = min(16, T - pg * 16)
+            k_table[where, :, :m] = k[pg * 16 : pg * 16 + m].transpose(0, 1)
+            v_table[where, :, :m] = v[pg * 16 : pg * 16 + m].transpose(0, 1)
+        s = torch.einsum("nhd,thd->hnt", q[at : at + n].double(), k.double().repeat_interleave(hq // hkv, 1)) * d ** -0.5
+        s = cap * torch.tanh(s / cap) if cap else s
+        count, t = torch.arange(before + 1, T + 1, device="cuda")[:, None], torch.arange(T, device="cuda")[None, :]
+        s = s.masked_fill(~((t < count) & (t >= (count - window if window else 0)))[None], -torch.inf)
+        if sink:
+            s = torch.cat([s, sinks.double()[:, None, None].expand(hq, n, 1)], 2)
+        want.append(torch.einsum("hnt,thd->nhd", torch.softmax(s, -1)[..., :T], v.double().repeat_interleave(hq // hkv, 1)))
+        counts += list(range(before + 1, T + 1))
+        entries += [e] * n
+        at += n
+    args = (q, k_table, v_table, table.cuda(), torch.tensor(entries, dtype=torch.int32, device="cuda"), torch.tensor(counts, dtype=torch.int32, device="cuda"),
+            16, window, d ** -0.5, cap, longest // K.attention_chunk() + 2)
+    want = torch.cat(want)
+    by_rows, by_tiles = K.paged_attention_rows(*args, sinks=sinks), K.paged_attention_rows(*args, sinks=sinks, tiles=cut(portions, 32 // (hq // hkv)))
+    off = lambda x: float((x.double() - want).abs().max() / want.abs().max())
+    # products of d terms and sums of up to 630 weights in 32-bit; a score of 30 moves by 2^-19 when it is rounded
+    assert off(by_tiles) <= 1e-5 and off(by_tiles) <= 3.0 * off(by_rows) + 1e-6, (off(by_tiles), off(by_rows))
