@@ -120,6 +120,48 @@ __global__ void head_gate_kernel(TO* __restrict__ out, const TY* __restrict__ y,
         for (int c = heads * e + lane; c < fill_to; c += 32) Elem<TO>::store(out + (size_t)r * out_stride + c, 0.f);
 }
 
+// The same for prompts where every row, column and width is a multiple of four and the gate is one 32-bit slice: a lane takes four
+// neighbouring values at a time. 2,048 rows of 16 heads of 128: 14 us against 22.
+template <typename TY, typename TW, typename TO>
+__global__ void head_gate_fours_kernel(TO* __restrict__ out, const TY* __restrict__ y, const float* __restrict__ gate, int row_width, int g_off,
+                                       const TW* __restrict__ w, int unit, float eps, long long pairs, int heads, int e, int out_stride, int fill_to,
+                                       int act, float scale) {
+    const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (pair >= pairs) return;
+    const int lane = threadIdx.x & 31;
+    const long long r = pair / heads;
+    const int h = (int)(pair - r * heads);
+    const TY* yp = y + (size_t)pair * e;
+    float inv = 1.f;
+    if (unit) {
+        float ss = 0.f;
+        for (int c = lane * 4; c < e; c += 128) {
+            const float4 v = load_four(yp + c);
+            ss += v.x * v.x + v.y * v.y + v.z * v.z + v.w * v.w;
+        }
+        ss = warp_sum(ss);
+        inv = 1.f / sqrtf(ss / (float)e + eps);
+    }
+    inv *= scale;
+    for (int c = lane * 4; c < e; c += 128) {
+        float4 v = load_four(yp + c);
+        v.x *= inv, v.y *= inv, v.z *= inv, v.w *= inv;
+        if (w != nullptr) {
+            const float4 x = load_four(w + (size_t)h * e + c);
+            v.x *= x.x, v.y *= x.y, v.z *= x.z, v.w *= x.w;
+        }
+        if (act != 2) {
+            const float4 z = load_four(gate + (size_t)r * row_width + g_off + (size_t)h * e + c);
+            const float4 s = make_float4(1.f + expf(-z.x), 1.f + expf(-z.y), 1.f + expf(-z.z), 1.f + expf(-z.w));
+            if (act == 1) v.x *= z.x / s.x, v.y *= z.y / s.y, v.z *= z.z / s.z, v.w *= z.w / s.w;
+            else v.x *= 1.f / s.x, v.y *= 1.f / s.y, v.z *= 1.f / s.z, v.w *= 1.f / s.w;
+        }
+        store_four(out + (size_t)r * out_stride + (size_t)h * e + c, v);
+    }
+    if (h == heads - 1)
+        for (int c = heads * e + lane; c < fill_to; c += 32) Elem<TO>::store(out + (size_t)r * out_stride + c, 0.f);
+}
+
 // The same for wide heads (a whole row normed as one, say): one block a (row, head).
 template <typename TY, typename TS, typename TW, typename TO>
 __global__ void __launch_bounds__(1024)
@@ -162,6 +204,56 @@ head_gate_wide_kernel(TO* __restrict__ out, const TY* __restrict__ y, const Src<
 
 // One block a row; a warp takes head vectors in turn (queries, then keys, then values) through a
 // piece of shared memory of its own.
+// The kernel below for prompts whose heads are 128 wide: a warp a (row, head of q, k or v), a lane four neighbouring components, the
+// rotation's partners by shuffles; the same roundings. 2,048 rows of 16 + 4 + 4 heads: 14 us against 31.
+template <typename TW, typename TO>
+__global__ void head_norm_rope_append_128_kernel(const float* __restrict__ src, int row_width, int q_off, int k_off, int v_off,
+                                                 const TW* __restrict__ wq, float eps_q, float off_q, const TW* __restrict__ wk, float eps_k, float off_k,
+                                                 const float2* __restrict__ cos_sin, int rotary, const int* __restrict__ lines, TO* __restrict__ q_out,
+                                                 TO* __restrict__ k_table, TO* __restrict__ v_table, int rows, int hq, int hkv, long long table_lines, int page_size) {
+    const int units = hq + 2 * hkv;
+    const long long at = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (at >= (long long)rows * units) return;
+    const int r = (int)(at / units), u = (int)(at - (long long)r * units), lane = threadIdx.x & 31;
+    const bool is_q = u < hq, is_v = u >= hq + hkv;
+    const int h = is_q ? u : (is_v ? u - hq - hkv : u - hq);
+    long long line = -1;
+    if (!is_q) {
+        if (k_table != nullptr) line = lines[r];
+        if (line < 0 || line >= table_lines) return;            // a row that writes nowhere
+    }
+    float4 v = load_four(src + (size_t)r * row_width + (is_q ? q_off : is_v ? v_off : k_off) + (size_t)h * 128 + lane * 4);
+    if (!is_v) {
+        const TW* w = is_q ? wq : wk;
+        if (w != nullptr) {
+            float ss = fmaf(v.w, v.w, fmaf(v.z, v.z, fmaf(v.y, v.y, v.x * v.x)));
+            ss = warp_sum(ss);
+            const float inv = 1.f / sqrtf(ss / 128.f + (is_q ? eps_q : eps_k)), off = is_q ? off_q : off_k;
+            const float4 g = load_four(w + lane * 4);
+            v.x = v.x * inv * (off + g.x), v.y = v.y * inv * (off + g.y), v.z = v.z * inv * (off + g.z), v.w = v.w * inv * (off + g.w);
+        }
+        if (rotary > 0) {
+            const int half = rotary >> 1, i = lane * 4, hop = half >> 2;
+            const int from = i < half ? lane + hop : (i < rotary ? lane - hop : lane);
+            const float4 o = make_float4(__shfl_sync(0xffffffffu, v.x, from), __shfl_sync(0xffffffffu, v.y, from),
+                                         __shfl_sync(0xffffffffu, v.z, from), __shfl_sync(0xffffffffu, v.w, from));
+            if (i < rotary) {
+                const float4* cs = reinterpret_cast<const float4*>(cos_sin + (size_t)r * half + (i < half ? i : i - half));
+                const float4 c01 = cs[0], c23 = cs[1];          // (cos, sin) of two neighbouring pairs each
+                if (i < half) {
+                    v.x = __fmaf_rn(v.x, c01.x, -__fmul_rn(o.x, c01.y)), v.y = __fmaf_rn(v.y, c01.z, -__fmul_rn(o.y, c01.w));
+                    v.z = __fmaf_rn(v.z, c23.x, -__fmul_rn(o.z, c23.y)), v.w = __fmaf_rn(v.w, c23.z, -__fmul_rn(o.w, c23.w));
+                } else {
+                    v.x = __fmaf_rn(v.x, c01.x, __fmul_rn(o.x, c01.y)), v.y = __fmaf_rn(v.y, c01.z, __fmul_rn(o.y, c01.w));
+                    v.z = __fmaf_rn(v.z, c23.x, __fmul_rn(o.z, c23.y)), v.w = __fmaf_rn(v.w, c23.z, __fmul_rn(o.w, c23.w));
+                }
+            }
+        }
+    }
+    TO* dst = is_q ? q_out + ((size_t)r * hq + h) * 128 : (is_v ? v_table : k_table) + kv_row(line, h, hkv, page_size) * 128;
+    store_four(dst + lane * 4, v);
+}
+
 template <typename TS, typename TW, typename TO>
 __global__ void head_norm_rope_append_kernel(const Src<TS> src, int row_width, int q_off, int k_off, int v_off,
                                              const TW* __restrict__ wq, float eps_q, float off_q,
@@ -587,6 +679,25 @@ extern "C" int kb_head_gate(void* out, int out_dt, const void* y, int y_dt, cons
     const long long blocks = (pairs + warps - 1) / warps;
     KB_REQUIRE(pairs <= 0x7fffffffll, "head_gate: too many rows for one launch");
     const int wide = e >= 512 ? (rows <= DEPENDENT_ROWS ? (e >= 1024 ? 1024 : 512) : 256) : 0;      // threads of a block a head; 0: a warp a head
+    if (!wide && rows > DEPENDENT_ROWS && ((g_dt == KB_DT_F32 && splits == 1 && !by_head) || act == 2) && (e | row_width | g_off | out_stride) % 4 == 0 &&
+        (((uintptr_t)out | (uintptr_t)y | (uintptr_t)gate | (uintptr_t)w) & 15) == 0) {
+#define KB_HG4(TY, TW, TO)                                                                                                 \
+    head_gate_fours_kernel<TY, TW, TO><<<(unsigned)((pairs + 7) / 8), 256, 0, s>>>((TO*)out, (const TY*)y, (const float*)gate, row_width, g_off, \
+                                                                                   (const TW*)w, unit, eps, pairs, heads, e, out_stride, fill_to, act, scale)
+        switch (y_dt * 4 + w_dt * 2 + out_dt) {
+            case 0: KB_HG4(float, float, float); break;
+            case 1: KB_HG4(float, float, bf16); break;
+            case 2: KB_HG4(float, bf16, float); break;
+            case 3: KB_HG4(float, bf16, bf16); break;
+            case 4: KB_HG4(bf16, float, float); break;
+            case 5: KB_HG4(bf16, float, bf16); break;
+            case 6: KB_HG4(bf16, bf16, float); break;
+            case 7: KB_HG4(bf16, bf16, bf16); break;
+            default: return fail("head_gate: dtype codes y %d, w %d, out %d are not known", y_dt, w_dt, out_dt);
+        }
+#undef KB_HG4
+        return check_launch("head_gate");
+    }
 #define KB_HG(TY, TS, TW, TO)                                                                                       \
     if (wide)                                                                                                       \
         launch_dependent_if(rows <= DEPENDENT_ROWS, head_gate_wide_kernel<TY, TS, TW, TO>, dim3((unsigned)pairs), dim3(wide), 0, s, (TO*)out, (const TY*)y,                   \
@@ -639,6 +750,20 @@ extern "C" int kb_head_norm_rope_append(const void* src, int in_dt, int splits, 
     void* kt = write_kv ? k_table : nullptr;
     const int warps = rows <= DEPENDENT_ROWS ? 16 : 4;          // few rows: a head vector a warp side by side
     const size_t smem = (size_t)warps * d * sizeof(float);
+    const bool fours = rows > DEPENDENT_ROWS && d == 128 && dv == 128 && in_dt == KB_DT_F32 && splits == 1 && rotary % 8 == 0 && (row_width | q_off | k_off | v_off) % 4 == 0 &&
+                       (((uintptr_t)src | (uintptr_t)wq | (uintptr_t)wk | (uintptr_t)cos_sin | (uintptr_t)q_out | (uintptr_t)kt | (uintptr_t)v_table) & 15) == 0;
+    if (fours) {
+        const unsigned blocks = (unsigned)(((long long)rows * (hq + 2 * hkv) + 7) / 8);
+#define KB_HNRA4(TW, TO)                                                                                                   \
+    head_norm_rope_append_128_kernel<TW, TO><<<blocks, 256, 0, s>>>((const float*)src, row_width, q_off, k_off, v_off, (const TW*)wq, eps_q, off_q, \
+        (const TW*)wk, eps_k, off_k, (const float2*)cos_sin, rotary, lines, (TO*)q_out, (TO*)kt, (TO*)v_table, rows, hq, hkv, table_lines, page_size)
+        if (w_dt == KB_DT_F32 && out_dt == KB_DT_F32) KB_HNRA4(float, float);
+        else if (w_dt == KB_DT_F32) KB_HNRA4(float, bf16);
+        else if (out_dt == KB_DT_F32) KB_HNRA4(bf16, float);
+        else KB_HNRA4(bf16, bf16);
+#undef KB_HNRA4
+        return check_launch("head_norm_rope_append");
+    }
 #define KB_HNRA(TS, TW, TO)                                                                                              \
     launch_dependent_if(rows <= DEPENDENT_ROWS, head_norm_rope_append_kernel<TS, TW, TO>, dim3(rows), dim3(warps * 32), smem, s,                                                  \
         Src<TS>{(const TS*)src, splits, (size_t)split_stride}, row_width, q_off, k_off, v_off, (const TW*)wq, eps_q, off_q,  \
