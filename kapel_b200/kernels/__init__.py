@@ -1790,6 +1790,26 @@ def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.f
     """Lists the pairs of `experts` [rows, top] by expert, those from number `n_experts` on (experts without weights) left out; `dtype` is the grouped products' (it and the
     rows an expert gets on average decide how many rows a tile of those products has)."""
     _need(experts, "moe_sort experts", torch.int32)
+def moe_skinny_takes(dtype: torch.dtype, rows: int, widths) -> bool:
+    """Whether a decoding step of `rows` tokens streams its experts' weights through `moe_skinny`."""
+    return dtype == torch.bfloat16 and 0 < rows <= 64 and GEMM_SMALL == "skinny" and all(w % 8 == 0 for w in widths)
+
+
+def moe_skinny(a: torch.Tensor, w: torch.Tensor, lists: "ExpertLists", out_by_pair: bool) -> torch.Tensor:
+    """The grouped product of a decoding step on tcgen05, 32-bit out [pairs, n]: a [pairs, k] in the lists' order, w [experts, n, k]; lists
+    with tiles of 32 rows."""
+    _need(a, "moe_skinny input", torch.bfloat16)
+    _need(w, "moe_skinny weights", torch.bfloat16)
+    if w.dim() != 3 or w.shape[2] != a.shape[1] or a.shape[0] != lists.pairs or lists.tile_rows != 32:
+        raise KernelError(f"moe_skinny: weights {tuple(w.shape)} against {tuple(a.shape)}, tiles of {lists.tile_rows} rows")
+    n, k = int(w.shape[1]), int(w.shape[2])
+    out = _fresh((lists.pairs, n), torch.float32, a.device)
+    t = lists.tiles
+    _check(library().kb_moe_skinny_tcgen05(_ptr(out), _ptr(a), _ptr(w), int(w.shape[0]), _ptr(t[0]), _ptr(t[1]), _ptr(t[2]), _ptr(t[3]), int(lists.tile_cap),
+                                           _ptr(lists.order) if out_by_pair else None, lists.pairs, n, k, lists.pairs // lists.top, _stream()))
+    return out
+
+
     rows, top = experts.shape
     pairs = rows * top
     lists = ExpertLists()

@@ -81,7 +81,8 @@ class MoE(Part):
                                        s.renormalize, s.route_scale)
         own = h if s.identity else None
         tiled = K.moe_tcgen05_takes(self.w_up.dtype, h.shape[0], s.top, s.experts, (s.hidden, s.intermediate), s.activation, s.gated)
-        lists = K.moe_sort(experts, s.experts, self.w_up.dtype, 128 if tiled else None)
+        few = not tiled and s.gated and K.moe_skinny_takes(self.w_up.dtype, h.shape[0], (s.hidden, s.intermediate))
+        lists = K.moe_sort(experts, s.experts, self.w_up.dtype, 128 if tiled else (32 if few else None))
         if h.dtype != self.w_up.dtype:
             h = K.cast(h, self.w_up.dtype)
         also = self.shared.forward(h) if self.shared is not None else None
@@ -90,12 +91,12 @@ class MoE(Part):
             y = K.moe_tcgen05(inner, self.w_down, lists, None, True, torch.float32)
             return K.moe_combine(y, weights, torch.float32, also=also, experts=experts if s.identity else None, real=s.experts, own=own)
         if s.gated:
-            both = K.moe_grouped(h, self.w_up, lists, "none", True, False, torch.float32)
+            both = K.moe_skinny(K.moe_gather(h, lists), self.w_up, lists, False) if few else K.moe_grouped(h, self.w_up, lists, "none", True, False, torch.float32)
             if self.clamped:
                 inner = K.glu_clamped(both, s.limit, s.swish_alpha, out_dtype=self.w_up.dtype)
             else:
                 inner = K.glu(both, s.activation, out_dtype=self.w_up.dtype)
         else:
             inner = K.moe_grouped(h, self.w_up, lists, s.activation, True, False, self.w_up.dtype)
-        y = K.moe_grouped(inner, self.w_down, lists, "none", False, True, torch.float32)
+        y = K.moe_skinny(inner, self.w_down, lists, True) if few else K.moe_grouped(inner, self.w_down, lists, "none", False, True, torch.float32)
         return K.moe_combine(y, weights, torch.float32, also=also, experts=experts if s.identity else None, real=s.experts, own=own)

@@ -42,3 +42,40 @@ def test_against_64_bit(act, counts, identity, width, inner):
     back = torch.einsum("pk,pnk->pn", got[:listed].double(), w_down[expert].double())
     assert (y[order].double() - back).abs().max() <= 1e-5 * back.abs().max()
     K.check_async_errors()
+
+
+@pytest.mark.parametrize("counts,identity", [([0, 32, 1, 7], 5), ([33], 0), ([3, 0, 65], 1)])
+@pytest.mark.parametrize("width,n", [(72, 40), (256, 136), (520, 128)])
+def test_few_rows_against_64_bit(counts, identity, width, n):
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(width + n)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)
+    experts = len(counts)
+    chosen = torch.cat([torch.full((c,), e) for e, c in enumerate(counts)] + [torch.full((identity,), experts)])
+    chosen = chosen[torch.randperm(len(chosen), generator=torch.Generator().manual_seed(2))].to(torch.int32).view(-1, 1).cuda()
+    h, w = make(chosen.shape[0], width).bfloat16(), make(experts, n, width).bfloat16()
+    lists = K.moe_sort(chosen, experts, torch.bfloat16, 32)
+    rows = K.moe_gather(h, lists)
+    listed = int(lists.offsets[-1])
+    order = lists.order[:listed].long()
+    want = torch.einsum("pk,pnk->pn", h[order].double(), w[chosen.view(-1)[order].long()].double())
+    for by_pair in (False, True):
+        got = K.moe_skinny(rows, w, lists, by_pair)
+        assert ((got[order] if by_pair else got[:listed]).double() - want).abs().max() <= 1e-5 * want.abs().max()      # 32-bit sums
+    K.check_async_errors()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("scoring", ["sigmoid", "softmax", "softmax_chosen"])
+def test_the_router_by_rows_and_a_row_a_block(dtype, scoring):
+    """The router of a prompt takes eight rows a block: the same choices and weights as the rows one decoding step at a time."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    h, router = torch.randn(77, 516, device="cuda", generator=gen).to(dtype), torch.randn(19, 516, device="cuda", generator=gen) * 0.1
+    correction = torch.randn(19, device="cuda", generator=gen) * 0.1
+    experts, weights = K.moe_route(h, router, correction, 5, 1, 1, 1, scoring, True, 1.5)
+    for at in range(0, 77, 40):
+        e, w = K.moe_route(h[at : at + 40].contiguous(), router, correction, 5, 1, 1, 1, scoring, True, 1.5)
+        assert torch.equal(e, experts[at : at + 40]) and torch.equal(w, weights[at : at + 40])
