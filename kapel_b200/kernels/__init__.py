@@ -1786,10 +1786,6 @@ def moe_tcgen05(a: torch.Tensor, w: torch.Tensor, lists: "ExpertLists", act: Opt
     return out
 
 
-def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.float32, tile_rows: Optional[int] = None) -> ExpertLists:
-    """Lists the pairs of `experts` [rows, top] by expert, those from number `n_experts` on (experts without weights) left out; `dtype` is the grouped products' (it and the
-    rows an expert gets on average decide how many rows a tile of those products has)."""
-    _need(experts, "moe_sort experts", torch.int32)
 def moe_skinny_takes(dtype: torch.dtype, rows: int, widths) -> bool:
     """Whether a decoding step of `rows` tokens streams its experts' weights through `moe_skinny`."""
     return dtype == torch.bfloat16 and 0 < rows <= 64 and GEMM_SMALL == "skinny" and all(w % 8 == 0 for w in widths)
@@ -1810,6 +1806,10 @@ def moe_skinny(a: torch.Tensor, w: torch.Tensor, lists: "ExpertLists", out_by_pa
     return out
 
 
+def moe_sort(experts: torch.Tensor, n_experts: int, dtype: torch.dtype = torch.float32, tile_rows: Optional[int] = None) -> ExpertLists:
+    """Lists the pairs of `experts` [rows, top] by expert, those from number `n_experts` on (experts without weights) left out; `dtype` is the grouped products' (it and the
+    rows an expert gets on average decide how many rows a tile of those products has)."""
+    _need(experts, "moe_sort experts", torch.int32)
     rows, top = experts.shape
     pairs = rows * top
     lists = ExpertLists()
