@@ -252,6 +252,39 @@ class StepBatch:
             self.memo[key] = (decode, tiles, split, slots, relative, host)
         return self.memo[key][:5]
 
+    def mixed_tiles(self, heads_per_kv: int, kv_heads: int, window: Optional[int], head_dim: int, prompt_kernel: str):
+        """How a pass of single tokens ahead of prompt portions is cut in two, or None where it is not: (rows of the first part, its
+        (decode, tiles, split, slots, relative) as `attention_tiles` gives them for a decoding step, the second part's with rows counted from
+        its first). Cut only where the single tokens' tiles, a handful of rows each, would be a wave of their own on the prompt
+        kernel, which takes some 20 us a block whatever its rows: 32 single tokens behind 500 to 1,500 positions beside a prompt
+        of 2,016, 16 heads over 8 of 256: 194 us a layer as one, 74 and 60 cut in two."""
+        key = ("mixed", heads_per_kv, kv_heads, window, head_dim, prompt_kernel)
+        if key not in self.memo:
+            from .. import kernels as K
+
+            plan = self.plan
+            q_len = np.asarray(plan.q_len, np.int64)
+            single = int(np.argmax(q_len > 1)) if (q_len > 1).any() else 0        # requests of one token ahead of the first portion
+            costs = prompt_costs_of(prompt_kernel, head_dim, K.prompt_pairs(plan.rows, int(plan.row_count.max())))
+            few = single == 0 or single * kv_heads * PROMPT_KERNEL_COSTS[costs][3] < sm_count(self.ids.device)
+            if few or int(q_len[single:].min()) * heads_per_kv <= K.attention_mma_rows(True) or not self.ids.is_cuda:
+                self.memo[key] = None
+            else:
+                pairs = K.prompt_pairs(plan.rows, int(plan.row_count.max()))
+                per_tile = max(1, K.attention_tile_rows(False, prompt_kernel, head_dim, pairs) // heads_per_kv)
+                tiles = cut_tiles(plan.q_start[single:], plan.q_len[single:], per_tile)
+                every = np.arange(single, dtype=np.int32)
+                parts = [every, every, np.ones(single, np.int32), tiles[0] + single, tiles[1] - single, tiles[2]]
+                host = torch.from_numpy(np.concatenate([a.astype(np.int32) for a in parts])).pin_memory()
+                views = host.to(self.ids.device, non_blocking=True).split([a.size for a in parts])
+                views = [v.clone() if v.data_ptr() % 16 else v for v in views]
+                first = decode_split(single * kv_heads, int(plan.row_count[:single].max()), sm_count(self.ids.device), window, True)
+                firsts = plan.row_count[tiles[1]]
+                second = prompt_split(firsts, firsts + tiles[2] - 1, kv_heads, sm_count(self.ids.device), window, plan.rows - single,
+                                      heads_per_kv * kv_heads, head_dim, costs)
+                self.memo[key] = (single, (heads_per_kv, tuple(views[:3]), *first, True), (0, tuple(views[3:]), *second, False), pairs, host)
+        return self.memo[key][:4] if self.memo[key] is not None else None
+
     def attention_slots(self, window: Optional[int], keep_first: int = 0) -> int:
         """Chunk slots the row-wise attention kernel needs for a layer with this window; with
         `keep_first` the slots of the kept first keys come on top."""

@@ -77,6 +77,9 @@ class StaticBatch:
     def row_tiles(self, heads_per_kv: int):
         return None
 
+    def mixed_tiles(self, *sizes):
+        return None
+
     def latent_tiles(self):
         return None
 

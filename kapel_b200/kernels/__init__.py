@@ -894,7 +894,8 @@ def paged_attention_decode_fused(qkv: "SplitSum", cos_sin, lines, k_table, v_tab
 def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page_size: int, window: Optional[int],
                         scale: float, softcap: Optional[float], decode: int, split: int, slots: int,
                         relative: bool = False, pairs: Optional[int] = None, keep_first: int = 0, block: int = 0,
-                        sinks: Optional[torch.Tensor] = None, prompt_kernel: Optional[str] = None) -> torch.Tensor:
+                        sinks: Optional[torch.Tensor] = None, prompt_kernel: Optional[str] = None,
+                        out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Attention over the paged cache on tensor cores (bfloat16). `tiles` = (tile_entry, tile_row0,
     tile_nq) int32 device tensors: each tile is up to `attention_mma_rows(decode) // group` tokens of
     one request at consecutive positions. `decode` is 0 for prompt portions, else the most rows
@@ -905,7 +906,7 @@ def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page
     window, `keep_first` keys from position 0 stay visible below it (prompt portions in one slot only).
     With `block` > 0 a row at position i sees only the keys from floor(i / block) * block on (prompt portions
     in one slot only). With `sinks` [hq] float32 e^sink joins each row's denominator.
-    `prompt_kernel` "flash" (whose tiles the caller then gives) runs prompt portions on the tcgen05 kernel for scores without a bound."""
+    `prompt_kernel` "flash" (whose tiles the caller then gives) runs prompt portions on the tcgen05 kernel for scores without a bound. `out`: where the result goes, like q."""
     rows, hq, d = q.shape
     if sinks is not None:
         _need(sinks, "attention sinks", torch.float32, (hq,))
@@ -921,7 +922,10 @@ def paged_attention_mma(q, k_table, v_table, block_table, row_count, tiles, page
         _need(t, "attention tiles", torch.int32, (n_tiles,))
     _need(block_table, "attention block table", torch.int32)
     _need(row_count, "attention row_count", torch.int32, (rows,))
-    out = _fresh(q.shape, q.dtype, q.device)
+    if out is None:
+        out = _fresh(q.shape, q.dtype, q.device)
+    else:
+        _need(out, "attention output", q.dtype, tuple(q.shape))
     lib = library()
     need = lib.kb_attention_mma_scratch_floats(rows, hq, d, int(slots))
     scratch = _fresh((need,), torch.float32, q.device) if need else None

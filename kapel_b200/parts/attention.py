@@ -394,12 +394,20 @@ class Attention(Part):
         )
         if K.attention_mma_takes(q.dtype, s.head_dim, heads_per_kv):
             prompt = K.attention_prompt_kernel(s.num_heads, s.num_kv_heads, s.head_dim, self.ctx.page_size, s.softcap, s.scale)
-            decode, tiles, split, slots, relative = batch.attention_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt)
-            y = K.paged_attention_mma(
-                q, k_table, v_table, group.block_table, batch.row_count, tiles,
-                self.ctx.page_size, s.window, s.scale, s.softcap, decode, split, slots, relative,
-                pairs=getattr(batch, "pairs", None), prompt_kernel=prompt,
-            )
+            mixed = batch.mixed_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt) if prompt != "mma" else None
+            if mixed is not None:       # single tokens ahead of portions: each by the kernel made for them
+                n, ahead, behind, pairs = mixed
+                y = torch.empty_like(q)
+                for rows, (decode, tiles, split, slots, relative) in ((slice(0, n), ahead), (slice(n, None), behind)):
+                    K.paged_attention_mma(q[rows], k_table, v_table, group.block_table, batch.row_count[rows], tiles, self.ctx.page_size, s.window, s.scale,
+                                          s.softcap, decode, split, slots, relative, pairs=pairs, prompt_kernel=prompt, out=y[rows])
+            else:
+                decode, tiles, split, slots, relative = batch.attention_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt)
+                y = K.paged_attention_mma(
+                    q, k_table, v_table, group.block_table, batch.row_count, tiles,
+                    self.ctx.page_size, s.window, s.scale, s.softcap, decode, split, slots, relative,
+                    pairs=getattr(batch, "pairs", None), prompt_kernel=prompt,
+                )
         else:                   # the 32-bit path, and sizes the tensor-core kernel does not take
             y = K.paged_attention_rows(
                 q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count,
