@@ -53,6 +53,7 @@ struct DeltaParams {
     float* scal;                // [rows, heads, 2] decay, step size;
     float* kq;                  // [rows, kv_heads]
     float* out;                 // [rows, heads, e]
+    int single;                 // every request brings one row: the convolutions' history is the first kernel's business too
     int chunk_rows;             // requests that bring at least so many rows are not the scan's (0: all are)
 };
 
@@ -75,11 +76,11 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
         slot = p.slots[entry];
     }
     const bool kept = slot > 0 && slot < p.n_slots;
-    const float* hist = p.state + (size_t)(kept ? slot : 0) * p.state_floats;
+    float* hist = p.state + (size_t)(kept ? slot : 0) * p.state_floats;
     const int taps = p.taps;
     for (int c = threadIdx.x; c < channels; c += blockDim.x) {
         const int col = c < nq ? p.q_off + c : (c < 2 * nq ? p.k_off + (c - nq) : p.v_off + (c - 2 * nq));
-        float y = 0.f;
+        float y = 0.f, newer = 0.f;
         for (int j = 0; j < taps; ++j) {                        // the input j rows back
             const int t = r - j;
             float x;
@@ -87,6 +88,9 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
             else if (kept) x = hist[(size_t)(taps - 1 + (t - r0)) * channels + c];     // t - r0 in [-(taps-1), -1]
             else x = 0.f;
             y = fmaf(p.conv[(size_t)c * taps + (taps - 1 - j)], x, y);
+            // a request's only row of the step: the history moves up by one on the way, its place j rows back takes the input a row later
+            if (p.single && kept && j > 0) hist[(size_t)(taps - 1 - j) * channels + c] = newer;
+            newer = x;
         }
         act[c] = delta_silu(y);
     }
@@ -453,15 +457,16 @@ extern "C" long long kb_delta_chunk_floats(int rows, int heads, int d, int e) { 
 // Whether long portions of these sizes can go by chunks.
 extern "C" int kb_delta_chunks_take(int d, int e) { return delta_chunks_take(d, e) ? 1 : 0; }
 
-// `chunk_scratch` not null: requests that bring at least `chunk_rows` rows go by chunks; `longest` and `shortest` are the most and the fewest
-// rows any request brings.
+// `longest` and `shortest` are the most and the fewest rows any request brings (0: not known). `chunk_scratch` not null: requests that bring at
+// least `chunk_rows` rows go by chunks.
 extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in_dt, int splits, long long split_stride, int row_width,
                              int q_off, int k_off, int v_off, int b_off, int a_off, const float* conv, const float* a_log,
                              const float* dt_bias, float* state, int n_slots, long long state_floats, const int* row_entry,
                              const int* entry_start, const int* entry_end, const int* slots, int entries, int rows, int heads,
                              int kv_heads, int d, int e, int taps, float q_scale, float unit_eps, float* chunk_scratch, int chunk_rows,
                              int longest, int shortest, void* stream) {
-    KB_REQUIRE(chunk_scratch == nullptr || (delta_chunks_take(d, e) && chunk_rows > 0 && longest <= rows), "delta: chunks of sizes %d / %d from %d rows on (longest %d of %d)",
+    KB_REQUIRE(longest >= 0 && longest <= rows, "delta: a request of %d rows in a step of %d", longest, rows);
+    KB_REQUIRE(chunk_scratch == nullptr || (delta_chunks_take(d, e) && chunk_rows > 0), "delta: chunks of sizes %d / %d from %d rows on (longest %d of %d)",
                d, e, chunk_rows, longest, rows);
     KB_REQUIRE(entries >= 0 && rows >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0 && d > 0 && e > 0,
                "delta: entries %d, rows %d, heads %d over %d, sizes %d / %d", entries, rows, heads, kv_heads, d, e);
@@ -492,6 +497,7 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     p.kq = p.scal + (size_t)rows * heads * 2;
     p.out = out;
     const bool by_chunks = chunk_scratch != nullptr && longest >= chunk_rows;
+    p.single = longest == 1 && rows <= DEPENDENT_ROWS;
     p.chunk_rows = by_chunks ? chunk_rows : 0;
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = (size_t)channels * sizeof(float);
@@ -509,7 +515,7 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
         launch_dependent_if(rows <= DEPENDENT_ROWS, delta_prep_kernel<TS>, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 256), smem, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \
         }                                                                                                                  \
         if (int err = check_launch("delta prep")) return err;                                                              \
-        if (taps > 1) {                                                                                                    \
+        if (taps > 1 && !p.single) {                                                                                       \
             launch_dependent_if(rows <= DEPENDENT_ROWS, delta_history_kernel<TS>, dim3((unsigned)((channels + 127) / 128), entries), dim3(128), 0, s,                      \
                 Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p);                                                 \
             if (int err = check_launch("delta history")) return err;                                                       \

@@ -56,6 +56,7 @@ class StaticBatch:
         # the tensor-core attention kernel's tiles: every row a tile of one token
         every = torch.arange(rows, dtype=torch.int32, device=device)
         self._tiles = (every, every.clone(), torch.ones(rows, dtype=torch.int32, device=device))
+        self._next_row = every + 1
         self._longest = width * page_size
         self._device = device
         self._mma = {}
@@ -91,11 +92,7 @@ class StaticBatch:
 
     def entry_ranges(self):
         """(start, end) on the device: rows [start[e], end[e]) are request e's (here every row is its own)."""
-        if "entry_ranges" not in self.memo:
-            from .. import kernels as K
-
-            self.memo["entry_ranges"] = K.entry_ranges(self.row_entry, self.entries)
-        return self.memo["entry_ranges"]
+        return self._tiles[1], self._next_row
 
     def attention_tiles(self, heads_per_kv: int, kv_heads: int, window: Optional[int] = None, head_dim: int = 256,
                         prompt_kernel: str = "mma", keep_first: int = 0):

@@ -1169,7 +1169,8 @@ def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: i
     step, request by request in row order, from and into `state` [slots, state floats]. `conv`
     [2 kv_heads d + heads e, taps] float32: the short convolutions' filters, the queries' channels
     first, then the keys', then the values'. `longest` and `shortest`, where the caller knows them: the most and
-    the fewest rows any request brings (long portions then go by chunks of rows)."""
+    the fewest rows any request brings (long portions then go by chunks of rows, and the history of single tokens moves on
+    without a kernel of its own)."""
     src, dt, splits, stride, rows, width = _stacked(stacked, "delta input")
     channels = 2 * kv_heads * d + heads * e
     _need(conv, "delta convolution filters", torch.float32, (channels, taps))
@@ -1196,7 +1197,7 @@ def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: i
         _ptr(out), _ptr(scratch), _ptr(src), dt, splits, ctypes.c_longlong(stride), width, int(q_off), int(k_off), int(v_off),
         int(b_off), int(a_off), _ptr(conv), _ptr(a_log), _ptr(dt_bias), _ptr(state), int(state.shape[0]), ctypes.c_longlong(per),
         _ptr(row_entry), _ptr(start), _ptr(end), _ptr(slots), int(entries), rows, heads, kv_heads, d, e, int(taps), _f(q_scale),
-        _f(unit_eps), _ptr(chunks), DELTA_CHUNK_ROWS, int(longest) if chunks is not None else 0, int(shortest), _stream()))
+        _f(unit_eps), _ptr(chunks), DELTA_CHUNK_ROWS, int(longest), int(shortest), _stream()))
     return out
 
 

@@ -54,3 +54,26 @@ def test_against_64_bit_and_the_scan(H, G, d, e, taps):
     out = K.delta_scan(dev(data["a"][:70]), 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, dev(conv), dev(a_log), dev(dt_bias), by_chunks, entry,
                        K.entry_ranges(entry, 1), dev([0], torch.int32), 1, H, G, d, e, taps, d ** -0.5, 1e-6, 70, 70)
     assert float(out.abs().max()) == 0.0 and torch.equal(before, by_chunks)
+
+
+@pytest.mark.parametrize("taps,rows", [(1, 3), (2, 1), (4, 64), (4, 65), (8, 5)])
+def test_single_tokens_move_their_own_history(taps, rows):
+    """Told that every request brings one row, the first kernel moves the history on; the bits are those of the kernel made for any portion."""
+    from kapel_b200 import kernels as K
+
+    H, G, d, e = 4, 2, 32, 16
+    rng = torch.Generator(device="cuda").manual_seed(taps * rows)
+    n, nv = G * d, H * e
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=rng)
+    conv, a_log, dt_bias = rand(2 * n + nv, taps), rand(H), rand(H)
+    entry = torch.arange(rows, dtype=torch.int32, device="cuda")
+    slots = torch.arange(1, rows + 1, dtype=torch.int32, device="cuda")
+    slots[rows // 2] = 0                                     # a row of no request
+    ranges, start = K.entry_ranges(entry, rows), rand(rows + 1, K.delta_state_floats(H, G, d, e, taps))
+    states = [start.clone(), start.clone()]
+    for _ in range(3):
+        x = rand(rows, 2 * n + nv + 2 * H)
+        a, b = (K.delta_scan(x, 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, conv, a_log, dt_bias, state, entry, ranges, slots, rows, H, G, d, e, taps,
+                             d ** -0.5, 1e-6, longest, longest) for state, longest in zip(states, (0, 1)))
+        assert torch.equal(a, b)
+    assert torch.equal(states[0], states[1]) and torch.equal(states[1][0], start[0])
