@@ -3,11 +3,12 @@
 // 128-byte swizzle, no multicast), the 128 x 256 accumulator in tensor memory (TMEM), read back
 // with tcgen05.ld for the epilogue. Kapel's counterpart is the cutile `batched_matmul_nt`
 // (crates/kapel-cuda/src/tile.rs:65-87), which has no sm_100 path. Four kernels, below in this order:
-// one block a 128 x 256 tile (products of about one tile a multiprocessor); persistent pairs of
+// one block a 128 x 256 tile (products of up to a wave and a half of tiles); persistent pairs of
 // blocks with cta_group::2 and two accumulators (all other products of more than 64 rows, also with
 // the gated unit in the epilogue); operands swapped for up to 64 rows, split over K; the same with
-// the gated unit. The last two (decoding) are launched as programmatic dependents and wait for the
-// kernel before them only before they touch the activations; the first two are launched plainly.
+// the gated unit; and, behind the first, the experts' forms of the first and the third, over lists of rows. Those for
+// up to 64 rows (decoding) are launched as programmatic dependents and wait for the
+// kernel before them only before they touch the activations; the others are launched plainly.
 //
 // The first: one block computes one 128 x 256 tile of C. Six warps:
 //   warp 0    one lane walks K in steps of 64 and asks TMA for the A and W tiles of each step, four
@@ -176,12 +177,35 @@ __device__ __forceinline__ void tc_store8(void* __restrict__ c, int c_dt, size_t
     }
 }
 
+// 32 neighbouring columns of 32-bit results of a warp's 32 rows, lane l holding those of row `row`, through the warp's own piece of shared
+// memory (`stage`): eight lanes then store a row's 128 bytes together. A lane that stored its own row asked for 16 bytes in each of 32
+// lines an instruction, half a sector each: 2,048 rows by 2,304 x 2,048 on pairs 24.3 us, 19.6 this way, by 9,216 x 2,304 82.8 and 65.1; where
+// rows are a power of two apart nothing much changes (by 2,048 x 2,048 20.0 and 19.4). Bfloat16 results, whole sectors a lane and
+// half of the bytes, gain in some widths what they lose in others (20.4 to 19.6 and 17.7 to 18.5) and leave lane by lane.
+constexpr int TC_STAGE_LD = 36;                                 // words: rows of 16 bytes that eight lanes meet without a conflict
+constexpr int TC_STAGE_FLOATS = 32 * TC_STAGE_LD;               // a warp's
+__device__ __forceinline__ void tc_store_rows(float* stage, const float (&v)[32], int row, int col, float* __restrict__ c, int m, int n) {
+    const int lane = threadIdx.x & 31;
+    float* mine = stage + lane * TC_STAGE_LD;
+#pragma unroll
+    for (int j = 0; j < 32; j += 4) *reinterpret_cast<float4*>(mine + j) = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int r = i * 4 + (lane >> 3), x = (lane & 7) * 4;
+        const int to = __shfl_sync(0xffffffffu, row, r);
+        const float4 w = *reinterpret_cast<const float4*>(stage + r * TC_STAGE_LD + x);
+        if (to < m) *reinterpret_cast<float4*>(c + (size_t)to * n + col + x) = w;
+    }
+    __syncwarp();                                               // read before the next columns come
+}
+
 // One warp's share of a 128 x 256 accumulator: its 32 TMEM lanes start at `lanes`, this thread's
 // row of C is `row`, the accumulator's first column is column `n0` of C. For the gated unit the
 // accumulator's columns 0-127 are gates and 128-255 the matching ups, C is [m, n] with n the unit's
-// width, and n0 counts in outputs.
+// width, and n0 counts in outputs. `stage`: this warp's TC_STAGE_FLOATS of shared memory.
 template <int EPI>
-__device__ __forceinline__ void tc_epilogue(uint32_t lanes, int row, int n0, void* __restrict__ c, int c_dt, int m, int n, float cap, float alpha = 0.f) {
+__device__ __forceinline__ void tc_epilogue(uint32_t lanes, int row, int n0, void* __restrict__ c, int c_dt, int m, int n, float* stage, float cap, float alpha = 0.f) {
     const bool vec = (c_dt == KB_DT_BF16) ? (n % 8 == 0) : (n % 4 == 0);
     if constexpr (epi_glu(EPI)) {
         for (int c0 = 0; c0 < 128; c0 += 16) {
@@ -210,6 +234,16 @@ __device__ __forceinline__ void tc_epilogue(uint32_t lanes, int row, int n0, voi
             uint32_t r[32];
             __syncwarp();
             tc_ld32(lanes + (uint32_t)c0, r);
+            if (c_dt == KB_DT_F32 && vec && n0 + c0 + 32 <= n) {    // the same for the whole warp
+                float v[32];
+#pragma unroll
+                for (int j = 0; j < 32; ++j) {
+                    v[j] = __uint_as_float(r[j]);
+                    if (EPI == EPI_SOFTCAP) v[j] = cap * tanhf(v[j] / cap);
+                }
+                tc_store_rows(stage, v, row, n0 + c0, static_cast<float*>(c), m, n);
+                continue;
+            }
             if (row >= m) continue;
 #pragma unroll
             for (int h = 0; h < 32; h += 8) {
@@ -299,7 +333,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
             failed = true;
         } else {
             tc_fence_after();
-            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16), m0 + quarter * 32 + lane, n0, c, c_dt, m, n, cap);
+            // every stage has been read: the first one's memory takes the rows on their way out
+            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16), m0 + quarter * 32 + lane, n0, c, c_dt, m, n,
+                             reinterpret_cast<float*>(smem) + quarter * TC_STAGE_FLOATS, cap);
         }
     }
     if (failed) atomicExch(&g_tcgen05_error, 1);
@@ -399,7 +435,8 @@ moe_tcgen05_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
             failed = true;
         } else {
             tc_fence_after();
-            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16), row, n0, c, c_dt, places, n, cap, alpha);
+            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16), row, n0, c, c_dt, places, n,
+                             reinterpret_cast<float*>(smem) + quarter * TC_STAGE_FLOATS, cap, alpha);
         }
     }
     if (failed) atomicExch(&g_tcgen05_error, 1);
@@ -538,7 +575,7 @@ __global__ void moe_gather_kernel(uint4* __restrict__ out, const uint4* __restri
 constexpr int TP_BN_HALF = 128;
 constexpr int TP_B_BYTES = TP_BN_HALF * TC_BK * 2;             // 16 KB: this block's half of the weight tile
 constexpr int TP_STAGE_BYTES = TC_A_BYTES + TP_B_BYTES;        // 32 KB
-constexpr int tp_smem_bytes(int stages) { return stages * TP_STAGE_BYTES + 1024 + 256; }
+constexpr int tp_smem_bytes(int stages) { return stages * TP_STAGE_BYTES + 1024 + 256 + 4 * TC_STAGE_FLOATS * 4; }
 constexpr uint32_t TP_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(256 >> 4) << 24);
 constexpr uint32_t TP_PEER_MASK = 0xFEFFFFFFu;                 // clears the bit that tells the two blocks' shared windows apart
 
@@ -580,6 +617,7 @@ gemm_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
     uint64_t* acc_full = empty + TPP_STAGES;             // [2] accumulator complete (MMA -> both blocks' epilogues)
     uint64_t* acc_empty = acc_full + 2;                  // [2] accumulator read out (both blocks' epilogues -> MMA), first block's
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+    float* out_rows = reinterpret_cast<float*>(smem + TPP_STAGES * TP_STAGE_BYTES + 256);      // the stages are in use by the next tile
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     uint32_t rank;
@@ -664,7 +702,8 @@ gemm_tcgen05_pair_persistent_kernel(const __grid_constant__ CUtensorMap map_a, c
             const int n0 = (t / m_pairs) * tile_cols;
             if (!__all_sync(0xffffffffu, tc_mbar_wait(acc_full + acc, (uint32_t)(i >> 1) & 1u))) { failed = true; break; }
             tc_fence_after();
-            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256), m0 + quarter * 32 + lane, n0, c, c_dt, m, n, cap, alpha);
+            tc_epilogue<EPI>(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * 256), m0 + quarter * 32 + lane, n0, c, c_dt, m, n,
+                             out_rows + quarter * TC_STAGE_FLOATS, cap, alpha);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) tp_arrive_on_first(acc_empty + acc);
