@@ -1176,9 +1176,20 @@ extern "C" int kb_gemm_tcgen05(void* c, int c_dt, const void* a, const void* w, 
     dim3 grid((m + TC_BM - 1) / TC_BM, (n + TC_BN - 1) / TC_BN);
     KB_REQUIRE(grid.y <= 65535, "gemm_tcgen05: %d columns is too many for one launch", n);
     const long long tiles = (long long)grid.x * grid.y;
-    // About one 128 x 256 tile a multiprocessor and a short K: pairs would leave half the tiles'
-    // worth of multiprocessors idle and there is no second tile whose MMAs could hide an epilogue.
-    if (kernel == 0) kernel = (tiles <= 3 * (long long)skinny_sms() / 2 && k <= 4096) ? 1 : 2;
+    // Up to a wave and a half of 128 x 256 tiles: whichever kernel needs fewer waves (1,088 rows by 4,096 x 9,216: 144 tiles, but 80 of pairs for
+    // 74 clusters, 65.8 us against 111; 2,048 by 3,104 x 2,048: 208 tiles and 104 of pairs, two waves each, 39.7 against 30.7). In one wave each
+    // the pairs take in half as much a tile and the single blocks start sooner: pairs from K = 3,072 on (2,048 rows by 2,048 columns
+    // 23.8 us against 26.6, 117 by 6,144 x 4,096 27.2 against 31.6), from 2,048 on where enough multiprocessors have a tile (2,048 by 2,304
+    // 19.6 against 20.9, 500 by 3,104 18.3 against 19.3, by 2,048 17.4 against 16.5; bfloat16, whose epilogue is shorter: 2,048 by 2,304
+    // 19.3 against 19.6, 1,088 by 2,048 16.3 against 15.3), not below (K = 1,024, 500 rows by 2,048: 12.5 against 11.7).
+    if (kernel == 0) {
+        const int sms = skinny_sms();
+        const long long pair_tiles = ((m + 2 * TC_BM - 1) / (2 * TC_BM)) * (long long)grid.y;
+        const long long waves = (tiles + sms - 1) / sms, pair_waves = (pair_tiles + sms / 2 - 1) / (sms / 2);
+        if (tiles > 3 * (long long)sms / 2) kernel = 2;
+        else if (waves != pair_waves) kernel = waves < pair_waves ? 1 : 2;
+        else kernel = waves > 1 || k >= 3072 || (k >= 2048 && tiles > (c_dt == KB_DT_F32 ? 48 : 96)) ? 2 : 1;
+    }
     if (kernel == 2) {
         if (int e = encode_map_bf16(&map_w, w, n, k, k, TP_BN_HALF)) return e;
         return epilogue == 0 ? launch_pair<EPI_NONE>(map_a, map_w, c, c_dt, m, n, k, cap, s)
