@@ -467,6 +467,63 @@ retention_prep_kernel(const Src<TS> src, const RetentionParams p, const ScanInpu
     for (int i = threadIdx.x; i < nv; i += blockDim.x) s.val[(size_t)r * nv + i] = at(base + p.v_off + i);
 }
 
+// The same for prompts whose sizes and columns are multiples of four, from one 32-bit slice: four neighbouring components a lane, the
+// other half of its pairs loaded beside them. 1,360 rows of 16 heads of 128: 17 us against 34.
+__global__ void __launch_bounds__(256)
+retention_prep_fours_kernel(const float* __restrict__ src, const RetentionParams p, const ScanInputs s) {
+    const int r = blockIdx.x;
+    const float* row = src + (size_t)r * p.row_width;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    const int half = p.rotary >> 1, d = p.d;
+    auto at = [&](const float* x) {
+        float4 v = load_four(x);
+        if (p.act == 1) v.x *= rc_sigmoid(v.x), v.y *= rc_sigmoid(v.y), v.z *= rc_sigmoid(v.z), v.w *= rc_sigmoid(v.w);
+        return v;
+    };
+    for (int h = warp; h < p.heads; h += warps) {
+        float kr = 0.f;
+        const float decay = p.decay[h];
+        float* vec = s.vec + ((size_t)r * p.heads + h) * 2 * d;
+        const float *qr = row + p.q_off + (size_t)h * d, *kp = row + p.k_off + (size_t)h * d;
+        for (int i = lane * 4; i < d; i += 128) {
+            const float4 qa = at(qr + i), ka = at(kp + i);
+            float q[4] = {qa.x, qa.y, qa.z, qa.w}, k[4] = {ka.x, ka.y, ka.z, ka.w};
+            if (i < 2 * half) {
+                const bool low = i < half;
+                const int j = low ? i + half : i - half, pair = low ? i : j;
+                const float4 qb = at(qr + j), kb4 = at(kp + j);
+                const float qo[4] = {qb.x, qb.y, qb.z, qb.w}, ko[4] = {kb4.x, kb4.y, kb4.z, kb4.w};
+                const float4* cs = reinterpret_cast<const float4*>(p.cos_sin + (size_t)r * half + pair);
+                const float4 c0 = cs[0], c1 = cs[1];
+                const float2 turn[4] = {make_float2(c0.x, c0.y), make_float2(c0.z, c0.w), make_float2(c1.x, c1.y), make_float2(c1.z, c1.w)};
+#pragma unroll
+                for (int y = 0; y < 4; ++y) {
+                    float q0 = low ? q[y] : qo[y], q1 = low ? qo[y] : q[y], k0 = low ? k[y] : ko[y], k1 = low ? ko[y] : k[y];
+                    rope_rotate(q0, q1, turn[y]);
+                    rope_rotate(k0, k1, turn[y]);
+                    q[y] = low ? q0 : q1;
+                    k[y] = low ? k0 : k1;
+                }
+            }
+#pragma unroll
+            for (int y = 0; y < 4; ++y) {
+                k[y] *= p.k_scale;
+                kr = fmaf(k[y], q[y], kr);
+                q[y] *= decay;
+            }
+            store_four(vec + i, make_float4(q[0], q[1], q[2], q[3]));
+            store_four(vec + d + i, make_float4(k[0], k[1], k[2], k[3]));
+        }
+        kr = warp_sum(kr);
+        if (lane == 0) {
+            s.scal[((size_t)r * p.heads + h) * 2] = 0.f;
+            s.scal[((size_t)r * p.heads + h) * 2 + 1] = kr;
+        }
+    }
+    const int nv = p.heads * p.e;
+    for (int i = threadIdx.x * 4; i < nv; i += blockDim.x * 4) store_four(s.val + (size_t)r * nv + i, at(row + p.v_off + i));
+}
+
 // ------------------------------------------------------------------------------------------ the scan
 // What the vectors of a row are, and what a row does:
 //   SCAN_GATE     (w r, w, k)         S <- diag(w) S + k v^T
@@ -960,7 +1017,7 @@ static bool by_chunks(int longest) { return g_retention_chunk_rows > 0 && longes
 
 // Floats of scratch kb_retention_scan takes for a step of `rows` rows whose longest portion has `longest`.
 extern "C" long long kb_retention_scratch_floats(int rows, int entries, int longest, int heads, int d, int e) {
-    return kb_decay_scan_scratch_floats(rows, heads, d, e, SCAN_FIXED) + (by_chunks(longest) ? retention_chunk_floats(rows, entries, heads, d, e) : 0);
+    return kb_decay_scan_scratch_floats(rows, heads, d, e, SCAN_FIXED) + (by_chunks(longest) ? retention_chunk_floats(rows, entries, heads, d, e) + 3 : 0);
 }
 
 // The read-out [rows, heads, e] of a matrix memory with a fixed decay a head behind rotated queries and keys. `longest`: the
@@ -988,13 +1045,16 @@ extern "C" int kb_retention_scan(float* out, float* scratch, const void* src, in
     in.nv = 2;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = rows <= DEPENDENT_ROWS ? 1024 : 256;      // few rows: latency counts
-    if (in_dt == KB_DT_F32) launch_dependent_if(rows <= DEPENDENT_ROWS, retention_prep_kernel<float>, dim3(rows), dim3(threads), 0, s, Src<float>{(const float*)src, splits, (size_t)split_stride}, g, in);
+    const bool fours = in_dt == KB_DT_F32 && splits == 1 && rows > DEPENDENT_ROWS && ((row_width | q_off | k_off | v_off | d | (int)nv | (rotary / 2)) & 3) == 0 &&
+                       (((uintptr_t)src | (uintptr_t)scratch | (uintptr_t)cos_sin) & 15) == 0;
+    if (fours) retention_prep_fours_kernel<<<rows, 256, 0, s>>>((const float*)src, g, in);
+    else if (in_dt == KB_DT_F32) launch_dependent_if(rows <= DEPENDENT_ROWS, retention_prep_kernel<float>, dim3(rows), dim3(threads), 0, s, Src<float>{(const float*)src, splits, (size_t)split_stride}, g, in);
     else if (in_dt == KB_DT_BF16) launch_dependent_if(rows <= DEPENDENT_ROWS, retention_prep_kernel<bf16>, dim3(rows), dim3(threads), 0, s, Src<bf16>{(const bf16*)src, splits, (size_t)split_stride}, g, in);
     else return fail("retention: dtype code %d is not known", in_dt);
     if (int err = check_launch("retention prep")) return err;
     if (by_chunks(longest))
-        return run_retention_chunks(out, in.vec, in.val, in.scal, decay, in.scal + (size_t)rows * heads * 2, state, n_slots, entry_start, entry_end,
-                                    slots, entries, longest, heads, d, e, s);
+        return run_retention_chunks(out, in.vec, in.val, in.scal, decay, in.scal + (((size_t)rows * heads * 2 + 3) & ~(size_t)3), state, n_slots,
+                                    entry_start, entry_end, slots, entries, longest, heads, d, e, s);
     return run_decay_scan(out, in, state, n_slots, entry_start, entry_end, slots, entries, heads, d, e, SCAN_FIXED, decay, s);
 }
 
