@@ -124,13 +124,13 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
     }
 }
 
-// The same for prompts with filters of four weights: a block takes DPR rows, so an input that serves four rows' convolutions is loaded
-// once for those of a block (7 loads a channel for 4 rows instead of 16). 2,048 rows of 3,072 channels: 43 us against 71.
-// VEC: a thread takes four neighbouring channels (the columns and widths are multiples of four, the input is one slice in 32-bit).
-constexpr int DPR = 4, DPR_TAPS = 4;
-template <typename TS, bool VEC>
+// The same for prompts with filters of four weights, from one 32-bit slice whose columns and widths are multiples of four: a block takes
+// DPR rows, so an input that serves four rows' convolutions is loaded once for those of a block, a thread four neighbouring channels of them
+// (7 loads of 16 bytes for 4 x 4 values instead of 64 of 4). 2,048 rows of 3,072 channels: 43 us against 71, 1,360 rows 37 against 55; a
+// block's own chain takes some 35 us where 172 rows of a row a block take 27, so from DPR_FROM rows on.
+constexpr int DPR = 4, DPR_TAPS = 4, DPR_FROM = 512;
 __global__ void __launch_bounds__(256)
-delta_prep_rows_kernel(const Src<TS> src, const DeltaParams p) {
+delta_prep_rows_kernel(const Src<float> src, const DeltaParams p) {
     extern __shared__ float act[];                              // [DPR][channels]
     const int first = blockIdx.x * DPR, nr = min(DPR, p.rows - first);
     const int nq = p.kv_heads * p.d, nv = p.heads * p.e;
@@ -150,7 +150,7 @@ delta_prep_rows_kernel(const Src<TS> src, const DeltaParams p) {
         }
         plain = plain && start[i] <= first - (DPR_TAPS - 1);
     }
-    constexpr int CW = VEC ? 4 : 1;
+    constexpr int CW = 4;
     for (int c = threadIdx.x * CW; c < channels; c += blockDim.x * CW) {
         const int col = c < nq ? p.q_off + c : (c < 2 * nq ? p.k_off + (c - nq) : p.v_off + (c - 2 * nq));
         float raw[DPR + DPR_TAPS - 1][CW], f[CW][DPR_TAPS];     // the inputs of rows first - 3 .. first + 3; the filters
@@ -158,12 +158,8 @@ delta_prep_rows_kernel(const Src<TS> src, const DeltaParams p) {
         for (int x = 0; x < DPR + DPR_TAPS - 1; ++x) {
             const int t = first - (DPR_TAPS - 1) + x;
             const bool there = t >= 0 && t < p.rows;
-            if constexpr (VEC) {
-                const float4 v = there ? *reinterpret_cast<const float4*>(src.p + (size_t)t * p.row_width + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-                raw[x][0] = v.x, raw[x][1] = v.y, raw[x][2] = v.z, raw[x][3] = v.w;
-            } else {
-                raw[x][0] = there ? src.at((size_t)t * p.row_width + col) : 0.f;
-            }
+            const float4 v = there ? *reinterpret_cast<const float4*>(src.p + (size_t)t * p.row_width + col) : make_float4(0.f, 0.f, 0.f, 0.f);
+            raw[x][0] = v.x, raw[x][1] = v.y, raw[x][2] = v.z, raw[x][3] = v.w;
         }
 #pragma unroll
         for (int w = 0; w < CW; ++w)
@@ -502,14 +498,12 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = (size_t)channels * sizeof(float);
     const bool fours = splits == 1 && (row_width | q_off | k_off | v_off | (int)nq | (int)nv) % 4 == 0 && ((uintptr_t)src & 15) == 0;
-    const bool by_rows = rows > DEPENDENT_ROWS && taps == DPR_TAPS && DPR * smem <= 100 * 1024;
+    const bool by_rows = in_dt == KB_DT_F32 && fours && rows >= DPR_FROM && taps == DPR_TAPS && DPR * smem <= 100 * 1024;
 #define KB_DELTA_PREP(TS)                                                                                                  \
     do {                                                                                                                   \
         if (by_rows) {                                                                                                     \
-            constexpr bool f32 = sizeof(TS) == 4;                                                                          \
-            auto kernel = f32 && fours ? delta_prep_rows_kernel<TS, f32> : delta_prep_rows_kernel<TS, false>;              \
-            if (DPR * smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DPR * smem)); \
-            kernel<<<(rows + DPR - 1) / DPR, 256, DPR * smem, s>>>(Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); \
+            if (DPR * smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DPR * smem)); \
+            delta_prep_rows_kernel<<<(rows + DPR - 1) / DPR, 256, DPR * smem, s>>>(Src<float>{(const float*)src, splits, (size_t)split_stride}, p); \
         } else {                                                                                                           \
         if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
         launch_dependent_if(rows <= DEPENDENT_ROWS, delta_prep_kernel<TS>, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 256), smem, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \

@@ -233,8 +233,9 @@ moe_route_kernel(const TH* __restrict__ h, const float* __restrict__ router, con
 constexpr int GM = 32;         // rows of a grouped product's tile: few rows an expert, and the 32-bit path
 constexpr int GM_LARGE = 64;   // and where an expert has many rows (bfloat16)
 // The router of prompts, without groups: a block takes ROUTE_ROWS rows, so the router's weights are read once for all of them (a block a row read
-// all of them again: 1,360 rows by 20 x 2,048 took 43 us, 30 like this). The same sums in the same order.
-constexpr int ROUTE_ROWS = 8;
+// all of them again: 1,360 rows by 20 x 2,048 took 43 us, 30 like this). The same sums in the same order. A block takes 29 us
+// whatever the rows, a row a block 23 us up to 172 rows: eight rows a block from ROUTE_ROWS_FROM rows on.
+constexpr int ROUTE_ROWS = 8, ROUTE_ROWS_FROM = 512;
 template <typename TH>
 __global__ void __launch_bounds__(ROUTE_THREADS)
 moe_route_rows_kernel(const TH* __restrict__ h, const float* __restrict__ router, const float* __restrict__ correction, int* __restrict__ experts_out,
@@ -572,7 +573,7 @@ extern "C" int kb_moe_route(int* experts, float* weights, const void* h, int h_d
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = rows <= DEPENDENT_ROWS ? ROUTE_THREADS_FEW : ROUTE_THREADS;
     const size_t rows_smem = ((size_t)ROUTE_ROWS * width + (size_t)2 * ROUTE_ROWS * n_experts) * sizeof(float);
-    if (rows > DEPENDENT_ROWS && (groups == 1 || keep_groups == groups) && width % 4 == 0 && rows_smem <= 200 * 1024 && (h_dt == KB_DT_F32 || h_dt == KB_DT_BF16) &&
+    if (rows >= ROUTE_ROWS_FROM && (groups == 1 || keep_groups == groups) && width % 4 == 0 && rows_smem <= 200 * 1024 && (h_dt == KB_DT_F32 || h_dt == KB_DT_BF16) &&
         (((uintptr_t)h | (uintptr_t)router) & 15) == 0) {
         const unsigned blocks = (unsigned)((rows + ROUTE_ROWS - 1) / ROUTE_ROWS);
 #define KB_ROUTE_ROWS(TH)                                                                                                  \

@@ -1157,9 +1157,10 @@ def delta_columns_per_warp(n: int = 0) -> None:
     library().kb_delta_columns_per_warp(int(n))
 
 
-# Rows a request brings from which the delta rule goes by chunks of 32 rows instead of row by row: a row of the scan takes
-# 0.3 us, a chunk 3.9 and the launch ahead of the chain some 20, so two chunks are where the two ways meet.
-DELTA_CHUNK_ROWS = 64
+# The delta rule goes by chunks of 32 rows instead of row by row where some request brings DELTA_CHUNK_LONGEST rows: a row of the scan takes
+# 0.33 us, a chunk 3.9 and the launch ahead of the chain 35 (100 rows of 16 heads of 128: 35 us row by row, 53 by chunks). Then every
+# request of DELTA_CHUNK_ROWS rows goes that way, side by side with the longest.
+DELTA_CHUNK_ROWS, DELTA_CHUNK_LONGEST = 64, 192
 
 
 def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: int, conv: torch.Tensor, a_log: torch.Tensor,
@@ -1191,7 +1192,7 @@ def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: i
     out = _fresh((rows, heads, e), torch.float32, src.device)
     scratch = _fresh((max(1, int(lib.kb_delta_scratch_floats(rows, heads, kv_heads, d, e))),), torch.float32, src.device)
     chunks = None
-    if longest >= DELTA_CHUNK_ROWS and lib.kb_delta_chunks_take(d, e):
+    if longest >= DELTA_CHUNK_LONGEST and lib.kb_delta_chunks_take(d, e):
         chunks = _fresh((int(lib.kb_delta_chunk_floats(rows, heads, d, e)),), torch.float32, src.device)
     _check(lib.kb_delta_scan(
         _ptr(out), _ptr(scratch), _ptr(src), dt, splits, ctypes.c_longlong(stride), width, int(q_off), int(k_off), int(v_off),

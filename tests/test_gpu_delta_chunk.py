@@ -10,8 +10,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("H,G,d,e,taps", [(4, 2, 32, 16, 4), (2, 1, 128, 48, 4), (3, 3, 64, 16, 3), (4, 1, 96, 32, 4)])
-def test_against_64_bit_and_the_scan(H, G, d, e, taps):
+def test_against_64_bit_and_the_scan(H, G, d, e, taps, monkeypatch):
     from kapel_b200 import kernels as K
+
+    monkeypatch.setattr(K, "DELTA_CHUNK_LONGEST", 64)       # shorter portions than where chunks pay
 
     dev = lambda x, dtype=torch.float32: torch.tensor(np.asarray(x), dtype=dtype, device="cuda")
     rng = np.random.default_rng(d + e)
@@ -77,3 +79,30 @@ def test_single_tokens_move_their_own_history(taps, rows):
                              d ** -0.5, 1e-6, longest, longest) for state, longest in zip(states, (0, 1)))
         assert torch.equal(a, b)
     assert torch.equal(states[0], states[1]) and torch.equal(states[1][0], start[0])
+
+
+@pytest.mark.parametrize("sizes", [(512,), (515,), (300, 1, 2, 260), (63, 510, 3)])
+def test_inputs_by_four_rows_and_by_rows(sizes):
+    """Prompts' convolutions and unit vectors four rows a block, against the same columns one place further, which the kernel of a row a
+    block reads: the same bits, behind a history and beside a row of no request."""
+    from kapel_b200 import kernels as K
+
+    H, G, d, e, taps = 4, 2, 32, 16, 4
+    rows, n, nv = sum(sizes), G * d, H * e
+    rng = torch.Generator(device="cuda").manual_seed(rows)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=rng)
+    conv, a_log, dt_bias = rand(2 * n + nv, taps), rand(H), rand(H)
+    entry = torch.tensor(np.repeat(np.arange(len(sizes)), sizes), dtype=torch.int32, device="cuda")
+    slots = torch.arange(1, len(sizes) + 1, dtype=torch.int32, device="cuda")
+    if len(sizes) > 3:
+        slots[2] = 0
+    ranges, start = K.entry_ranges(entry, len(sizes)), rand(len(sizes) + 1, K.delta_state_floats(H, G, d, e, taps))
+    states = [start.clone(), start.clone()]
+    for _ in range(2):
+        x = rand(rows, 2 * n + nv + 2 * H)
+        shifted = torch.zeros(rows, 2 * n + nv + 2 * H + 4, device="cuda")
+        shifted[:, 1:-3] = x
+        a, b = (K.delta_scan(src, off, off + n, off + 2 * n, off + 2 * n + nv, off + 2 * n + nv + H, conv, a_log, dt_bias, state, entry, ranges, slots,
+                             len(sizes), H, G, d, e, taps, d ** -0.5, 1e-6) for src, off, state in ((x, 0, states[0]), (shifted, 1, states[1])))
+        assert torch.equal(a, b)
+    assert torch.equal(states[0], states[1])

@@ -69,13 +69,13 @@ def test_few_rows_against_64_bit(counts, identity, width, n):
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("scoring", ["sigmoid", "softmax", "softmax_chosen"])
 def test_the_router_by_rows_and_a_row_a_block(dtype, scoring):
-    """The router of a prompt takes eight rows a block: the same choices and weights as the rows one decoding step at a time."""
+    """The router of a long prompt (512 rows and more) takes eight rows a block: the same choices and weights as the rows one decoding step at a time."""
     from kapel_b200 import kernels as K
 
     gen = torch.Generator(device="cuda").manual_seed(5)
-    h, router = torch.randn(77, 516, device="cuda", generator=gen).to(dtype), torch.randn(19, 516, device="cuda", generator=gen) * 0.1
+    h, router = torch.randn(531, 516, device="cuda", generator=gen).to(dtype), torch.randn(19, 516, device="cuda", generator=gen) * 0.1
     correction = torch.randn(19, device="cuda", generator=gen) * 0.1
     experts, weights = K.moe_route(h, router, correction, 5, 1, 1, 1, scoring, True, 1.5)
-    for at in range(0, 77, 40):
+    for at in range(0, 531, 40):
         e, w = K.moe_route(h[at : at + 40].contiguous(), router, correction, 5, 1, 1, 1, scoring, True, 1.5)
         assert torch.equal(e, experts[at : at + 40]) and torch.equal(w, weights[at : at + 40])
