@@ -14,8 +14,14 @@ int fail(const char* fmt, ...) {
 }
 
 static unsigned long long g_launches = 0;
+static unsigned long long g_dependent_launches = 0;
 static bool g_pdl = false;
-bool pdl_enabled() { return g_pdl; }
+static thread_local int g_pass_rows = 0;
+bool chains(bool dependent) {
+    if (!dependent || !g_pdl || g_pass_rows > DEPENDENT_ROWS) return false;
+    ++g_dependent_launches;
+    return true;
+}
 
 int check_launch(const char* what) {
     ++g_launches;                         // every kernel launch of this library passes here once
@@ -33,6 +39,13 @@ extern "C" unsigned long long kb_launch_count() { return kb::g_launches; }
 
 // 1: the kernels of a decode step are launched as programmatic dependents of one another.
 extern "C" void kb_set_pdl(int on) { kb::g_pdl = on != 0; }
+
+// How many rows the pass has that this thread launches kernels of from now on, until it is told otherwise (0: a launch alone, which
+// goes by its own rows). Launches of a pass of more than DEPENDENT_ROWS rows are plain also where they cover a few of its rows.
+extern "C" void kb_pass_rows(int rows) { kb::g_pass_rows = rows; }
+
+// Kernels launched (or recorded) as programmatic dependents so far.
+extern "C" unsigned long long kb_dependent_launch_count() { return kb::g_dependent_launches; }
 
 // The compute capability this library was built for, as major * 10 + minor.
 extern "C" int kb_built_for() { return 100; }

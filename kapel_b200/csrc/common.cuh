@@ -27,9 +27,11 @@ int check_launch(const char* what);      // cudaGetLastError -> fail(...)
 //
 // Only the kernels of a step of at most DEPENDENT_ROWS rows (decoding) are chained this way. The
 // kernels of a prompt are launched plainly (`launch_dependent_if(false, ...)`): that is a rule of
-// this library, not a tuning choice, and it holds for every prompt kernel.
+// this library, not a tuning choice, and it holds for every prompt kernel. A launch knows the rows it
+// covers, which in a pass with prompts may be a few of many (single tokens beside a prompt, the rows whose
+// logits are wanted): `kb_pass_rows` tells the thread's launches how many the whole pass has, and that decides.
 constexpr int DEPENDENT_ROWS = 64;
-bool pdl_enabled();
+bool chains(bool dependent);             // whether a launch that may be a dependent is one (and counts it)
 template <typename... KArgs, typename... Args>
 inline void launch_dependent_if(bool dependent, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
@@ -41,7 +43,7 @@ inline void launch_dependent_if(bool dependent, void (*kernel)(KArgs...), dim3 g
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = dependent && pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = chains(dependent) ? 1 : 0;
     cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);      // the caller checks with check_launch
 }
 template <typename... KArgs, typename... Args>

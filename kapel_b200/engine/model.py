@@ -64,6 +64,10 @@ class ModelParts:
 
     def forward(self, batch, cache_manager) -> torch.Tensor:
         """float32 logits [wanted rows, vocab] of a step."""
+        with K.pass_of(batch.rows):
+            return self._forward(batch, cache_manager)
+
+    def _forward(self, batch, cache_manager) -> torch.Tensor:
         copies = {"copies": self.streams} if self.streams else {}
         if getattr(self.embedding, "needs_positions", False):
             x = self.embedding.forward(batch.ids, batch.positions, **copies)

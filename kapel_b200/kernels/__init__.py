@@ -7,6 +7,7 @@ device memory; no torch operator computes anything on this path.
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import threading
 from typing import Optional
@@ -67,6 +68,7 @@ def library():
                              "kb_retention_scratch_floats"):
                     getattr(lib, name).restype = ctypes.c_longlong
                 lib.kb_launch_count.restype = ctypes.c_ulonglong
+                lib.kb_dependent_launch_count.restype = ctypes.c_ulonglong
                 lib.kb_set_pdl(1 if PDL else 0)
                 if _os.environ.get("KAPEL_B200_DELTA_COLUMNS"):      # 1, 2 or 4 columns a warp in the delta scan instead of the launcher's choice
                     lib.kb_delta_columns_per_warp(int(_os.environ["KAPEL_B200_DELTA_COLUMNS"]))
@@ -105,6 +107,23 @@ def wait_probe(limit_clocks: int = 2_000_000) -> None:
 def launch_count() -> int:
     """Kernels launched (or recorded under a graph capture) by this library so far."""
     return int(library().kb_launch_count())
+
+
+def dependent_launch_count() -> int:
+    """Kernels launched (or recorded) as programmatic dependents of the kernel before them so far."""
+    return int(library().kb_dependent_launch_count())
+
+
+@contextlib.contextmanager
+def pass_of(rows: int):
+    """The launches of this thread inside belong to a pass of `rows` rows: in a pass of more rows than a decoding step has every
+    kernel is launched plainly, also those over a few of its rows."""
+    lib = library()
+    lib.kb_pass_rows(int(rows))
+    try:
+        yield
+    finally:
+        lib.kb_pass_rows(0)
 
 
 def library_path() -> str:

@@ -1,0 +1,31 @@
+"""Only decoding steps chain their kernels: in a pass with a prompt every kernel is launched plainly, also those over a few of its rows
+(single tokens beside the prompt, the wanted rows' norm and product)."""
+import numpy as np
+import pytest
+
+from test_gpu_flash import LATENT
+from test_gpu_mixed_attention import config
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("model,singles", [(config(128, 16, 50.0), 10), (LATENT, 3)])
+def test_dependent_launches_of_each_kind_of_pass(model, singles):
+    from kapel_b200 import kernels as K
+    from kapel_b200.engine import Engine
+
+    rng = np.random.default_rng(4)
+    eng = Engine.random(model, seed=1, dtype="bfloat16", max_tokens=singles * 64 + 512, max_sequences=singles + 1, graphs=False)
+    draw = lambda n: rng.integers(0, 90, n).tolist()
+    ones = lambda: [(f"s{i}", draw(1), [0]) for i in range(singles)]
+
+    def chained(entries):
+        before = K.dependent_launch_count()
+        eng.step(entries)
+        return K.dependent_launch_count() - before
+
+    assert chained([(f"s{i}", draw(30), [29]) for i in range(singles)]) == 0
+    assert chained(ones() + [("p", draw(100), [99])]) == 0
+    assert (chained(ones()) > 0) == K.PDL
+    assert chained([("p", draw(70), [3, 69])]) == 0
+    eng.check()
