@@ -139,7 +139,7 @@ class LatentAttention(Part):
                                        entries, longest, ctx.page_size, s.scale, batch.attention_slots(None),
                                        self.sinks, s.kv_rank)
         else:                   # the 32-bit path, and sizes the tensor-core kernel does not take
-            y = K.paged_attention_rows(q_lat.view(-1, H, s.kv_rank + r), k_table, k_table, group.block_table, batch.row_entry,
+            y = K.paged_attention_rows(q_lat.view(-1, H, s.kv_rank + r), k_table, k_table, group.block_table, batch.row_entry[: row_count.numel()],
                                        row_count, ctx.page_size, None, s.scale, None, batch.attention_slots(None),
                                        sinks=self.sinks, value_dim=s.kv_rank)
         return K.head_linear(y.view(-1, H * s.kv_rank), H, s.kv_rank, 0, self.m_uv, gate=stacked if s.gated else None,

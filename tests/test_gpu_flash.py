@@ -146,3 +146,24 @@ def test_latent_attention_by_heads_and_over_lines():
     for e, l, h in zip(exact, lines, heads):
         off = lambda x: float((x - e).norm() / e.norm())
         assert off(h) <= 2e-2 and off(h) <= 1.5 * off(l) + 1e-3, (off(h), off(l))
+
+
+@pytest.mark.parametrize("kv_rank", [512, 576, 640])
+def test_single_tokens_beside_a_prompt_at_wide_ranks(kv_rank):
+    """Lines wider than the tensor-core kernel over lines takes: the single tokens of a mixed pass go row by row, the prompt by heads."""
+    import copy
+
+    from kapel_b200.engine import Engine
+
+    model = copy.deepcopy(LATENT)
+    model["layers"][0]["mixer"]["kv_rank"] = kv_rank
+    rng = np.random.default_rng(6)
+    draw = lambda n: rng.integers(0, 97, n).tolist()
+    steps = [[("a", draw(40), []), ("b", draw(25), [])], [("a", draw(1), [0]), ("b", draw(1), [0]), ("c", draw(90), list(range(90)))]]
+
+    def run(dtype):
+        eng = Engine.random(model, seed=2, dtype=dtype, max_tokens=512, max_sequences=3)
+        return [eng.step(s).double().cpu() for s in steps][1]
+
+    exact, got = run("float32"), run("bfloat16")
+    assert got.shape == (92, 97) and float((got - exact).norm() / exact.norm()) <= 2e-2
