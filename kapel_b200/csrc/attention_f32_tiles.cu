@@ -5,7 +5,8 @@
 // multiply-adds from shared memory, the running maximum and the weights eight threads a row, then the weighted sum into registers. Keys and values come
 // by asynchronous copies, the next keys while the values are multiplied, the values while the scores are made. No tensor-core instruction: nothing
 // rounds an input; exponentials and soft caps are the library's. Shared memory's 32 words a clock bound it (0.75 and 0.38 words a multiply-add),
-// and how few blocks a short prompt gives: 136 us for those 500 tokens, which is what the 8 steps of the last rows' block take.
+// and how few blocks a short prompt gives: 139 us for those 500 tokens, which is what the 8 steps of the last rows' block take.
+#include <type_traits>
 #include "common.cuh"
 
 namespace kb {
@@ -37,6 +38,7 @@ attention_f32_tiles_kernel(const F32TileParams p) {
     float* sv = sk + AFT_KEYS * LD;                              // [64][LD]
     float* sp = sv + AFT_KEYS * LD;                              // [32][68] scores, then weights
     float* fade = sp + AFT_ROWS * (AFT_KEYS + 4);                // [32] what a row's sums are scaled by this step; at the end its reciprocal
+    int* paged = reinterpret_cast<int*>(fade + AFT_ROWS);        // [2][64] whether a key of this step, of the next, has a page: one without is seen by nobody
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int kvh = blockIdx.x, tile = gridDim.y - 1 - blockIdx.y;       // later tiles of a prompt see more keys: they start first
     const int group = p.hq / p.hkv;
@@ -51,6 +53,7 @@ attention_f32_tiles_kernel(const F32TileParams p) {
             int page = -1;
             if (pos < khi && lp < p.table_width) page = p.block_table[(size_t)entry * p.table_width + lp];
             const bool there = page >= 0 && page < p.n_pages;
+            if (table == p.k_table && lane == 0) paged[((k0 - klo) / AFT_KEYS & 1) * AFT_KEYS + key] = there;
             const float* from = there ? table + kv_row((long long)page * p.page_size + pos % p.page_size, kvh, p.hkv, p.page_size) * D : table;
             for (int x = lane; x < D4; x += 32)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to + key * LD + x * 4)), "l"(from + x * 4), "r"(there ? 16 : 0) : "memory");
@@ -63,6 +66,16 @@ attention_f32_tiles_kernel(const F32TileParams p) {
         if (r < rows_valid) v = *reinterpret_cast<const float4*>(p.q + ((size_t)(row0 + r / group) * p.hq + kvh * group + r % group) * D + x);
         *reinterpret_cast<float4*>(sq + r * LD + x) = v;
     }
+    // This warp's four rows of the weighted sum see the keys [lo4, hi4). A weight of zero times a value that is no finite number is no
+    // zero, so where not every row sees every key of a step the others are left out of the sum.
+    int lo4[4], hi4[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 4 * warp + i;
+        hi4[i] = r < rows_valid ? c_first + r / group : 0;
+        lo4[i] = p.window > 0 ? max(0, hi4[i] - p.window) : 0;
+    }
+    const int all_from = p.window > 0 ? max(0, khi - p.window) : 0;      // every row sees the keys [all_from, c_first)
     // the row whose softmax this thread shares with its seven neighbours
     const int sr = tid >> 3, sc = tid & 7;
     const bool own = sr < rows_valid;
@@ -101,12 +114,13 @@ attention_f32_tiles_kernel(const F32TileParams p) {
         else asm volatile("cp.async.commit_group;" ::: "memory");
         {
             float w[8], top = -INFINITY;
+            const int* there = paged + ((k0 - klo) / AFT_KEYS & 1) * AFT_KEYS;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int key = k0 + sc + 8 * j;
                 float x = sp[sr * (AFT_KEYS + 4) + sc + 8 * j] * p.scale;
                 if (p.cap > 0.f) x = p.cap * tanhf(x / p.cap);
-                w[j] = key >= fst && key < cnt ? x : -INFINITY;
+                w[j] = key >= fst && key < cnt && there[sc + 8 * j] ? x : -INFINITY;
                 top = fmaxf(top, w[j]);
             }
 #pragma unroll
@@ -134,26 +148,31 @@ attention_f32_tiles_kernel(const F32TileParams p) {
 #pragma unroll
             for (int c = 0; c < 4 * CG; ++c) o[i][c] *= f;
         }
+        auto sum = [&](auto all) {
 #pragma unroll 4
-        for (int k = 0; k < AFT_KEYS; k += 4) {
-            float4 w[4];
+            for (int k = 0; k < AFT_KEYS; k += 4) {
+                float4 w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (4 * warp + i) * (AFT_KEYS + 4) + k);
+                for (int i = 0; i < 4; ++i) w[i] = *reinterpret_cast<const float4*>(sp + (4 * warp + i) * (AFT_KEYS + 4) + k);
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk)
+                for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-                for (int g = 0; g < CG; ++g) {
-                    const float4 v = *reinterpret_cast<const float4*>(sv + (k + kk) * LD + 4 * (lane + 32 * g));
+                    for (int g = 0; g < CG; ++g) {
+                        const float4 v = *reinterpret_cast<const float4*>(sv + (k + kk) * LD + 4 * (lane + 32 * g));
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float x = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                        o[i][4 * g] = fmaf(x, v.x, o[i][4 * g]);
-                        o[i][4 * g + 1] = fmaf(x, v.y, o[i][4 * g + 1]);
-                        o[i][4 * g + 2] = fmaf(x, v.z, o[i][4 * g + 2]);
-                        o[i][4 * g + 3] = fmaf(x, v.w, o[i][4 * g + 3]);
+                        for (int i = 0; i < 4; ++i) {
+                            if (!decltype(all)::value && (k0 + k + kk < lo4[i] || k0 + k + kk >= hi4[i])) continue;      // the same for the whole warp
+                            const float x = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
+                            o[i][4 * g] = fmaf(x, v.x, o[i][4 * g]);
+                            o[i][4 * g + 1] = fmaf(x, v.y, o[i][4 * g + 1]);
+                            o[i][4 * g + 2] = fmaf(x, v.z, o[i][4 * g + 2]);
+                            o[i][4 * g + 3] = fmaf(x, v.w, o[i][4 * g + 3]);
+                        }
                     }
-                }
-        }
+            }
+        };
+        if (k0 >= all_from && k0 + AFT_KEYS <= c_first) sum(std::true_type{});
+        else sum(std::false_type{});
         __syncthreads();                                         // the values and the weights are done with
         if (more) fetch(sv, p.v_table, k0 + AFT_KEYS);
         else asm volatile("cp.async.commit_group;" ::: "memory");
@@ -186,7 +205,7 @@ attention_f32_tiles_kernel(const F32TileParams p) {
 
 template <int D>
 static int launch_f32_tiles(const F32TileParams& p, int tiles, cudaStream_t s) {
-    constexpr int smem = ((AFT_ROWS + 2 * AFT_KEYS) * (D + 4) + AFT_ROWS * (AFT_KEYS + 4) + AFT_ROWS) * (int)sizeof(float);
+    constexpr int smem = ((AFT_ROWS + 2 * AFT_KEYS) * (D + 4) + AFT_ROWS * (AFT_KEYS + 4) + AFT_ROWS + 2 * AFT_KEYS) * (int)sizeof(float);
     static bool attr_set = false;
     if (!attr_set) {
         if (cudaFuncSetAttribute(attention_f32_tiles_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)

@@ -51,3 +51,34 @@ def test_against_64_bit_and_by_rows(portions, hq, hkv, d, window, cap, sink):
     off = lambda x: float((x.double() - want).abs().max() / want.abs().max())
     # products of d terms and sums of up to 630 weights in 32-bit; a score of 30 moves by 2^-19 when it is rounded
     assert off(by_tiles) <= 1e-5 and off(by_tiles) <= 3.0 * off(by_rows) + 1e-6, (off(by_tiles), off(by_rows))
+
+
+@pytest.mark.parametrize("window", [None, 40])
+@pytest.mark.parametrize("hq,hkv,d", [(4, 2, 256), (8, 2, 128)])
+def test_what_a_row_does_not_see_does_not_reach_it(hq, hkv, d, window):
+    """Values that are no finite numbers reach the rows that see them and no other, and a key without a page is seen by nobody: as row by row."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(8)
+    before, n = 70, 60
+    T = before + n
+    width = -(-T // 16)
+    k_table, v_table = (torch.randn(width, hkv, 16, d, device="cuda", generator=gen) for _ in range(2))
+    at = lambda t: (t // 16, slice(None), t % 16)
+    v_table[at(100)] = float("nan")
+    v_table[at(111)] = float("inf")
+    v_table[at(5)] = float("nan")                            # below the window; without one every row sees it
+    k_table[at(120)] = float("nan")
+    if window is None:
+        v_table[at(5)] = 1.0
+    table = torch.arange(width, dtype=torch.int32, device="cuda")[None].contiguous()
+    table[0, 3] = -1                                         # positions 48 to 63
+    q = torch.randn(n, hq, d, device="cuda", generator=gen)
+    counts = torch.arange(before + 1, T + 1, dtype=torch.int32, device="cuda")
+    args = (q, k_table, v_table, table, torch.zeros(n, dtype=torch.int32, device="cuda"), counts, 16, window, d ** -0.5, None, T // K.attention_chunk() + 2)
+    by_rows, by_tiles = K.paged_attention_rows(*args), K.paged_attention_rows(*args, tiles=cut([(before, n)], 32 // (hq // hkv)))
+    seen = counts > 100                                      # these rows see position 100
+    assert torch.isfinite(by_rows[~seen]).all() and not torch.isfinite(by_rows[seen]).any()
+    assert torch.equal(torch.isfinite(by_rows), torch.isfinite(by_tiles))
+    # sums of at most 100 weights in 32-bit, in another order
+    assert (by_rows - by_tiles)[~seen].abs().max() <= 1e-5 * by_rows[~seen].abs().max()
