@@ -151,7 +151,7 @@ attention_flash_kernel(const FlashParams p, const __grid_constant__ CUtensorMap 
                 const int s = brings_keys ? kt % KS : kt % VS, round = brings_keys ? kt / KS : kt / VS;
                 uint64_t* full = (brings_keys ? k_full : v_full) + s;
                 if (!at_mbar_wait((brings_keys ? k_empty : v_empty) + s, ((uint32_t)round & 1u) ^ 1u)) { failed = true; break; }
-                const int row = base + k_begin + kt * AF_KEYS;   // rows beyond the matrix read as zeros
+                const int row = base + k_begin + kt * AF_KEYS;   // the last tile's keys behind the request's end: zeros (`latent_gather`)
                 at_mbar_expect_tx(full, brings_keys ? C::K_BYTES : C::V_BYTES);
                 if (brings_keys) {
                     const uint32_t dst = at_saddr(k_ring) + (uint32_t)s * C::K_BYTES;

@@ -9,18 +9,20 @@ namespace kb {
 typedef __nv_bfloat16 bf16;
 
 // Lines [kv_rank + rot] of the positions 0 .. length - 1 of each request, the latent into c [positions, kv_rank], the rotated part into
-// rot_keys [positions, rot], rows entry_base[e] + position. A position without a page gives zeros. 16 bytes a thread.
+// rot_keys [positions, rot], rows entry_base[e] + position; zeros behind them up to a multiple of `align` rows. A position without a page
+// gives zeros. 16 bytes a thread.
 __global__ void latent_gather_kernel(const uint4* __restrict__ table, const int* __restrict__ block_table, int table_width, int n_pages,
-                                     int page_size, const int* __restrict__ entry_base, const int* __restrict__ entry_length,
+                                     int page_size, const int* __restrict__ entry_base, const int* __restrict__ entry_length, int align,
                                      uint4* __restrict__ c, uint4* __restrict__ rot_keys, int c_pieces, int rot_pieces) {
     const int entry = blockIdx.y;
     const int pieces = c_pieces + rot_pieces;
-    const long long total = (long long)entry_length[entry] * pieces;
+    const int length = entry_length[entry];
+    const long long total = (long long)((length + align - 1) / align * align) * pieces;
     const size_t base = (size_t)entry_base[entry];
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long long)gridDim.x * blockDim.x) {
         const int pos = (int)(i / pieces), at = (int)(i - (long long)pos * pieces);
         const int lp = pos / page_size;
-        const int page = lp < table_width ? block_table[(size_t)entry * table_width + lp] : -1;
+        const int page = pos < length && lp < table_width ? block_table[(size_t)entry * table_width + lp] : -1;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if (page >= 0 && page < n_pages) v = table[((size_t)page * page_size + pos % page_size) * pieces + at];
         if (at < c_pieces) c[(base + pos) * c_pieces + at] = v;
@@ -58,9 +60,11 @@ __global__ void latent_query_kernel(const Src<TS> src, const float2* __restrict_
 
 using namespace kb;
 
-// table [pages, 1, page_size, kv_rank + rot] bfloat16; `longest`: the most positions of any request; c [positions, kv_rank], rot_keys [positions, rot].
+// table [pages, 1, page_size, kv_rank + rot] bfloat16; `longest`: the most positions of any request; c [positions, kv_rank], rot_keys [positions, rot],
+// a request's rows followed by zeros up to a multiple of `align`.
 extern "C" int kb_latent_gather(void* c, void* rot_keys, const void* table, const int* block_table, int table_width, int n_pages, int page_size,
-                                const int* entry_base, const int* entry_length, int entries, int longest, int kv_rank, int rot, void* stream) {
+                                const int* entry_base, const int* entry_length, int entries, int longest, int align, int kv_rank, int rot, void* stream) {
+    KB_REQUIRE(align >= 1, "latent_gather: rows up to a multiple of %d", align);
     KB_REQUIRE(entries >= 0 && longest >= 0 && kv_rank > 0 && rot > 0 && kv_rank % 8 == 0 && rot % 8 == 0, "latent_gather: lines of %d + %d (multiples of 8)", kv_rank, rot);
     KB_REQUIRE(table_width > 0 && n_pages > 0 && page_size > 0 && entries <= 65535, "latent_gather: table width %d, pages %d of %d, %d requests", table_width, n_pages, page_size, entries);
     KB_REQUIRE(c && rot_keys && table && block_table && entry_base && entry_length, "latent_gather: a null input");
@@ -69,7 +73,7 @@ extern "C" int kb_latent_gather(void* c, void* rot_keys, const void* table, cons
     const long long work = (long long)longest * ((kv_rank + rot) / 8);
     const unsigned blocks = (unsigned)std::min<long long>((work + 255) / 256, 4096);
     latent_gather_kernel<<<dim3(blocks, entries), 256, 0, (cudaStream_t)stream>>>((const uint4*)table, block_table, table_width, n_pages, page_size,
-                                                                                   entry_base, entry_length, (uint4*)c, (uint4*)rot_keys, kv_rank / 8, rot / 8);
+                                                                                   entry_base, entry_length, align, (uint4*)c, (uint4*)rot_keys, kv_rank / 8, rot / 8);
     return check_launch("latent_gather");
 }
 

@@ -350,20 +350,24 @@ class StepBatch:
         """How the prompt path of latent attention cuts this step, or None where no request brings enough rows for it: (rows before
         the first such request's, requests before it, the most rows one of those brings, (tile_entry, tile_row0, tile_nq), entry_base,
         entry_length, positions, longest): tiles of 128 rows, counted from the first such request's; where each request's positions begin
-        among those laid out densely, and how many it has there (none where it brings few rows)."""
+        among those laid out densely, and how many it has there (none where it brings few rows). Each begins at a multiple of the positions
+        that the kernel reads at a time, so that it reads zeros behind a request's last and nothing of the next request's."""
         key = "latent_tiles"
         if key not in self.memo:
+            from .. import kernels as K
+
             plan = self.plan
             q_len = np.asarray(plan.q_len, np.int64)
             many = q_len >= LATENT_PROMPT_ROWS
             first = int(np.argmax(many)) if many.any() else 0
             lengths = np.where(many, plan.row_count[np.asarray(plan.q_start, np.int64) + np.maximum(q_len, 1) - 1], 0) if q_len.size else q_len
-            positions = int(lengths.sum())
+            room = -(-lengths // K.LATENT_KEYS) * K.LATENT_KEYS
+            positions = int(room.sum())
             # Requests with few rows have to lie before the others (as the scheduler orders a pass).
             if not many.any() or not many[first:].all() or positions > LATENT_PROMPT_POSITIONS or not self.ids.is_cuda:
                 self.memo[key] = None
             else:
-                base = np.cumsum(lengths) - lengths
+                base = np.cumsum(room) - room
                 tiles = cut_tiles(plan.q_start[first:], plan.q_len[first:], 128)
                 arrays = [tiles[0] + first, tiles[1] - int(plan.q_start[first]), tiles[2], base.astype(np.int32), lengths.astype(np.int32)]
                 host = torch.from_numpy(np.concatenate([a.astype(np.int32) for a in arrays])).pin_memory()

@@ -744,6 +744,9 @@ def latent_attention_mma(q, table, block_table, row_count, ranges, entries: int,
     return out
 
 
+LATENT_KEYS = 128       # positions that `latent_prompt` reads at a time
+
+
 def latent_prompt_takes(dtype, hq: int, d: int, rot: int, dv: int, kv_rank: int, scale: float) -> bool:
     """Whether `latent_prompt` takes these sizes."""
     return dtype == torch.bfloat16 and kv_rank % 64 == 0 and bool(library().kb_attention_flash_latent_takes(int(hq), int(d), int(rot), int(dv), _f(scale)))
@@ -761,9 +764,10 @@ def latent_query(q, heads: int, d: int, rot: int, cos_sin) -> torch.Tensor:
     return out
 
 
-def latent_gather(table, block_table, entry_base, entry_length, positions: int, longest: int, page_size: int, kv_rank: int, rot: int):
+def latent_gather(table, block_table, entry_base, entry_length, positions: int, longest: int, page_size: int, kv_rank: int, rot: int, align: int = 1):
     """(c [positions, kv_rank], rotated keys [positions, rot]) of the cached lines of whole requests: position p of request e at row
-    entry_base[e] + p, for p below entry_length[e]."""
+    entry_base[e] + p, for p below entry_length[e], and zeros behind a request's rows up to a multiple of `align` (for which the bases
+    leave room)."""
     _need(table, "latent_gather table", torch.bfloat16)
     if table.dim() != 4 or table.shape[1] != 1 or table.shape[2] != page_size or table.shape[3] != kv_rank + rot:
         raise KernelError(f"latent_gather: a table of {tuple(table.shape)} for lines of {kv_rank} + {rot}, pages of {page_size}")
@@ -776,14 +780,15 @@ def latent_gather(table, block_table, entry_base, entry_length, positions: int, 
     c = _fresh((positions, kv_rank), torch.bfloat16, table.device)
     rot_keys = _fresh((positions, rot), torch.bfloat16, table.device)
     _check(library().kb_latent_gather(_ptr(c), _ptr(rot_keys), _ptr(table), _ptr(block_table), int(block_table.shape[1]), int(table.shape[0]),
-                                      int(page_size), _ptr(entry_base), _ptr(entry_length), entries, int(longest), int(kv_rank), int(rot), _stream()))
+                                      int(page_size), _ptr(entry_base), _ptr(entry_length), entries, int(longest), int(align), int(kv_rank), int(rot), _stream()))
     return c, rot_keys
 
 
 def latent_prompt(q, kv, rot_keys, entry_base, row_count, tiles, scale: float, sinks, d: int, dv: int) -> torch.Tensor:
     """Attention of prompt portions over every head's own keys and values: q [rows, hq, d + rot] bfloat16, `kv` [positions,
     hq d + hq dv] (all heads' plain keys, then their values), `rot_keys` [positions, rot]; `tiles` of 128 rows; [rows, hq, dv] float32.
-    Rows that no tile names are left as they are."""
+    Rows that no tile names are left as they are. Keys are read LATENT_KEYS positions at a time, the last of them beyond the request's end:
+    what lies there meets weights of zero and has to be finite."""
     rows, hq, width = q.shape
     rot = width - d
     positions = kv.shape[0]

@@ -121,7 +121,7 @@ class LatentAttention(Part):
         multiply-adds of attention over the lines, which a portion of LATENT_PROMPT_ROWS rows pays back."""
         s, ctx = self.spec, self.ctx
         few, _, _, tiles, entry_base, entry_length, positions, longest = cut
-        c, rot_keys = K.latent_gather(k_table, group.block_table, entry_base, entry_length, positions, longest, ctx.page_size, s.kv_rank, s.rot_dim)
+        c, rot_keys = K.latent_gather(k_table, group.block_table, entry_base, entry_length, positions, longest, ctx.page_size, s.kv_rank, s.rot_dim, K.LATENT_KEYS)
         kv = linear(ctx, c, self.w_ukv)
         heads = K.latent_query(q, s.num_heads, s.head_dim, s.rot_dim, cos_sin)
         y = K.latent_prompt(heads, kv, rot_keys, entry_base, batch.row_count[few:], tiles, s.scale, self.sinks,

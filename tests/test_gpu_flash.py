@@ -167,3 +167,17 @@ def test_single_tokens_beside_a_prompt_at_wide_ranks(kv_rank):
 
     exact, got = run("float32"), run("bfloat16")
     assert got.shape == (92, 97) and float((got - exact).norm() / exact.norm()) <= 2e-2
+
+
+def test_a_request_reads_nothing_of_its_neighbour():
+    """Two prompts of lengths that fill no tile in one pass, laid out densely one behind the other, the second's lines no finite numbers: the
+    first's logits are what they are alone."""
+    from kapel_b200.engine import Engine
+
+    eng = Engine.random(LATENT, seed=2, dtype="bfloat16", max_tokens=1024, max_sequences=4, graphs=False)
+    eng.model.embedding.table[96] = float("nan")             # a token that the second prompt alone has
+    tokens = np.random.default_rng(7).integers(0, 96, 100).tolist()
+    want = list(range(100))
+    alone = eng.step([("a", tokens, want), ("b", [3] * 70, [])])[:, :96]
+    beside = eng.step([("c", tokens, want), ("d", [96] * 70, [69])])[:, :96]
+    assert torch.isfinite(alone).all() and torch.equal(alone, beside[:100]) and not torch.isfinite(beside[100]).any()
