@@ -58,7 +58,8 @@ def decode_split(pairs: int, longest: int, sms: int, window: Optional[int] = Non
 
 # Latent attention: a request's rows from which its keys and values are made for every head: that costs about 6 ns a position (16 heads of
 # 128 / 128 from 512 components), and then a pair of a row and a key costs 0.02 ns instead of the 0.4 that it costs over the cached
-# lines, so a portion of some twenty rows pays for it; 64 leaves room for the launches. And the most positions laid out so in a pass (9 KB each at 16 heads; the partial sums that the kernel over shared lines would write for them are more).
+# lines, so a portion of some twenty rows pays for it; 64 leaves room for the launches. And the most positions laid out so in a pass
+# (the part bounds their bytes).
 LATENT_PROMPT_ROWS = 64
 LATENT_PROMPT_POSITIONS = 131072
 

@@ -30,6 +30,20 @@ from .base import Part, linear, matrix_named, pad_columns, product_width, stack_
 from .registry import build_part
 
 
+PROMPT_BYTES = 512 << 20
+
+
+def room_for_heads(positions: int, longest: int, rows: int, heads: int, d: int, dv: int, kv_rank: int, rot: int) -> bool:
+    """Whether the keys and values of `positions` positions, made for every head, are small enough to be made: up to PROMPT_BYTES (57,000
+    positions of 16 heads of 128 / 128), or no more than the partial sums that attention over the lines would write for the pass's
+    `rows` instead (16 bytes a row and position at 16 heads, so from some 600 rows on whatever the history). Beyond it short portions
+    behind a long history stay with the lines, so that a pass takes no more memory than there was room for before it was cut this way."""
+    made = positions * (heads * (d + dv) + kv_rank + rot) * 2
+    slots = -(-longest // (K.attention_chunk() * K.LATENT_PROMPT_CHUNKS))
+    partial = rows * heads * slots * (kv_rank + 2) * 4 if slots > 1 else 0
+    return made <= max(PROMPT_BYTES, partial)
+
+
 class LatentAttention(Part):
     graph_safe = True
 
@@ -99,6 +113,8 @@ class LatentAttention(Part):
         s, ctx = self.spec, self.ctx
         H, d, r = s.num_heads, s.head_dim, s.rot_dim
         cut = batch.latent_tiles() if self.expands else None
+        if cut is not None and not room_for_heads(cut[6], cut[7], batch.rows, H, d, s.v_head_dim, s.kv_rank, r):
+            cut = None
         few = cut[0] if cut is not None else 0               # rows of requests that bring few, ahead of the others
         stacked = linear(ctx, h, self.w_down, out_dtype=torch.float32, keep_split=few == 0)
         k_table, _ = cache.tables()

@@ -92,3 +92,19 @@ def test_chunks_touched_counts_absolute_chunks():
     assert _chunks_touched(counts, 100, 64) == 2                            # keys 900..999 touch chunks 14 and 15
     assert _chunks_touched(np.array([1025], np.int32), 100, 64) == 3        # keys 925..1024 touch chunks 14, 15 and 16
     assert _chunks_touched(np.zeros(3, np.int32), None, 64) == 1
+
+
+def test_heads_of_a_long_history_are_made_only_where_they_fit():
+    """Latent attention's own keys and values for every head: bounded in bytes, whatever the number of heads, unless the pass's partial sums
+    over the lines would take as much."""
+    from kapel_b200.parts.latent_attention import PROMPT_BYTES, room_for_heads
+
+    size = lambda positions, heads: positions * (heads * 256 + 576) * 2
+    for heads in (4, 16, 64, 128):
+        for rows in (64, 100, 2048):
+            for positions in (64, 2048, 16384, 131072):
+                over_lines = rows * heads * -(-positions // 2048) * 514 * 4
+                fits = room_for_heads(positions, positions, rows, heads, 128, 128, 512, 64)
+                assert fits == (size(positions, heads) <= max(PROMPT_BYTES, over_lines if positions > 2048 else 0))
+    assert not room_for_heads(131072, 131072, 64, 16, 128, 128, 512, 64)           # 1.2 GB for 64 rows, whose partial sums are 135 MB
+    assert room_for_heads(131072, 131072, 2048, 16, 128, 128, 512, 64) and room_for_heads(16384, 16384, 64, 16, 128, 128, 512, 64)
