@@ -217,14 +217,28 @@ delta_chain_kernel(const DeltaChunks p) {
             const int t = row - DCH_C;
             const float G = b.fade[t][0];
             float4 o = make_float4(G * total.x, G * total.y, G * total.z, G * total.w);
+            // Up to the row itself: a later row's write may be no finite number, and then a weight of zero does not keep it out. A warp has
+            // eight rows, t0 .. t0 + 7: whole pieces of four sources below t0, the eight that lie among its rows each to the rows from it on.
+            const int t0 = (t >> 3) << 3;
 #pragma unroll
             for (int s = 0; s < DCH_C; s += 4) {
+                if (s >= t0 + 8) break;                         // the same for the whole warp
                 const float4 a = *reinterpret_cast<const float4*>(&b.within[t][s]);
                 const float aw[4] = {a.x, a.y, a.z, a.w};
+                if (s < t0) {
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 u = *reinterpret_cast<const float4*>(&m.u[s + j][col]);
-                    o.x = fmaf(aw[j], u.x, o.x), o.y = fmaf(aw[j], u.y, o.y), o.z = fmaf(aw[j], u.z, o.z), o.w = fmaf(aw[j], u.w, o.w);
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 u = *reinterpret_cast<const float4*>(&m.u[s + j][col]);
+                        o.x = fmaf(aw[j], u.x, o.x), o.y = fmaf(aw[j], u.y, o.y), o.z = fmaf(aw[j], u.z, o.z), o.w = fmaf(aw[j], u.w, o.w);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 u = *reinterpret_cast<const float4*>(&m.u[s + j][col]);
+                        const bool takes = s + j <= t;
+                        o.x = takes ? fmaf(aw[j], u.x, o.x) : o.x, o.y = takes ? fmaf(aw[j], u.y, o.y) : o.y;
+                        o.z = takes ? fmaf(aw[j], u.z, o.z) : o.z, o.w = takes ? fmaf(aw[j], u.w, o.w) : o.w;
+                    }
                 }
             }
             if (t < n) *reinterpret_cast<float4*>(p.out + ((size_t)(first + t) * p.heads + head) * e + c0 + col) = o;

@@ -106,3 +106,21 @@ def test_inputs_by_four_rows_and_by_rows(sizes):
                              len(sizes), H, G, d, e, taps, d ** -0.5, 1e-6) for src, off, state in ((x, 0, states[0]), (shifted, 1, states[1])))
         assert torch.equal(a, b)
     assert torch.equal(states[0], states[1])
+
+
+def test_a_row_takes_nothing_from_later_rows():
+    """A value that is no finite number reaches its own row and the rows behind it, by chunks as row by row."""
+    from kapel_b200 import kernels as K
+
+    H, G, d, e, taps, rows = 2, 1, 32, 16, 4, 200
+    rng = torch.Generator(device="cuda").manual_seed(3)
+    n, nv = G * d, H * e
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=rng)
+    conv, a_log, dt_bias, x = rand(2 * n + nv, taps), rand(H), rand(H), rand(rows, 2 * n + nv + 2 * H)
+    x[75, 2 * n + 3] = float("nan")                          # a value's component of the first head, in the middle of a chunk
+    entry = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    one, ranges = torch.ones(1, dtype=torch.int32, device="cuda"), K.entry_ranges(entry, 1)
+    out = [K.delta_scan(x, 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, conv, a_log, dt_bias, torch.zeros(2, K.delta_state_floats(H, G, d, e, taps), device="cuda"),
+                        entry, ranges, one, 1, H, G, d, e, taps, d ** -0.5, 1e-6, longest, longest) for longest in (0, rows)]
+    assert torch.isfinite(out[0][:75]).all() and not torch.isfinite(out[0][75:, 0, 3]).any()
+    assert torch.equal(torch.isfinite(out[0]), torch.isfinite(out[1]))
