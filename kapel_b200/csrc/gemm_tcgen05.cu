@@ -134,13 +134,16 @@ __device__ __forceinline__ void tc_ld16(uint32_t taddr, uint32_t (&r)[16]) {
 
 // Epilogues, chosen at compile time so that each kernel carries only its own code:
 // 0 none, 1 soft cap c * tanh(x / c), 2 and 3 the gated unit gelu_tanh(gate) * up and silu(gate) * up, 4 the unit with
-// both halves bounded, g sigmoid(alpha g) (u + 1) with g = min(gate, cap) and u = clamp(up, -cap, cap).
-constexpr int EPI_NONE = 0, EPI_SOFTCAP = 1, EPI_GLU_GELU = 2, EPI_GLU_SILU = 3, EPI_GLU_BOUNDED = 4;
-__host__ __device__ constexpr bool epi_glu(int epi) { return epi == EPI_GLU_GELU || epi == EPI_GLU_SILU || epi == EPI_GLU_BOUNDED; }
+// both halves bounded, g sigmoid(alpha g) (u + 1) with g = min(gate, cap) and u = clamp(up, -cap, cap); 5 the same with the
+// library's exponential: the experts', whose unit is that one's (`glu_clamped_kernel`) wherever it is applied.
+constexpr int EPI_NONE = 0, EPI_SOFTCAP = 1, EPI_GLU_GELU = 2, EPI_GLU_SILU = 3, EPI_GLU_BOUNDED = 4, EPI_GLU_BOUNDED_EXP = 5;
+__host__ __device__ constexpr bool epi_bounded(int epi) { return epi == EPI_GLU_BOUNDED || epi == EPI_GLU_BOUNDED_EXP; }
+__host__ __device__ constexpr bool epi_glu(int epi) { return epi == EPI_GLU_GELU || epi == EPI_GLU_SILU || epi_bounded(epi); }
+template <bool EXP = false>
 __device__ __forceinline__ float glu_bounded(float g, float u, float cap, float alpha) {
     g = fminf(g, cap);
     u = fminf(fmaxf(u, -cap), cap);
-    return g / (1.f + __expf(-alpha * g)) * (u + 1.f);
+    return g / (1.f + (EXP ? expf(-alpha * g) : __expf(-alpha * g))) * (u + 1.f);
 }
 
 __device__ __forceinline__ uint4 tc_pack8(const float (&v)[8]) {
@@ -222,7 +225,7 @@ __device__ __forceinline__ void tc_epilogue(uint32_t lanes, int row, int n0, voi
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
                     const float x = __uint_as_float(g[h + j]), up = __uint_as_float(u[h + j]);
-                    v[j] = EPI == EPI_GLU_BOUNDED ? glu_bounded(x, up, cap, alpha) : (EPI == EPI_GLU_GELU ? gelu_tanh(x) : silu(x)) * up;
+                    v[j] = epi_bounded(EPI) ? glu_bounded<EPI == EPI_GLU_BOUNDED_EXP>(x, up, cap, alpha) : (EPI == EPI_GLU_GELU ? gelu_tanh(x) : silu(x)) * up;
                 }
                 const int col = n0 + c0 + h;
                 tc_store8(c, c_dt, (size_t)row * n + col, col, n, vec && col + 8 <= n, v);
@@ -1359,7 +1362,7 @@ extern "C" int kb_moe_tcgen05(void* out, int out_dt, const void* a, const void* 
         case EPI_NONE: KB_MOE_TC(EPI_NONE); break;
         case EPI_GLU_GELU: KB_MOE_TC(EPI_GLU_GELU); break;
         case EPI_GLU_SILU: KB_MOE_TC(EPI_GLU_SILU); break;
-        case EPI_GLU_BOUNDED: KB_MOE_TC(EPI_GLU_BOUNDED); break;
+        case EPI_GLU_BOUNDED: KB_MOE_TC(EPI_GLU_BOUNDED_EXP); break;
         default: return fail("moe_tcgen05: epilogue %d is not known", epilogue);
     }
 #undef KB_MOE_TC

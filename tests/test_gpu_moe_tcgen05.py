@@ -79,3 +79,19 @@ def test_the_router_by_rows_and_a_row_a_block(dtype, scoring):
     for at in range(0, 531, 40):
         e, w = K.moe_route(h[at : at + 40].contiguous(), router, correction, 5, 1, 1, 1, scoring, True, 1.5)
         assert torch.equal(e, experts[at : at + 40]) and torch.equal(w, weights[at : at + 40])
+
+
+def test_the_bounded_unit_keeps_the_librarys_exponential():
+    """Rows that pick one weight each, so that the products are exact and the unit's own error shows."""
+    from kapel_b200 import kernels as K
+
+    width, inner = 160, 8
+    gate = -0.25 * torch.arange(width, device="cuda", dtype=torch.float32)[None, :] - torch.arange(inner, device="cuda")[:, None] * 0.25
+    w = torch.cat([gate, torch.full((inner, width), 0.5, device="cuda")])[None].bfloat16()
+    h = torch.eye(width, device="cuda").bfloat16()
+    lists = K.moe_sort(torch.zeros((width, 1), dtype=torch.int32, device="cuda"), 1, torch.bfloat16, 128)
+    got = K.moe_tcgen05(K.moe_gather(h, lists), w, lists, "clamped_swish", False, torch.float32, 50.0, 1.0)
+    g = gate.T[lists.order[:width].long()].double()
+    want = g * torch.sigmoid(g) * 1.5
+    # an exponential within an ulp, a sum, a quotient and a product: 4 roundings of 2^-24 and that ulp
+    assert ((got.double() - want).abs() <= 6.0 * 2.0 ** -24 * want.abs()).all()
