@@ -63,10 +63,29 @@ def decode_split(pairs: int, longest: int, sms: int, window: Optional[int] = Non
 LATENT_PROMPT_ROWS = 64
 LATENT_PROMPT_POSITIONS = 131072
 
-# The 32-bit attention by tiles: rows a tile, and the fewest tokens a request may bring (a tile takes 17 us a 64 keys however few its rows,
-# the row-wise kernel a twentieth of that a row and chunk side by side).
+# The 32-bit attention by tiles: rows a tile, and the fewest tokens a request may bring.
 ROW_TILE = 32
 ROW_TILE_TOKENS = 16
+
+
+def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: int, head_dim: int, window: Optional[int], sms: int) -> bool:
+    """Whether the 32-bit attention of these rows is faster by tiles than row by row. A block of the tile kernel walks all the keys of its
+    tile, 64 a step, however few its rows: few tiles behind a long history leave the GPU idle, where the row-wise kernel has a block
+    a row, kv head and 256 keys. Both as measured on a B200 for 16 to 1,024 tokens behind 0 to 16,384, groups of 1 to 16 heads of 128 and 256:
+    a step 16.6 us (heads of 256) or 11.0 (of 128), a block a multiprocessor; a key 0.07 us + 1.45 ns a component + 0.06 us a head of the group,
+    7 (groups of 1) to 4 (of 8) blocks a multiprocessor. 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 139 and 407; 16 tokens
+    behind 256, 1,024 and 4,096 positions 86 and 145, 281 and 149, 1,062 and 219; 128 tokens behind 1,024 and 16,384 298 and 373, 4,219 and 5,675."""
+    count = np.asarray(row_count, np.int64)
+    row0 = np.asarray(tile_row0, np.int64)
+    first, last = count[row0], count[row0 + np.asarray(tile_nq, np.int64) - 1]
+    steps = -(-(last - (np.maximum(0, first - window) if window else 0)) // 64)
+    by_tiles = 6.0 + (5.4 + 0.0438 * head_dim) * max(float(steps.max()), 1.1 * float(steps.sum()) * kv_heads / sms)
+    seen = np.where(count > window, window + 200, count) if window else count      # a window begins within a block's keys: one more, partly idle
+    slices, heads = -(-heads_per_kv // 8), min(heads_per_kv, 8)      # the row-wise kernel's blocks have up to eight heads
+    at_once = (7.5 - 0.42 * heads) * sms
+    by_rows = 3.0 + (0.07 + 0.00145 * head_dim + 0.06 * heads) * max(min(256.0, float(count.max())), float(seen.sum()) * kv_heads * slices / at_once)
+    return by_tiles <= by_rows
+
 
 # What a block costs beyond its 64-key steps, what the merge of partial sums costs beyond its traffic
 # (both in steps), microseconds a step, and how many multiprocessors a block takes, by prompt kernel;
@@ -330,16 +349,21 @@ class StepBatch:
         tiles = self.memo[key]
         return tiles[:3] if tiles is not None else None
 
-    def row_tiles(self, heads_per_kv: int):
+    def row_tiles(self, heads_per_kv: int, kv_heads: int, head_dim: int, window: Optional[int]):
         """(tile_entry, tile_row0, tile_nq) on the device for the 32-bit attention by tiles of ROW_TILE rows (tokens x query heads of a kv
-        head), or None where some request brings fewer than ROW_TILE_TOKENS tokens (its tile would hold a few rows and walk all its keys alone)."""
-        key = ("row_tiles", heads_per_kv)
+        head), or None where some request brings fewer than ROW_TILE_TOKENS tokens (its tile would hold a few rows and walk all its keys
+        alone) or the tiles take longer than row by row (`row_tiles_pay`)."""
+        key = ("row_tiles", heads_per_kv, kv_heads, head_dim, window)
         if key not in self.memo:
             plan = self.plan
-            if not len(plan.q_len) or self.shortest_portion() < ROW_TILE_TOKENS or heads_per_kv > ROW_TILE or not self.ids.is_cuda:
+            arrays = None
+            if len(plan.q_len) and self.shortest_portion() >= ROW_TILE_TOKENS and heads_per_kv <= ROW_TILE and self.ids.is_cuda:
+                arrays = cut_tiles(plan.q_start, plan.q_len, ROW_TILE // heads_per_kv)
+                if not row_tiles_pay(plan.row_count, arrays[1], arrays[2], kv_heads, heads_per_kv, head_dim, window, sm_count(self.ids.device)):
+                    arrays = None
+            if arrays is None:
                 self.memo[key] = None
             else:
-                arrays = cut_tiles(plan.q_start, plan.q_len, ROW_TILE // heads_per_kv)
                 n = arrays[0].size
                 host = torch.from_numpy(np.concatenate(arrays)).pin_memory()
                 dev = host.to(self.ids.device, non_blocking=True)

@@ -75,7 +75,7 @@ class StaticBatch:
     def shortest_portion(self) -> int:
         return 1
 
-    def row_tiles(self, heads_per_kv: int):
+    def row_tiles(self, *sizes):
         return None
 
     def mixed_tiles(self, *sizes):

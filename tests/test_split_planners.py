@@ -108,3 +108,17 @@ def test_heads_of_a_long_history_are_made_only_where_they_fit():
                 assert fits == (size(positions, heads) <= max(PROMPT_BYTES, over_lines if positions > 2048 else 0))
     assert not room_for_heads(131072, 131072, 64, 16, 128, 128, 512, 64)           # 1.2 GB for 64 rows, whose partial sums are 135 MB
     assert room_for_heads(131072, 131072, 2048, 16, 128, 128, 512, 64) and room_for_heads(16384, 16384, 64, 16, 128, 128, 512, 64)
+
+
+@pytest.mark.parametrize("heads_per_kv,kv_heads,d,window,tokens,before,tiles", [
+    (2, 4, 256, None, 500, 0, 1), (2, 4, 256, None, 16, 256, 1), (2, 4, 256, None, 16, 1024, 0), (2, 4, 256, None, 16, 6144, 0), (2, 4, 256, None, 64, 4096, 0),
+    (2, 4, 256, None, 128, 4096, 1), (2, 4, 256, None, 512, 16384, 1), (2, 8, 256, None, 64, 1024, 1), (2, 8, 256, None, 32, 4096, 0),
+    (4, 4, 128, None, 128, 16384, 1), (4, 4, 128, None, 32, 4096, 0), (1, 4, 128, None, 128, 4096, 0), (1, 4, 128, None, 1024, 4096, 1),
+    (8, 1, 256, None, 64, 4096, 0), (16, 1, 128, None, 256, 16384, 1), (16, 2, 128, None, 16, 4096, 0), (2, 4, 256, 512, 128, 16384, 1)])
+def test_32_bit_attention_goes_by_tiles_where_they_are_faster(heads_per_kv, kv_heads, d, window, tokens, before, tiles):
+    """As measured on a B200, one request: a few tiles behind a long history are slower than row by row."""
+    from kapel_b200.engine.batch import ROW_TILE, row_tiles_pay
+
+    _, row0, nq = cut_tiles(np.asarray([0]), np.asarray([tokens]), ROW_TILE // heads_per_kv)
+    count = np.arange(before + 1, before + tokens + 1)
+    assert row_tiles_pay(count, row0, nq, kv_heads, heads_per_kv, d, window, 148) == bool(tiles)
