@@ -214,6 +214,11 @@ def _fresh(shape, dtype, device) -> torch.Tensor:
     return t
 
 
+def buffer(shape, dtype, device) -> torch.Tensor:
+    """A buffer for kernels to write that a caller hands to several of them (`out`); like every other it is poisoned and refused on demand."""
+    return _fresh(shape, dtype, device)
+
+
 def fill_rows(table: torch.Tensor, rows: torch.Tensor, value: float = 0.0) -> None:
     """table[rows[i]] = value for a float32 table [n, ...] and int32 row numbers on the device."""
     _need(table, "fill_rows table", torch.float32)
@@ -1132,13 +1137,13 @@ def latent_append(stacked, q_off: int, kv_off: int, q_rank: int, kv_rank: int, r
 
 
 def head_linear(x, heads: int, x_head: int, x_off: int, m: torch.Tensor, y_head: Optional[int] = None, tail_off: int = 0,
-                tail: int = 0, cos_sin=None, gate=None, g_off: int = 0, pad_to: int = 0, transposed: bool = False) -> torch.Tensor:
+                tail: int = 0, cos_sin=None, gate=None, g_off: int = 0, pad_to: int = 0, transposed: bool = False, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """y[r, h, :n_out] = x[r, h, x_off : x_off + n_in] . m[h] for `m` [heads, n_in, n_out] (its dtype is
     the output's); `x` [rows, heads * x_head] is a tensor or a SplitSum. With `tail`, the components
     x[r, h, tail_off : tail_off + tail] follow the product in y, turned by `cos_sin` [rows, tail/2, 2].
     With `gate` (a float32 stacked product, tensor or SplitSum) the result is multiplied by the sigmoid
     of its columns g_off + h * n_out ... The result is [rows, heads * y_head] (y_head defaults to
-    n_out + tail), or [rows, pad_to] with zeros behind the heads. With `transposed`, `m` is bfloat16
+    n_out + tail), or [rows, pad_to] with zeros behind the heads, and goes to `out` where that is given. With `transposed`, `m` is bfloat16
     [heads, n_out, n_in] and the product runs on tensor cores."""
     src, x_dt, splits, stride, rows, x_row = _stacked(x, "head_linear input")
     _need(m, "head_linear matrices", torch.bfloat16 if transposed else None)
@@ -1154,7 +1159,7 @@ def head_linear(x, heads: int, x_head: int, x_off: int, m: torch.Tensor, y_head:
         g_src, g_dt, g_splits, g_stride, g_rows, g_row = _stacked(gate, "head_linear gate")
         if g_dt != F32 or g_rows != rows:
             raise KernelError("head_linear: the gate must be a float32 product of as many rows")
-    y = _fresh((rows, y_row), m.dtype, src.device)
+    y = _fresh((rows, y_row), m.dtype, src.device) if out is None else _need(out, "head_linear output", m.dtype, (rows, y_row))
     if transposed:
         _check(library().kb_head_linear_mma(
             _ptr(y), y_row, y_head, _ptr(src), x_dt, splits, ctypes.c_longlong(stride), x_row, int(x_head), int(x_off), _ptr(m), n_in, n_out,

@@ -397,7 +397,7 @@ class Attention(Part):
             mixed = batch.mixed_tiles(heads_per_kv, s.num_kv_heads, s.window, s.head_dim, prompt) if prompt != "mma" else None
             if mixed is not None:       # single tokens ahead of portions: each by the kernel made for them
                 n, ahead, behind, pairs = mixed
-                y = torch.empty_like(q)
+                y = K.buffer(q.shape, q.dtype, q.device)
                 for rows, (decode, tiles, split, slots, relative) in ((slice(0, n), ahead), (slice(n, None), behind)):
                     K.paged_attention_mma(q[rows], k_table, v_table, group.block_table, batch.row_count[rows], tiles, self.ctx.page_size, s.window, s.scale,
                                           s.softcap, decode, split, slots, relative, pairs=pairs, prompt_kernel=prompt, out=y[rows])

@@ -123,15 +123,17 @@ class LatentAttention(Part):
         c_q = K.latent_append(stacked, 0, s.q_rank, s.q_rank, s.kv_rank, r, self.norm_q, self.norm_kv, s.eps,
                               cos_sin, group.lines, k_table, cache.owns, ctx.dtype, pad_to=self.w_uq.shape[1])
         q = linear(ctx, c_q, self.w_uq, out_dtype=torch.float32, keep_split=few == 0)
-        if cut is not None:
-            o = self._expanded(q[few:] if few else q, cos_sin[few:] if few else cos_sin, stacked[few:] if few else stacked, batch, group, k_table, cut)
-            if few:
-                o = torch.cat([self._over_lines(q[:few], cos_sin[:few], stacked[:few], batch, group, k_table, batch.row_count[:few], cut[1], cut[2]), o])
+        if cut is not None and few:
+            o = K.buffer((batch.rows, product_width(ctx, H * s.v_head_dim)), ctx.dtype, q.device)
+            self._over_lines(q[:few], cos_sin[:few], stacked[:few], batch, group, k_table, batch.row_count[:few], cut[1], cut[2], o[:few])
+            self._expanded(q[few:], cos_sin[few:], stacked[few:], batch, group, k_table, cut, o[few:])
+        elif cut is not None:
+            o = self._expanded(q, cos_sin, stacked, batch, group, k_table, cut)
         else:
             o = self._over_lines(q, cos_sin, stacked, batch, group, k_table, batch.row_count, batch.entries, batch.longest_portion())
         return linear(ctx, o, self.w_o, keep_split=True)
 
-    def _expanded(self, q, cos_sin, stacked, batch, group, k_table, cut):
+    def _expanded(self, q, cos_sin, stacked, batch, group, k_table, cut, out=None):
         """Prompt portions: the lines of the whole requests are laid out densely, one product makes every head's own keys and
         values of them, and attention runs at the heads' own sizes. Per pair of a row and a key that is a third of the
         multiply-adds of attention over the lines, which a portion of LATENT_PROMPT_ROWS rows pays back."""
@@ -143,9 +145,9 @@ class LatentAttention(Part):
         y = K.latent_prompt(heads, kv, rot_keys, entry_base, batch.row_count[few:], tiles, s.scale, self.sinks,
                             s.head_dim, s.v_head_dim)
         return K.head_gate(y, stacked, s.q_rank + s.kv_rank + s.rot_dim if s.gated else 0, None, False, 0.0, ctx.dtype,
-                           pad_to=product_width(ctx, s.num_heads * s.v_head_dim), gate_act="sigmoid" if s.gated else "none")
+                           pad_to=product_width(ctx, s.num_heads * s.v_head_dim), gate_act="sigmoid" if s.gated else "none", out=out)
 
-    def _over_lines(self, q, cos_sin, stacked, batch, group, k_table, row_count, entries, longest):
+    def _over_lines(self, q, cos_sin, stacked, batch, group, k_table, row_count, entries, longest, out=None):
         """Single tokens and short portions: all heads over the cached lines themselves."""
         s, ctx = self.spec, self.ctx
         H, d, r = s.num_heads, s.head_dim, s.rot_dim
@@ -159,4 +161,4 @@ class LatentAttention(Part):
                                        row_count, ctx.page_size, None, s.scale, None, batch.attention_slots(None),
                                        sinks=self.sinks, value_dim=s.kv_rank)
         return K.head_linear(y.view(-1, H * s.kv_rank), H, s.kv_rank, 0, self.m_uv, gate=stacked if s.gated else None,
-                          g_off=s.q_rank + s.kv_rank + r, pad_to=product_width(ctx, H * s.v_head_dim), transposed=self.turned)
+                          g_off=s.q_rank + s.kv_rank + r, pad_to=product_width(ctx, H * s.v_head_dim), transposed=self.turned, out=out)
