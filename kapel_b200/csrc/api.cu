@@ -13,6 +13,12 @@ int fail(const char* fmt, ...) {
     return 1;
 }
 
+int multiprocessors() {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) sms = 0;
+    return sms > 0 ? sms : 148;
+}
+
 static unsigned long long g_launches = 0;
 static unsigned long long g_dependent_launches = 0;
 static bool g_pdl = false;
@@ -49,6 +55,8 @@ extern "C" unsigned long long kb_dependent_launch_count() { return kb::g_depende
 
 // The compute capability this library was built for, as major * 10 + minor.
 extern "C" int kb_built_for() { return 100; }
+
+extern "C" int kb_multiprocessors() { return kb::multiprocessors(); }
 
 extern "C" int kb_device_info(int* sms, int* cc_major, int* cc_minor) {
     int dev = 0;

@@ -18,6 +18,7 @@ namespace kb {
 
 int fail(const char* fmt, ...);          // stores the message, returns 1
 int check_launch(const char* what);      // cudaGetLastError -> fail(...)
+int multiprocessors();                   // the current device's (148 where there is none)
 
 // Programmatic dependent launch. A kernel started through `launch_dependent` may begin while the
 // kernel before it on the stream still runs: it must call `dependent_wait()` before it reads what

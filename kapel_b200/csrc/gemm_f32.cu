@@ -266,10 +266,11 @@ static int launch_f32(float* c, const float* a, const float* w, int m, int n, in
             // largest's rate (500 rows by 18,432 x 2,304: 828, 925, 942, 1,083 and 1,519 us in this order).
             const int bm[5] = {128, 128, 64, 64, 32}, bn[5] = {128, 64, 128, 64, 64};
             const double reach[5] = {1.0, 0.9, 0.88, 0.76, 0.55};
+            const int sms = multiprocessors();
             double best = 0;
             for (int v = 0; v < 5; ++v) {
                 const long long tiles = (long long)((m + bm[v] - 1) / bm[v]) * ((n + bn[v] - 1) / bn[v]);
-                const double cost = (double)((tiles + 147) / 148) * bm[v] * bn[v] / reach[v];
+                const double cost = (double)((tiles + sms - 1) / sms) * bm[v] * bn[v] / reach[v];
                 if (v == 0 || cost < best) best = cost, variant = v + 1;
             }
         }

@@ -1324,7 +1324,7 @@ extern "C" int kb_moe_gather(void* out, const void* a, const int* order, const i
     KB_REQUIRE((((uintptr_t)out | (uintptr_t)a) & 15) == 0, "moe_gather: tensors must be 16-byte aligned");
     if (pairs == 0) return 0;
     const long long work = (long long)pairs * (k / 8);
-    launch_dependent_if(pairs <= DEPENDENT_ROWS * top, moe_gather_kernel, dim3((unsigned)std::min<long long>((work + 255) / 256, 148 * 16)), dim3(256), 0, (cudaStream_t)stream,
+    launch_dependent_if(pairs <= DEPENDENT_ROWS * top, moe_gather_kernel, dim3((unsigned)std::min<long long>((work + 255) / 256, multiprocessors() * 16)), dim3(256), 0, (cudaStream_t)stream,
                         (uint4*)out, (const uint4*)a, order, listed, k / 8, top);
     return check_launch("moe_gather");
 }

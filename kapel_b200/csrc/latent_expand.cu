@@ -85,7 +85,7 @@ extern "C" int kb_latent_query(void* q, const void* src, int in_dt, int splits, 
     KB_REQUIRE(((uintptr_t)q & 3) == 0 && cos_sin != nullptr, "latent_query: an aligned output and a table are needed");
     if (rows == 0) return 0;
     const long long work = (long long)rows * heads * ((d + rot / 2) / 2);
-    const unsigned blocks = (unsigned)std::min<long long>((work + 255) / 256, 148 * 16);
+    const unsigned blocks = (unsigned)std::min<long long>((work + 255) / 256, multiprocessors() * 16);
     if (in_dt == KB_DT_F32) latent_query_kernel<float><<<blocks, 256, 0, (cudaStream_t)stream>>>(Src<float>{(const float*)src, splits, (size_t)split_stride}, (const float2*)cos_sin, (bf16*)q, rows, heads, d, rot);
     else if (in_dt == KB_DT_BF16) latent_query_kernel<bf16><<<blocks, 256, 0, (cudaStream_t)stream>>>(Src<bf16>{(const bf16*)src, splits, (size_t)split_stride}, (const float2*)cos_sin, (bf16*)q, rows, heads, d, rot);
     else return fail("latent_query: dtype code %d is not known", in_dt);

@@ -878,7 +878,8 @@ extern "C" int kb_head_linear_mma(void* y, int y_row, int y_head, const void* x,
     if (rows <= HF_ROWS && few_smem <= 48 * 1024 && (n_out + HF_WARPS - 1) / HF_WARPS <= 65535) {     // a decode step: a warp a column
         // columns a warp: every block adds up the rows' inputs of its head again, so several where the blocks still fill the GPU
         int columns = 1;
-        while (columns < 8 && (long long)heads * (n_out / (2 * columns * HF_WARPS)) >= 148) columns *= 2;
+        const int sms = multiprocessors();
+        while (columns < 8 && (long long)heads * (n_out / (2 * columns * HF_WARPS)) >= sms) columns *= 2;
         dim3 few(heads, (n_out + HF_WARPS * columns - 1) / (HF_WARPS * columns));
         if (x_dt == KB_DT_F32)
             launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<float>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, Src<float>{(const float*)x, x_splits, (size_t)x_split_stride}, x_row,

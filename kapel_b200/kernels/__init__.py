@@ -737,7 +737,7 @@ def latent_attention_mma(q, table, block_table, row_count, ranges, entries: int,
     chunk = attention_chunk()
     if longest == 1:        # single tokens: a block a chunk of 128 keys, while the launch stays within four waves of blocks
         finer = -(-int(slots) * chunk // int(lib.kb_latent_decode_keys()))
-        if rows * (-(-hq // 16)) * finer <= 4 * 148:
+        if rows * (-(-hq // 16)) * finer <= 4 * int(lib.kb_multiprocessors()):
             chunk, slots = int(lib.kb_latent_decode_keys()), finer
     if longest > 1:         # measured at 2,048 tokens, 16 heads, lines of 576: 4.91, 4.68, 4.52, 4.43 ms a four-layer prefill with 1, 2, 4, 8
         chunk, slots = chunk * LATENT_PROMPT_CHUNKS, -(-int(slots) // LATENT_PROMPT_CHUNKS)

@@ -35,3 +35,9 @@ def test_every_kernel_gives_the_same_bits(m, n, k):
         assert (capped.double() - 5.0 * torch.tanh(got[0].double() / 5.0)).abs().max() <= 5.0 * 2.0 ** -21
         if m > 1:                                            # a row does not depend on the others
             assert torch.equal(product(a[: m // 2].contiguous(), w, -1, 0.0), got[0][: m // 2])
+
+
+def test_the_launchers_rules_ask_the_device():
+    from kapel_b200 import kernels as K
+
+    assert K.library().kb_multiprocessors() == torch.cuda.get_device_properties(0).multi_processor_count
