@@ -29,8 +29,10 @@ int multiprocessors();                   // the current device's (148 where ther
 // Only the kernels of a step of at most DEPENDENT_ROWS rows (decoding) are chained this way. The
 // kernels of a prompt are launched plainly (`launch_dependent_if(false, ...)`): that is a rule of
 // this library, not a tuning choice, and it holds for every prompt kernel. A launch knows the rows it
-// covers, which in a pass with prompts may be a few of many (single tokens beside a prompt, the rows whose
-// logits are wanted): `kb_pass_rows` tells the thread's launches how many the whole pass has, and that decides.
+// covers, which in a pass with prompts may be a few of many (the single tokens beside a prompt): `kb_pass_rows` tells the
+// thread's launches how many the whole pass has, and that decides. What comes behind the last kernel over all rows of a pass, the norm and
+// the product of the rows whose logits are wanted, goes by those rows' number: the gather ahead of them is launched plainly, so they
+// overlap with one another and with no kernel of a prompt.
 constexpr int DEPENDENT_ROWS = 64;
 bool chains(bool dependent);             // whether a launch that may be a dependent is one (and counts it)
 template <typename... KArgs, typename... Args>
