@@ -8,15 +8,15 @@
 //                  over S as bfloat16;
 //   O += P V       tcgen05.mma with P as the A operand straight from TMEM, the value tile [128 x DV] an MN-major B operand; O
 //                  [128 x DV] float32 stays in TMEM.
-// m is a row's reference. The first tile sets it to that tile's largest score; later tiles move it only when their largest score
-// lies more than 8 (in powers of two) above it, which hardly ever happens after a few tiles: P is then at most 2^8, as
-// exact in bfloat16 as below 1, and the sums stay far inside 32 bits. When it moves, the warps of the row's quarter wait until
+// m is a row's reference, its largest score so far. When a tile raises it, the warps of the row's quarter wait until
 // the product of the tile before has gone through, scale their rows of O in TMEM and go on: the product of this tile cannot
-// start before their P is there, so nobody else touches O meanwhile.
+// start before their P is there, so nobody else touches O meanwhile. Letting m lag by up to 2^8 would save most of these waits and less than
+// 0.5 % of a prompt's pass, but then the largest weight of a row is no power of two and is rounded: an error up to 1.24 times as large where one
+// key has nearly all the weight. The row's sum adds up the rounded P, as the product does.
 //
 // What bounds it: a tile takes 64 clocks a 16-element step, (DQK + DV) / 16 of them, on the tensor cores and 1,024 clocks of
-// exponentials (16 a clock a multiprocessor). 2,048 tokens, 16 heads of 192 / 128: 47 us (458 Tflop/s; the kernel over shared lines
-// took 867 us and the two products a head around it 248); 16 heads over 4 of 128: 42 us (the mma.sync kernel: 111). A launch of 256
+// exponentials (16 a clock a multiprocessor). 2,048 tokens, 16 heads of 192 / 128: 49 us (440 Tflop/s; the kernel over shared lines
+// took 867 us and the two products a head around it 248); 16 heads over 4 of 128: 44 us (the mma.sync kernel: 111). A launch of 256
 // blocks is 1.7 waves, and a block of few tiles spends most of its time on what precedes its first product and follows its last.
 //
 // Keys and values come from the paged cache (boxes of 16 keys x 64 elements, four warps asking, a half of the keys or values each) or,
@@ -299,7 +299,7 @@ attention_flash_kernel(const FlashParams p, const __grid_constant__ CUtensorMap 
             turn[half * AF_ROWS + r] = top;
             asm volatile("bar.sync %0, 64;" ::"r"(2 + quarter) : "memory");
             top = fmaxf(top, turn[(half ^ 1) * AF_ROWS + r]) * c;
-            const bool moves = top > ref + 8.f || (ref == -INFINITY && top > -INFINITY);
+            const bool moves = top > ref;
             const float was = ref;
             if (moves) ref = top;
             const float fade = moves ? (was == -INFINITY ? 0.f : at_exp2(was - ref)) : 1.f;      // a row that has seen nothing holds zeros
@@ -325,16 +325,18 @@ attention_flash_kernel(const FlashParams p, const __grid_constant__ CUtensorMap 
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
                 const float p0 = at_exp2(fmaf(__uint_as_float(sa[j]), c, -m)), p1 = at_exp2(fmaf(__uint_as_float(sa[j + 1]), c, -m));
-                la += p0;
-                lb += p1;
-                pr[j >> 1] = at_pack(p0, p1);
+                const uint32_t w = at_pack(p0, p1);
+                la += __uint_as_float(w << 16);
+                lb += __uint_as_float(w & 0xffff0000u);
+                pr[j >> 1] = w;
             }
 #pragma unroll
             for (int j = 0; j < 32; j += 2) {
                 const float p0 = at_exp2(fmaf(__uint_as_float(sb[j]), c, -m)), p1 = at_exp2(fmaf(__uint_as_float(sb[j + 1]), c, -m));
-                la += p0;
-                lb += p1;
-                pr[16 + (j >> 1)] = at_pack(p0, p1);
+                const uint32_t w = at_pack(p0, p1);
+                la += __uint_as_float(w << 16);
+                lb += __uint_as_float(w & 0xffff0000u);
+                pr[16 + (j >> 1)] = w;
             }
             l += la + lb;
             at_st32(lanes + (uint32_t)(C::COL_S + b * AF_KEYS + half * 32), pr);
