@@ -4,8 +4,11 @@
 // over 4 of 256). Here a block takes 32 rows -- (token, query head) pairs of one kv head -- and walks their keys 64 at a time: scores by 32-bit
 // multiply-adds from shared memory, the running maximum and the weights eight threads a row, then the weighted sum into registers. Keys and values come
 // by asynchronous copies, the next keys while the values are multiplied, the values while the scores are made. No tensor-core instruction: nothing
-// rounds an input; exponentials and soft caps are the library's. Shared memory's 32 words a clock bound it (0.75 and 0.38 words a multiply-add),
-// and how few blocks a short prompt gives: 139 us for those 500 tokens, which is what the 8 steps of the last rows' block take.
+// rounds an input; exponentials and soft caps are the library's. Sums go by pieces (chains of 8 components; of 64 keys, then of 256), so that their
+// rounding is no larger than the row-wise kernel's, whose lanes and chunks cut them as short: 0.7 to 0.99 of its error against 64 bits at 500
+// to 4,608 keys, where one chain a sum had 1.8 to 4.7 times as much and took 139 us instead of 147. Shared memory's 32 words a clock bound it (0.75
+// and 0.38 words a multiply-add), and how few blocks a short prompt gives: 147 us for those 500 tokens, which is what the 8 steps of the last
+// rows' block take. With heads of 128 two blocks share a multiprocessor.
 #include <type_traits>
 #include "common.cuh"
 
@@ -29,7 +32,7 @@ struct F32TileParams {
 };
 
 template <int D>
-__global__ void __launch_bounds__(AFT_THREADS, 1)
+__global__ void __launch_bounds__(AFT_THREADS, D == 128 ? 2 : 1)
 attention_f32_tiles_kernel(const F32TileParams p) {
     constexpr int LD = D + 4, D4 = D / 4, CG = D / 128;          // column groups of four a lane holds: 4 (lane + 32 g)
     extern __shared__ __align__(16) float aft_smem[];
@@ -81,9 +84,19 @@ attention_f32_tiles_kernel(const F32TileParams p) {
     const bool own = sr < rows_valid;
     const int cnt = own ? c_first + sr / group : 0;
     const int fst = (own && p.window > 0 && cnt > p.window) ? cnt - p.window : 0;
-    float m = -INFINITY, l = 0.f;
+    float m = -INFINITY, l = 0.f, l_near = 0.f, l_fade = 1.f;
     const int qy = tid >> 4, qx = tid & 15;                      // scores: rows 2 qy and 2 qy + 1, keys qx + 16 j
-    float o[4][4 * CG] = {};                                     // sums: rows 4 warp .. + 3
+    // Sums over the keys of rows 4 warp .. + 3: a step's 64 keys, those of up to four steps, and all before; o is still to be scaled by o_fade.
+    float o[4][4 * CG] = {}, near[4][4 * CG] = {}, o_fade[4] = {1.f, 1.f, 1.f, 1.f};
+    auto gather = [&]() {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int c = 0; c < 4 * CG; ++c) o[i][c] = fmaf(o[i][c], o_fade[i], near[i][c]), near[i][c] = 0.f;
+            o_fade[i] = 1.f;
+        }
+        l = fmaf(l, l_fade, l_near), l_near = 0.f, l_fade = 1.f;
+    };
     if (klo < khi) {
         fetch(sk, p.k_table, klo);
         fetch(sv, p.v_table, klo);
@@ -93,16 +106,29 @@ attention_f32_tiles_kernel(const F32TileParams p) {
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();                                         // the keys are there
         {
-            float s[2][4] = {};
+            float s[2][4] = {}, half[2][4] = {};
+#pragma unroll 1
+            for (int x0 = 0; x0 < D; x0 += 32) {                 // 32 components in four chains of eight; pieces meet in pairs
+                float4 c[2][4] = {};
 #pragma unroll 4
-            for (int x = 0; x < D; x += 4) {
-                const float4 a = *reinterpret_cast<const float4*>(sq + (2 * qy) * LD + x), b = *reinterpret_cast<const float4*>(sq + (2 * qy + 1) * LD + x);
+                for (int x = x0; x < x0 + 32; x += 4) {
+                    const float4 a = *reinterpret_cast<const float4*>(sq + (2 * qy) * LD + x), b = *reinterpret_cast<const float4*>(sq + (2 * qy + 1) * LD + x);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float4 k = *reinterpret_cast<const float4*>(sk + (qx + 16 * j) * LD + x);
-                    s[0][j] = fmaf(a.w, k.w, fmaf(a.z, k.z, fmaf(a.y, k.y, fmaf(a.x, k.x, s[0][j]))));
-                    s[1][j] = fmaf(b.w, k.w, fmaf(b.z, k.z, fmaf(b.y, k.y, fmaf(b.x, k.x, s[1][j]))));
+                    for (int j = 0; j < 4; ++j) {
+                        const float4 k = *reinterpret_cast<const float4*>(sk + (qx + 16 * j) * LD + x);
+                        c[0][j].x = fmaf(a.x, k.x, c[0][j].x), c[0][j].y = fmaf(a.y, k.y, c[0][j].y), c[0][j].z = fmaf(a.z, k.z, c[0][j].z), c[0][j].w = fmaf(a.w, k.w, c[0][j].w);
+                        c[1][j].x = fmaf(b.x, k.x, c[1][j].x), c[1][j].y = fmaf(b.y, k.y, c[1][j].y), c[1][j].z = fmaf(b.z, k.z, c[1][j].z), c[1][j].w = fmaf(b.w, k.w, c[1][j].w);
+                    }
                 }
+                const bool second = x0 & 32;
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const float piece = (c[i][j].x + c[i][j].y) + (c[i][j].z + c[i][j].w);
+                        s[i][j] += second ? half[i][j] + piece : 0.f;
+                        half[i][j] = piece;
+                    }
             }
 #pragma unroll
             for (int i = 0; i < 2; ++i)
@@ -136,18 +162,14 @@ attention_f32_tiles_kernel(const F32TileParams p) {
             }
 #pragma unroll
             for (int d = 1; d < 8; d <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
-            l = l * f + sum;
+            l_near = l_near * f + sum;
+            l_fade *= f;
             m = now;
             if (sc == 0) fade[sr] = f;
         }
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();                                         // the weights and the values are there
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float f = fade[4 * warp + i];
-#pragma unroll
-            for (int c = 0; c < 4 * CG; ++c) o[i][c] *= f;
-        }
+        float now[4][4 * CG] = {};
         auto sum = [&](auto all) {
 #pragma unroll 4
             for (int k = 0; k < AFT_KEYS; k += 4) {
@@ -163,21 +185,30 @@ attention_f32_tiles_kernel(const F32TileParams p) {
                         for (int i = 0; i < 4; ++i) {
                             if (!decltype(all)::value && (k0 + k + kk < lo4[i] || k0 + k + kk >= hi4[i])) continue;      // the same for the whole warp
                             const float x = kk == 0 ? w[i].x : kk == 1 ? w[i].y : kk == 2 ? w[i].z : w[i].w;
-                            o[i][4 * g] = fmaf(x, v.x, o[i][4 * g]);
-                            o[i][4 * g + 1] = fmaf(x, v.y, o[i][4 * g + 1]);
-                            o[i][4 * g + 2] = fmaf(x, v.z, o[i][4 * g + 2]);
-                            o[i][4 * g + 3] = fmaf(x, v.w, o[i][4 * g + 3]);
+                            now[i][4 * g] = fmaf(x, v.x, now[i][4 * g]);
+                            now[i][4 * g + 1] = fmaf(x, v.y, now[i][4 * g + 1]);
+                            now[i][4 * g + 2] = fmaf(x, v.z, now[i][4 * g + 2]);
+                            now[i][4 * g + 3] = fmaf(x, v.w, now[i][4 * g + 3]);
                         }
                     }
             }
         };
         if (k0 >= all_from && k0 + AFT_KEYS <= c_first) sum(std::true_type{});
         else sum(std::false_type{});
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float f = fade[4 * warp + i];
+#pragma unroll
+            for (int c = 0; c < 4 * CG; ++c) near[i][c] = fmaf(near[i][c], f, now[i][c]);
+            o_fade[i] *= f;
+        }
+        if (((k0 - klo) / AFT_KEYS & 3) == 3) gather();
         __syncthreads();                                         // the values and the weights are done with
         if (more) fetch(sv, p.v_table, k0 + AFT_KEYS);
         else asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
+    gather();
     if (sc == 0) {
         float inv = 0.f;
         if (l > 0.f) {

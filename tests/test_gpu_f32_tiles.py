@@ -82,3 +82,26 @@ def test_what_a_row_does_not_see_does_not_reach_it(hq, hkv, d, window):
     assert torch.equal(torch.isfinite(by_rows), torch.isfinite(by_tiles))
     # sums of at most 100 weights in 32-bit, in another order
     assert (by_rows - by_tiles)[~seen].abs().max() <= 1e-5 * by_rows[~seen].abs().max()
+
+
+@pytest.mark.parametrize("hq,hkv,d,cap", [(8, 4, 256, 50.0), (16, 4, 128, None)])
+@pytest.mark.parametrize("before,n,peak", [(0, 500, 1.0), (2500, 96, 1.0), (2500, 96, 4.0)])
+def test_as_near_to_64_bit_as_row_by_row(hq, hkv, d, cap, before, n, peak):
+    """The 2-norm of the error: short chains of products and of keys, as the row-wise kernel's lanes and chunks have them."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(9)
+    T = before + n
+    width = -(-T // 16)
+    k_table, v_table = (torch.randn(width, hkv, 16, d, device="cuda", generator=gen) for _ in range(2))
+    k, v = (t.transpose(1, 2).reshape(width * 16, hkv, d)[:T].double().repeat_interleave(hq // hkv, 1) for t in (k_table, v_table))
+    q = torch.randn(n, hq, d, device="cuda", generator=gen) * peak
+    counts = torch.arange(before + 1, T + 1, dtype=torch.int32, device="cuda")
+    s = torch.einsum("nhd,thd->hnt", q.double(), k) * d ** -0.5
+    s = cap * torch.tanh(s / cap) if cap else s
+    s = s.masked_fill((torch.arange(T, device="cuda")[None, :] >= counts[:, None])[None], -torch.inf)
+    want = torch.einsum("hnt,thd->nhd", torch.softmax(s, -1), v)
+    args = (q, k_table, v_table, torch.arange(width, dtype=torch.int32, device="cuda")[None].contiguous(), torch.zeros(n, dtype=torch.int32, device="cuda"),
+            counts, 16, None, d ** -0.5, cap, -(-T // K.attention_chunk()))
+    off = [float((K.paged_attention_rows(*args, tiles=t).double() - want).norm() / want.norm()) for t in (None, cut([(before, n)], 32 // (hq // hkv)))]
+    assert off[1] <= 1.03 * off[0], off                      # 190,000 results and more: the norms of two random errors of one size agree to 1 %
