@@ -521,7 +521,7 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
 #undef KB_DELTA_PREP
     if (by_chunks) {
         DeltaChunks c;
-        c.qn = p.qn; c.kn = p.kn; c.vn = p.vn; c.scal = p.scal;
+        c.qn = p.qn; c.kn = p.kn; c.vn = p.vn; c.scal = p.scal; c.kq = p.kq;
         c.w = chunk_scratch;
         c.u0 = c.w + (size_t)rows * heads * d;
         c.within = c.u0 + (size_t)rows * nv;

@@ -44,17 +44,27 @@ delta_chunk_kernel(const DeltaChunks p) {
     {   // a thread: row t against four rows s of the chunk
         const int t = tid >> 3, s0 = (tid & 7) * 4;
         float a[4] = {}, b[4] = {};
-        for (int x = 0; x < d; x += 4) {
-            const float4 k = *reinterpret_cast<const float4*>(&sk[t][x]), q = *reinterpret_cast<const float4*>(&sq[t][x]);
+        for (int x0 = 0; x0 < d; x0 += 32) {                    // 32 components in four chains of eight: the rounding of a warp's sum of lanes
+            float4 ka[4] = {}, qa[4] = {};
+#pragma unroll 2
+            for (int x = x0; x < x0 + 32; x += 4) {
+                const float4 k = *reinterpret_cast<const float4*>(&sk[t][x]), q = *reinterpret_cast<const float4*>(&sq[t][x]);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float4 o = *reinterpret_cast<const float4*>(&sk[s0 + j][x]);
+                    ka[j].x = fmaf(k.x, o.x, ka[j].x), ka[j].y = fmaf(k.y, o.y, ka[j].y), ka[j].z = fmaf(k.z, o.z, ka[j].z), ka[j].w = fmaf(k.w, o.w, ka[j].w);
+                    qa[j].x = fmaf(q.x, o.x, qa[j].x), qa[j].y = fmaf(q.y, o.y, qa[j].y), qa[j].z = fmaf(q.z, o.z, qa[j].z), qa[j].w = fmaf(q.w, o.w, qa[j].w);
+                }
+            }
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const float4 o = *reinterpret_cast<const float4*>(&sk[s0 + j][x]);
-                a[j] = fmaf(k.w, o.w, fmaf(k.z, o.z, fmaf(k.y, o.y, fmaf(k.x, o.x, a[j]))));
-                b[j] = fmaf(q.w, o.w, fmaf(q.z, o.z, fmaf(q.y, o.y, fmaf(q.x, o.x, b[j]))));
+                a[j] += (ka[j].x + ka[j].y) + (ka[j].z + ka[j].w);
+                b[j] += (qa[j].x + qa[j].y) + (qa[j].z + qa[j].w);
             }
         }
 #pragma unroll
-        for (int j = 0; j < 4; ++j) kk[t][s0 + j] = a[j], qk[t][s0 + j] = b[j];
+        for (int j = 0; j < 4; ++j)                             // a row against itself: as the scan has it, from before the vectors were rounded
+            kk[t][s0 + j] = a[j], qk[t][s0 + j] = s0 + j == t && t < n ? p.kq[(size_t)(first + t) * p.kv_heads + kvh] : b[j];
     }
     auto am = sq;                                               // [t][s] the substitution's matrix, once the queries are done with
     const int per = p.heads / p.kv_heads;
@@ -201,9 +211,9 @@ delta_chain_kernel(const DeltaChunks p) {
         const int row = tid >> 2, col = (tid & 3) * 4;
         float4 total = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-        for (int w8 = 0; w8 < 8; ++w8) {
-            const float4 v = *reinterpret_cast<const float4*>(&m.part[w8][row][col]);
-            total.x += v.x, total.y += v.y, total.z += v.z, total.w += v.w;
+        for (int w8 = 0; w8 < 8; w8 += 2) {
+            const float4 v = *reinterpret_cast<const float4*>(&m.part[w8][row][col]), w = *reinterpret_cast<const float4*>(&m.part[w8 + 1][row][col]);
+            total.x += v.x + w.x, total.y += v.y + w.y, total.z += v.z + w.z, total.w += v.w + w.w;
         }
         if (row < DCH_C) {                                      // U = U0 - W S
             const float4 v = *reinterpret_cast<const float4*>(&b.u0[row][col]);
@@ -220,6 +230,7 @@ delta_chain_kernel(const DeltaChunks p) {
             // Up to the row itself: a later row's write may be no finite number, and then a weight of zero does not keep it out. A warp has
             // eight rows, t0 .. t0 + 7: whole pieces of four sources below t0, the eight that lie among its rows each to the rows from it on.
             const int t0 = (t >> 3) << 3;
+            float4 below = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
             for (int s = 0; s < DCH_C; s += 4) {
                 if (s >= t0 + 8) break;                         // the same for the whole warp
@@ -229,7 +240,7 @@ delta_chain_kernel(const DeltaChunks p) {
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
                         const float4 u = *reinterpret_cast<const float4*>(&m.u[s + j][col]);
-                        o.x = fmaf(aw[j], u.x, o.x), o.y = fmaf(aw[j], u.y, o.y), o.z = fmaf(aw[j], u.z, o.z), o.w = fmaf(aw[j], u.w, o.w);
+                        below.x = fmaf(aw[j], u.x, below.x), below.y = fmaf(aw[j], u.y, below.y), below.z = fmaf(aw[j], u.z, below.z), below.w = fmaf(aw[j], u.w, below.w);
                     }
                 } else {
 #pragma unroll
@@ -240,6 +251,7 @@ delta_chain_kernel(const DeltaChunks p) {
                         o.z = takes ? fmaf(aw[j], u.z, o.z) : o.z, o.w = takes ? fmaf(aw[j], u.w, o.w) : o.w;
                     }
                 }
+                if (s + 4 == t0) o.x += below.x, o.y += below.y, o.z += below.z, o.w += below.w;
             }
             if (t < n) *reinterpret_cast<float4*>(p.out + ((size_t)(first + t) * p.heads + head) * e + c0 + col) = o;
         } else if ((tid >> 2) < d4) {                           // the memory behind the chunk: four of its rows x four columns a thread

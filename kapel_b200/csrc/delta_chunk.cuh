@@ -11,6 +11,7 @@ struct DeltaChunks {
     const float* kn;            // [rows, kv_heads, d] unit keys
     const float* vn;            // [rows, heads, e]
     const float* scal;          // [rows, heads, 2] decay, step size
+    const float* kq;            // [rows, kv_heads] a row's key times its query
     float* w;                   // [rows, heads, d]: what a chunk's writes owe to the memory before it
     float* u0;                  // [rows, heads, e]: the writes with an empty memory before
     float* within;              // [rows, heads, DCH_C]: what row t reads of the chunk's row s

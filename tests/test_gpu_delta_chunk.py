@@ -124,3 +124,31 @@ def test_a_row_takes_nothing_from_later_rows():
                         entry, ranges, one, 1, H, G, d, e, taps, d ** -0.5, 1e-6, longest, longest) for longest in (0, rows)]
     assert torch.isfinite(out[0][:75]).all() and not torch.isfinite(out[0][75:, 0, 3]).any()
     assert torch.equal(torch.isfinite(out[0]), torch.isfinite(out[1]))
+
+
+@pytest.mark.parametrize("decay", [0.0, -3.0, -6.0])
+def test_as_near_to_64_bit_as_the_scan(decay):
+    """The 2-norm of the error over memories that forget within a row, within a chunk and hardly at all (64-bit sums row by row)."""
+    from kapel_b200 import kernels as K
+
+    H, G, d, e, taps, rows = 8, 2, 128, 128, 4, 400
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)
+    n, nv = G * d, H * e
+    conv, a_log, dt_bias, x = rand(2 * n + nv, taps) * 0.5, rand(H) * 0.5 + decay, rand(H) * 0.5, rand(rows, 2 * n + nv + 2 * H)
+    entry = torch.zeros(rows, dtype=torch.int32, device="cuda")
+    one, ranges = torch.ones(1, dtype=torch.int32, device="cuda"), K.entry_ranges(entry, 1)
+    scan, chunks = (K.delta_scan(x, 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, conv, a_log, dt_bias, torch.zeros(2, K.delta_state_floats(H, G, d, e, taps), device="cuda"),
+                                 entry, ranges, one, 1, H, G, d, e, taps, d ** -0.5, 1e-6, longest, longest).double() for longest in (0, rows))
+    np64 = lambda t: t.double().cpu().numpy()
+    q, k, v, g, beta = (torch.as_tensor(np.asarray(t), device="cuda") for t in PK.delta_inputs(np64(x), np64(conv), np64(a_log), np64(dt_bias), H, G, d, e))
+    q, k = q.repeat_interleave(H // G, 1), k.repeat_interleave(H // G, 1)
+    S, want = torch.zeros(H, d, e, dtype=torch.float64, device="cuda"), []
+    for t in range(rows):
+        S = S * g[t][:, None, None]
+        S = S + k[t][:, :, None] * (beta[t][:, None] * (v[t] - torch.einsum("hde,hd->he", S, k[t])))[:, None, :]
+        want.append(torch.einsum("hde,hd->he", S, q[t]))
+    off = [float((o - torch.stack(want)).norm() / torch.stack(want).norm()) for o in (scan, chunks)]
+    # a warp's sums of four components a lane and a tree, against chains of eight to sixteen and pairs: some roundings more, 1.36 to 1.6 with
+    # chains over all components
+    assert off[1] <= 1.15 * off[0], off
