@@ -2,11 +2,12 @@
 // tcgen05.mma issued by one thread, operands staged in shared memory by TMA (cp.async.bulk.tensor,
 // 128-byte swizzle, no multicast), the 128 x 256 accumulator in tensor memory (TMEM), read back
 // with tcgen05.ld for the epilogue. Kapel's counterpart is the cutile `batched_matmul_nt`
-// (crates/kapel-cuda/src/tile.rs:65-87), which has no sm_100 path. Four kernels, below in this order:
-// one block a 128 x 256 tile (products of up to a wave and a half of tiles); persistent pairs of
+// (crates/kapel-cuda/src/tile.rs:65-87), which has no sm_100 path. Six kernels, below in this order:
+// one block a 128 x 256 tile (products of up to a wave and a half of tiles); the experts' products of prompts, the same over lists of
+// rows, and of decoding steps, operands swapped; persistent pairs of
 // blocks with cta_group::2 and two accumulators (all other products of more than 64 rows, also with
 // the gated unit in the epilogue); operands swapped for up to 64 rows, split over K; the same with
-// the gated unit; and, behind the first, the experts' forms of the first and the third, over lists of rows. Those for
+// the gated unit. Those for
 // up to 64 rows (decoding) are launched as programmatic dependents and wait for the
 // kernel before them only before they touch the activations; the others are launched plainly.
 //
@@ -1184,7 +1185,9 @@ extern "C" int kb_gemm_tcgen05(void* c, int c_dt, const void* a, const void* w, 
     // the pairs take in half as much a tile and the single blocks start sooner: pairs from K = 3,072 on (2,048 rows by 2,048 columns
     // 23.8 us against 26.6, 117 by 6,144 x 4,096 27.2 against 31.6), from 2,048 on where enough multiprocessors have a tile (2,048 by 2,304
     // 19.6 against 20.9, 500 by 3,104 18.3 against 19.3, by 2,048 17.4 against 16.5; bfloat16, whose epilogue is shorter: 2,048 by 2,304
-    // 19.3 against 19.6, 1,088 by 2,048 16.3 against 15.3), not below (K = 1,024, 500 rows by 2,048: 12.5 against 11.7).
+    // 19.3 against 19.6, 1,088 by 2,048 16.3 against 15.3), not below (K = 1,024, 500 rows by 2,048: 12.5 against 11.7). Over 14 weights of 1,024
+    // to 8,192 columns and 1,024 to 9,216 inputs by 117 to 2,048 rows in both result types the choice is within 6 % of the faster kernel but once
+    // (1,088 rows by 8,192 x 4,096, 288 tiles: 70 us, single blocks 60).
     if (kernel == 0) {
         const int sms = skinny_sms();
         const long long pair_tiles = ((m + 2 * TC_BM - 1) / (2 * TC_BM)) * (long long)grid.y;

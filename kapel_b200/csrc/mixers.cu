@@ -202,9 +202,7 @@ head_gate_wide_kernel(TO* __restrict__ out, const TY* __restrict__ y, const Src<
         for (int c = heads * e + threadIdx.x; c < fill_to; c += blockDim.x) Elem<TO>::store(out + (size_t)r * out_stride + c, 0.f);
 }
 
-// One block a row; a warp takes head vectors in turn (queries, then keys, then values) through a
-// piece of shared memory of its own.
-// The kernel below for prompts whose heads are 128 wide: a warp a (row, head of q, k or v), a lane four neighbouring components, the
+// Queries, keys and values of prompts whose heads are 128 wide, as the kernel behind this one has them for any size: a warp a (row, head of q, k or v), a lane four neighbouring components, the
 // rotation's partners by shuffles; the same roundings. 2,048 rows of 16 + 4 + 4 heads: 14 us against 31.
 template <typename TW, typename TO>
 __global__ void head_norm_rope_append_128_kernel(const float* __restrict__ src, int row_width, int q_off, int k_off, int v_off,
@@ -254,6 +252,8 @@ __global__ void head_norm_rope_append_128_kernel(const float* __restrict__ src, 
     store_four(dst + lane * 4, v);
 }
 
+// One block a row; a warp takes head vectors in turn (queries, then keys, then values) through a
+// piece of shared memory of its own.
 template <typename TS, typename TW, typename TO>
 __global__ void head_norm_rope_append_kernel(const Src<TS> src, int row_width, int q_off, int k_off, int v_off,
                                              const TW* __restrict__ wq, float eps_q, float off_q,

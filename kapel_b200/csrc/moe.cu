@@ -229,9 +229,6 @@ moe_route_kernel(const TH* __restrict__ h, const float* __restrict__ router, con
         }
 }
 
-// ------------------------------------------------------------------------------------------- sort
-constexpr int GM = 32;         // rows of a grouped product's tile: few rows an expert, and the 32-bit path
-constexpr int GM_LARGE = 64;   // and where an expert has many rows (bfloat16)
 // The router of prompts, without groups: a block takes ROUTE_ROWS rows, so the router's weights are read once for all of them (a block a row read
 // all of them again: 1,360 rows by 20 x 2,048 took 43 us, 30 like this). The same sums in the same order. A block takes 29 us
 // whatever the rows, a row a block 23 us up to 172 rows: eight rows a block from ROUTE_ROWS_FROM rows on.
@@ -276,6 +273,9 @@ moe_route_rows_kernel(const TH* __restrict__ h, const float* __restrict__ router
                       weights_out + (size_t)(first + warp) * top, n_experts, top, softmax, renormalize, scale);
 }
 
+// ------------------------------------------------------------------------------------------- sort
+constexpr int GM = 32;         // rows of a grouped product's tile: few rows an expert, and the 32-bit path
+constexpr int GM_LARGE = 64;   // and where an expert has many rows (bfloat16)
 constexpr int SORT_THREADS = 1024;
 
 // One block. offsets [E + 1]; order [pairs]: pair numbers by expert (any order within an expert);

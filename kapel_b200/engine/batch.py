@@ -93,7 +93,9 @@ def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: in
 # that starts among running ones costs 20 to 27 us before its first and after its last step, twice
 # what it costs in a launch of its own). The tcgen05 kernels' steps are short, so their fixed costs
 # weigh more and they are cut into slots only when a few tiles face a long history; "tcgen05_pair" is
-# the kernel on pairs of blocks (a tile of 256 rows on two multiprocessors, half the time a step).
+# the kernel on pairs of blocks (a tile of 256 rows on two multiprocessors, half the time a step). "flash", the kernel without a soft cap, has
+# the tcgen05 kernel's fixed costs and half its step, not fitted but measured after: of 48 shapes (128, 512 and 2,048 tokens behind 0 to 30,720, 8 to 32
+# heads of 64 and 128, with a window and without) the choice is the fastest split in 42 and within 7 us of it in the others.
 PROMPT_KERNEL_COSTS = {"mma": (0.5, 1.0, 4.5, 1), "flash": (18.0, 15.0, 0.6, 1), "tcgen05": (18.0, 15.0, 1.2, 1), "tcgen05_pair": (32.0, 18.0, 0.85, 2)}
 
 

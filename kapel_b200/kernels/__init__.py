@@ -1784,8 +1784,9 @@ class ExpertLists:
 
 
 # Rows an expert gets on average from which its products run on tcgen05 tiles of 128 rows: 272 rows an expert
-# took 77 + 52 us where the 64-row tiles of mma.sync took 145 + 145 and 23 for the unit between them; at 48 a tile is filled to three
-# eighths, which the five times faster products still pay for. Below, the tiles of 32 and 64 rows.
+# took 77 + 52 us where the 64-row tiles of mma.sync took 145 + 145 and 23 for the unit between them. At the line, 48 rows each of 16, 32 and 64 experts
+# (2,048 x 1,024 twice, 1,024 x 512), both products with sort and unit: 70, 98 and 71 us, the tiles below it 110, 147 and 99. They are ahead at 16 rows
+# an expert too (66, 91 and 65 against 86, 134 and 82, pairs spread evenly); the line leaves room for passes whose pairs are not.
 MOE_TCGEN05_ROWS = 48
 
 
