@@ -1186,7 +1186,7 @@ extern "C" int kb_gemm_tcgen05(void* c, int c_dt, const void* a, const void* w, 
     // 23.8 us against 26.6, 117 by 6,144 x 4,096 27.2 against 31.6), from 2,048 on where enough multiprocessors have a tile (2,048 by 2,304
     // 19.6 against 20.9, 500 by 3,104 18.3 against 19.3, by 2,048 17.4 against 16.5; bfloat16, whose epilogue is shorter: 2,048 by 2,304
     // 19.3 against 19.6, 1,088 by 2,048 16.3 against 15.3), not below (K = 1,024, 500 rows by 2,048: 12.5 against 11.7). Over 14 weights of 1,024
-    // to 8,192 columns and 1,024 to 9,216 inputs by 117 to 2,048 rows in both result types the choice is within 6 % of the faster kernel but once
+    // to 8,192 columns and 1,024 to 9,216 inputs by 300 to 2,048 rows in both result types the choice is within 6 % of the faster kernel but once
     // (1,088 rows by 8,192 x 4,096, 288 tiles: 70 us, single blocks 60).
     if (kernel == 0) {
         const int sms = skinny_sms();

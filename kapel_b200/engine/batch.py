@@ -73,8 +73,8 @@ def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: in
     tile, 64 a step, however few its rows: few tiles behind a long history leave the GPU idle, where the row-wise kernel has a block
     a row, kv head and 256 keys. Both as measured on a B200 for 16 to 1,024 tokens behind 0 to 16,384, groups of 1 to 16 heads of 128 and 256:
     a step 17.0 us (heads of 256) or 11.4 (of 128), a block a multiprocessor; a key 0.07 us + 1.45 ns a component + 0.06 us a head of the group,
-    7 (groups of 1) to 4 (of 8) blocks a multiprocessor. 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 139 and 407; 16 tokens
-    behind 256, 1,024 and 4,096 positions 86 and 145, 281 and 149, 1,062 and 219; 128 tokens behind 1,024 and 16,384 298 and 373, 4,219 and 5,675."""
+    7 (groups of 1) to 4 (of 8) blocks a multiprocessor. 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 146 and 391; 16 tokens
+    behind 256, 1,024 and 4,096 positions 89 and 145, 292 and 149, 1,101 and 219; 128 tokens behind 1,024 and 16,384 311 and 372, 4,374 and 5,685."""
     count = np.asarray(row_count, np.int64)
     row0 = np.asarray(tile_row0, np.int64)
     first, last = count[row0], count[row0 + np.asarray(tile_nq, np.int64) - 1]

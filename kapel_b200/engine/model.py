@@ -68,8 +68,8 @@ class ModelParts:
             rows = self._wanted_rows(batch, cache_manager)
         # The norm and the product of the wanted rows go by their own number: a few of a prompt's are its tail, behind a plainly launched
         # gather that every kernel over the prompt has ended before, so none of those overlaps with a dependent. A recorded
-        # pass that ends so replays with shorter gaps between all of its kernels (117 tokens at Gemma 2 2B sizes, 210 kernels: 2,449 us; with
-        # the norm, or both, launched plainly 2,526 and 2,537).
+        # pass that ends so mostly replays with shorter gaps between all of its kernels (117 tokens at Gemma 2 2B sizes, 210 kernels: 2,455 us in
+        # most processes, 2,530 in some; with the norm, or both, launched plainly 2,526 to 2,537 in all).
         return self.head.forward(self.final_norm.forward(rows))
 
     def _wanted_rows(self, batch, cache_manager) -> torch.Tensor:
