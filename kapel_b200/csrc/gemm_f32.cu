@@ -1,5 +1,6 @@
-// C[M,N] = A[M,K] . W[N,K]^T in true 32-bit: FFMA only, no tensor-core instruction, so nothing
-// rounds an input (the 32-bit path of the whole model; Kapel's f32 tiles: crates/kapel-cuda/src/tile.rs:196).
+// C[M,N] = A[M,K] . W[N,K]^T in true 32-bit (the 32-bit path of the whole model; Kapel's f32 tiles: crates/kapel-cuda/src/tile.rs:196). The
+// kernels of this file use multiply-adds only; `kb_gemm_f32_fast` hands what is large enough to those of gemm_f32_split.cu, which
+// cut every input into pieces that hold it exactly. Of the kernels of this file:
 //
 // Each output element is one accumulator that takes its K products in ascending k, whatever M
 // and N are, whichever kernel computes it and wherever the element lies in its tile: the result for
@@ -18,7 +19,7 @@
 //   dependent multiply-adds where N has few columns: 16 columns a block (2,304 columns are then 144 blocks for 148
 //   multiprocessors). Warps of their own copy, so that the others do nothing but multiply. One row by 18,432 x 2,304: 39 us (4.3
 //   TB/s; the tile kernel took 331), by 2,304 x 9,216: 33 us (780), where the chain alone is 19.
-#include "common.cuh"
+#include "gemm_f32_split.cuh"
 
 namespace kb {
 
@@ -307,5 +308,17 @@ extern "C" int kb_gemm_f32_variant(float* c, const float* a, const float* w, int
     return e ? e : check_launch("gemm_f32");
 }
 extern "C" int kb_gemm_f32(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, void* stream) {
+    return kb_gemm_f32_variant(c, a, w, m, n, k, epilogue, cap, -1, stream);
+}
+
+// The same by whatever is fastest, the tensor cores included. `scratch`: `kb_gemm_f32_scratch_floats` floats (0: none).
+extern "C" long long kb_gemm_f32_scratch_floats(const float* a, const float* w, int m, int n, int k) {
+    return m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(m, n, k, a, w) ? gemm_f32_pieces_floats(m, k) : 0;
+}
+extern "C" int kb_gemm_f32_fast(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, float* scratch, void* stream) {
+    if (m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(m, n, k, a, w)) {
+        KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
+        return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, gemm_f32_segments(m, n, k), scratch, (cudaStream_t)stream);
+    }
     return kb_gemm_f32_variant(c, a, w, m, n, k, epilogue, cap, -1, stream);
 }

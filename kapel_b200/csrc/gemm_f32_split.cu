@@ -1,0 +1,426 @@
+// C[M,N] = A[M,K] . W[N,K]^T of 32-bit values on the fifth-generation tensor cores, with no less precision than a chain of 32-bit
+// multiply-adds: every input is cut into three bfloat16 pieces (pieces.cuh) and of the nine products of pieces the six that matter are added up,
+//     w3 a1 + w1 a3 + w2 a2 + w2 a1 + w1 a2 + w1 a1        (in this order, the small ones first).
+// The tensor cores add in 32 bits but round towards zero, so a long sum must not be theirs: an accumulator in tensor memory takes one
+// chunk of 64 k, of which only the last four additions are to a sum of full size, and the chunks are added up in registers, rounded to
+// nearest.
+//
+// The operands are swapped, 128 weight rows are the MMA's M and 16, 32, 64 or 128 rows of A its N, for a handful of rows and for thousands
+// alike: an element's products and additions are the same in all of them. Where the tiles are too few, K is cut into segments, a block each in a
+// cluster of up to eight, which add up their sums through shared memory in the segments' order.
+//
+// Twenty warps:
+//   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep, as 32-bit values (and of up to 32 rows of A)
+//   warps 3-10    cut the weights, each half of them every second stage: a thread has a row, its pieces go to tensor memory, from where the
+//                 MMA takes its A operand
+//   warps 1, 2    issue the 24 MMAs of a chunk, one the even chunks, the other the odd ones (issuing takes a thread longer than the tensor
+//                 cores need for a small product; each chunk has pieces and an accumulator of its own)
+//   warp 19       asks TMA for the pieces of A, the MMA's B operand, which a kernel ahead of this one has cut: every block of a row of
+//                 tiles needs them. Up to 32 rows are cut here instead, by warps 11-14, which saves that launch
+//   warps 11-18   (15-18) add a finished chunk to the sums they hold in registers, and store them at the end
+//
+// Values that are no finite numbers (and those that round to infinity in bfloat16) have no pieces: infinity less infinity is NaN. A
+// row that holds one is noticed when it is cut, and its elements are computed again by multiply-adds, as the other kernels do.
+// Every wait gives up after about a second, raises a flag that `kb_gemm_f32_split_error` reports, and the block still meets at its
+// barriers, frees its TMEM and returns.
+#include "attention_tc.cuh"
+#include "gemm_f32_split.cuh"
+#include "pieces.cuh"
+#include "tensor_map.cuh"
+
+namespace kb {
+
+__device__ int g_gemm_f32_split_error = 0;
+
+constexpr int FP_M = 128, FP_K = 64, FP_STAGE_K = 32, FP_THREADS = 20 * 32;
+constexpr int FP_WARP_W = 3, FP_WARP_A = 11, FP_WARP_PIECES = 19;
+constexpr int FP_CUT_ROWS = 32;                                    // up to so many rows of A are cut by the block that needs them
+
+template <int NP> struct Pieces {
+    static constexpr bool CUTS = NP <= FP_CUT_ROWS;
+    static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
+    static constexpr int STAGES = 8;
+    static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
+    static constexpr int SMEM = STAGES * STAGE + 2 * PIECES + 1024 /* alignment */ + 512 /* barriers, rows that are not finite */;
+    static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, TMEM_COLS = COL_W + 192 <= 256 ? 256 : 512;
+    static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
+    static_assert(SMEM <= 232448, "more shared memory than a block can have");
+    static_assert(STAGES * STAGE >= NP * FP_M * 4, "the sums take the stages' place");
+};
+
+__device__ __forceinline__ void fp_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                   "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr) : "memory");
+}
+
+// `odd` becomes NaN when one of the two values has no pieces.
+__device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t& two, uint32_t& three, float& odd) {
+    cut_pair(x, y, one, two, three);
+    odd = fmaf(x, y, odd);
+}
+
+__device__ __forceinline__ void fp_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// epilogue 0: none; 1: cap * tanh(acc / cap)
+template <int NP, int EPI>
+__global__ void __launch_bounds__(FP_THREADS, 1)
+gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ c,
+                       const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ a_odd, int m, int n, int k, int chunks_a_segment, float cap) {
+    // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]; a_odd then says which rows have none
+    using C = Pieces<NP>;
+    extern __shared__ unsigned char fp_raw[];
+    unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)fp_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* pieces = smem + C::STAGES * C::STAGE;           // [2][3][NP rows][128 bytes]
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + 2 * C::PIECES);
+    uint64_t* empty = full + C::STAGES;                            // the warps that cut it have read the stage
+    uint64_t* cut = empty + C::STAGES;                             // [2] a chunk's pieces are there that are cut here
+    uint64_t* a_full = cut + 2;                                    // [2] its pieces of A that are not
+    uint64_t* done = a_full + 2;                                   // [2] a chunk's products are complete: its pieces' place is free, its sum there
+    uint64_t* added = done + 2;                                    // [2] the sum has been read
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(added + 2);
+    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 224;      // [128] of W, [NP] of A
+    int* any_odd = reinterpret_cast<int*>(tmem_slot + 1);
+    static_assert((2 * C::STAGES + 8) * 8 + 8 <= 224, "the barriers outgrew their room");
+
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int m0 = blockIdx.x * NP, n0 = blockIdx.y * FP_M, segment = blockIdx.z, segments = gridDim.z;
+    const int chunks_all = (k + FP_K - 1) / FP_K;
+    const int chunk0 = segment * chunks_a_segment, chunks = max(0, min(chunks_a_segment, chunks_all - chunk0));
+
+    if (tid == 0) {
+        for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 8 : 4); }
+        for (int b = 0; b < 2; ++b) {
+            at_mbar_init(cut + b, C::CUTS ? 12 : 8);
+            at_mbar_init(a_full + b, 1);
+            at_mbar_init(done + b, 1);
+            at_mbar_init(added + b, C::CUTS ? 4 : 8);
+        }
+        *any_odd = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (tid < FP_M + NP) odd_rows[tid] = 0;
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_saddr(tmem_slot)), "r"(C::TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    at_fence_before();
+    __syncthreads();
+    at_fence_after();
+    const uint32_t tmem = *tmem_slot;
+    bool failed = false;
+    constexpr int COLS = C::COLS;
+    float sum[COLS];
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int it = 0;
+            for (; it < 2 * chunks; ++it) {
+                const int s = it % C::STAGES;
+                if (!at_mbar_wait(empty + s, ((uint32_t)(it / C::STAGES) & 1u) ^ 1u)) { failed = true; break; }
+                const uint32_t dst = at_saddr(smem + s * C::STAGE);
+                at_mbar_expect_tx(full + s, C::STAGE);
+                at_tma_box(dst, &map_w, chunk0 * FP_K + it * FP_STAGE_K, n0, full + s);
+                if (C::CUTS) at_tma_box(dst + C::W_BYTES, &map_a, chunk0 * FP_K + it * FP_STAGE_K, m0, full + s);
+            }
+            if (failed)                                            // the copies in flight land before the block goes on
+                for (int i = max(0, it - C::STAGES); i < it; ++i) at_mbar_wait(full + i % C::STAGES, (uint32_t)(i / C::STAGES) & 1u);
+        }
+    } else if (warp < FP_WARP_W) {
+        // ---------------------------------------------------------------- the products of every second chunk, from one lane
+        if (lane == 0) {
+            constexpr uint32_t IDESC = at_idesc(FP_M, NP, false);
+            const int b = warp - 1;
+            for (int ch = b; ch < chunks; ch += 2) {
+                if (!at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u)) { failed = true; break; }
+                if (!C::CUTS && !at_mbar_wait(a_full + b, (uint32_t)(ch >> 1) & 1u)) { failed = true; break; }
+                if (!at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
+                at_fence_after();
+                const uint32_t d = tmem + (uint32_t)(b * C::ACC), aw = tmem + (uint32_t)(C::COL_W + b * 96);
+                const uint64_t ba = at_desc(at_saddr(pieces + b * C::PIECES), 16, 1024);
+#pragma unroll
+                for (int p = 0; p < PIECE_PRODUCTS; ++p)
+#pragma unroll
+                    for (int kk = 0; kk < FP_K / 16; ++kk)
+                        at_mma_ts(d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
+                at_commit(done + b);
+            }
+        }
+    } else if (warp < FP_WARP_A) {
+        // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
+        const int quarter = warp & 3, half = (warp - FP_WARP_W) >> 2;      // of the TMEM lanes, which are the weight rows; of the chunk
+        const int row = quarter * 32 + lane;
+        float odd = 0.f;
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
+            const unsigned char* from = smem + s * C::STAGE + row * 128;
+            uint32_t one[16], two[16], three[16];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                const float4 x = *reinterpret_cast<const float4*>(from + ((j ^ (row & 7)) << 4));
+                fp_cut(x.x, x.y, one[2 * j], two[2 * j], three[2 * j], odd);
+                fp_cut(x.z, x.w, one[2 * j + 1], two[2 * j + 1], three[2 * j + 1], odd);
+            }
+            __syncwarp();
+            if (lane == 0) at_mbar_arrive(empty + s);
+            // the chunk two before this one was the last to lie here
+            if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u))) { failed = true; break; }
+            at_fence_after();
+            const uint32_t to = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(C::COL_W + b * 96 + half * 16);
+            at_st16(to, one);
+            at_st16(to + 32, two);
+            at_st16(to + 64, three);
+            asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+            at_fence_before();
+            __syncwarp();
+            if (lane == 0) at_mbar_arrive(cut + b);
+        }
+        if (odd != odd) odd_rows[row] = 1, *any_odd = 1;
+    } else if (C::CUTS && warp < C::WARP_SUM) {
+        // ---------------------------------------------------------------- cutting a few rows of A
+        const int t = (warp - FP_WARP_A) * 32 + lane, row = t % NP;
+        float odd = 0.f;
+        for (int it = 0; it < 2 * chunks; ++it) {
+            const int s = it % C::STAGES, ch = it >> 1, b = ch & 1, half = it & 1;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
+            if (half == 0 && !__all_sync(0xffffffffu, at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u))) { failed = true; break; }
+            const unsigned char* from = smem + s * C::STAGE + C::W_BYTES + row * 128;
+            unsigned char* to = pieces + b * C::PIECES + row * 128;
+            for (int i = t; i < NP * 4; i += 128) {                // eight values at a time
+                const int g = i / NP;
+                const float4 x = *reinterpret_cast<const float4*>(from + (((2 * g) ^ (row & 7)) << 4));
+                const float4 y = *reinterpret_cast<const float4*>(from + (((2 * g + 1) ^ (row & 7)) << 4));
+                uint4 one, two, three;
+                fp_cut(x.x, x.y, one.x, two.x, three.x, odd);
+                fp_cut(x.z, x.w, one.y, two.y, three.y, odd);
+                fp_cut(y.x, y.y, one.z, two.z, three.z, odd);
+                fp_cut(y.z, y.w, one.w, two.w, three.w, odd);
+                const int at = ((half * 4 + g) ^ (row & 7)) << 4;
+                *reinterpret_cast<uint4*>(to + at) = one;
+                *reinterpret_cast<uint4*>(to + C::PIECE + at) = two;
+                *reinterpret_cast<uint4*>(to + 2 * C::PIECE + at) = three;
+            }
+            if (half == 1) at_fence_async_smem();                  // the MMAs read what was written here
+            __syncwarp();
+            if (lane == 0) {
+                at_mbar_arrive(empty + s);
+                if (half == 1) at_mbar_arrive(cut + b);
+            }
+        }
+        if (odd != odd) odd_rows[FP_M + row] = 1, *any_odd = 1;
+    } else if (warp == FP_WARP_PIECES) {
+        if (!C::CUTS) {
+            // ------------------------------------------------------------ A's pieces, and which of its rows have none
+            if (lane == 0) {
+                int ch = 0;
+                for (; ch < chunks; ++ch) {
+                    const int b = ch & 1;
+                    if (!at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
+                    at_mbar_expect_tx(a_full + b, C::PIECES);
+                    for (int p = 0; p < 3; ++p)
+                        at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch) * FP_K, p * m + m0, a_full + b);
+                }
+                if (failed)
+                    for (int i = max(0, ch - 2); i < ch; ++i) at_mbar_wait(a_full + (i & 1), (uint32_t)(i >> 1) & 1u);
+            }
+            __syncwarp();
+            for (int j = lane; j < NP && m0 + j < m; j += 32)
+                if (a_odd[m0 + j] != 0) odd_rows[FP_M + j] = 1, *any_odd = 1;
+        }
+    } else {
+        // ---------------------------------------------------------------- adding up: a weight row and COLS of A's rows a thread
+        const int quarter = warp & 3, half = (warp - C::WARP_SUM) >> 2;
+        const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * COLS);
+#pragma unroll
+        for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int b = ch & 1;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, (uint32_t)(ch >> 1) & 1u))) { failed = true; break; }
+            at_fence_after();
+#pragma unroll
+            for (int c0 = 0; c0 < COLS; c0 += 16) {
+                uint32_t r[16];
+                fp_ld16(lanes + (uint32_t)(b * C::ACC + c0), r);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (c0 + 16 == COLS) {
+                    at_fence_before();
+                    __syncwarp();
+                    if (lane == 0) at_mbar_arrive(added + b);
+                }
+#pragma unroll
+                for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+            }
+        }
+    }
+    __syncthreads();                                               // the stages have been read, the rows that are not finite are marked
+    float* sums = reinterpret_cast<float*>(smem);                  // [NP][128], where K is cut
+    if (warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
+        const int r = (warp & 3) * 32 + lane, j0 = ((warp - C::WARP_SUM) >> 2) * COLS;
+        if (segments == 1) {
+            if (n0 + r < n)
+#pragma unroll
+                for (int j = 0; j < COLS; ++j) {
+                    float v = sum[j];
+                    if (EPI == 1) v = cap * tanhf(v / cap);
+                    if (m0 + j0 + j < m) c[(size_t)(m0 + j0 + j) * n + n0 + r] = v;
+                }
+        } else {
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) sums[(j0 + j) * FP_M + r] = sum[j];
+        }
+        if (*any_odd != 0 && n0 + r < n) {                         // this thread's elements of rows without pieces again
+            const int k0 = chunk0 * FP_K, k1 = min(k, (chunk0 + chunks) * FP_K);
+#pragma unroll 1
+            for (int j = j0; j < min(j0 + COLS, m - m0); ++j) {
+                if ((odd_rows[r] | odd_rows[FP_M + j]) == 0) continue;
+                const float *x = a + (size_t)(m0 + j) * k, *y = w + (size_t)(n0 + r) * k;
+                float v = 0.f;
+#pragma unroll 1
+                for (int kk = k0; kk < k1; ++kk) v = fmaf(x[kk], y[kk], v);
+                if (segments > 1) sums[j * FP_M + r] = v;
+                else c[(size_t)(m0 + j) * n + n0 + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
+            }
+        }
+    }
+    if (segments > 1) {
+        fp_cluster_sync();
+        const int per = NP / segments;                             // rows of A this block adds up
+        for (int i = tid; i < per * FP_M; i += FP_THREADS) {
+            const int j = segment * per + i / FP_M, r = i % FP_M;
+            const uint32_t at = at_saddr(sums + j * FP_M + r);
+            float v = 0.f;
+            for (int s = 0; s < segments; ++s) {
+                float x;
+                asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
+                             : "=f"(x) : "r"(at), "r"(s) : "memory");
+                v = s == 0 ? x : v + x;
+            }
+            if (EPI == 1) v = cap * tanhf(v / cap);
+            if (m0 + j < m && n0 + r < n) c[(size_t)(m0 + j) * n + n0 + r] = v;
+        }
+        fp_cluster_sync();                                         // nobody leaves while its sums are read
+    }
+    if (failed) atomicExch(&g_gemm_f32_split_error, 1);
+    at_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        at_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(C::TMEM_COLS) : "memory");
+    }
+}
+
+// A's rows cut for a product of more than FP_CUT_ROWS: pieces [3, m, kp], kp the next multiple of 8 (the columns beyond k are zeros), and
+// whether a row has none. A block a row.
+__global__ void __launch_bounds__(256)
+f32_cut_rows_kernel(const float* __restrict__ a, uint32_t* __restrict__ pieces, int* __restrict__ odd_rows, int m, int k, int kp) {
+    const int row = blockIdx.x;
+    const float* from = a + (size_t)row * k;
+    uint32_t* to = pieces + (size_t)row * (kp / 2);
+    const size_t piece = (size_t)m * (kp / 2);
+    float odd = 0.f;
+    for (int x = threadIdx.x * 4; x < kp; x += 1024) {             // k is a multiple of four
+        const float4 v = x < k ? *reinterpret_cast<const float4*>(from + x) : make_float4(0.f, 0.f, 0.f, 0.f);
+        uint2 one, two, three;
+        fp_cut(v.x, v.y, one.x, two.x, three.x, odd);
+        fp_cut(v.z, v.w, one.y, two.y, three.y, odd);
+        *reinterpret_cast<uint2*>(to + x / 2) = one;
+        *reinterpret_cast<uint2*>(to + piece + x / 2) = two;
+        *reinterpret_cast<uint2*>(to + 2 * piece + x / 2) = three;
+    }
+    const int any = __syncthreads_or(odd != odd);
+    if (threadIdx.x == 0) odd_rows[row] = any;
+}
+
+template <int NP, int EPI>
+static int launch_pieces(float* c, const float* a, const float* w, int m, int n, int k, int segments, float cap, float* scratch, cudaStream_t s) {
+    using C = Pieces<NP>;
+    CUtensorMap map_a, map_w;
+    const int kp = (k + 7) & ~7;
+    int* odd_rows = nullptr;
+    KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535, "gemm_f32: a weight of %d rows is too much for one launch", n);
+    if (cudaFuncSetAttribute(gemm_f32_pieces_kernel<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+        return fail("gemm_f32: cannot have %d bytes of shared memory", C::SMEM);
+    if (int e = encode_map_f32(&map_w, w, n, k, k, FP_M)) return e;
+    if (C::CUTS) {
+        if (int e = encode_map_f32(&map_a, a, m, k, k, NP)) return e;
+    } else {
+        KB_REQUIRE(scratch != nullptr && ((uintptr_t)scratch & 15) == 0, "gemm_f32: %d rows by pieces without scratch", m);
+        odd_rows = reinterpret_cast<int*>(scratch) + (size_t)3 * m * (kp / 2);
+        if (int e = encode_map_bf16(&map_a, scratch, 3ull * m, kp, kp, NP)) return e;
+        f32_cut_rows_kernel<<<m, 256, 0, s>>>(a, reinterpret_cast<uint32_t*>(scratch), odd_rows, m, k, kp);
+        if (int e = check_launch("gemm_f32 cut")) return e;
+    }
+    const int chunks = (k + FP_K - 1) / FP_K;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((m + NP - 1) / NP, (n + FP_M - 1) / FP_M, segments);
+    cfg.blockDim = FP_THREADS;
+    cfg.dynamicSmemBytes = C::SMEM;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = segments;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, gemm_f32_pieces_kernel<NP, EPI>, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap);
+    return check_launch("gemm_f32 pieces");
+}
+
+// Segments of K: the waves of blocks times what a block takes, a chunk 0.85 us with up to 32 rows, 1.1 with 64, 1.5 with 128, and 6 or (in a
+// cluster) 8 us to begin and end. A block takes a multiprocessor; clusters of four and eight do not fit every group of them, so that seven
+// eighths and three quarters run at once (144 blocks in clusters of eight: two waves). Of 95 sizes (512 to 18,432 weight rows of 1,024 to 9,216, 1
+// to 500 rows) the choice is the fastest of the four in all, or within 3 % of it.
+int gemm_f32_segments(int m, int n, int k) {
+    const int tiles = ((m + 127) / 128) * ((n + FP_M - 1) / FP_M), chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
+    const double chunk_us = m > 64 ? 1.5 : m > 32 ? 1.12 : 0.85;
+    int best = 1;
+    double least = 0;
+    for (int s = 1; s <= 8 && s <= chunks; s *= 2) {
+        const int at_once = s <= 2 ? sms : (s == 4 ? sms * 7 / 8 : sms * 3 / 4) / s * s;
+        const double us = (double)((tiles * s + at_once - 1) / at_once) * ((chunks + s - 1) / s * chunk_us + (s == 1 ? 6.0 : 8.0));
+        if (s == 1 || us < least) least = us, best = s;
+    }
+    return best;
+}
+// From 512 weight rows of 1,024 on and more than two rows: one accumulator an element in ascending k, a kernel for each, is limited by
+// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 32. One row stays with the chains (18,432 x
+// 2,304: 37 us by chains, 39 by pieces; 2,304 x 9,216: 32 and 39), four go either way (44 and 39, 51 and 39) as long as the tiles are one
+// wave (256,000 x 2,304: 440 and 500), six and more go by pieces (54 and 39, 72 and 39, 639 and 499), 500 rows far ahead: 824 and 223, 545 and 122, by 2,304 x
+// 2,048 131 and 35, by 512 x 1,024 32 and 15. The error against 64 bits is 0.07 to 0.2 of the chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6).
+bool gemm_f32_pieces_take(int m, int n, int k, const void* a, const void* w) {
+    return (m > 4 || (m > 2 && n <= FP_M * multiprocessors())) && n >= 512 && k >= 1024 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
+}
+long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * (3 * ((k + 7) / 8 * 4) + 1); }
+
+int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, cudaStream_t s) {
+    KB_REQUIRE(k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0, "gemm_f32: rows of %d values must begin at 16-byte boundaries", k);
+    KB_REQUIRE(segments == 1 || segments == 2 || segments == 4 || segments == 8, "gemm_f32: %d segments", segments);
+#define KB_PIECES(NP) \
+    return epilogue == 0 ? launch_pieces<NP, 0>(c, a, w, m, n, k, segments, cap, scratch, s) : launch_pieces<NP, 1>(c, a, w, m, n, k, segments, cap, scratch, s)
+    if (m <= 16) KB_PIECES(16);
+    if (m <= 32) KB_PIECES(32);
+    if (m <= 64) KB_PIECES(64);
+    KB_PIECES(128);
+#undef KB_PIECES
+}
+
+}  // namespace kb
+
+using namespace kb;
+
+extern "C" int kb_gemm_f32_split_error() {
+    int flag = 0, zero = 0;
+    if (cudaMemcpyFromSymbol(&flag, g_gemm_f32_split_error, sizeof(int)) != cudaSuccess) return -1;
+    if (flag) cudaMemcpyToSymbol(g_gemm_f32_split_error, &zero, sizeof(int));
+    return flag;
+}
+// The kernel over pieces whatever the sizes, with `segments` blocks to K (0: as the rule has it).
+extern "C" int kb_gemm_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, void* stream) {
+    KB_REQUIRE(m >= 0 && n > 0 && k > 0, "gemm_f32: m %d, n %d, k %d", m, n, k);
+    KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
+    if (m == 0) return 0;
+    return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, segments > 0 ? segments : gemm_f32_segments(m, n, k), scratch, (cudaStream_t)stream);
+}

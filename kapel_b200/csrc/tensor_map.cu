@@ -39,20 +39,30 @@ int encode_map_bf16_chunks(CUtensorMap* map, const void* base, unsigned long lon
     return 0;
 }
 
-int encode_map_bf16(CUtensorMap* map, const void* base, unsigned long long rows, unsigned long long cols,
-                    unsigned long long pitch_elems, unsigned box_rows) {
+static int encode_rows(CUtensorMap* map, CUtensorMapDataType type, unsigned bytes, const void* base, unsigned long long rows, unsigned long long cols,
+                       unsigned long long pitch_elems, unsigned box_rows) {
     if (int e = find_encoder()) return e;
-    if (((uintptr_t)base & 15) != 0 || (pitch_elems * 2) % 16 != 0)
-        return fail("tensor map: base %p and row pitch %llu bytes must be multiples of 16", base, pitch_elems * 2);
+    if (((uintptr_t)base & 15) != 0 || (pitch_elems * bytes) % 16 != 0)
+        return fail("tensor map: base %p and row pitch %llu bytes must be multiples of 16", base, pitch_elems * bytes);
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)pitch_elems * 2};
-    const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)pitch_elems * bytes};
+    const cuuint32_t box[2] = {128u / bytes, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
-    const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
+    const CUresult r = g_encode(map, type, 2, const_cast<void*>(base), dims, strides, box, elem,
                                 CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                 CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail("tensor map: cuTensorMapEncodeTiled failed with code %d for [%llu, %llu]", (int)r, rows, cols);
     return 0;
+}
+
+int encode_map_bf16(CUtensorMap* map, const void* base, unsigned long long rows, unsigned long long cols,
+                    unsigned long long pitch_elems, unsigned box_rows) {
+    return encode_rows(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, base, rows, cols, pitch_elems, box_rows);
+}
+
+int encode_map_f32(CUtensorMap* map, const void* base, unsigned long long rows, unsigned long long cols, unsigned long long pitch_elems,
+                   unsigned box_rows) {
+    return encode_rows(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, rows, cols, pitch_elems, box_rows);
 }
 
 }  // namespace kb

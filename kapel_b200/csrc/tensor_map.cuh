@@ -1,4 +1,4 @@
-// TMA tensor maps over row-major bfloat16 matrices, shared by the kernels that load through them.
+// TMA tensor maps over row-major matrices, shared by the kernels that load through them.
 #pragma once
 #include <cuda.h>
 
@@ -9,6 +9,10 @@ namespace kb {
 // as zero. Returns 0, or 1 after storing a message.
 int encode_map_bf16(CUtensorMap* map, const void* base, unsigned long long rows, unsigned long long cols,
                     unsigned long long pitch_elems, unsigned box_rows);
+
+// The same over float32, in boxes of box_rows x 32 elements (128 bytes); the row pitch a multiple of four elements.
+int encode_map_f32(CUtensorMap* map, const void* base, unsigned long long rows, unsigned long long cols, unsigned long long pitch_elems,
+                   unsigned box_rows);
 
 // A dense [rows, cols] bfloat16 matrix (cols a multiple of 64) seen as three dimensions: 64 elements,
 // rows, chunks of 64 columns. A box of box_rows rows lands in shared memory chunk by chunk:

@@ -63,7 +63,7 @@ def library():
                 lib = ctypes.CDLL(str(path))
                 lib.kb_last_error.restype = ctypes.c_char_p
                 for name in ("kb_gemm_bf16_scratch_floats", "kb_paged_attention_scratch_floats", "kb_attention_mma_scratch_floats", "kb_sample_scratch_floats",
-                             "kb_mlstm_state_floats", "kb_delta_state_floats", "kb_delta_scratch_floats", "kb_delta_chunk_floats", "kb_pooled_attention_scratch_floats",
+                             "kb_mlstm_state_floats", "kb_delta_state_floats", "kb_delta_scratch_floats", "kb_delta_chunk_floats", "kb_gemm_f32_scratch_floats", "kb_pooled_attention_scratch_floats",
                              "kb_pooled_attention_mma_scratch_floats", "kb_pooled_attention_mma_kept_floats", "kb_decay_scan_scratch_floats",
                              "kb_retention_scratch_floats"):
                     getattr(lib, name).restype = ctypes.c_longlong
@@ -89,6 +89,8 @@ def check_async_errors() -> None:
         bad.append("tcgen05 attention (a TMA load, an MMA commit or a softmax warp never arrived)")
     if lib.kb_attention_flash_error() != 0:
         bad.append("tcgen05 attention without a soft cap (a TMA load, an MMA commit or a softmax warp never arrived)")
+    if lib.kb_gemm_f32_split_error() != 0:
+        bad.append("32-bit product (a TMA load, an MMA commit or a warp of the block never arrived)")
     if lib.kb_rope_error() != 0:
         bad.append("rotate and append (a bulk copy of partial sums into shared memory never completed)")
     if lib.kb_norm_error() != 0:
@@ -572,7 +574,9 @@ def gemm(a: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = No
     lib = library()
     if a.dtype == torch.float32:
         out = _fresh((m, n), torch.float32, a.device)
-        _check(lib.kb_gemm_f32(_ptr(out), _ptr(a), _ptr(w), m, n, k, epi, _f(cap), _stream()))
+        need = int(lib.kb_gemm_f32_scratch_floats(_ptr(a), _ptr(w), m, n, k))
+        scratch = _fresh((need,), torch.float32, a.device) if need else None
+        _check(lib.kb_gemm_f32_fast(_ptr(out), _ptr(a), _ptr(w), m, n, k, epi, _f(cap), _ptr(scratch), _stream()))
         if out_dtype is not None and out_dtype != torch.float32:
             out = cast(out, out_dtype)
         return out
