@@ -448,7 +448,9 @@ extern "C" long long kb_delta_scratch_floats(int rows, int heads, int kv_heads, 
 }
 
 // Floats of scratch that `rows` rows take on the way by chunks (`kb_delta_scan`'s `chunk_scratch`).
-extern "C" long long kb_delta_chunk_floats(int rows, int heads, int d, int e) { return (long long)rows * heads * (d + e + DCH_C + 2); }
+extern "C" long long kb_delta_chunk_floats(int rows, int entries, int heads, int kv_heads, int d, int e) {
+    return delta_chunk_floats(rows, entries, heads, kv_heads, d, e);
+}
 
 // Whether long portions of these sizes can go by chunks.
 extern "C" int kb_delta_chunks_take(int d, int e) { return delta_chunks_take(d, e) ? 1 : 0; }
@@ -522,14 +524,10 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     if (by_chunks) {
         DeltaChunks c;
         c.qn = p.qn; c.kn = p.kn; c.vn = p.vn; c.scal = p.scal; c.kq = p.kq;
-        c.w = chunk_scratch;
-        c.u0 = c.w + (size_t)rows * heads * d;
-        c.within = c.u0 + (size_t)rows * nv;
-        c.fade = c.within + (size_t)rows * heads * DCH_C;
         c.state = state; c.state_floats = state_floats; c.state_off = (long long)(taps - 1) * channels;
         c.entry_start = entry_start; c.entry_end = entry_end; c.slots = slots; c.n_slots = n_slots; c.entries = entries;
         c.heads = heads; c.kv_heads = kv_heads; c.d = d; c.e = e; c.from_rows = chunk_rows; c.out = out;
-        if (int err = launch_delta_chunks(c, longest, s)) return err;
+        if (int err = launch_delta_chunks(c, chunk_scratch, rows, longest, s)) return err;
         if (shortest >= chunk_rows) return 0;                   // nobody is left for the scan
     }
     // columns a warp: the most that still gives the GPU about eight warps a multiprocessor (a prompt of one request has

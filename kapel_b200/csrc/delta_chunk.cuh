@@ -5,6 +5,13 @@
 namespace kb {
 
 constexpr int DCH_C = 32;              // rows a chunk
+constexpr int DCH_LD_W = DCH_C + 4;    // a row of 32 weights, and four more so that rows begin in different banks
+constexpr int DCH_G = DCH_C * DCH_LD_W, DCH_F = DCH_G + DCH_C, DCH_ALL = DCH_F + DCH_C, DCH_WITHIN = DCH_ALL + 4;      // the decays' places behind them
+
+// Where a chunk's inputs lie: the chunk of request `entry` that begins at row `first`. Requests of a step follow one another, so every
+// chunk has a place of its own below rows / 32 + entries.
+__host__ __device__ inline int delta_chunk_place(int first, int entry) { return first / DCH_C + entry; }
+__host__ __device__ inline int delta_piece_row(int d) { return 3 * d + 8; }             // 8 more: eight rows begin in different banks
 
 struct DeltaChunks {
     const float* qn;            // [rows, kv_heads, d] unit queries times the query scale
@@ -12,10 +19,12 @@ struct DeltaChunks {
     const float* vn;            // [rows, heads, e]
     const float* scal;          // [rows, heads, 2] decay, step size
     const float* kq;            // [rows, kv_heads] a row's key times its query
-    float* w;                   // [rows, heads, d]: what a chunk's writes owe to the memory before it
-    float* u0;                  // [rows, heads, e]: the writes with an empty memory before
-    float* within;              // [rows, heads, DCH_C]: what row t reads of the chunk's row s
-    float* fade;                // [rows, heads, 2]: decay from the chunk's start to the row, from the row to the chunk's end
+    // A chunk's inputs to the chain as they lie in its shared memory, chunk by chunk (`delta_chunk_place`); rows beyond the last are zeros.
+    __nv_bfloat16* w;           // [places, heads, DCH_C, 3 d + 8]: what a row's write owes to the memory before the chunk, in three pieces of d
+    __nv_bfloat16* qk;          // [places, kv_heads, 2, DCH_C, 3 d + 8]: unit queries times their scale, then unit keys, likewise
+    float* within;              // [places, heads, DCH_WITHIN]: what row t reads of the chunk's row s, [DCH_C][DCH_LD_W]; then the decays from the
+                                // chunk's start to the rows, from the rows to its end, over the whole chunk
+    float* u0;                  // [places, heads, e, DCH_LD_W]: the writes with an empty memory before, by component
     float* state;               // [slots, state_floats], a head's memory [e, d] at state_off + head e d
     long long state_floats, state_off;
     const int* entry_start;
@@ -27,7 +36,10 @@ struct DeltaChunks {
 
 // Whether the chunk kernels take these sizes.
 bool delta_chunks_take(int d, int e);
+// Floats of scratch for a step of `rows` rows.
+long long delta_chunk_floats(int rows, int entries, int heads, int kv_heads, int d, int e);
 // Requests that bring at least p.from_rows rows, `longest` being the most any brings.
-int launch_delta_chunks(const DeltaChunks& p, int longest, cudaStream_t s);
+// The inputs' places are taken from `scratch`.
+int launch_delta_chunks(DeltaChunks p, float* scratch, int rows, int longest, cudaStream_t s);
 
 }  // namespace kb

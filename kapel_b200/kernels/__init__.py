@@ -91,6 +91,8 @@ def check_async_errors() -> None:
         bad.append("tcgen05 attention without a soft cap (a TMA load, an MMA commit or a softmax warp never arrived)")
     if lib.kb_gemm_f32_split_error() != 0:
         bad.append("32-bit product (a TMA load, an MMA commit or a warp of the block never arrived)")
+    if lib.kb_delta_chain_error() != 0:
+        bad.append("the delta rule's chain over chunks (a bulk copy into shared memory never completed)")
     if lib.kb_rope_error() != 0:
         bad.append("rotate and append (a bulk copy of partial sums into shared memory never completed)")
     if lib.kb_norm_error() != 0:
@@ -1191,9 +1193,9 @@ def delta_columns_per_warp(n: int = 0) -> None:
 
 
 # The delta rule goes by chunks of 32 rows instead of row by row where some request brings DELTA_CHUNK_LONGEST rows: a row of the scan takes
-# 0.33 us, a chunk 3.9 and the launch ahead of the chain 35 (100 rows of 16 heads of 128: 35 us row by row, 53 by chunks). Then every
-# request of DELTA_CHUNK_ROWS rows goes that way, side by side with the longest.
-DELTA_CHUNK_ROWS, DELTA_CHUNK_LONGEST = 64, 192
+# 0.33 us, a chunk 1.65 and the launch ahead of the chain 14 (16 heads of 128: 64 rows 24 us row by row, 21 by chunks; 100 rows 34 and 24, 192 rows 63
+# and 27). Then every request of DELTA_CHUNK_ROWS rows goes that way, side by side with the longest.
+DELTA_CHUNK_ROWS, DELTA_CHUNK_LONGEST = 64, 64
 
 
 def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: int, conv: torch.Tensor, a_log: torch.Tensor,
@@ -1226,7 +1228,7 @@ def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: i
     scratch = _fresh((max(1, int(lib.kb_delta_scratch_floats(rows, heads, kv_heads, d, e))),), torch.float32, src.device)
     chunks = None
     if longest >= DELTA_CHUNK_LONGEST and lib.kb_delta_chunks_take(d, e):
-        chunks = _fresh((int(lib.kb_delta_chunk_floats(rows, heads, d, e)),), torch.float32, src.device)
+        chunks = _fresh((int(lib.kb_delta_chunk_floats(rows, int(entries), heads, kv_heads, d, e)),), torch.float32, src.device)
     _check(lib.kb_delta_scan(
         _ptr(out), _ptr(scratch), _ptr(src), dt, splits, ctypes.c_longlong(stride), width, int(q_off), int(k_off), int(v_off),
         int(b_off), int(a_off), _ptr(conv), _ptr(a_log), _ptr(dt_bias), _ptr(state), int(state.shape[0]), ctypes.c_longlong(per),
