@@ -385,13 +385,15 @@ int gemm_f32_segments(int m, int n, int k) {
     }
     return best;
 }
-// From 512 weight rows of 1,024 on and more than two rows: one accumulator an element in ascending k, a kernel for each, is limited by
-// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 32. One row stays with the chains (18,432 x
-// 2,304: 37 us by chains, 39 by pieces; 2,304 x 9,216: 32 and 39), four go either way (44 and 39, 51 and 39) as long as the tiles are one
-// wave (256,000 x 2,304: 440 and 500), six and more go by pieces (54 and 39, 72 and 39, 639 and 499), 500 rows far ahead: 824 and 223, 545 and 122, by 2,304 x
-// 2,048 131 and 35, by 512 x 1,024 32 and 15. The error against 64 bits is 0.07 to 0.2 of the chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6).
+// More than 16 rows of 256 and more, and three to 16 of 1,024 and more: one accumulator an element in ascending k, a kernel for each, is limited by
+// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 32. 500 rows by 18,432 x 2,304: 824 us by
+// chains, 223 by pieces; by 2,304 x 9,216 545 and 122, by 2,304 x 2,048 131 and 35, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
+// 12 (64 rows 9.3 and 8.8). Six rows: 54 and 40, 72 and 39, 18 and 14, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 39, 51 and 39, 14 and 14, 13 and
+// 9 as long as the tiles are one wave (256,000 x 2,304: 440 and 500); one row 37 and 39, 32 and 39. The error against 64 bits is 0.07 to 0.3 of the
+// chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
 bool gemm_f32_pieces_take(int m, int n, int k, const void* a, const void* w) {
-    return (m > 4 || (m > 2 && n <= FP_M * multiprocessors())) && n >= 512 && k >= 1024 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
+    const bool pays = m > 16 ? k >= 256 : k >= 1024 && (m > 4 || (m > 2 && n <= FP_M * multiprocessors()));
+    return pays && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
 }
 long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * (3 * ((k + 7) / 8 * 4) + 1); }
 
