@@ -23,6 +23,7 @@
 //
 // Sums, norms, rotations and the gates are 32-bit.
 #include "common.cuh"
+#include "pieces.cuh"
 
 namespace kb {
 
@@ -523,56 +524,99 @@ head_linear_mma_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
     }
 }
 
-// The same product for a few rows (a decode step): one warp a column of M[h] for all rows. The lanes walk the
-// column's n_in values (they lie together in mt [heads, n_out, n_in]), every row's inputs lie in shared memory;
-// a warp sum a row. 32-bit sums; inputs and matrices as they come (no rounding of the inputs).
-constexpr int HF_ROWS = 16;
-constexpr int HF_WARPS = 8;
-template <typename TX>
+// The same product for a few rows (a decode step): the rows are the 16 of an MMA, a warp has eight columns of M[h], which lie together in mt
+// [heads, n_out, n_in] and come straight into registers, 16 bytes a lane, ahead of the wait on the kernel before. A lane's 16 bytes are eight neighbouring
+// inputs of one column, so two MMAs take 32 inputs in the order that gives, and the rows' inputs are read in the same. 32-bit inputs are
+// cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16): nothing is rounded but the sums. 8 rows, 16 heads of
+// 128 -> 512 (20.7 us by a column a warp, its sums by shuffles), 512 -> 128 with the gate (19.2): what is left is a launch's latency.
+constexpr int HF_ROWS = 16, HF_WARPS = 8, HF_COLS = HF_WARPS * 8, HF_HELD = 16;        // HF_HELD: groups of 32 inputs whose weights a lane holds at once
+// Elements between two rows of the inputs: 64 bytes further into the banks from row to row.
+__host__ __device__ constexpr int hf_ld(int n_in) { return (n_in + 31) / 32 * 32 + ((n_in + 31) / 32 % 2 == 0 ? 32 : 0); }
+template <typename TX> __host__ __device__ constexpr int hf_pieces() { return sizeof(TX) == 4 ? 3 : 1; }
+
+__device__ __forceinline__ void hf_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// VEC: columns of mt begin at 16-byte boundaries and n_in is a multiple of eight.
+template <typename TX, bool VEC>
 __global__ void __launch_bounds__(HF_WARPS * 32)
 head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX> x, int x_row, int x_head, int x_off,
-                       const bf16* __restrict__ mt, int n_in, int n_out, int columns, int rows, int heads,
+                       const bf16* __restrict__ mt, int n_in, int n_out, int rows, int heads,
                        int tail_off, int tail, const float2* __restrict__ cos_sin,
                        const Src<float> gate, int g_row, int g_off) {
-    extern __shared__ float xf[];                               // [rows][n_in]
+    constexpr int PIECES = hf_pieces<TX>();
+    extern __shared__ __align__(16) unsigned char hf_smem[];
+    uint32_t* xs = reinterpret_cast<uint32_t*>(hf_smem);        // [PIECES][16][ld] bfloat16
     const int h = blockIdx.x;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int c0 = (blockIdx.y * HF_WARPS + warp) * columns;
-    // the matrix is nobody's output: its columns set out for L2 ahead of the wait on the kernel before
-    for (int i = lane * 64; i < columns * n_in && c0 + i / n_in < n_out; i += 32 * 64)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(mt + ((size_t)h * n_out + c0) * n_in + i));
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
+    const int groups = (n_in + 31) / 32, ld = hf_ld(n_in);
+    const int c0 = blockIdx.y * HF_COLS + warp * 8, mine = c0 + row;      // the column whose weights this lane holds
+    const bf16* column = mt + ((size_t)h * n_out + min(mine, n_out - 1)) * n_in;
+    auto weights = [&](int group) {
+        const int k = group * 32 + quad * 8;
+        uint4 w = make_uint4(0u, 0u, 0u, 0u);
+        if (mine < n_out && group < groups) {
+            if (VEC) {
+                if (k < n_in) w = *reinterpret_cast<const uint4*>(column + k);
+            } else {
+                uint32_t u[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    if (k + j < n_in) u[j >> 1] |= (uint32_t)__bfloat16_as_ushort(column[k + j]) << (16 * (j & 1));
+                w = make_uint4(u[0], u[1], u[2], u[3]);
+            }
+        }
+        return w;
+    };
+    uint4 held[HF_HELD];
+#pragma unroll
+    for (int i = 0; i < HF_HELD; ++i) held[i] = weights(i);     // nobody's output
     dependent_wait();                                       // returns at once after a plain launch
     dependent_trigger();
-    for (int idx = tid; idx < rows * n_in; idx += HF_WARPS * 32) {
-        const int t = idx / n_in, i = idx - t * n_in;
-        xf[idx] = x.at((size_t)t * x_row + (size_t)h * x_head + x_off + i);
+    const int pairs = groups * 16;                              // of inputs a row; beyond n_in and the last row zeros
+    for (int idx = tid; idx < 16 * pairs; idx += HF_WARPS * 32) {
+        const int t = idx / pairs, k = (idx - t * pairs) * 2;
+        const size_t at = (size_t)t * x_row + (size_t)h * x_head + x_off + k;
+        float a = t < rows && k < n_in ? x.at(at) : 0.f, b = t < rows && k + 1 < n_in ? x.at(at + 1) : 0.f;
+        uint32_t* to = xs + (t * ld + k) / 2;
+        if (PIECES == 1) {
+            const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+            to[0] = *reinterpret_cast<const uint32_t*>(&v);
+        } else {
+            uint32_t two, three;
+            cut_pair(a, b, to[0], two, three);
+            const uint32_t keep = (a == a ? 0xffffu : 0u) | (b == b ? 0xffff0000u : 0u);      // infinity is its first piece alone
+            to[8 * ld] = two & keep, to[16 * ld] = three & keep;
+        }
     }
     __syncthreads();
-    for (int c = c0; c < min(c0 + columns, n_out); ++c) {
-        float acc[HF_ROWS];
+    float acc[PIECES][4] = {};
+    auto multiply = [&](int group, const uint4& w) {
 #pragma unroll
-        for (int t = 0; t < HF_ROWS; ++t) acc[t] = 0.f;
-        const bf16* col = mt + ((size_t)h * n_out + c) * n_in;
-        for (int i = lane; i < n_in; i += 32) {
-            const float w = __bfloat162float(col[i]);
+        for (int q = 0; q < PIECES; ++q) {
+            const uint32_t* from = xs + (q * 16 + row) * (ld / 2) + group * 16 + quad * 4;
+            const uint4 a = *reinterpret_cast<const uint4*>(from), b = *reinterpret_cast<const uint4*>(from + 4 * ld);      // rows `row` and `row` + 8
+            hf_mma(acc[q], a.x, b.x, a.y, b.y, w.x, w.y);
+            hf_mma(acc[q], a.z, b.z, a.w, b.w, w.z, w.w);
+        }
+    };
 #pragma unroll
-            for (int t = 0; t < HF_ROWS; ++t)
-                if (t < rows) acc[t] = fmaf(xf[t * n_in + i], w, acc[t]);
-        }
-        float v = 0.f;                                          // lane t ends up with row t
+    for (int i = 0; i < HF_HELD; ++i)
+        if (i < groups) multiply(i, held[i]);
+    for (int i = HF_HELD; i < groups; ++i) multiply(i, weights(i));
 #pragma unroll
-        for (int t = 0; t < HF_ROWS; ++t) {
-            if (t >= rows) continue;
-            const float total = warp_sum(acc[t]);
-            if (lane == t) v = total;
+    for (int i = 0; i < 4; ++i) {
+        const int t = row + (i >> 1) * 8, c = c0 + quad * 2 + (i & 1);
+        if (t >= rows || c >= n_out) continue;
+        float v = acc[0][i];
+        if (PIECES == 3) v = (acc[PIECES - 1][i] + acc[PIECES / 2][i]) + v;
+        if (gate.p != nullptr) {
+            const float z = gate.at((size_t)t * g_row + g_off + (size_t)h * n_out + c);
+            v *= 1.f / (1.f + expf(-z));
         }
-        if (lane < rows) {
-            if (gate.p != nullptr) {
-                const float z = gate.at((size_t)lane * g_row + g_off + (size_t)h * n_out + c);
-                v *= 1.f / (1.f + expf(-z));
-            }
-            y[(size_t)lane * y_row + (size_t)h * y_head + c] = __float2bfloat16_rn(v);
-        }
+        y[(size_t)t * y_row + (size_t)h * y_head + c] = __float2bfloat16_rn(v);
     }
     if (blockIdx.y != 0) return;
     const int half = tail >> 1;
@@ -874,21 +918,29 @@ extern "C" int kb_head_linear_mma(void* y, int y_row, int y_head, const void* x,
     if (rows == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const Src<float> g{gate, gate ? g_splits : 1, (size_t)g_split_stride};
-    const size_t few_smem = (size_t)rows * n_in * sizeof(float);
-    if (rows <= HF_ROWS && few_smem <= 48 * 1024 && (n_out + HF_WARPS - 1) / HF_WARPS <= 65535) {     // a decode step: a warp a column
-        // columns a warp: every block adds up the rows' inputs of its head again, so several where the blocks still fill the GPU
-        int columns = 1;
-        const int sms = multiprocessors();
-        while (columns < 8 && (long long)heads * (n_out / (2 * columns * HF_WARPS)) >= sms) columns *= 2;
-        dim3 few(heads, (n_out + HF_WARPS * columns - 1) / (HF_WARPS * columns));
-        if (x_dt == KB_DT_F32)
-            launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<float>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, Src<float>{(const float*)x, x_splits, (size_t)x_split_stride}, x_row,
-                                                                             x_head, x_off, (const bf16*)mt, n_in, n_out, columns, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
-        else if (x_dt == KB_DT_BF16)
-            launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<bf16>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, Src<bf16>{(const bf16*)x, x_splits, (size_t)x_split_stride}, x_row,
-                                                                            x_head, x_off, (const bf16*)mt, n_in, n_out, columns, rows, heads, tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);
-        else return fail("head_linear_mma: dtype code %d is not known", x_dt);
-        return check_launch("head_linear_few");
+    const size_t few_smem = (size_t)(x_dt == KB_DT_F32 ? hf_pieces<float>() : 1) * 16 * hf_ld(n_in) * sizeof(bf16);
+    if (rows <= HF_ROWS && few_smem <= 200 * 1024 && (n_out + HF_COLS - 1) / HF_COLS <= 65535) {     // a decode step
+        const dim3 few(heads, (n_out + HF_COLS - 1) / HF_COLS);
+        const bool vec = n_in % 8 == 0 && ((uintptr_t)mt & 15) == 0;
+#define KB_HF(TX, VEC)                                                                                                                                  \
+        do {                                                                                                                                            \
+            if (few_smem > 48 * 1024 && cudaFuncSetAttribute(head_linear_few_kernel<TX, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)few_smem) != cudaSuccess) \
+                return fail("head_linear: cannot have %zu bytes of shared memory", few_smem);                                                           \
+            launch_dependent_if(rows <= DEPENDENT_ROWS, head_linear_few_kernel<TX, VEC>, few, dim3(HF_WARPS * 32), few_smem, s, (bf16*)y, y_row, y_head, \
+                                Src<TX>{(const TX*)x, x_splits, (size_t)x_split_stride}, x_row, x_head, x_off, (const bf16*)mt, n_in, n_out, rows, heads, \
+                                tail_off, tail, (const float2*)cos_sin, g, g_row, g_off);                                                               \
+            return check_launch("head_linear_few");                                                                                                     \
+        } while (0)
+        if (x_dt == KB_DT_F32) {
+            if (vec) KB_HF(float, true);
+            else KB_HF(float, false);
+        }
+        if (x_dt == KB_DT_BF16) {
+            if (vec) KB_HF(bf16, true);
+            else KB_HF(bf16, false);
+        }
+#undef KB_HF
+        return fail("head_linear_mma: dtype code %d is not known", x_dt);
     }
     dim3 grid((rows + HM_ROWS - 1) / HM_ROWS, heads, (n_out + HM_COLS - 1) / HM_COLS);
     if (x_dt == KB_DT_F32)
