@@ -60,9 +60,22 @@ struct DeltaParams {
 __device__ __forceinline__ float delta_softplus(float x) { return x > 20.f ? x : log1pf(expf(x)); }
 __device__ __forceinline__ float delta_silu(float x) { return x / (1.f + expf(-x)); }
 
-template <typename TS>
+// SINGLE: every request brings one row, and filters have DELTA_SINGLE_TAPS weights. A thread then asks for its channels' filters ahead of the wait on
+// the kernel before and for all their inputs at once: tap by tap, behind the history's stores, a step took 13 us, of which the trips to memory were most.
+constexpr int DELTA_SINGLE_TAPS = 4, DELTA_SINGLE_CHANNELS = 4;
+template <typename TS, bool SINGLE>
 __global__ void __launch_bounds__(1024)
 delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
+    constexpr int CH = DELTA_SINGLE_CHANNELS;
+    float4 filter[CH];
+    if (SINGLE) {
+        const int channels = 2 * p.kv_heads * p.d + p.heads * p.e;
+#pragma unroll
+        for (int i = 0; i < CH; ++i) {
+            const int c = threadIdx.x + i * blockDim.x;
+            if (c < channels) filter[i] = *reinterpret_cast<const float4*>(p.conv + (size_t)c * DELTA_SINGLE_TAPS);
+        }
+    }
     dependent_wait();                                       // returns at once after a plain launch
     dependent_trigger();
     extern __shared__ float act[];                              // [channels]
@@ -78,21 +91,48 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
     const bool kept = slot > 0 && slot < p.n_slots;
     float* hist = p.state + (size_t)(kept ? slot : 0) * p.state_floats;
     const int taps = p.taps;
-    for (int c = threadIdx.x; c < channels; c += blockDim.x) {
-        const int col = c < nq ? p.q_off + c : (c < 2 * nq ? p.k_off + (c - nq) : p.v_off + (c - 2 * nq));
-        float y = 0.f, newer = 0.f;
-        for (int j = 0; j < taps; ++j) {                        // the input j rows back
-            const int t = r - j;
-            float x;
-            if (t >= r0) x = src.at((size_t)t * p.row_width + col);
-            else if (kept) x = hist[(size_t)(taps - 1 + (t - r0)) * channels + c];     // t - r0 in [-(taps-1), -1]
-            else x = 0.f;
-            y = fmaf(p.conv[(size_t)c * taps + (taps - 1 - j)], x, y);
-            // a request's only row of the step: the history moves up by one on the way, its place j rows back takes the input a row later
-            if (p.single && kept && j > 0) hist[(size_t)(taps - 1 - j) * channels + c] = newer;
-            newer = x;
+    auto column = [&](int c) { return c < nq ? p.q_off + c : (c < 2 * nq ? p.k_off + (c - nq) : p.v_off + (c - 2 * nq)); };
+    if (SINGLE) {
+        for (int c0 = threadIdx.x; c0 < channels; c0 += CH * blockDim.x) {
+            float x[CH], h[CH][DELTA_SINGLE_TAPS - 1];
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                const int c = c0 + i * blockDim.x;
+                const bool there = c < channels;
+                if (there && c0 >= (int)blockDim.x) filter[i] = *reinterpret_cast<const float4*>(p.conv + (size_t)c * DELTA_SINGLE_TAPS);
+#pragma unroll
+                for (int j = 0; j < DELTA_SINGLE_TAPS - 1; ++j) h[i][j] = there && kept ? hist[(size_t)j * channels + c] : 0.f;
+                x[i] = there ? src.at((size_t)r * p.row_width + column(c)) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < CH; ++i) {
+                const int c = c0 + i * blockDim.x;
+                if (c >= channels) break;
+                float y = fmaf(filter[i].w, x[i], 0.f);
+                y = fmaf(filter[i].z, h[i][2], y);
+                y = fmaf(filter[i].y, h[i][1], y);
+                y = fmaf(filter[i].x, h[i][0], y);
+                if (kept) hist[c] = h[i][1], hist[channels + c] = h[i][2], hist[(size_t)2 * channels + c] = x[i];      // the history moves up by one
+                act[c] = delta_silu(y);
+            }
         }
-        act[c] = delta_silu(y);
+    } else {
+        for (int c = threadIdx.x; c < channels; c += blockDim.x) {
+            const int col = column(c);
+            float y = 0.f, newer = 0.f;
+            for (int j = 0; j < taps; ++j) {                        // the input j rows back
+                const int t = r - j;
+                float x;
+                if (t >= r0) x = src.at((size_t)t * p.row_width + col);
+                else if (kept) x = hist[(size_t)(taps - 1 + (t - r0)) * channels + c];     // t - r0 in [-(taps-1), -1]
+                else x = 0.f;
+                y = fmaf(p.conv[(size_t)c * taps + (taps - 1 - j)], x, y);
+                // a request's only row of the step: the history moves up by one on the way, its place j rows back takes the input a row later
+                if (p.single && kept && j > 0) hist[(size_t)(taps - 1 - j) * channels + c] = newer;
+                newer = x;
+            }
+            act[c] = delta_silu(y);
+        }
     }
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
@@ -116,7 +156,7 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
         if (lane == 0) p.kq[(size_t)r * p.kv_heads + h] = qk * iq * ik;
     }
     for (int i = threadIdx.x; i < nv; i += blockDim.x) p.vn[(size_t)r * nv + i] = act[2 * nq + i];
-    for (int h = threadIdx.x; h < p.heads; h += blockDim.x) {
+    for (int h = blockDim.x - 1 - threadIdx.x; h < p.heads; h += blockDim.x) {      // by the last threads: the first make the unit vectors
         const float a = src.at((size_t)r * p.row_width + p.a_off + h) + p.dt_bias[h];
         const float b = src.at((size_t)r * p.row_width + p.b_off + h);
         p.scal[((size_t)r * p.heads + h) * 2] = expf(-expf(p.a_log[h]) * delta_softplus(a));
@@ -124,93 +164,138 @@ delta_prep_kernel(const Src<TS> src, const DeltaParams p) {
     }
 }
 
-// The same for prompts with filters of four weights, from one 32-bit slice whose columns and widths are multiples of four: a block takes
-// DPR rows, so an input that serves four rows' convolutions is loaded once for those of a block, a thread four neighbouring channels of them
-// (7 loads of 16 bytes for 4 x 4 values instead of 64 of 4). 2,048 rows of 3,072 channels: 43 us against 71, 1,360 rows 37 against 55; a
-// block's own chain takes some 35 us where 172 rows of a row a block take 27, so from DPR_FROM rows on.
-constexpr int DPR = 4, DPR_TAPS = 4, DPR_FROM = 512;
-__global__ void __launch_bounds__(256)
-delta_prep_rows_kernel(const Src<float> src, const DeltaParams p) {
-    extern __shared__ float act[];                              // [DPR][channels]
-    const int first = blockIdx.x * DPR, nr = min(DPR, p.rows - first);
-    const int nq = p.kv_heads * p.d, nv = p.heads * p.e;
-    const int channels = 2 * nq + nv;
-    int start[DPR];                                             // each row's request's first row of the step
-    const float* hist[DPR];                                     // its slot's history, or null
-    bool plain = true;                                          // no row of the block looks back beyond its request's first
+// The same for prompts with filters of four weights, from one 32-bit slice whose columns and widths are multiples of four. A warp takes DPR
+// rows of one kv head's queries and keys (a lane their components l, l + 32, ..: the norms' sums are those of the kernel above, bit for bit)
+// or of 128 value channels (four neighbouring ones a lane), and a last warp the rows' decays and step sizes: a filter and an input are
+// loaded once for all the rows they serve, and nothing passes through shared memory. More rows than DEPENDENT_ROWS only: launched plainly.
+constexpr int DPR = 8, DPR_TAPS = 4;
+
+// Convolution and silu of E channels of a lane over the warp's rows: `load(t, x)` an input row, `history(slot's history, place, x)` one of those
+// kept. One small loop over the rows, the inputs of some more asked for ahead: unrolled over the rows, the warps waited for instructions.
+template <int E, typename Load, typename History, typename Done>
+__device__ __forceinline__ void delta_conv_rows(const DeltaParams& p, int first, int nr, int my_start, int my_slot, const float (&f)[E][DPR_TAPS],
+                                                Load load, History history, Done done) {
+    constexpr int AHEAD = E <= 4 ? 4 : 2;
+    float raw[DPR_TAPS + AHEAD][E];                             // the inputs of rows r - 3 .. r + AHEAD
 #pragma unroll
-    for (int i = 0; i < DPR; ++i) {
-        const int r = min(first + i, p.rows - 1), entry = p.row_entry[r];
-        start[i] = r;
-        hist[i] = nullptr;
-        if (entry >= 0 && entry < p.entries) {
-            start[i] = p.entry_start[entry];
-            const int slot = p.slots[entry];
-            if (slot > 0 && slot < p.n_slots) hist[i] = p.state + (size_t)slot * p.state_floats;
-        }
-        plain = plain && start[i] <= first - (DPR_TAPS - 1);
-    }
-    constexpr int CW = 4;
-    for (int c = threadIdx.x * CW; c < channels; c += blockDim.x * CW) {
-        const int col = c < nq ? p.q_off + c : (c < 2 * nq ? p.k_off + (c - nq) : p.v_off + (c - 2 * nq));
-        float raw[DPR + DPR_TAPS - 1][CW], f[CW][DPR_TAPS];     // the inputs of rows first - 3 .. first + 3; the filters
+    for (int x = 0; x < DPR_TAPS + AHEAD - 1; ++x) load(min(max(first - (DPR_TAPS - 1) + x, 0), p.rows - 1), raw[x]);
+#pragma unroll 1
+    for (int i = 0; i < nr; ++i) {
+        load(min(first + i + AHEAD, p.rows - 1), raw[DPR_TAPS + AHEAD - 1]);
+        const int back = first + i - __shfl_sync(0xffffffffu, my_start, i);      // rows of its request before it in this step
+        const int slot = __shfl_sync(0xffffffffu, my_slot, i);
+        float y[E];
 #pragma unroll
-        for (int x = 0; x < DPR + DPR_TAPS - 1; ++x) {
-            const int t = first - (DPR_TAPS - 1) + x;
-            const bool there = t >= 0 && t < p.rows;
-            const float4 v = there ? *reinterpret_cast<const float4*>(src.p + (size_t)t * p.row_width + col) : make_float4(0.f, 0.f, 0.f, 0.f);
-            raw[x][0] = v.x, raw[x][1] = v.y, raw[x][2] = v.z, raw[x][3] = v.w;
-        }
+        for (int c = 0; c < E; ++c) y[c] = 0.f;
 #pragma unroll
-        for (int w = 0; w < CW; ++w)
+        for (int j = 0; j < DPR_TAPS; ++j) {
+            float in[E];
 #pragma unroll
-            for (int j = 0; j < DPR_TAPS; ++j) f[w][j] = p.conv[(size_t)(c + w) * DPR_TAPS + (DPR_TAPS - 1 - j)];
+            for (int c = 0; c < E; ++c) in[c] = raw[DPR_TAPS - 1 - j][c];
+            if (back < j) {                                     // the same for the whole warp
 #pragma unroll
-        for (int i = 0; i < DPR; ++i)
-#pragma unroll
-            for (int w = 0; w < CW; ++w) {
-                float y = 0.f;
-#pragma unroll
-                for (int j = 0; j < DPR_TAPS; ++j) {
-                    float x = raw[i + DPR_TAPS - 1 - j][w];
-                    const int back = first + i - j - start[i];  // below zero: before the request's first row of the step
-                    if (!plain && back < 0) x = hist[i] != nullptr ? hist[i][(size_t)(DPR_TAPS - 1 + back) * channels + c + w] : 0.f;
-                    y = fmaf(f[w][j], x, y);
-                }
-                act[i * channels + c + w] = delta_silu(y);
+                for (int c = 0; c < E; ++c) in[c] = 0.f;
+                if (slot > 0) history(p.state + (size_t)slot * p.state_floats, DPR_TAPS - 1 + back - j, in);
             }
-    }
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-    for (int hi = warp; hi < nr * p.kv_heads; hi += warps) {
-        const int i = hi / p.kv_heads, h = hi - i * p.kv_heads;
-        const size_t r = (size_t)(first + i);
-        const float* a = act + i * channels;
-        float sq = 0.f, sk = 0.f, qk = 0.f;
-        for (int x = lane; x < p.d; x += 32) {
-            const float q = a[h * p.d + x], k = a[nq + h * p.d + x];
-            sq = fmaf(q, q, sq);
-            sk = fmaf(k, k, sk);
-            qk = fmaf(q, k, qk);
+#pragma unroll
+            for (int c = 0; c < E; ++c) y[c] = fmaf(f[c][j], in[c], y[c]);
         }
-        sq = warp_sum(sq);
-        sk = warp_sum(sk);
-        qk = warp_sum(qk);
-        const float iq = p.q_scale / sqrtf(sq + p.unit_eps), ik = 1.f / sqrtf(sk + p.unit_eps);
-        for (int x = lane; x < p.d; x += 32) {
-            p.qn[(r * p.kv_heads + h) * p.d + x] = a[h * p.d + x] * iq;
-            p.kn[(r * p.kv_heads + h) * p.d + x] = a[nq + h * p.d + x] * ik;
-        }
-        if (lane == 0) p.kq[r * p.kv_heads + h] = qk * iq * ik;
+#pragma unroll
+        for (int c = 0; c < E; ++c) y[c] = delta_silu(y[c]);
+        done(first + i, y);
+#pragma unroll
+        for (int x = 0; x < DPR_TAPS + AHEAD - 1; ++x)
+#pragma unroll
+            for (int c = 0; c < E; ++c) raw[x][c] = raw[x + 1][c];
     }
-    for (int x = threadIdx.x; x < nr * nv; x += blockDim.x) p.vn[(size_t)first * nv + x] = act[(x / nv) * channels + 2 * nq + x % nv];
-    for (int x = threadIdx.x; x < nr * p.heads; x += blockDim.x) {
-        const int h = x % p.heads;
-        const size_t r = (size_t)(first + x / p.heads);
-        const float a = src.at(r * p.row_width + p.a_off + h) + p.dt_bias[h];
-        const float b = src.at(r * p.row_width + p.b_off + h);
-        p.scal[(r * p.heads + h) * 2] = expf(-expf(p.a_log[h]) * delta_softplus(a));
-        p.scal[(r * p.heads + h) * 2 + 1] = 1.f / (1.f + expf(-b));
+}
+
+// R: components of a head a lane has. `parts`: warps a group of rows takes.
+template <int R>
+__global__ void __launch_bounds__(256, R <= 4 ? 2 : 1)
+delta_prep_rows_kernel(const Src<float> src, const DeltaParams p, int parts) {
+    const int lane = threadIdx.x & 31;
+    const long long item = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int first = (int)(item / parts) * DPR, part = (int)(item % parts);
+    if (first >= p.rows) return;
+    const int nr = min(DPR, p.rows - first), nq = p.kv_heads * p.d, nv = p.heads * p.e, channels = 2 * nq + nv;
+    int my_start = first + lane, my_slot = 0;                   // of row first + lane: its request's first row of the step, its slot or 0
+    if (lane < nr) {
+        const int entry = p.row_entry[first + lane];
+        if (entry >= 0 && entry < p.entries) {
+            my_start = p.entry_start[entry];
+            const int slot = p.slots[entry];
+            if (slot > 0 && slot < p.n_slots) my_slot = slot;
+        }
+    }
+    if (part < p.kv_heads) {
+        const int h = part, d = p.d;
+        float f[2 * R][DPR_TAPS];                               // queries' components, then keys'
+#pragma unroll
+        for (int i = 0; i < 2 * R; ++i) {
+            const int x = lane + 32 * (i % R), c = (i < R ? 0 : nq) + h * d + x;
+            const float4 w = x < d ? *reinterpret_cast<const float4*>(p.conv + (size_t)c * DPR_TAPS) : make_float4(0.f, 0.f, 0.f, 0.f);
+            f[i][0] = w.w, f[i][1] = w.z, f[i][2] = w.y, f[i][3] = w.x;
+        }
+        delta_conv_rows<2 * R>(p, first, nr, my_start, my_slot, f,
+            [&](int t, float (&to)[2 * R]) {
+                const float* row = src.p + (size_t)t * p.row_width + h * d + lane;
+#pragma unroll
+                for (int i = 0; i < 2 * R; ++i) to[i] = lane + 32 * (i % R) < d ? row[(i < R ? p.q_off : p.k_off) + 32 * (i % R)] : 0.f;
+            },
+            [&](const float* hist, int place, float (&to)[2 * R]) {
+#pragma unroll
+                for (int i = 0; i < 2 * R; ++i) {
+                    const int x = lane + 32 * (i % R);
+                    to[i] = x < d ? hist[(size_t)place * channels + (i < R ? 0 : nq) + h * d + x] : 0.f;
+                }
+            },
+            [&](int r, const float (&y)[2 * R]) {
+                float sq = 0.f, sk = 0.f, qk = 0.f;
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (lane + 32 * i < d) sq = fmaf(y[i], y[i], sq), sk = fmaf(y[R + i], y[R + i], sk), qk = fmaf(y[i], y[R + i], qk);
+                sq = warp_sum(sq);
+                sk = warp_sum(sk);
+                qk = warp_sum(qk);
+                const float iq = p.q_scale / sqrtf(sq + p.unit_eps), ik = 1.f / sqrtf(sk + p.unit_eps);
+                const size_t to = ((size_t)r * p.kv_heads + h) * d + lane;
+#pragma unroll
+                for (int i = 0; i < R; ++i)
+                    if (lane + 32 * i < d) p.qn[to + 32 * i] = y[i] * iq, p.kn[to + 32 * i] = y[R + i] * ik;
+                if (lane == 0) p.kq[(size_t)r * p.kv_heads + h] = qk * iq * ik;
+            });
+    } else if (part < parts - 1) {
+        const int c = ((part - p.kv_heads) * 32 + lane) * 4;    // value channel: widths are multiples of four
+        const bool there = c < nv;
+        const int cc = there ? c : 0;
+        float f[4][DPR_TAPS];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 w = *reinterpret_cast<const float4*>(p.conv + (size_t)(2 * nq + cc + i) * DPR_TAPS);
+            f[i][0] = w.w, f[i][1] = w.z, f[i][2] = w.y, f[i][3] = w.x;
+        }
+        delta_conv_rows<4>(p, first, nr, my_start, my_slot, f,
+            [&](int t, float (&to)[4]) {
+                const float4 v = *reinterpret_cast<const float4*>(src.p + (size_t)t * p.row_width + p.v_off + cc);
+                to[0] = v.x, to[1] = v.y, to[2] = v.z, to[3] = v.w;
+            },
+            [&](const float* hist, int place, float (&to)[4]) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) to[i] = hist[(size_t)place * channels + 2 * nq + cc + i];
+            },
+            [&](int r, const float (&y)[4]) {
+                if (there) *reinterpret_cast<float4*>(p.vn + (size_t)r * nv + c) = make_float4(y[0], y[1], y[2], y[3]);
+            });
+    } else {
+        for (int x = lane; x < nr * p.heads; x += 32) {
+            const int h = x % p.heads;
+            const size_t r = (size_t)(first + x / p.heads);
+            const float a = src.at(r * p.row_width + p.a_off + h) + p.dt_bias[h];
+            const float b = src.at(r * p.row_width + p.b_off + h);
+            p.scal[(r * p.heads + h) * 2] = expf(-expf(p.a_log[h]) * delta_softplus(a));
+            p.scal[(r * p.heads + h) * 2 + 1] = 1.f / (1.f + expf(-b));
+        }
     }
 }
 
@@ -500,15 +585,21 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     cudaStream_t s = (cudaStream_t)stream;
     const size_t smem = (size_t)channels * sizeof(float);
     const bool fours = splits == 1 && (row_width | q_off | k_off | v_off | (int)nq | (int)nv) % 4 == 0 && ((uintptr_t)src & 15) == 0;
-    const bool by_rows = in_dt == KB_DT_F32 && fours && rows >= DPR_FROM && taps == DPR_TAPS && DPR * smem <= 100 * 1024;
+    const bool by_rows = in_dt == KB_DT_F32 && fours && rows > DEPENDENT_ROWS && taps == DPR_TAPS && (((uintptr_t)conv | (uintptr_t)p.vn) & 15) == 0;
+    const int parts = kv_heads + (int)((nv + 127) / 128) + 1;   // warps that DPR rows take
+    const unsigned prep_blocks = (unsigned)(((long long)((rows + DPR - 1) / DPR) * parts + 7) / 8);
+#define KB_DELTA_PREP_ROWS(R) delta_prep_rows_kernel<R><<<prep_blocks, 256, 0, s>>>(Src<float>{(const float*)src, splits, (size_t)split_stride}, p, parts)
 #define KB_DELTA_PREP(TS)                                                                                                  \
     do {                                                                                                                   \
         if (by_rows) {                                                                                                     \
-            if (DPR * smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(DPR * smem)); \
-            delta_prep_rows_kernel<<<(rows + DPR - 1) / DPR, 256, DPR * smem, s>>>(Src<float>{(const float*)src, splits, (size_t)split_stride}, p); \
+            if (d <= 32) KB_DELTA_PREP_ROWS(1);                                                                            \
+            else if (d <= 64) KB_DELTA_PREP_ROWS(2);                                                                       \
+            else if (d <= 128) KB_DELTA_PREP_ROWS(4);                                                                      \
+            else KB_DELTA_PREP_ROWS(DELTA_R);                                                                              \
         } else {                                                                                                           \
-        if (smem > 48 * 1024) cudaFuncSetAttribute(delta_prep_kernel<TS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); \
-        launch_dependent_if(rows <= DEPENDENT_ROWS, delta_prep_kernel<TS>, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 256), smem, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \
+        auto prep = p.single && taps == DELTA_SINGLE_TAPS && ((uintptr_t)conv & 15) == 0 ? delta_prep_kernel<TS, true> : delta_prep_kernel<TS, false>; \
+        if (smem > 48 * 1024) cudaFuncSetAttribute(prep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+        launch_dependent_if(rows <= DEPENDENT_ROWS, prep, dim3(rows), dim3(rows <= DEPENDENT_ROWS ? 1024 : 256), smem, s, Src<TS>{(const TS*)src, splits, (size_t)split_stride}, p); /* few rows: a channel or two a thread */ \
         }                                                                                                                  \
         if (int err = check_launch("delta prep")) return err;                                                              \
         if (taps > 1 && !p.single) {                                                                                       \
@@ -521,6 +612,7 @@ extern "C" int kb_delta_scan(float* out, float* scratch, const void* src, int in
     else if (in_dt == KB_DT_BF16) KB_DELTA_PREP(bf16);
     else return fail("delta: dtype code %d is not known", in_dt);
 #undef KB_DELTA_PREP
+#undef KB_DELTA_PREP_ROWS
     if (by_chunks) {
         DeltaChunks c;
         c.qn = p.qn; c.kn = p.kn; c.vn = p.vn; c.scal = p.scal; c.kq = p.kq;
