@@ -526,7 +526,7 @@ extern "C" int kb_latent_attention_mma(void* out, const void* q, const void* tab
         launch_dependent_if(rows <= DEPENDENT_ROWS, latent_decode_kernel, dim3(slots, entries * slices), dim3(LM_THREADS), latent_decode_smem(d, dv), s, p, entry_start, entry_end, slices);
         if (int e = check_launch("latent_attention_mma decode")) return e;
         if (slots > 1) {
-            launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(128), 0, s, p);
+            launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(combine_threads(p.dv, (long long)rows * hq)), 0, s, p);
             return check_launch("latent_attention_mma combine");
         }
         return 0;
@@ -534,7 +534,7 @@ extern "C" int kb_latent_attention_mma(void* out, const void* q, const void* tab
     launch_dependent_if(rows <= DEPENDENT_ROWS, latent_mma_kernel, dim3((unsigned)tiles, entries, slots), dim3(LM_THREADS), smem, s, p, entry_start, entry_end, tokens_per_tile, heads_per_tile, head_slices);
     if (int e = check_launch("latent_attention_mma")) return e;
     if (slots > 1) {
-        launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(128), 0, s, p);
+        launch_dependent_if(rows <= DEPENDENT_ROWS, combine_kernel<bf16>, dim3(rows, hq), dim3(combine_threads(p.dv, (long long)rows * hq)), 0, s, p);
         return check_launch("latent_attention_mma combine");
     }
     return 0;

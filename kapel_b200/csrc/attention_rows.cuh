@@ -122,14 +122,14 @@ rows_kernel(const AttParams p) {
         return;
     }
 
-    // shared: q [GMAX][dq] | scores [GMAX][CHUNK] | lines [CHUNK] | stats [2*GMAX] | acc [groups][GMAX][dv]
+    // shared: q [GMAX][dq] | scores [GMAX][CHUNK] | rows [CHUNK] | stats [2*GMAX] | acc [groups][GMAX][dv]
     // (dq: d rounded up to whole 16-byte pieces, the rest zeros)
     const int nvec = (d + VN - 1) / VN;
     const int dq = nvec * VN;
     float* sq = smem;
     float* ss = sq + GMAX * dq;
-    int* sline = reinterpret_cast<int*>(ss + GMAX * ATT_CHUNK);
-    float* sstat = reinterpret_cast<float*>(sline + ATT_CHUNK);
+    long long* srow = reinterpret_cast<long long*>(ss + GMAX * ATT_CHUNK);      // a key's row of the tables: divided out once, not by every thread that reads it
+    float* sstat = reinterpret_cast<float*>(srow + ATT_CHUNK);
     float* sacc = sstat + 2 * GMAX;
 
     const int entry = p.row_entry[r];
@@ -143,8 +143,8 @@ rows_kernel(const AttParams p) {
         const int lp = pos / p.page_size;
         const int page = lp < p.table_width ? p.block_table[(size_t)entry * p.table_width + lp] : -1;
         // A page outside the table would be a fault of the cache manager; such a key is skipped
-        // by giving it line -1, and its score becomes -inf below.
-        sline[j] = (page >= 0 && page < p.n_pages) ? page * p.page_size + pos % p.page_size : -1;
+        // by giving it row -1, and its score becomes -inf below.
+        srow[j] = (page >= 0 && page < p.n_pages) ? ((long long)page * p.hkv + kvh) * p.page_size + pos % p.page_size : -1;
     }
     __syncthreads();
 
@@ -152,42 +152,64 @@ rows_kernel(const AttParams p) {
     const T* kt = static_cast<const T*>(p.k_table);
     constexpr int KPW = 32 / LPK;                          // keys a warp handles at a time
     const int sub = lane / LPK, li = lane % LPK;
-    for (int j0 = warp * KPW; j0 < nkeys; j0 += ATT_WARPS * KPW) {
-        const int j = j0 + sub;
-        const bool live = j < nkeys;
-        const int line = live ? sline[j] : -1;
-        float kv[VPL][VN];
+    constexpr int AT_ONCE = VPL * VN <= 8 ? 8 : (VPL * VN <= 16 ? 4 : 2);      // keys of a warp asked for before the first is used
+    for (int j0 = warp * KPW; j0 < nkeys; j0 += AT_ONCE * ATT_WARPS * KPW) {
+        float kv[AT_ONCE][VPL][VN];
+        bool has[AT_ONCE];
 #pragma unroll
-        for (int v = 0; v < VPL; ++v) {
-            const int vi = li + v * LPK;
-            if (line >= 0 && vi < nvec && p.vec) {
-                Vec<T>::load(kt + kv_row(line, kvh, p.hkv, p.page_size) * d + vi * VN, kv[v]);
-            } else if (line >= 0 && vi < nvec) {
-                const T* kp = kt + kv_row(line, kvh, p.hkv, p.page_size) * d;
+        for (int u = 0; u < AT_ONCE; ++u) {
+            const int j = j0 + u * ATT_WARPS * KPW + sub;
+            const long long at = j < nkeys ? srow[j] : -1;
+            has[u] = at >= 0;
 #pragma unroll
-                for (int e = 0; e < VN; ++e) kv[v][e] = vi * VN + e < d ? Elem<T>::load(kp + vi * VN + e) : 0.f;
-            } else {
+            for (int v = 0; v < VPL; ++v) {
+                const int vi = li + v * LPK;
 #pragma unroll
-                for (int e = 0; e < VN; ++e) kv[v][e] = 0.f;
+                for (int e = 0; e < VN; ++e) kv[u][v][e] = 0.f;
+                if (has[u] && vi < nvec) {
+                    const T* kp = kt + (size_t)at * d + vi * VN;
+                    if (p.vec) {
+                        Vec<T>::load(kp, kv[u][v]);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < VN; ++e)
+                            if (vi * VN + e < d) kv[u][v][e] = Elem<T>::load(kp + e);
+                    }
+                }
             }
         }
         for (int g = 0; g < gn; ++g) {
-            float dot = 0.f;
+            float dot[AT_ONCE];
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) dot[u] = 0.f;
 #pragma unroll
             for (int v = 0; v < VPL; ++v) {
                 const int vi = li + v * LPK;
                 if (vi < nvec) {
 #pragma unroll
-                    for (int e = 0; e < VN; ++e) dot = fmaf(kv[v][e], sq[g * dq + vi * VN + e], dot);
+                    for (int e = 0; e < VN; ++e) {
+                        const float x = sq[g * dq + vi * VN + e];
+#pragma unroll
+                        for (int u = 0; u < AT_ONCE; ++u) dot[u] = fmaf(kv[u][v][e], x, dot[u]);
+                    }
                 }
             }
 #pragma unroll
-            for (int o = LPK / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-            if (live && li == 0) {
-                float s = dot * p.scale;
-                if (p.cap > 0.f) s = p.cap * tanhf(s / p.cap);
-                ss[g * ATT_CHUNK + j] = line >= 0 ? s : -INFINITY;
+            for (int o = LPK / 2; o > 0; o >>= 1)           // the keys' sums of lanes side by side
+#pragma unroll
+                for (int u = 0; u < AT_ONCE; ++u) dot[u] += __shfl_xor_sync(0xffffffffu, dot[u], o);
+#pragma unroll
+            for (int u = 0; u < AT_ONCE; ++u) {
+                const int j = j0 + u * ATT_WARPS * KPW + sub;
+                if (j < nkeys && li == 0) ss[g * ATT_CHUNK + j] = has[u] ? dot[u] * p.scale : -INFINITY;
             }
+        }
+    }
+    if (p.cap > 0.f) {                                      // a thread a key, not one of the lanes that share it
+        __syncthreads();
+        for (int i = tid; i < gn * nkeys; i += ATT_THREADS) {
+            float& s = ss[i / nkeys * ATT_CHUNK + i % nkeys];
+            if (srow[i % nkeys] >= 0) s = p.cap * tanhf(s / p.cap);
         }
     }
     __syncthreads();
@@ -222,17 +244,32 @@ rows_kernel(const AttParams p) {
         for (int g = 0; g < GMAX; ++g) acc[g][0] = acc[g][1] = 0.f;
         if (tgroups == 1 || tg < tgroups) {
             const int jstart = tgroups == 1 ? 0 : tg;
-            for (int j = jstart; j < nkeys; j += tgroups) {
-                const int line = sline[j];
-                if (line < 0) continue;
-                const T* vp = vt + kv_row(line, kvh, p.hkv, p.page_size) * p.v_stride + 2 * pi;
-                const float v0 = Elem<T>::load(vp), v1 = 2 * pi + 1 < dv ? Elem<T>::load(vp + 1) : 0.f;
+            constexpr int AT_ONCE_V = 8;                    // likewise of the values; added up in the keys' order all the same
+            for (int j0 = jstart; j0 < nkeys; j0 += AT_ONCE_V * tgroups) {
+                float v0[AT_ONCE_V], v1[AT_ONCE_V];
+                bool has[AT_ONCE_V];
 #pragma unroll
-                for (int g = 0; g < GMAX; ++g) {
-                    if (g < gn) {
-                        const float w = ss[g * ATT_CHUNK + j];
-                        acc[g][0] = fmaf(w, v0, acc[g][0]);
-                        acc[g][1] = fmaf(w, v1, acc[g][1]);
+                for (int u = 0; u < AT_ONCE_V; ++u) {
+                    const int j = j0 + u * tgroups;
+                    const long long at = j < nkeys ? srow[j] : -1;
+                    has[u] = at >= 0;
+                    v0[u] = v1[u] = 0.f;
+                    if (has[u]) {
+                        const T* vp = vt + (size_t)at * p.v_stride + 2 * pi;
+                        v0[u] = Elem<T>::load(vp);
+                        if (2 * pi + 1 < dv) v1[u] = Elem<T>::load(vp + 1);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < AT_ONCE_V; ++u) {
+                    if (!has[u]) continue;
+#pragma unroll
+                    for (int g = 0; g < GMAX; ++g) {
+                        if (g < gn) {
+                            const float w = ss[g * ATT_CHUNK + j0 + u * tgroups];
+                            acc[g][0] = fmaf(w, v0[u], acc[g][0]);
+                            acc[g][1] = fmaf(w, v1[u], acc[g][1]);
+                        }
                     }
                 }
             }
@@ -328,9 +365,16 @@ __global__ void combine_kernel(const AttParams p) {
     for (int i = threadIdx.x; i < dv; i += blockDim.x) {
         float acc = 0.f;
         const int known = min(p.slots, COMBINE_SLOTS);
-        for (int z = 0; z < known; ++z) {
-            const float w = weight[z];
-            if (w != 0.f) acc = fmaf(w, base[(size_t)z * (dv + 2) + i], acc);
+        for (int z0 = 0; z0 < known; z0 += 8) {             // eight slots asked for before the first is added
+            float v[8], w[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                w[u] = z0 + u < known ? weight[z0 + u] : 0.f;
+                v[u] = w[u] != 0.f ? base[(size_t)(z0 + u) * (dv + 2) + i] : 0.f;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (w[u] != 0.f) acc = fmaf(w[u], v[u], acc);
         }
         for (int z = known; z < p.slots; ++z) {
             int lo, hi;
@@ -344,11 +388,15 @@ __global__ void combine_kernel(const AttParams p) {
     }
 }
 
+// A thread a component, up to 512, where blocks are few (a decoding step): with 128 threads a component after the other waits for its slots' values (8 rows, 16 heads of
+// 512, 24 slots: 13 us). Many blocks (300 rows of 16 heads: 16 us) lose more to the larger blocks' sums (53).
+static int combine_threads(int dv, long long blocks) { return dv <= 128 || blocks > 4 * multiprocessors() ? 128 : dv <= 256 ? 256 : 512; }
+
 static size_t rows_smem_bytes(int gmax, int d, int dv) {
     const int pairs = (dv + 1) / 2;
     const int tgroups = pairs >= ATT_THREADS ? 1 : ATT_THREADS / pairs;
     const int dq = (d + 7) / 8 * 8;                          // room for d rounded up to either element type's pieces
-    size_t floats = (size_t)gmax * dq + (size_t)gmax * ATT_CHUNK + ATT_CHUNK + 2 * gmax;
+    size_t floats = (size_t)gmax * dq + (size_t)gmax * ATT_CHUNK + 2 * ATT_CHUNK + 2 * gmax;
     if (tgroups > 1) floats += (size_t)tgroups * gmax * (dv + 1);
     return floats * sizeof(float);
 }
@@ -413,8 +461,7 @@ template <typename T>
 static int run_rows(const AttParams& p, cudaStream_t s, bool combine) {
     if (int e = dispatch_group<T>(p, s)) return e;
     if (combine) {
-        dim3 grid(p.rows, p.hq);
-        combine_kernel<T><<<grid, 128, 0, s>>>(p);
+        combine_kernel<T><<<dim3(p.rows, p.hq), combine_threads(p.dv, (long long)p.rows * p.hq), 0, s>>>(p);
         return check_launch("paged_attention combine");
     }
     return 0;

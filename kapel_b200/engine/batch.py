@@ -68,13 +68,18 @@ ROW_TILE = 32
 ROW_TILE_TOKENS = 16
 
 
-def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: int, head_dim: int, window: Optional[int], sms: int) -> bool:
+def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: int, head_dim: int, window: Optional[int], sms: int,
+                  ahead: bool = False) -> bool:
     """Whether the 32-bit attention of these rows is faster by tiles than row by row. A block of the tile kernel walks all the keys of its
     tile, 64 a step, however few its rows: few tiles behind a long history leave the GPU idle, where the row-wise kernel has a block
     a row, kv head and 256 keys. Both as measured on a B200 for 16 to 1,024 tokens behind 0 to 16,384, groups of 1 to 16 heads of 128 and 256:
     a step 17.0 us (heads of 256) or 11.4 (of 128), a block a multiprocessor; a key 0.07 us + 1.45 ns a component + 0.06 us a head of the group,
     7 (groups of 1) to 4 (of 8) blocks a multiprocessor. 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 146 and 391; 16 tokens
-    behind 256, 1,024 and 4,096 positions 89 and 145, 292 and 149, 1,101 and 219; 128 tokens behind 1,024 and 16,384 311 and 372, 4,374 and 5,685."""
+    behind 256, 1,024 and 4,096 positions 89 and 145, 292 and 149, 1,101 and 219; 128 tokens behind 1,024 and 16,384 311 and 372, 4,374 and 5,685.
+    With `ahead` against the row-wise kernel as it is for what the engine gives it, which asks for several keys before it uses the first: the longest block's
+    keys, 0.08 us (one head of 128) to 0.17 (two of 256, four of 128) each, or all keys, 0.018 to 0.051 us a key and multiprocessor, and a quarter of the
+    shorter; 1 to 500 tokens behind 0 to 4,096, groups of 1 to 4. The same sizes by tiles and row by row: 500 tokens 146 and 217; 16 tokens 90 and 47, 291 and 51,
+    1,100 and 109; 128 tokens behind 0, 1,024 and 4,096 40 and 27, 310 and 205, 1,123 and 730; 500 behind 1,024 430 and 894 (the faster one in 71 of 72)."""
     count = np.asarray(row_count, np.int64)
     row0 = np.asarray(tile_row0, np.int64)
     first, last = count[row0], count[row0 + np.asarray(tile_nq, np.int64) - 1]
@@ -84,6 +89,10 @@ def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: in
     slices, heads = -(-heads_per_kv // 8), min(heads_per_kv, 8)      # the row-wise kernel's blocks have up to eight heads
     at_once = (7.5 - 0.42 * heads) * sms
     by_rows = 3.0 + (0.07 + 0.00145 * head_dim + 0.06 * heads) * max(min(256.0, float(count.max())), float(seen.sum()) * kv_heads * slices / at_once)
+    if ahead:
+        longest = (0.00046 * head_dim + 0.0293 * heads - 0.008) * min(256.0, float(count.max()))
+        every = head_dim * (0.0000794 + 0.000065 * heads) * float(seen.sum()) * kv_heads * slices / sms
+        by_rows = 3.0 + max(longest, every) + 0.25 * min(longest, every)
     return by_tiles <= by_rows
 
 
@@ -361,7 +370,7 @@ class StepBatch:
             arrays = None
             if len(plan.q_len) and self.shortest_portion() >= ROW_TILE_TOKENS and heads_per_kv <= ROW_TILE and self.ids.is_cuda:
                 arrays = cut_tiles(plan.q_start, plan.q_len, ROW_TILE // heads_per_kv)
-                if not row_tiles_pay(plan.row_count, arrays[1], arrays[2], kv_heads, heads_per_kv, head_dim, window, sm_count(self.ids.device)):
+                if not row_tiles_pay(plan.row_count, arrays[1], arrays[2], kv_heads, heads_per_kv, head_dim, window, sm_count(self.ids.device), ahead=True):
                     arrays = None
             if arrays is None:
                 self.memo[key] = None
