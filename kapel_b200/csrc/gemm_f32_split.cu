@@ -61,18 +61,43 @@ __device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t
     odd = fmaf(x, y, odd);
 }
 
+// 1 in one lane of the warp, the same one every time.
+__device__ __forceinline__ uint32_t fp_elect() {
+    uint32_t one;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
+    return one;
+}
+// at_mma_ts in the lane that has `one`
+__device__ __forceinline__ void fp_mma(uint32_t one, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
+}
+
 __device__ __forceinline__ void fp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// epilogue 0: none; 1: cap * tanh(acc / cap)
-template <int NP, int EPI>
+// Row tiles of a grouped product, an expert's rows each (moe.cu's lists): A's rows lie in the lists' order, the weights are [experts, n, k].
+struct F32Tiles {
+    const int* expert;
+    const int* first;
+    const int* rows;
+    const int* count;
+    const int* order;          // the pair at each place, where the result's rows are placed by pair; else null
+};
+
+// epilogue 0: none; 1: cap * tanh(acc / cap). GROUPED: blockIdx.x is a tile of `tiles`, NP rows at most, m the places there are.
+template <int NP, int EPI, bool GROUPED>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ c,
-                       const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ a_odd, int m, int n, int k, int chunks_a_segment, float cap) {
+                       const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ a_odd, int m, int n, int k, int chunks_a_segment, float cap, const F32Tiles tiles) {
     // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]; a_odd then says which rows have none
     using C = Pieces<NP>;
+    static_assert(!GROUPED || C::CUTS, "a tile's rows are cut by the blocks that need them");
     extern __shared__ unsigned char fp_raw[];
+    if (GROUPED && (int)blockIdx.x >= tiles.count[0]) return;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)fp_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* pieces = smem + C::STAGES * C::STAGE;           // [2][3][NP rows][128 bytes]
     uint64_t* full = reinterpret_cast<uint64_t*>(pieces + 2 * C::PIECES);
@@ -87,7 +112,8 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     static_assert((2 * C::STAGES + 8) * 8 + 8 <= 224, "the barriers outgrew their room");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * NP, n0 = blockIdx.y * FP_M, segment = blockIdx.z, segments = gridDim.z;
+    const int m0 = GROUPED ? tiles.first[blockIdx.x] : blockIdx.x * NP, rows = GROUPED ? min(tiles.rows[blockIdx.x], m - m0) : m - m0;      // what lies behind is not stored
+    const int n0 = blockIdx.y * FP_M, w0 = GROUPED ? tiles.expert[blockIdx.x] * n + n0 : n0, segment = blockIdx.z, segments = gridDim.z;
     const int chunks_all = (k + FP_K - 1) / FP_K;
     const int chunk0 = segment * chunks_a_segment, chunks = max(0, min(chunks_a_segment, chunks_all - chunk0));
 
@@ -123,31 +149,35 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 if (!at_mbar_wait(empty + s, ((uint32_t)(it / C::STAGES) & 1u) ^ 1u)) { failed = true; break; }
                 const uint32_t dst = at_saddr(smem + s * C::STAGE);
                 at_mbar_expect_tx(full + s, C::STAGE);
-                at_tma_box(dst, &map_w, chunk0 * FP_K + it * FP_STAGE_K, n0, full + s);
+                at_tma_box(dst, &map_w, chunk0 * FP_K + it * FP_STAGE_K, w0, full + s);
                 if (C::CUTS) at_tma_box(dst + C::W_BYTES, &map_a, chunk0 * FP_K + it * FP_STAGE_K, m0, full + s);
             }
             if (failed)                                            // the copies in flight land before the block goes on
                 for (int i = max(0, it - C::STAGES); i < it; ++i) at_mbar_wait(full + i % C::STAGES, (uint32_t)(i / C::STAGES) & 1u);
         }
     } else if (warp < FP_WARP_W) {
-        // ---------------------------------------------------------------- the products of every second chunk, from one lane
-        if (lane == 0) {
-            constexpr uint32_t IDESC = at_idesc(FP_M, NP, false);
-            const int b = warp - 1;
-            for (int ch = b; ch < chunks; ch += 2) {
-                if (!at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u)) { failed = true; break; }
-                if (!C::CUTS && !at_mbar_wait(a_full + b, (uint32_t)(ch >> 1) & 1u)) { failed = true; break; }
-                if (!at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
-                at_fence_after();
-                const uint32_t d = tmem + (uint32_t)(b * C::ACC), aw = tmem + (uint32_t)(C::COL_W + b * 96);
-                const uint64_t ba = at_desc(at_saddr(pieces + b * C::PIECES), 16, 1024);
+        // ---------------------------------------------------------------- the products of every second chunk
+        // The whole warp walks the loop and one lane's products go: inside a branch of one lane the operands have to be brought into the
+        // uniform registers that the instruction takes them from one by one, and a product of 128 rows took 118 clocks, not 64.
+        constexpr uint32_t IDESC = at_idesc(FP_M, NP, false);
+        const int b = __shfl_sync(0xffffffffu, warp, 0) - 1;
+        const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+        const uint32_t d = tm + (uint32_t)(b * C::ACC), aw = tm + (uint32_t)(C::COL_W + b * 96);
+        const uint64_t ba = at_desc(at_saddr(pieces + b * C::PIECES), 16, 1024);
+        for (int ch = b; ch < chunks; ch += 2) {
+            bool there = at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u);
+            if (!C::CUTS) there = there && at_mbar_wait(a_full + b, (uint32_t)(ch >> 1) & 1u);
+            there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
+            if (!__all_sync(0xffffffffu, there)) { failed = true; break; }
+            at_fence_after();
+            const uint32_t one = fp_elect();
 #pragma unroll
-                for (int p = 0; p < PIECE_PRODUCTS; ++p)
+            for (int p = 0; p < PIECE_PRODUCTS; ++p)
 #pragma unroll
-                    for (int kk = 0; kk < FP_K / 16; ++kk)
-                        at_mma_ts(d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
-                at_commit(done + b);
-            }
+                for (int kk = 0; kk < FP_K / 16; ++kk)
+                    fp_mma(one, d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
+            if (one) at_commit(done + b);
+            __syncwarp();
         }
     } else if (warp < FP_WARP_A) {
         // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
@@ -258,6 +288,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     __syncthreads();                                               // the stages have been read, the rows that are not finite are marked
     float* sums = reinterpret_cast<float*>(smem);                  // [NP][128], where K is cut
+    auto to = [&](int j) { return (size_t)(GROUPED && tiles.order != nullptr ? tiles.order[m0 + j] : m0 + j) * n + n0; };
     if (warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
         const int r = (warp & 3) * 32 + lane, j0 = ((warp - C::WARP_SUM) >> 2) * COLS;
         if (segments == 1) {
@@ -266,7 +297,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 for (int j = 0; j < COLS; ++j) {
                     float v = sum[j];
                     if (EPI == 1) v = cap * tanhf(v / cap);
-                    if (m0 + j0 + j < m) c[(size_t)(m0 + j0 + j) * n + n0 + r] = v;
+                    if (j0 + j < rows) c[to(j0 + j) + r] = v;
                 }
         } else {
 #pragma unroll
@@ -275,14 +306,14 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         if (*any_odd != 0 && n0 + r < n) {                         // this thread's elements of rows without pieces again
             const int k0 = chunk0 * FP_K, k1 = min(k, (chunk0 + chunks) * FP_K);
 #pragma unroll 1
-            for (int j = j0; j < min(j0 + COLS, m - m0); ++j) {
+            for (int j = j0; j < min(j0 + COLS, rows); ++j) {
                 if ((odd_rows[r] | odd_rows[FP_M + j]) == 0) continue;
-                const float *x = a + (size_t)(m0 + j) * k, *y = w + (size_t)(n0 + r) * k;
+                const float *x = a + (size_t)(m0 + j) * k, *y = w + (size_t)(w0 + r) * k;
                 float v = 0.f;
 #pragma unroll 1
                 for (int kk = k0; kk < k1; ++kk) v = fmaf(x[kk], y[kk], v);
                 if (segments > 1) sums[j * FP_M + r] = v;
-                else c[(size_t)(m0 + j) * n + n0 + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
+                else c[to(j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
             }
         }
     }
@@ -300,7 +331,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 v = s == 0 ? x : v + x;
             }
             if (EPI == 1) v = cap * tanhf(v / cap);
-            if (m0 + j < m && n0 + r < n) c[(size_t)(m0 + j) * n + n0 + r] = v;
+            if (j < rows && n0 + r < n) c[to(j) + r] = v;
         }
         fp_cluster_sync();                                         // nobody leaves while its sums are read
     }
@@ -342,7 +373,7 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     const int kp = (k + 7) & ~7;
     int* odd_rows = nullptr;
     KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535, "gemm_f32: a weight of %d rows is too much for one launch", n);
-    if (cudaFuncSetAttribute(gemm_f32_pieces_kernel<NP, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    if (cudaFuncSetAttribute(gemm_f32_pieces_kernel<NP, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
         return fail("gemm_f32: cannot have %d bytes of shared memory", C::SMEM);
     if (int e = encode_map_f32(&map_w, w, n, k, k, FP_M)) return e;
     if (C::CUTS) {
@@ -365,7 +396,7 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = segments;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, gemm_f32_pieces_kernel<NP, EPI>, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap);
+    cudaLaunchKernelEx(&cfg, gemm_f32_pieces_kernel<NP, EPI, false>, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
     return check_launch("gemm_f32 pieces");
 }
 
@@ -409,9 +440,32 @@ int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, in
 #undef KB_PIECES
 }
 
+// Whether the experts' 32-bit products of this inner size go by pieces.
+bool moe_f32_pieces_take(int k, const void* a, const void* w) { return k >= 256 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0; }
+
 }  // namespace kb
 
 using namespace kb;
+
+// c [places, n]: a [places, k] (in the lists' order) by the expert's weights w [experts, n, k], tiles of at most FP_CUT_ROWS rows; `order` not null: rows
+// placed by pair number. A block a tile and 128 columns, K in one: the tiles alone fill the GPU. 1,200 pairs of 16 experts of 2,048 x 1,024: see `moe_grouped`.
+extern "C" int kb_moe_f32_pieces_takes(const float* a, const float* w, int k) { return moe_f32_pieces_take(k, a, w) ? 1 : 0; }
+extern "C" int kb_moe_f32_pieces(float* c, const float* a, const float* w, int experts, const int* tile_expert, const int* tile_first, const int* tile_rows,
+                                 const int* n_tiles, int tile_cap, const int* order, int places, int n, int k, void* stream) {
+    using C = Pieces<FP_CUT_ROWS>;
+    KB_REQUIRE(experts > 0 && places >= 0 && n > 0 && k > 0 && tile_cap >= 0, "moe_f32: %d experts, %d places, n %d, k %d, %d tiles", experts, places, n, k, tile_cap);
+    KB_REQUIRE(k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0, "moe_f32: rows of %d values must begin at 16-byte boundaries", k);
+    KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535 && (long long)experts * n <= 0x7fffffffll, "moe_f32: %d experts of %d rows are too much for one launch", experts, n);
+    if (tile_cap == 0 || places == 0) return 0;
+    auto kernel = gemm_f32_pieces_kernel<FP_CUT_ROWS, 0, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) return fail("moe_f32: cannot have %d bytes of shared memory", C::SMEM);
+    CUtensorMap map_a, map_w;
+    if (int e = encode_map_f32(&map_a, a, places, k, k, FP_CUT_ROWS)) return e;
+    if (int e = encode_map_f32(&map_w, w, (unsigned long long)experts * n, k, k, FP_M)) return e;
+    kernel<<<dim3(tile_cap, (n + FP_M - 1) / FP_M), FP_THREADS, C::SMEM, (cudaStream_t)stream>>>(map_a, map_w, c, a, w, nullptr, places, n, k, (k + FP_K - 1) / FP_K, 0.f,
+                                                                                                  F32Tiles{tile_expert, tile_first, tile_rows, n_tiles, order});
+    return check_launch("moe_f32 pieces");
+}
 
 extern "C" int kb_gemm_f32_split_error() {
     int flag = 0, zero = 0;

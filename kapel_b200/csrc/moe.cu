@@ -529,9 +529,10 @@ moe_grouped_bf16_kernel(const GroupedParams p) {
 // `also` (a tensor or split-K partial sums of the output's shape, or none) is added behind the experts' sum: an
 // expert that every token uses.
 template <typename TO, typename TA>
-__global__ void moe_combine_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights,
-                                   long long rows, int width, int top, const Src<TA> also, const int* __restrict__ experts, int real,
-                                   const void* __restrict__ self, int self_dt) {
+__global__ void __launch_bounds__(256)
+moe_combine_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights,
+                   long long rows, int width, int top, const Src<TA> also, const int* __restrict__ experts, int real,
+                   const void* __restrict__ self, int self_dt) {
     dependent_wait();                                       // returns at once after a plain launch
     dependent_trigger();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -547,6 +548,43 @@ __global__ void moe_combine_kernel(TO* __restrict__ out, const float* __restrict
     }
     if (also.p != nullptr) acc += also.at((size_t)i);
     Elem<TO>::store(out + i, acc);
+}
+
+// The same, four neighbouring columns a thread and four experts' values asked for before the first is added: a column and an expert at a time, 1,360 rows of 2,048
+// with four experts took 27 us. For widths of a multiple of four and an addend of one slice.
+template <typename TO, typename TA>
+__global__ void __launch_bounds__(256)
+moe_combine_fours_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights, long long rows, int width, int top,
+                         const TA* __restrict__ also, const int* __restrict__ experts, int real, const void* __restrict__ self, int self_dt) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
+    const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * 4;
+    if (i >= rows * width) return;
+    const long long r = i / width;
+    const int c = (int)(i - r * width);
+    float4 own = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (experts != nullptr) own = self_dt == KB_DT_F32 ? load_four(static_cast<const float*>(self) + i) : load_four(static_cast<const bf16*>(self) + i);
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int t0 = 0; t0 < top; t0 += 4) {
+        float4 v[4];
+        float w[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            const bool there = t0 + u < top;
+            w[u] = there ? weights[r * top + t0 + u] : 0.f;
+            v[u] = own;
+            if (there && (experts == nullptr || experts[r * top + t0 + u] < real)) v[u] = load_four(y + ((size_t)r * top + t0 + u) * width + c);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (t0 + u < top)
+                acc.x = fmaf(w[u], v[u].x, acc.x), acc.y = fmaf(w[u], v[u].y, acc.y), acc.z = fmaf(w[u], v[u].z, acc.z), acc.w = fmaf(w[u], v[u].w, acc.w);
+    }
+    if (also != nullptr) {
+        const float4 a = load_four(also + i);
+        acc.x += a.x, acc.y += a.y, acc.z += a.z, acc.w += a.w;
+    }
+    store_four(out + i, acc);
 }
 
 }  // namespace kb
@@ -666,12 +704,14 @@ extern "C" int kb_moe_combine(void* out, int out_dt, const float* y, const float
     const long long blocks = (rows * width + 255) / 256;
     KB_REQUIRE(blocks <= 0x7fffffffll, "moe_combine: too many rows for one launch");
     cudaStream_t s = (cudaStream_t)stream;
+    const bool fours = width % 4 == 0 && (also == nullptr || also_splits == 1) && (((uintptr_t)out | (uintptr_t)y | (uintptr_t)also | (uintptr_t)self) & 15) == 0;
 #define KB_COMBINE(TO, TA) \
-    launch_dependent_if(rows <= DEPENDENT_ROWS, moe_combine_kernel<TO, TA>, dim3((unsigned)blocks), dim3(256), 0, s, (TO*)out, y, weights, rows, width, top, Src<TA>{(const TA*)also, also ? also_splits : 1, (size_t)also_stride}, experts, real, self, self_dt)
+    if (fours) launch_dependent_if(rows <= DEPENDENT_ROWS, moe_combine_fours_kernel<TO, TA>, dim3((unsigned)((rows * width / 4 + 255) / 256)), dim3(256), 0, s, (TO*)out, y, weights, rows, width, top, (const TA*)also, experts, real, self, self_dt); \
+    else launch_dependent_if(rows <= DEPENDENT_ROWS, moe_combine_kernel<TO, TA>, dim3((unsigned)blocks), dim3(256), 0, s, (TO*)out, y, weights, rows, width, top, Src<TA>{(const TA*)also, also ? also_splits : 1, (size_t)also_stride}, experts, real, self, self_dt)
     const bool narrow = also != nullptr && also_dt == KB_DT_BF16;
     KB_REQUIRE(also == nullptr || also_dt == KB_DT_F32 || also_dt == KB_DT_BF16, "moe_combine: addend dtype code %d is not known", also_dt);
-    if (out_dt == KB_DT_F32) { if (narrow) KB_COMBINE(float, bf16); else KB_COMBINE(float, float); }
-    else if (out_dt == KB_DT_BF16) { if (narrow) KB_COMBINE(bf16, bf16); else KB_COMBINE(bf16, float); }
+    if (out_dt == KB_DT_F32) { if (narrow) { KB_COMBINE(float, bf16); } else { KB_COMBINE(float, float); } }
+    else if (out_dt == KB_DT_BF16) { if (narrow) { KB_COMBINE(bf16, bf16); } else { KB_COMBINE(bf16, float); } }
     else return fail("moe_combine: output dtype code %d is not known", out_dt);
 #undef KB_COMBINE
     return check_launch("moe_combine");

@@ -82,3 +82,54 @@ def test_which_products_go_that_way():
     got, want = K.gemm(a, w, softcap=30.0).double(), 30.0 * torch.tanh(a.double() @ w.double().T / 30.0)
     assert (got - want).abs().max() <= 1e-4
     K.check_async_errors()
+
+
+@pytest.mark.parametrize("tokens,top,experts,n,k", [(1, 1, 3, 130, 256), (9, 4, 5, 128, 1028), (150, 2, 4, 300, 512), (70, 3, 20, 64, 260)])
+def test_experts_products(tokens, top, experts, n, k):
+    """By lists of rows with gaps (experts without rows, pairs of no expert) against 64-bit and against the multiply-adds, rows by token and by place."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    chosen = torch.randint(0, experts + 2, (tokens, top), device="cuda", generator=gen, dtype=torch.int32)     # the last two have no weights
+    if experts > 3:
+        chosen[chosen == 1] = 2
+    a, w = torch.randn(tokens, k, device="cuda", generator=gen), torch.randn(experts, n, k, device="cuda", generator=gen)
+    a[tokens // 2, 3] = float("inf")
+    lists = K.moe_sort(chosen, experts, torch.float32)
+    pairs = (chosen.reshape(-1) < experts).nonzero()[:, 0]
+    rows, which = pairs // top, chosen.reshape(-1)[pairs].long()
+    want = torch.einsum("pk,pnk->pn", a[rows].double(), w[which].double())
+    sizes = torch.einsum("pk,pnk->pn", a[rows].abs().double(), w[which].abs().double())
+    got = K.moe_grouped(a, w, lists, "none", True, True, torch.float32)[pairs]
+    known = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), known)
+    assert ((got - want)[known].abs() <= ((4 * 2.0 ** -23 + (k // 64 + 2) * 2.0 ** -24) * sizes)[known]).all()
+    by_place = K.moe_grouped(a, w, lists, "none", True, False, torch.float32)
+    listed = int(lists.offsets[-1])
+    order = lists.order[:listed].long()
+    where = torch.empty(tokens * top, dtype=torch.long, device="cuda")
+    where[order] = torch.arange(listed, device="cuda")
+    assert torch.equal(torch.nan_to_num(by_place[where[pairs]]), torch.nan_to_num(got))
+    # the second product: rows by place in, rows by pair out
+    back = torch.randn(experts, 36, n // 4 * 4, device="cuda", generator=gen)
+    inner = torch.nan_to_num(by_place[:, : n // 4 * 4], 0.0, 0.0, 0.0).contiguous()
+    out = K.moe_grouped(inner, back, lists, "none", False, True, torch.float32)[pairs]
+    want = torch.einsum("pk,pnk->pn", inner[where[pairs]].double(), back[which].double())
+    assert float((out - want).norm()) <= 1e-6 * float(want.norm())
+    K.check_async_errors()
+
+
+@pytest.mark.parametrize("tokens,width,top", [(1, 4, 1), (33, 2048, 4), (513, 12, 5), (7, 7, 3)])
+def test_experts_sum_by_fours_and_one_by_one(tokens, width, top):
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(width)
+    y, weights = torch.randn(tokens * top, width, device="cuda", generator=gen), torch.rand(tokens, top, device="cuda", generator=gen)
+    own, also = torch.randn(tokens, width, device="cuda", generator=gen), torch.randn(tokens, width, device="cuda", generator=gen)
+    experts = torch.randint(0, 6, (tokens, top), device="cuda", generator=gen, dtype=torch.int32)
+    pad = lambda t: torch.cat([torch.zeros(1, device="cuda"), t.reshape(-1)])[1:].view(t.shape)                # one element further: not by fours
+    for kw in ({}, {"experts": experts, "real": 4, "own": own}):
+        for extra in (None, also):
+            a = K.moe_combine(y, weights, torch.float32, also=extra, **kw)
+            b = K.moe_combine(pad(y), weights, torch.float32, also=extra, **kw)
+            assert torch.equal(a, b)
