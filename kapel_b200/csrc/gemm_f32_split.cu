@@ -61,20 +61,6 @@ __device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t
     odd = fmaf(x, y, odd);
 }
 
-// 1 in one lane of the warp, the same one every time.
-__device__ __forceinline__ uint32_t fp_elect() {
-    uint32_t one;
-    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(one));
-    return one;
-}
-// at_mma_ts in the lane that has `one`
-__device__ __forceinline__ void fp_mma(uint32_t one, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
-}
-
 __device__ __forceinline__ void fp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -118,7 +104,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     const int chunk0 = segment * chunks_a_segment, chunks = max(0, min(chunks_a_segment, chunks_all - chunk0));
 
     if (tid == 0) {
-        for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 8 : 4); }
+        for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 6 : 4); }      // the warps that cut the stage
         for (int b = 0; b < 2; ++b) {
             at_mbar_init(cut + b, C::CUTS ? 12 : 8);
             at_mbar_init(a_full + b, 1);
@@ -170,12 +156,12 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
             if (!__all_sync(0xffffffffu, there)) { failed = true; break; }
             at_fence_after();
-            const uint32_t one = fp_elect();
+            const uint32_t one = at_elect();
 #pragma unroll
             for (int p = 0; p < PIECE_PRODUCTS; ++p)
 #pragma unroll
                 for (int kk = 0; kk < FP_K / 16; ++kk)
-                    fp_mma(one, d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
+                    at_mma_ts_if(one, d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
             if (one) at_commit(done + b);
             __syncwarp();
         }
@@ -211,16 +197,17 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
         if (odd != odd) odd_rows[row] = 1, *any_odd = 1;
     } else if (C::CUTS && warp < C::WARP_SUM) {
-        // ---------------------------------------------------------------- cutting a few rows of A
-        const int t = (warp - FP_WARP_A) * 32 + lane, row = t % NP;
+        // ---------------------------------------------------------------- cutting a few rows of A, two warps a half of the chunk
+        const int half = (warp - FP_WARP_A) >> 1, t = ((warp - FP_WARP_A) & 1) * 32 + lane, row = t % NP;
         float odd = 0.f;
-        for (int it = 0; it < 2 * chunks; ++it) {
-            const int s = it % C::STAGES, ch = it >> 1, b = ch & 1, half = it & 1;
+        for (int ch = 0; ch < chunks; ++ch) {
+            const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
-            if (half == 0 && !__all_sync(0xffffffffu, at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u))) { failed = true; break; }
+            if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u))) { failed = true; break; }
             const unsigned char* from = smem + s * C::STAGE + C::W_BYTES + row * 128;
             unsigned char* to = pieces + b * C::PIECES + row * 128;
-            for (int i = t; i < NP * 4; i += 128) {                // eight values at a time
+#pragma unroll
+            for (int i = t; i < NP * 4; i += 64) {                 // eight values at a time
                 const int g = i / NP;
                 const float4 x = *reinterpret_cast<const float4*>(from + (((2 * g) ^ (row & 7)) << 4));
                 const float4 y = *reinterpret_cast<const float4*>(from + (((2 * g + 1) ^ (row & 7)) << 4));
@@ -234,11 +221,11 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 *reinterpret_cast<uint4*>(to + C::PIECE + at) = two;
                 *reinterpret_cast<uint4*>(to + 2 * C::PIECE + at) = three;
             }
-            if (half == 1) at_fence_async_smem();                  // the MMAs read what was written here
+            at_fence_async_smem();                                 // the MMAs read what was written here
             __syncwarp();
             if (lane == 0) {
                 at_mbar_arrive(empty + s);
-                if (half == 1) at_mbar_arrive(cut + b);
+                at_mbar_arrive(cut + b);
             }
         }
         if (odd != odd) odd_rows[FP_M + row] = 1, *any_odd = 1;
@@ -400,30 +387,30 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     return check_launch("gemm_f32 pieces");
 }
 
-// Segments of K: the waves of blocks times what a block takes, a chunk 0.85 us with up to 32 rows, 1.1 with 64, 1.5 with 128, and 6 or (in a
-// cluster) 8 us to begin and end. A block takes a multiprocessor; clusters of four and eight do not fit every group of them, so that seven
+// Segments of K: the waves of blocks times what a block takes, a chunk 0.65 us with up to 32 rows, 0.7 with 64, 1.2 with 128, and 5 or (in a
+// cluster) 6.5 us to begin and end. A block takes a multiprocessor; clusters of four and eight do not fit every group of them, so that seven
 // eighths and three quarters run at once (144 blocks in clusters of eight: two waves). Of 95 sizes (512 to 18,432 weight rows of 1,024 to 9,216, 1
 // to 500 rows) the choice is the fastest of the four in all, or within 3 % of it.
 int gemm_f32_segments(int m, int n, int k) {
     const int tiles = ((m + 127) / 128) * ((n + FP_M - 1) / FP_M), chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
-    const double chunk_us = m > 64 ? 1.5 : m > 32 ? 1.12 : 0.85;
+    const double chunk_us = m > 64 ? 1.2 : m > 32 ? 0.68 : 0.65;
     int best = 1;
     double least = 0;
     for (int s = 1; s <= 8 && s <= chunks; s *= 2) {
         const int at_once = s <= 2 ? sms : (s == 4 ? sms * 7 / 8 : sms * 3 / 4) / s * s;
-        const double us = (double)((tiles * s + at_once - 1) / at_once) * ((chunks + s - 1) / s * chunk_us + (s == 1 ? 6.0 : 8.0));
+        const double us = (double)((tiles * s + at_once - 1) / at_once) * ((chunks + s - 1) / s * chunk_us + (s == 1 ? 5.0 : 6.5));
         if (s == 1 || us < least) least = us, best = s;
     }
     return best;
 }
 // More than 16 rows of 256 and more, and three to 16 of 1,024 and more: one accumulator an element in ascending k, a kernel for each, is limited by
-// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 32. 500 rows by 18,432 x 2,304: 824 us by
-// chains, 223 by pieces; by 2,304 x 9,216 545 and 122, by 2,304 x 2,048 131 and 35, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
-// 12 (64 rows 9.3 and 8.8). Six rows: 54 and 40, 72 and 39, 18 and 14, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 39, 51 and 39, 14 and 14, 13 and
-// 9 as long as the tiles are one wave (256,000 x 2,304: 440 and 500); one row 37 and 39, 32 and 39. The error against 64 bits is 0.07 to 0.3 of the
+// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
+// chains, 204 by pieces; by 2,304 x 9,216 545 and 118, by 2,304 x 2,048 131 and 31, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
+// 12 (64 rows 9.3 and 8.8). Six rows: 54 and 31, 72 and 30, 18 and 11, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 31, 51 and 30, 14 and 12,
+// 13 and 9, by 256,000 x 2,304 440 and 384; one row 37 and 31, 32 and 30, 9.5 and 11.6, 355 and 384. The error against 64 bits is 0.07 to 0.3 of the
 // chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
-bool gemm_f32_pieces_take(int m, int n, int k, const void* a, const void* w) {
-    const bool pays = m > 16 ? k >= 256 : k >= 1024 && (m > 4 || (m > 2 && n <= FP_M * multiprocessors()));
+bool gemm_f32_pieces_take(int m, int k, const void* a, const void* w) {
+    const bool pays = m > 16 ? k >= 256 : m > 2 && k >= 1024;
     return pays && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
 }
 long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * (3 * ((k + 7) / 8 * 4) + 1); }
