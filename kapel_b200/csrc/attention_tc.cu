@@ -248,53 +248,55 @@ attention_tc_kernel(const AttTcParams p, const __grid_constant__ CUtensorMap map
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- the score products, from one lane
-        if (lane == 0) {
+        {                                                       // the whole warp: see at_elect()
+            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t IDESC_S = at_idesc(AT_ROWS, AT_KEYS, false);
             const uint32_t ring_addr = at_saddr(ring);
             for (int kt = 0; kt < n_tiles; ++kt) {               // S[kt & 1] = Q K(kt)^T
                 const int s = kt % KS, b = kt & 1;
-                if (!at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u)) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
                 // the buffer still holds tile kt - 2's P until the product that reads it is complete
-                if (kt >= 2 && !at_mbar_wait(s_free + b, (uint32_t)((kt - 2) >> 1) & 1u)) { failed = true; break; }
+                if (kt >= 2 && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)((kt - 2) >> 1) & 1u))) { failed = true; break; }
                 at_fence_after();
                 const uint32_t k_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t d_tmem = tmem + (uint32_t)(C::COL_S + b * AT_KEYS);
+                const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);
 #pragma unroll
                 for (int bx = 0; bx < NBOX; ++bx) {
-                    const uint32_t a_tmem = tmem + (uint32_t)(C::COL_Q + bx * 32);          // 64 elements of Q: 32 columns
+                    const uint32_t a_tmem = tm + (uint32_t)(C::COL_Q + bx * 32);          // 64 elements of Q: 32 columns
                     const uint64_t bdesc = at_desc(k_addr + bx * (AT_KEYS * 128), 16, 1024);
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        at_mma_ts(d_tmem, a_tmem + (uint32_t)(kk * 8), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
+                        at_mma_ts_if(one, d_tmem, a_tmem + (uint32_t)(kk * 8), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
                 }
-                at_commit(empty + s);                            // the key slot is free when S is complete
-                at_commit(s_full + b);
+                if (one) at_commit(empty + s);                            // the key slot is free when S is complete
+                if (one) at_commit(s_full + b);
             }
         }
     } else if (warp == AT_WARP_PV) {
         // ---------------------------------------------------------------- the P V products, from one lane
-        if (lane == 0) {
+        {                                                       // the whole warp: see at_elect()
+            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t PAGE_BYTES = NBOX * 2048u;
             constexpr uint32_t IDESC_O = at_idesc(AT_ROWS, HD, true);
             const uint32_t ring_addr = at_saddr(ring);
             for (int kt = 0; kt < n_tiles; ++kt) {
                 const int b = kt & 1;
                 const int s = KS + kt % VS;
-                if (!at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u)) { failed = true; break; }
-                if (!at_mbar_wait(p_full + b, (uint32_t)(kt >> 1) & 1u)) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt >> 1) & 1u))) { failed = true; break; }
                 at_fence_after();
                 const uint32_t v_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t a_tmem = tmem + (uint32_t)(C::COL_S + b * AT_KEYS);          // P lies over its S
+                const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);          // P lies over its S
 #pragma unroll
                 for (int kk = 0; kk < 4; ++kk) {
                     // keys 16 kk ..: page kk of the tile, its two eight-key groups 1 KB apart, chunks 2 KB apart
                     const uint64_t bdesc = at_desc(v_addr + (uint32_t)kk * PAGE_BYTES, 2048, 1024);
-                    at_mma_ts(tmem + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
+                    at_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
                 }
-                at_commit(empty + s);
-                at_commit(s_free + b);                           // P has been read: the scores of tile kt + 2 may land
+                if (one) at_commit(empty + s);
+                if (one) at_commit(s_free + b);                           // P has been read: the scores of tile kt + 2 may land
             }
-            if (!failed) at_commit(o_full);
+            if (!failed && one) at_commit(o_full);
         }
     } else if (warp >= 2 && warp < 10) {
         // ---------------------------------------------------------------- softmax and epilogue, half a row a thread
@@ -448,11 +450,11 @@ __device__ __forceinline__ void atp_arrive_on_first(uint64_t* bar) {
         "mbarrier.arrive.release.cluster.shared::cluster.b64 _, [ra];\n\t}"
         ::"r"(at_saddr(bar)) : "memory");
 }
-__device__ __forceinline__ void atp_mma_ss(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void atp_mma_ss_if(uint32_t one, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
 }
 // The same without the release: for a signal that only says "my tcgen05.st has completed" (the store was
 // waited for and fenced with tcgen05.fence::before_thread_sync), which needs no ordering of ordinary
@@ -466,11 +468,11 @@ __device__ __forceinline__ void atp_arrive_on_first_relaxed(uint64_t* bar) {
 __device__ __forceinline__ void atp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void atp_mma_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+__device__ __forceinline__ void atp_mma_ts_if(uint32_t one, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %4, 0;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(one) : "memory");
 }
 
 constexpr int ATP_ROWS = 256;                                   // rows a tile of the pair kernel
@@ -665,53 +667,55 @@ attention_tc_pair_kernel(const AttTcParams p, const __grid_constant__ CUtensorMa
         }
     } else if (warp == 1) {
         // ---------------------------------------------------------------- the score products of both blocks, from one lane of the first
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                                        // the whole warp: see at_elect()
+            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t IDESC_S = at_idesc(ATP_ROWS, ATP_KEYS, false);
             const uint32_t ring_addr = at_saddr(ring);
             const uint32_t q_addr = at_saddr(q_smem);
             for (int kt = 0; kt < n_tiles; ++kt) {               // S[kt % SB] = Q K(kt)^T
                 const int s = kt % KS, b = kt % SB;
-                if (!at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u)) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
                 // the buffer still holds tile kt - SB's P until the product that reads it is complete
-                if (kt >= SB && !at_mbar_wait(s_free + b, (uint32_t)(kt / SB - 1) & 1u)) { failed = true; break; }
+                if (kt >= SB && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)(kt / SB - 1) & 1u))) { failed = true; break; }
                 at_fence_after();
                 const uint32_t k_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t d_tmem = tmem + (uint32_t)(C::COL_S + b * ATP_KEYS);
+                const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * ATP_KEYS);
 #pragma unroll
                 for (int bx = 0; bx < NBOX; ++bx) {
                     const uint64_t adesc = at_desc(q_addr + bx * (AT_ROWS * 128), 16, 1024);        // 64 elements of the 128 rows
                     const uint64_t bdesc = at_desc(k_addr + bx * (ATP_KEYS / 2 * 128), 16, 1024);  // this chunk's 64 keys a block
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
-                        atp_mma_ss(d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
+                        atp_mma_ss_if(one, d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
                 }
-                atp_commit_both(empty + s);                      // the key slot is free in both blocks when S is complete
-                atp_commit_both(s_full + b);
+                if (one) atp_commit_both(empty + s);                      // the key slot is free in both blocks when S is complete
+                if (one) atp_commit_both(s_full + b);
             }
         }
     } else if (warp == AT_WARP_PV) {
         // ---------------------------------------------------------------- the P V products of both blocks
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {                                        // the whole warp: see at_elect()
+            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t IDESC_O = at_idesc(ATP_ROWS, HD, true);
             const uint32_t ring_addr = at_saddr(ring);
             for (int kt = 0; kt < n_tiles; ++kt) {
                 const int b = kt % SB;
                 const int s = KS + kt % VS;
-                if (!at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u)) { failed = true; break; }
-                if (!at_mbar_wait(p_full + b, (uint32_t)(kt / SB) & 1u)) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
+                if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt / SB) & 1u))) { failed = true; break; }
                 at_fence_after();
                 const uint32_t v_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t a_tmem = tmem + (uint32_t)(C::COL_S + b * ATP_KEYS);         // P lies over the first half of its S
+                const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * ATP_KEYS);         // P lies over the first half of its S
 #pragma unroll
                 for (int kk = 0; kk < ATP_KEYS / 16; ++kk) {
                     // keys 16 kk ..: page kk, its two eight-key groups 1 KB apart, this block's chunks 2 KB apart
                     const uint64_t bdesc = at_desc(v_addr + (uint32_t)kk * PAGE_HALF, 2048, 1024);
-                    atp_mma_ts(tmem + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
+                    atp_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
                 }
-                atp_commit_both(empty + s);
-                atp_commit_here(s_free + b);                     // P has been read: the scores of tile kt + SB may land
+                if (one) atp_commit_both(empty + s);
+                if (one) atp_commit_here(s_free + b);                     // P has been read: the scores of tile kt + SB may land
             }
-            if (!failed) atp_commit_both(o_full);
+            if (!failed && one) atp_commit_both(o_full);
         }
     } else if ((warp >= 2 && warp < 10) || warp >= 13) {
         // ---------------------------------------------------------------- softmax and epilogue: a row's 32 keys of a step a thread
