@@ -37,6 +37,30 @@ __global__ void embed_kernel(float* __restrict__ out, const T* __restrict__ tabl
     for (int i = threadIdx.x; i < width; i += blockDim.x) o[i] = Elem<T>::load(t + i) * scale;
 }
 
+// The same, four neighbouring values a thread and a row's copies by one block, which reads the row once: 1,360 rows of 2,048 in four streams 23 us
+// by a value and a copy at a time. For widths of a multiple of four.
+template <typename T>
+__global__ void __launch_bounds__(512)
+embed_fours_kernel(float* __restrict__ out, const T* __restrict__ table, const int* __restrict__ ids, int width, int vocab, float scale,
+                   const T* __restrict__ pos_table, const int* __restrict__ positions, int max_positions, int copies) {
+    const int r = blockIdx.x, id = ids[r], pos = pos_table != nullptr ? positions[r] : -1;
+    const bool there = id >= 0 && id < vocab, moved = pos >= 0 && pos < max_positions;
+    float* o = out + (size_t)r * copies * width;
+    for (int i = threadIdx.x * 4; i < width; i += blockDim.x * 4) {
+        float4 v = make_float4(__int_as_float(0x7fc00000), __int_as_float(0x7fc00000), __int_as_float(0x7fc00000), __int_as_float(0x7fc00000));
+        if (there) {
+            const float4 t = load_four(table + (size_t)id * width + i);
+            if (moved) {
+                const float4 p = load_four(pos_table + (size_t)pos * width + i);
+                v = make_float4(t.x * scale + p.x, t.y * scale + p.y, t.z * scale + p.z, t.w * scale + p.w);
+            } else {
+                v = make_float4(t.x * scale, t.y * scale, t.z * scale, t.w * scale);
+            }
+        }
+        for (int c = 0; c < copies; ++c) store_four(o + (size_t)c * width + i, v);
+    }
+}
+
 // ---------------------------------------------------------------------------------------
 // cos_sin[r, j] = (cos, sin)(positions[r] * theta^(-2j / rotary) / divisor), angle in 64-bit
 // (`divisor` 1: plain; f: every frequency divided by f, "linear scaling" of the positions).
@@ -395,6 +419,14 @@ extern "C" int kb_embed(float* out, const void* table, int table_dt, const int* 
     if (rows == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const int threads = width >= 1024 ? 256 : 128;
+    if (width % 4 == 0 && (((uintptr_t)out | (uintptr_t)table | (uintptr_t)pos_table) & 15) == 0 && (table_dt == KB_DT_F32 || table_dt == KB_DT_BF16)) {
+        const int fours = width >= 2048 ? 512 : threads;
+        if (table_dt == KB_DT_F32)
+            embed_fours_kernel<float><<<rows, fours, 0, s>>>(out, (const float*)table, ids, width, vocab, scale, (const float*)pos_table, positions, max_positions, copies);
+        else
+            embed_fours_kernel<bf16><<<rows, fours, 0, s>>>(out, (const bf16*)table, ids, width, vocab, scale, (const bf16*)pos_table, positions, max_positions, copies);
+        return check_launch("embed");
+    }
     if (table_dt == KB_DT_F32)
         embed_kernel<float><<<rows * copies, threads, 0, s>>>(out, (const float*)table, ids, rows, width, vocab, scale, (const float*)pos_table, positions, max_positions, copies);
     else if (table_dt == KB_DT_BF16)
