@@ -7,8 +7,9 @@
 // rounds an input; exponentials and soft caps are the library's. Sums go by pieces (chains of 8 components; of 64 keys, then of 256), so that their
 // rounding is no larger than the row-wise kernel's, whose lanes and chunks cut them as short: 0.7 to 0.99 of its error against 64 bits at 500
 // to 4,608 keys, where one chain a sum had 1.8 to 4.7 times as much and took 139 us instead of 147. Shared memory's 32 words a clock bound it (0.75
-// and 0.38 words a multiply-add), and how few blocks a short prompt gives: 147 us for those 500 tokens, which is what the 8 steps of the last
-// rows' block take. With heads of 128 two blocks share a multiprocessor.
+// and 0.38 words a multiply-add), and how few blocks a short prompt gives: 146 us for those 500 tokens by a block a tile, which is what the 8 steps of
+// the last rows' block take. With heads of 128 two blocks share a multiprocessor. Where the tiles are few, a cluster of two blocks takes one, every second
+// step each, and the first merges what the second leaves in its shared memory: 99 us.
 #include <type_traits>
 #include "common.cuh"
 
@@ -31,7 +32,25 @@ struct F32TileParams {
     float scale, cap;
 };
 
-template <int D>
+__device__ __forceinline__ void aft_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A float at the same place in the cluster's block `rank`.
+__device__ __forceinline__ float aft_remote(const float* at, int rank) {
+    float v;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
+                 : "=f"(v) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(rank) : "memory");
+    return v;
+}
+__device__ __forceinline__ float4 aft_remote_four(const float* at, int rank) {
+    float4 v;
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %4, %5;\n\tld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [ra];\n\t}"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"((uint32_t)__cvta_generic_to_shared(at)), "r"(rank) : "memory");
+    return v;
+}
+
+// PARTS: blocks (of a cluster, along z) a tile, 1 or 2
+template <int D, int PARTS>
 __global__ void __launch_bounds__(AFT_THREADS, D == 128 ? 2 : 1)
 attention_f32_tiles_kernel(const F32TileParams p) {
     constexpr int LD = D + 4, D4 = D / 4, CG = D / 128;          // column groups of four a lane holds: 4 (lane + 32 g)
@@ -50,13 +69,15 @@ attention_f32_tiles_kernel(const F32TileParams p) {
     const int c_first = p.row_count[row0];
     const int klo = (p.window > 0 && c_first > p.window) ? c_first - p.window : 0;
     const int khi = c_first > 0 ? c_first + nq - 1 : 0;          // a padding row sees nothing
+    constexpr int stride = AFT_KEYS * PARTS;
+    const int part = PARTS == 1 ? 0 : blockIdx.z, from_key = klo + part * AFT_KEYS;      // this block's steps
     auto fetch = [&](float* to, const float* table, int k0) {
         for (int key = warp; key < AFT_KEYS; key += AFT_THREADS / 32) {      // a warp a line; keys nobody sees are zeros
             const int pos = k0 + key, lp = pos / p.page_size;
             int page = -1;
             if (pos < khi && lp < p.table_width) page = p.block_table[(size_t)entry * p.table_width + lp];
             const bool there = page >= 0 && page < p.n_pages;
-            if (table == p.k_table && lane == 0) paged[((k0 - klo) / AFT_KEYS & 1) * AFT_KEYS + key] = there;
+            if (table == p.k_table && lane == 0) paged[((k0 - klo) / stride & 1) * AFT_KEYS + key] = there;
             const float* from = there ? table + kv_row((long long)page * p.page_size + pos % p.page_size, kvh, p.hkv, p.page_size) * D : table;
             for (int x = lane; x < D4; x += 32)
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(to + key * LD + x * 4)), "l"(from + x * 4), "r"(there ? 16 : 0) : "memory");
@@ -97,12 +118,12 @@ attention_f32_tiles_kernel(const F32TileParams p) {
         }
         l = fmaf(l, l_fade, l_near), l_near = 0.f, l_fade = 1.f;
     };
-    if (klo < khi) {
-        fetch(sk, p.k_table, klo);
-        fetch(sv, p.v_table, klo);
+    if (from_key < khi) {
+        fetch(sk, p.k_table, from_key);
+        fetch(sv, p.v_table, from_key);
     }
-    for (int k0 = klo; k0 < khi; k0 += AFT_KEYS) {
-        const bool more = k0 + AFT_KEYS < khi;
+    for (int k0 = from_key; k0 < khi; k0 += stride) {
+        const bool more = k0 + stride < khi;
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();                                         // the keys are there
         {
@@ -136,11 +157,11 @@ attention_f32_tiles_kernel(const F32TileParams p) {
                 for (int j = 0; j < 4; ++j) sp[(2 * qy + i) * (AFT_KEYS + 4) + qx + 16 * j] = s[i][j];
         }
         __syncthreads();                                         // the scores are there, the keys are done with
-        if (more) fetch(sk, p.k_table, k0 + AFT_KEYS);
+        if (more) fetch(sk, p.k_table, k0 + stride);
         else asm volatile("cp.async.commit_group;" ::: "memory");
         {
             float w[8], top = -INFINITY;
-            const int* there = paged + ((k0 - klo) / AFT_KEYS & 1) * AFT_KEYS;
+            const int* there = paged + ((k0 - klo) / stride & 1) * AFT_KEYS;
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const int key = k0 + sc + 8 * j;
@@ -202,13 +223,47 @@ attention_f32_tiles_kernel(const F32TileParams p) {
             for (int c = 0; c < 4 * CG; ++c) near[i][c] = fmaf(near[i][c], f, now[i][c]);
             o_fade[i] *= f;
         }
-        if (((k0 - klo) / AFT_KEYS & 3) == 3) gather();
+        if (((k0 - klo) / stride & 3) == 3) gather();
         __syncthreads();                                         // the values and the weights are done with
-        if (more) fetch(sv, p.v_table, k0 + AFT_KEYS);
+        if (more) fetch(sv, p.v_table, k0 + stride);
         else asm volatile("cp.async.commit_group;" ::: "memory");
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     gather();
+    if constexpr (PARTS == 2) {
+        float* ml = sp;                                          // [2][32] a row's maximum and sum, where scores were
+        __syncthreads();                                         // the last step's weights and values have been read
+        if (part == 1) {
+            if (sc == 0) ml[sr] = m, ml[AFT_ROWS + sr] = l;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                for (int g = 0; g < CG; ++g)
+                    *reinterpret_cast<float4*>(sk + (4 * warp + i) * LD + 4 * (lane + 32 * g)) = make_float4(o[i][4 * g], o[i][4 * g + 1], o[i][4 * g + 2], o[i][4 * g + 3]);
+        }
+        aft_cluster_sync();
+        if (part == 0) {
+            if (sc == 0) {                                       // both parts' sums against the larger maximum
+                const float m1 = aft_remote(ml + sr, 1), l1 = aft_remote(ml + AFT_ROWS + sr, 1), top = fmaxf(m, m1);
+                const float f0 = m == -INFINITY ? 0.f : expf(m - top), f1 = m1 == -INFINITY ? 0.f : expf(m1 - top);
+                m = top, l = fmaf(l, f0, l1 * f1);
+                ml[sr] = f0, ml[AFT_ROWS + sr] = f1;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float f0 = ml[4 * warp + i], f1 = ml[AFT_ROWS + 4 * warp + i];
+#pragma unroll
+                for (int g = 0; g < CG; ++g) {
+                    const float4 v = aft_remote_four(sk + (4 * warp + i) * LD + 4 * (lane + 32 * g), 1);
+                    o[i][4 * g] = fmaf(o[i][4 * g], f0, v.x * f1), o[i][4 * g + 1] = fmaf(o[i][4 * g + 1], f0, v.y * f1);
+                    o[i][4 * g + 2] = fmaf(o[i][4 * g + 2], f0, v.z * f1), o[i][4 * g + 3] = fmaf(o[i][4 * g + 3], f0, v.w * f1);
+                }
+            }
+        }
+        aft_cluster_sync();                                      // nobody leaves while its sums are read
+        if (part == 1) return;
+    }
     if (sc == 0) {
         float inv = 0.f;
         if (l > 0.f) {
@@ -234,17 +289,38 @@ attention_f32_tiles_kernel(const F32TileParams p) {
     }
 }
 
-template <int D>
-static int launch_f32_tiles(const F32TileParams& p, int tiles, cudaStream_t s) {
+template <int D, int PARTS>
+static int launch_f32_tiles_parts(const F32TileParams& p, int tiles, cudaStream_t s) {
     constexpr int smem = ((AFT_ROWS + 2 * AFT_KEYS) * (D + 4) + AFT_ROWS * (AFT_KEYS + 4) + AFT_ROWS + 2 * AFT_KEYS) * (int)sizeof(float);
     static bool attr_set = false;
     if (!attr_set) {
-        if (cudaFuncSetAttribute(attention_f32_tiles_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(attention_f32_tiles_kernel<D, PARTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return fail("attention_f32_tiles: cannot have %d bytes of shared memory", smem);
         attr_set = true;
     }
-    attention_f32_tiles_kernel<D><<<dim3(p.hkv, tiles), AFT_THREADS, smem, s>>>(p);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.hkv, tiles, PARTS);
+    cfg.blockDim = AFT_THREADS;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = PARTS;
+    cfg.attrs = attr;
+    cfg.numAttrs = PARTS > 1 ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, attention_f32_tiles_kernel<D, PARTS>, p);
     return check_launch("attention_f32_tiles");
+}
+
+// Two blocks a tile while the tiles are no more than the GPU takes at once; if a window makes them alike, while the blocks are. In us, one block and two: 16
+// tokens of 8 heads over 4 of 256 behind 1,024 (4 tiles) 291 and 164, 500 tokens behind 0 and 1,024 (128 tiles) 146 and 99, 431 and 373; of 16 over 4 of
+// 128 (252) 121 and 90, 392 and 356. 500 behind 1,024 with a window of 512: 162 and 186, 155 and 177. More tiles: 800 tokens of 256 (200 tiles) 227 and
+// 213, with a window of 512 158 and 197; 1,000 tokens of 128 (500) 246 and 287, of 256 (252) 288 and 304.
+template <int D>
+static int launch_f32_tiles(const F32TileParams& p, int tiles, cudaStream_t s) {
+    const long long at_once = (long long)multiprocessors() * (D == 128 ? 2 : 1), blocks = (long long)p.hkv * tiles;
+    const bool alike = p.window > 0 && p.window < (long long)p.table_width * p.page_size;
+    return (alike ? 2 : 1) * blocks <= at_once ? launch_f32_tiles_parts<D, 2>(p, tiles, s) : launch_f32_tiles_parts<D, 1>(p, tiles, s);
 }
 
 }  // namespace kb

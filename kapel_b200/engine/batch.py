@@ -78,8 +78,9 @@ def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: in
     behind 256, 1,024 and 4,096 positions 89 and 145, 292 and 149, 1,101 and 219; 128 tokens behind 1,024 and 16,384 311 and 372, 4,374 and 5,685.
     With `ahead` against the row-wise kernel as it is for what the engine gives it, which asks for several keys before it uses the first: the longest block's
     keys, 0.08 us (one head of 128) to 0.17 (two of 256, four of 128) each, or all keys, 0.018 to 0.051 us a key and multiprocessor, and a quarter of the
-    shorter; 1 to 500 tokens behind 0 to 4,096, groups of 1 to 4. The same sizes by tiles and row by row: 500 tokens 146 and 217; 16 tokens 90 and 47, 291 and 51,
-    1,100 and 109; 128 tokens behind 0, 1,024 and 4,096 40 and 27, 310 and 205, 1,123 and 730; 500 behind 1,024 430 and 894 (the faster one in 71 of 72)."""
+    shorter; 1 to 500 tokens behind 0 to 4,096, groups of 1 to 4; and with two blocks a tile where the tiles are few, half its steps of 17.2 us (heads of 256) or
+    12.9 (of 128). The same sizes by tiles and row by row: 500 tokens 99 and 215; 16 tokens 60 and 47, 164 and 51, 579 and 110; 128 tokens behind 0, 1,024
+    and 4,096 27 and 27, 166 and 206, 582 and 731; 500 behind 1,024 373 and 895 (the faster one in all of 72)."""
     count = np.asarray(row_count, np.int64)
     row0 = np.asarray(tile_row0, np.int64)
     first, last = count[row0], count[row0 + np.asarray(tile_nq, np.int64) - 1]
@@ -90,6 +91,9 @@ def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: in
     at_once = (7.5 - 0.42 * heads) * sms
     by_rows = 3.0 + (0.07 + 0.00145 * head_dim + 0.06 * heads) * max(min(256.0, float(count.max())), float(seen.sum()) * kv_heads * slices / at_once)
     if ahead:
+        alike = 2 if window and window < float(count.max()) else 1
+        if alike * len(steps) * kv_heads <= sms * (2 if head_dim == 128 else 1):         # as the launcher: two blocks a tile
+            by_tiles = 3.0 + 0.02 * head_dim + (8.6 + 0.0337 * head_dim) * max(-(-float(steps.max()) // 2), 1.1 * float(steps.sum()) * kv_heads / sms)
         longest = (0.00046 * head_dim + 0.0293 * heads - 0.008) * min(256.0, float(count.max()))
         every = head_dim * (0.0000794 + 0.000065 * heads) * float(seen.sum()) * kv_heads * slices / sms
         by_rows = 3.0 + max(longest, every) + 0.25 * min(longest, every)

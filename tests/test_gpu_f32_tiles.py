@@ -105,3 +105,23 @@ def test_as_near_to_64_bit_as_row_by_row(hq, hkv, d, cap, before, n, peak):
             counts, 16, None, d ** -0.5, cap, -(-T // K.attention_chunk()))
     off = [float((K.paged_attention_rows(*args, tiles=t).double() - want).norm() / want.norm()) for t in (None, cut([(before, n)], 32 // (hq // hkv)))]
     assert off[1] <= 1.03 * off[0], off                      # 190,000 results and more: the norms of two random errors of one size agree to 1 %
+
+
+@pytest.mark.parametrize("hq,hkv,d,at_once", [(8, 4, 256, 1), (16, 4, 128, 2)])
+@pytest.mark.parametrize("more,window", [(0, None), (1, None), (0, 600), (0, 100), (1, 100)])
+def test_on_both_sides_of_two_blocks_a_tile(hq, hkv, d, at_once, more, window):
+    """Up to a wave of tiles two blocks take one, every second step of 64 keys each; the first tiles have one step, so that the second has none."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(10)
+    per = 32 // (hq // hkv)
+    n = at_once * torch.cuda.get_device_properties(0).multi_processor_count // hkv * per + more
+    width = -(-n // 16)
+    k_table, v_table = (torch.randn(width, hkv, 16, d, device="cuda", generator=gen) for _ in range(2))
+    q = torch.randn(n, hq, d, device="cuda", generator=gen)
+    counts = torch.arange(1, n + 1, dtype=torch.int32, device="cuda")
+    args = (q, k_table, v_table, torch.arange(width, dtype=torch.int32, device="cuda")[None].contiguous(), torch.zeros(n, dtype=torch.int32, device="cuda"),
+            counts, 16, window, d ** -0.5, 50.0, -(-n // K.attention_chunk()) + 1)
+    by_rows, by_tiles = K.paged_attention_rows(*args), K.paged_attention_rows(*args, tiles=cut([(0, n)], per))
+    # sums of up to 600 weights in 32-bit in another order; each side is within 1e-5 of 64 bits (above)
+    assert (by_rows - by_tiles).abs().max() <= 2e-5 * by_rows.abs().max()
