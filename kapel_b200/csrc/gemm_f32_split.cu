@@ -7,7 +7,8 @@
 //
 // The operands are swapped, 128 weight rows are the MMA's M and 16, 32, 64 or 128 rows of A its N, for a handful of rows and for thousands
 // alike: an element's products and additions are the same in all of them. Where the tiles are too few, K is cut into segments, a block each in a
-// cluster of up to eight, which add up their sums through shared memory in the segments' order.
+// cluster of up to eight, which add up their sums through shared memory in the segments' order. Where they are more than the multiprocessors, a block
+// walks over several, and beginning and ending (some 6 us) are there once: 500 rows by 18,432 x 2,304 204 us by a block a tile, 187 so.
 //
 // Twenty warps:
 //   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep, as 32-bit values (and of up to 32 rows of A)
@@ -41,7 +42,7 @@ template <int NP> struct Pieces {
     static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
     static constexpr int STAGES = 8;
     static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
-    static constexpr int SMEM = STAGES * STAGE + 2 * PIECES + 1024 /* alignment */ + 512 /* barriers, rows that are not finite */;
+    static constexpr int SMEM = STAGES * STAGE + 2 * PIECES + 1024 /* alignment */ + 1536 /* barriers, rows that are not finite */;
     static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, TMEM_COLS = COL_W + 192 <= 256 ? 256 : 512;
     static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
     static_assert(SMEM <= 232448, "more shared memory than a block can have");
@@ -75,13 +76,15 @@ struct F32Tiles {
 };
 
 // epilogue 0: none; 1: cap * tanh(acc / cap). GROUPED: blockIdx.x is a tile of `tiles`, NP rows at most, m the places there are.
-template <int NP, int EPI, bool GROUPED>
+// WALK: a block takes tile after tile, gridDim.x apart; its warps go on to the next one's chunks while the last one's sums are stored.
+template <int NP, int EPI, bool GROUPED, bool WALK>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ c,
                        const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ a_odd, int m, int n, int k, int chunks_a_segment, float cap, const F32Tiles tiles) {
     // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]; a_odd then says which rows have none
     using C = Pieces<NP>;
     static_assert(!GROUPED || C::CUTS, "a tile's rows are cut by the blocks that need them");
+    static_assert(!WALK || !C::CUTS, "the walk is for many rows");
     extern __shared__ unsigned char fp_raw[];
     if (GROUPED && (int)blockIdx.x >= tiles.count[0]) return;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)fp_raw + 1023) & ~(uintptr_t)1023);
@@ -92,14 +95,20 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     uint64_t* a_full = cut + 2;                                    // [2] its pieces of A that are not
     uint64_t* done = a_full + 2;                                   // [2] a chunk's products are complete: its pieces' place is free, its sum there
     uint64_t* added = done + 2;                                    // [2] the sum has been read
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(added + 2);
-    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 224;      // [128] of W, [NP] of A
+    uint64_t* marked = added + 2;                                  // WALK: [2] a tile's rows without pieces are marked, every second tile in one place
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(marked + 2);
+    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 224;      // [128] of W, [NP] of A; WALK: [2][128 of W by either half's warps, NP]
+    unsigned char* odd_warps = odd_rows + 2 * (2 * FP_M + 128);    // WALK: [2][16] whether a warp marked any
     int* any_odd = reinterpret_cast<int*>(tmem_slot + 1);
-    static_assert((2 * C::STAGES + 8) * 8 + 8 <= 224, "the barriers outgrew their room");
+    static_assert((2 * C::STAGES + 10) * 8 + 8 <= 224, "the barriers outgrew their room");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = GROUPED ? tiles.first[blockIdx.x] : blockIdx.x * NP, rows = GROUPED ? min(tiles.rows[blockIdx.x], m - m0) : m - m0;      // what lies behind is not stored
-    const int n0 = blockIdx.y * FP_M, w0 = GROUPED ? tiles.expert[blockIdx.x] * n + n0 : n0, segment = blockIdx.z, segments = gridDim.z;
+    const int n0 = blockIdx.y * FP_M, w0 = GROUPED ? tiles.expert[blockIdx.x] * n + n0 : n0, segment = WALK ? 0 : blockIdx.z, segments = WALK ? 1 : gridDim.z;
+    const int m_tiles = (m + NP - 1) / NP, all_tiles = m_tiles * ((n + FP_M - 1) / FP_M);
+    const int walk = WALK ? (all_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;      // this block's tiles
+    auto tile_m0 = [&](int t) { return WALK ? ((int)blockIdx.x + t * (int)gridDim.x) % m_tiles * NP : m0; };
+    auto tile_w0 = [&](int t) { return WALK ? ((int)blockIdx.x + t * (int)gridDim.x) / m_tiles * FP_M : w0; };
     const int chunks_all = (k + FP_K - 1) / FP_K;
     const int chunk0 = segment * chunks_a_segment, chunks = max(0, min(chunks_a_segment, chunks_all - chunk0));
 
@@ -110,6 +119,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             at_mbar_init(a_full + b, 1);
             at_mbar_init(done + b, 1);
             at_mbar_init(added + b, C::CUTS ? 4 : 8);
+            at_mbar_init(marked + b, 9);
         }
         *any_odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -129,13 +139,14 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0;
-            for (; it < 2 * chunks; ++it) {
+            int it = 0, t = 0, step = 0, row = tile_w0(0);
+            for (; it < 2 * chunks * walk; ++it, ++step) {
+                if (WALK && step == 2 * chunks) step = 0, row = tile_w0(++t);
                 const int s = it % C::STAGES;
                 if (!at_mbar_wait(empty + s, ((uint32_t)(it / C::STAGES) & 1u) ^ 1u)) { failed = true; break; }
                 const uint32_t dst = at_saddr(smem + s * C::STAGE);
                 at_mbar_expect_tx(full + s, C::STAGE);
-                at_tma_box(dst, &map_w, chunk0 * FP_K + it * FP_STAGE_K, w0, full + s);
+                at_tma_box(dst, &map_w, chunk0 * FP_K + step * FP_STAGE_K, row, full + s);
                 if (C::CUTS) at_tma_box(dst + C::W_BYTES, &map_a, chunk0 * FP_K + it * FP_STAGE_K, m0, full + s);
             }
             if (failed)                                            // the copies in flight land before the block goes on
@@ -150,7 +161,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         const uint32_t d = tm + (uint32_t)(b * C::ACC), aw = tm + (uint32_t)(C::COL_W + b * 96);
         const uint64_t ba = at_desc(at_saddr(pieces + b * C::PIECES), 16, 1024);
-        for (int ch = b; ch < chunks; ch += 2) {
+        for (int ch = b; ch < chunks * walk; ch += 2) {
             bool there = at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u);
             if (!C::CUTS) there = there && at_mbar_wait(a_full + b, (uint32_t)(ch >> 1) & 1u);
             there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
@@ -170,7 +181,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int quarter = warp & 3, half = (warp - FP_WARP_W) >> 2;      // of the TMEM lanes, which are the weight rows; of the chunk
         const int row = quarter * 32 + lane;
         float odd = 0.f;
-        for (int ch = 0; ch < chunks; ++ch) {
+        for (int ch = 0, t = 0, last = chunks - 1; ch < chunks * walk; ++ch) {
             const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
             const unsigned char* from = smem + s * C::STAGE + row * 128;
@@ -194,8 +205,16 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             at_fence_before();
             __syncwarp();
             if (lane == 0) at_mbar_arrive(cut + b);
+            if (WALK && ch == last) {                              // the tile two before this one was stored before its neighbour's last sums were taken
+                odd_rows[(t & 1) * (2 * FP_M + 128) + half * FP_M + row] = odd != odd;
+                const bool any = __any_sync(0xffffffffu, odd != odd);
+                if (lane == 0) odd_warps[(t & 1) * 16 + warp - FP_WARP_W] = any;
+                __syncwarp();
+                if (lane == 0) at_mbar_arrive(marked + (t & 1));
+                ++t, last += chunks, odd = 0.f;
+            }
         }
-        if (odd != odd) odd_rows[row] = 1, *any_odd = 1;
+        if (!WALK && odd != odd) odd_rows[row] = 1, *any_odd = 1;
     } else if (C::CUTS && warp < C::WARP_SUM) {
         // ---------------------------------------------------------------- cutting a few rows of A, two warps a half of the chunk
         const int half = (warp - FP_WARP_A) >> 1, t = ((warp - FP_WARP_A) & 1) * 32 + lane, row = t % NP;
@@ -232,51 +251,97 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     } else if (warp == FP_WARP_PIECES) {
         if (!C::CUTS) {
             // ------------------------------------------------------------ A's pieces, and which of its rows have none
-            if (lane == 0) {
-                int ch = 0;
-                for (; ch < chunks; ++ch) {
-                    const int b = ch & 1;
-                    if (!at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
-                    at_mbar_expect_tx(a_full + b, C::PIECES);
-                    for (int p = 0; p < 3; ++p)
-                        at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch) * FP_K, p * m + m0, a_full + b);
+            int ch = 0;
+            for (int t = 0; t < walk && !failed; ++t) {
+                const int first = tile_m0(t);
+                if (lane == 0) {
+                    for (const int begin = ch; ch < begin + chunks; ++ch) {
+                        const int b = ch & 1;
+                        if (!at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
+                        at_mbar_expect_tx(a_full + b, C::PIECES);
+                        for (int p = 0; p < 3; ++p)
+                            at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch - begin) * FP_K, p * m + first, a_full + b);
+                    }
+                    if (failed)
+                        for (int i = max(0, ch - 2); i < ch; ++i) at_mbar_wait(a_full + (i & 1), (uint32_t)(i >> 1) & 1u);
                 }
-                if (failed)
-                    for (int i = max(0, ch - 2); i < ch; ++i) at_mbar_wait(a_full + (i & 1), (uint32_t)(i >> 1) & 1u);
+                failed = __any_sync(0xffffffffu, failed);
+                if (WALK) {
+                    bool any = false;
+                    for (int j = lane; j < NP; j += 32) {
+                        const bool o = first + j < m && a_odd[first + j] != 0;
+                        odd_rows[(t & 1) * (2 * FP_M + 128) + 2 * FP_M + j] = o;
+                        any = any || o;
+                    }
+                    any = __any_sync(0xffffffffu, any);
+                    if (lane == 0) odd_warps[(t & 1) * 16 + 8] = any;
+                    __syncwarp();
+                    if (lane == 0) at_mbar_arrive(marked + (t & 1));
+                } else {
+                    for (int j = lane; j < NP && m0 + j < m; j += 32)
+                        if (a_odd[m0 + j] != 0) odd_rows[FP_M + j] = 1, *any_odd = 1;
+                }
             }
-            __syncwarp();
-            for (int j = lane; j < NP && m0 + j < m; j += 32)
-                if (a_odd[m0 + j] != 0) odd_rows[FP_M + j] = 1, *any_odd = 1;
         }
     } else {
         // ---------------------------------------------------------------- adding up: a weight row and COLS of A's rows a thread
         const int quarter = warp & 3, half = (warp - C::WARP_SUM) >> 2;
         const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * COLS);
+        for (int t = 0; t < walk && !failed; ++t) {
 #pragma unroll
-        for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
-        for (int ch = 0; ch < chunks; ++ch) {
-            const int b = ch & 1;
-            if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, (uint32_t)(ch >> 1) & 1u))) { failed = true; break; }
-            at_fence_after();
+            for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
+            for (int ch = t * chunks; ch < (t + 1) * chunks; ++ch) {
+                const int b = ch & 1;
+                if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, (uint32_t)(ch >> 1) & 1u))) { failed = true; break; }
+                at_fence_after();
 #pragma unroll
-            for (int c0 = 0; c0 < COLS; c0 += 16) {
-                uint32_t r[16];
-                fp_ld16(lanes + (uint32_t)(b * C::ACC + c0), r);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (c0 + 16 == COLS) {
-                    at_fence_before();
-                    __syncwarp();
-                    if (lane == 0) at_mbar_arrive(added + b);
+                for (int c0 = 0; c0 < COLS; c0 += 16) {
+                    uint32_t r[16];
+                    fp_ld16(lanes + (uint32_t)(b * C::ACC + c0), r);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (c0 + 16 == COLS) {
+                        at_fence_before();
+                        __syncwarp();
+                        if (lane == 0) at_mbar_arrive(added + b);
+                    }
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
                 }
+            }
+            if constexpr (WALK) {
+                if (failed || !__all_sync(0xffffffffu, at_mbar_wait(marked + (t & 1), (uint32_t)(t >> 1) & 1u))) { failed = true; break; }
+                const int first = tile_m0(t), w_row = tile_w0(t) + quarter * 32 + lane, j0 = half * COLS, many = min(COLS, m - first - j0);
+                if (w_row < n) {
+                    float* to = c + (size_t)(first + j0) * n + w_row;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) sum[c0 + j] += __uint_as_float(r[j]);
+                    for (int j = 0; j < COLS; ++j) {
+                        float v = sum[j];
+                        if (EPI == 1) v = cap * tanhf(v / cap);
+                        if (j < many) to[(size_t)j * n] = v;
+                    }
+                    bool any = false;
+                    for (int i = 0; i < 9; ++i) any = any || odd_warps[(t & 1) * 16 + i] != 0;
+                    const unsigned char* marks = odd_rows + (t & 1) * (2 * FP_M + 128);
+                    const int r = quarter * 32 + lane;
+                    if (any) {                                     // this thread's elements of rows without pieces again
+#pragma unroll 1
+                        for (int j = 0; j < many; ++j) {
+                            if ((marks[r] | marks[FP_M + r] | marks[2 * FP_M + j0 + j]) == 0) continue;
+                            const float *x = a + (size_t)(first + j0 + j) * k, *y = w + (size_t)w_row * k;
+                            float v = 0.f;
+#pragma unroll 1
+                            for (int kk = 0; kk < k; ++kk) v = fmaf(x[kk], y[kk], v);
+                            to[(size_t)j * n] = EPI == 1 ? cap * tanhf(v / cap) : v;
+                        }
+                    }
+                }
             }
         }
     }
     __syncthreads();                                               // the stages have been read, the rows that are not finite are marked
     float* sums = reinterpret_cast<float*>(smem);                  // [NP][128], where K is cut
     auto to = [&](int j) { return (size_t)(GROUPED && tiles.order != nullptr ? tiles.order[m0 + j] : m0 + j) * n + n0; };
-    if (warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
+    if (!WALK && warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
         const int r = (warp & 3) * 32 + lane, j0 = ((warp - C::WARP_SUM) >> 2) * COLS;
         if (segments == 1) {
             if (n0 + r < n)
@@ -304,7 +369,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
         }
     }
-    if (segments > 1) {
+    if (!WALK && segments > 1) {
         fp_cluster_sync();
         const int per = NP / segments;                             // rows of A this block adds up
         for (int i = tid; i < per * FP_M; i += FP_THREADS) {
@@ -360,7 +425,14 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     const int kp = (k + 7) & ~7;
     int* odd_rows = nullptr;
     KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535, "gemm_f32: a weight of %d rows is too much for one launch", n);
-    if (cudaFuncSetAttribute(gemm_f32_pieces_kernel<NP, EPI, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
+    // More tiles than multiprocessors: blocks walk over them. (The marks of a tile's rows have two places: four chunks a tile keep them apart.)
+    const long long all_tiles = (long long)((m + NP - 1) / NP) * ((n + FP_M - 1) / FP_M);
+    const int chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
+    const bool walk = !C::CUTS && segments == 1 && all_tiles > sms && all_tiles <= 0x7fffffff - sms && all_tiles / sms * chunks < 0x3fffffff && chunks >= 4;
+    auto kernel = gemm_f32_pieces_kernel<NP, EPI, false, false>;
+    if constexpr (!C::CUTS)
+        if (walk) kernel = gemm_f32_pieces_kernel<NP, EPI, false, true>;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess)
         return fail("gemm_f32: cannot have %d bytes of shared memory", C::SMEM);
     if (int e = encode_map_f32(&map_w, w, n, k, k, FP_M)) return e;
     if (C::CUTS) {
@@ -372,9 +444,8 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
         f32_cut_rows_kernel<<<m, 256, 0, s>>>(a, reinterpret_cast<uint32_t*>(scratch), odd_rows, m, k, kp);
         if (int e = check_launch("gemm_f32 cut")) return e;
     }
-    const int chunks = (k + FP_K - 1) / FP_K;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((m + NP - 1) / NP, (n + FP_M - 1) / FP_M, segments);
+    cfg.gridDim = walk ? dim3(sms) : dim3((m + NP - 1) / NP, (n + FP_M - 1) / FP_M, segments);
     cfg.blockDim = FP_THREADS;
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = s;
@@ -383,7 +454,7 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = segments;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, gemm_f32_pieces_kernel<NP, EPI, false>, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
+    cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
     return check_launch("gemm_f32 pieces");
 }
 
@@ -398,14 +469,15 @@ int gemm_f32_segments(int m, int n, int k) {
     double least = 0;
     for (int s = 1; s <= 8 && s <= chunks; s *= 2) {
         const int at_once = s <= 2 ? sms : (s == 4 ? sms * 7 / 8 : sms * 3 / 4) / s * s;
-        const double us = (double)((tiles * s + at_once - 1) / at_once) * ((chunks + s - 1) / s * chunk_us + (s == 1 ? 5.0 : 6.5));
+        const int waves = (tiles * s + at_once - 1) / at_once, ends = s == 1 && m > FP_CUT_ROWS ? 1 : waves;      // a block that walks begins and ends once
+        const double us = (double)waves * ((chunks + s - 1) / s * chunk_us) + ends * (s == 1 ? 5.0 : 6.5);
         if (s == 1 || us < least) least = us, best = s;
     }
     return best;
 }
 // More than 16 rows of 256 and more, and three to 16 of 1,024 and more: one accumulator an element in ascending k, a kernel for each, is limited by
 // its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
-// chains, 204 by pieces; by 2,304 x 9,216 545 and 118, by 2,304 x 2,048 131 and 31, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
+// chains, 187 by pieces; by 2,304 x 9,216 545 and 118, by 2,304 x 2,048 131 and 31, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
 // 12 (64 rows 9.3 and 8.8). Six rows: 54 and 31, 72 and 30, 18 and 11, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 31, 51 and 30, 14 and 12,
 // 13 and 9, by 256,000 x 2,304 440 and 384; one row 37 and 31, 32 and 30, 9.5 and 11.6, 355 and 384. The error against 64 bits is 0.07 to 0.3 of the
 // chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
@@ -444,7 +516,7 @@ extern "C" int kb_moe_f32_pieces(float* c, const float* a, const float* w, int e
     KB_REQUIRE(k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0, "moe_f32: rows of %d values must begin at 16-byte boundaries", k);
     KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535 && (long long)experts * n <= 0x7fffffffll, "moe_f32: %d experts of %d rows are too much for one launch", experts, n);
     if (tile_cap == 0 || places == 0) return 0;
-    auto kernel = gemm_f32_pieces_kernel<FP_CUT_ROWS, 0, true>;
+    auto kernel = gemm_f32_pieces_kernel<FP_CUT_ROWS, 0, true, false>;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) != cudaSuccess) return fail("moe_f32: cannot have %d bytes of shared memory", C::SMEM);
     CUtensorMap map_a, map_w;
     if (int e = encode_map_f32(&map_a, a, places, k, k, FP_CUT_ROWS)) return e;

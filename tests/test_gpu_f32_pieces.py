@@ -133,3 +133,23 @@ def test_experts_sum_by_fours_and_one_by_one(tokens, width, top):
             a = K.moe_combine(y, weights, torch.float32, also=extra, **kw)
             b = K.moe_combine(pad(y), weights, torch.float32, also=extra, **kw)
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("m,more,k", [(33, 0, 260), (64, 1, 256), (65, 5, 256), (300, 300, 324), (500, 1, 1028)])
+def test_blocks_that_walk_over_tiles(m, more, k):
+    """More tiles of 128 weight rows than multiprocessors: every block takes several, and the results are a tile's own, rows without pieces included."""
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    n = -(-sms // -(-m // (64 if m <= 64 else 128))) * 128 + more + 128
+    a, w = torch.randn(m, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    for odd in (False, True):
+        if odd:
+            a[m - 1, k - 1], a[2, 0] = float("inf"), float("nan")
+            w[n - 1, 3], w[130, 7], w[n // 2, k - 2] = -float("inf"), float("nan"), 3.4e38
+        got = pieces(a, w, 1, 5.0 if m == 65 else 0.0)
+        for n0 in range(0, n, 4096):                         # few tiles: a block has one
+            assert torch.equal(torch.nan_to_num(got[:, n0 : n0 + 4096], nan=1e30),
+                               torch.nan_to_num(pieces(a, w[n0 : n0 + 4096].contiguous(), 1, 5.0 if m == 65 else 0.0), nan=1e30))
+        if not odd and m != 65:
+            want, sizes = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
+            assert ((got - want).abs() <= (4 * 2.0 ** -23 + (k // 64 + 2) * 2.0 ** -24) * sizes + 1e-30).all()      # as above
