@@ -8,16 +8,18 @@
 // The operands are swapped, 128 weight rows are the MMA's M and 16, 32, 64 or 128 rows of A its N, for a handful of rows and for thousands
 // alike: an element's products and additions are the same in all of them. Where the tiles are too few, K is cut into segments, a block each in a
 // cluster of up to eight, which add up their sums through shared memory in the segments' order. Where they are more than the multiprocessors, a block
-// walks over several, and beginning and ending (some 6 us) are there once: 500 rows by 18,432 x 2,304 204 us by a block a tile, 187 so.
+// walks over several, and beginning and ending (some 6 us) are there once: 500 rows by 18,432 x 2,304 204 us by a block a tile, 187 so (now 184).
 //
 // Twenty warps:
-//   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep, as 32-bit values (and of up to 32 rows of A)
+//   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep (five with 128 rows), as 32-bit values (and of up to 32 rows of A)
 //   warps 3-10    cut the weights, each half of them every second stage: a thread has a row, its pieces go to tensor memory, from where the
 //                 MMA takes its A operand
 //   warps 1, 2    issue the 24 MMAs of a chunk, one the even chunks, the other the odd ones (issuing takes a thread longer than the tensor
 //                 cores need for a small product; each chunk has pieces and an accumulator of its own)
 //   warp 19       asks TMA for the pieces of A, the MMA's B operand, which a kernel ahead of this one has cut: every block of a row of
-//                 tiles needs them. Up to 32 rows are cut here instead, by warps 11-14, which saves that launch
+//                 tiles needs them. They come three chunks ahead (four with 64 rows), which takes the place of stages: two ahead, a chunk of
+//                 500 rows by 2,304 x 9,216 waited for them (118 us, now 99; four times as many rows 416 and 363). Up to 32
+//                 rows are cut here instead, by warps 11-14, which saves that launch
 //   warps 11-18   (15-18) add a finished chunk to the sums they hold in registers, and store them at the end
 //
 // Values that are no finite numbers (and those that round to infinity in bfloat16) have no pieces: infinity less infinity is NaN. A
@@ -40,9 +42,9 @@ constexpr int FP_CUT_ROWS = 32;                                    // up to so m
 template <int NP> struct Pieces {
     static constexpr bool CUTS = NP <= FP_CUT_ROWS;
     static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
-    static constexpr int STAGES = 8;
     static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
-    static constexpr int SMEM = STAGES * STAGE + 2 * PIECES + 1024 /* alignment */ + 1536 /* barriers, rows that are not finite */;
+    static constexpr int STAGES = NP == 128 ? 5 : 8, PLACES = CUTS ? 2 : (NP == 128 ? 3 : 4);      // of the pieces of A
+    static constexpr int SMEM = STAGES * STAGE + PLACES * PIECES + 1024 /* alignment */ + 1536 /* barriers, rows that are not finite */;
     static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, TMEM_COLS = COL_W + 192 <= 256 ? 256 : 512;
     static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
     static_assert(SMEM <= 232448, "more shared memory than a block can have");
@@ -88,19 +90,20 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     extern __shared__ unsigned char fp_raw[];
     if (GROUPED && (int)blockIdx.x >= tiles.count[0]) return;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)fp_raw + 1023) & ~(uintptr_t)1023);
-    unsigned char* pieces = smem + C::STAGES * C::STAGE;           // [2][3][NP rows][128 bytes]
-    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + 2 * C::PIECES);
+    unsigned char* pieces = smem + C::STAGES * C::STAGE;           // [PLACES][3][NP rows][128 bytes]
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::PLACES * C::PIECES);
     uint64_t* empty = full + C::STAGES;                            // the warps that cut it have read the stage
     uint64_t* cut = empty + C::STAGES;                             // [2] a chunk's pieces are there that are cut here
-    uint64_t* a_full = cut + 2;                                    // [2] its pieces of A that are not
-    uint64_t* done = a_full + 2;                                   // [2] a chunk's products are complete: its pieces' place is free, its sum there
+    uint64_t* a_full = cut + 2;                                    // [PLACES] its pieces of A that are not
+    uint64_t* a_empty = a_full + C::PLACES;                        // [PLACES] and their place is free
+    uint64_t* done = a_empty + C::PLACES;                                 // [2] a chunk's products are complete: its pieces' place is free, its sum there
     uint64_t* added = done + 2;                                    // [2] the sum has been read
     uint64_t* marked = added + 2;                                  // WALK: [2] a tile's rows without pieces are marked, every second tile in one place
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(marked + 2);
-    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 224;      // [128] of W, [NP] of A; WALK: [2][128 of W by either half's warps, NP]
+    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 288;      // [128] of W, [NP] of A; WALK: [2][128 of W by either half's warps, NP]
     unsigned char* odd_warps = odd_rows + 2 * (2 * FP_M + 128);    // WALK: [2][16] whether a warp marked any
     int* any_odd = reinterpret_cast<int*>(tmem_slot + 1);
-    static_assert((2 * C::STAGES + 10) * 8 + 8 <= 224, "the barriers outgrew their room");
+    static_assert((2 * C::STAGES + 2 * C::PLACES + 8) * 8 + 8 <= 288, "the barriers outgrew their room");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = GROUPED ? tiles.first[blockIdx.x] : blockIdx.x * NP, rows = GROUPED ? min(tiles.rows[blockIdx.x], m - m0) : m - m0;      // what lies behind is not stored
@@ -116,11 +119,11 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 6 : 4); }      // the warps that cut the stage
         for (int b = 0; b < 2; ++b) {
             at_mbar_init(cut + b, C::CUTS ? 12 : 8);
-            at_mbar_init(a_full + b, 1);
             at_mbar_init(done + b, 1);
             at_mbar_init(added + b, C::CUTS ? 4 : 8);
             at_mbar_init(marked + b, 9);
         }
+        for (int b = 0; b < C::PLACES; ++b) { at_mbar_init(a_full + b, 1); at_mbar_init(a_empty + b, 1); }
         *any_odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -160,21 +163,25 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const int b = __shfl_sync(0xffffffffu, warp, 0) - 1;
         const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
         const uint32_t d = tm + (uint32_t)(b * C::ACC), aw = tm + (uint32_t)(C::COL_W + b * 96);
-        const uint64_t ba = at_desc(at_saddr(pieces + b * C::PIECES), 16, 1024);
+        const uint64_t first = at_desc(at_saddr(pieces), 16, 1024);
+        int place = b;
         for (int ch = b; ch < chunks * walk; ch += 2) {
             bool there = at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u);
-            if (!C::CUTS) there = there && at_mbar_wait(a_full + b, (uint32_t)(ch >> 1) & 1u);
+            if (!C::CUTS) there = there && at_mbar_wait(a_full + place, (uint32_t)(ch / C::PLACES) & 1u);
             there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
             if (!__all_sync(0xffffffffu, there)) { failed = true; break; }
             at_fence_after();
             const uint32_t one = at_elect();
+            const uint64_t ba = first + (uint64_t)(place * (C::PIECES >> 4));
 #pragma unroll
             for (int p = 0; p < PIECE_PRODUCTS; ++p)
 #pragma unroll
                 for (int kk = 0; kk < FP_K / 16; ++kk)
                     at_mma_ts_if(one, d, aw + (uint32_t)(piece_a(p) * 32 + kk * 8), ba + (uint64_t)(piece_b(p) * (C::PIECE >> 4) + kk * 2), IDESC, (p | kk) != 0 ? 1u : 0u);
             if (one) at_commit(done + b);
+            if (!C::CUTS && one) at_commit(a_empty + place);
             __syncwarp();
+            if (!C::CUTS) place = place + 2 >= C::PLACES ? place + 2 - C::PLACES : place + 2;
         }
     } else if (warp < FP_WARP_A) {
         // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
@@ -256,14 +263,14 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 const int first = tile_m0(t);
                 if (lane == 0) {
                     for (const int begin = ch; ch < begin + chunks; ++ch) {
-                        const int b = ch & 1;
-                        if (!at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u)) { failed = true; break; }
+                        const int b = ch % C::PLACES;
+                        if (!at_mbar_wait(a_empty + b, ((uint32_t)(ch / C::PLACES) & 1u) ^ 1u)) { failed = true; break; }
                         at_mbar_expect_tx(a_full + b, C::PIECES);
                         for (int p = 0; p < 3; ++p)
                             at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch - begin) * FP_K, p * m + first, a_full + b);
                     }
                     if (failed)
-                        for (int i = max(0, ch - 2); i < ch; ++i) at_mbar_wait(a_full + (i & 1), (uint32_t)(i >> 1) & 1u);
+                        for (int i = max(0, ch - C::PLACES); i < ch; ++i) at_mbar_wait(a_full + i % C::PLACES, (uint32_t)(i / C::PLACES) & 1u);
                 }
                 failed = __any_sync(0xffffffffu, failed);
                 if (WALK) {
@@ -477,7 +484,7 @@ int gemm_f32_segments(int m, int n, int k) {
 }
 // More than 16 rows of 256 and more, and three to 16 of 1,024 and more: one accumulator an element in ascending k, a kernel for each, is limited by
 // its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
-// chains, 187 by pieces; by 2,304 x 9,216 545 and 118, by 2,304 x 2,048 131 and 31, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
+// chains, 184 by pieces; by 2,304 x 9,216 545 and 99, by 2,304 x 2,048 131 and 29, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
 // 12 (64 rows 9.3 and 8.8). Six rows: 54 and 31, 72 and 30, 18 and 11, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 31, 51 and 30, 14 and 12,
 // 13 and 9, by 256,000 x 2,304 440 and 384; one row 37 and 31, 32 and 30, 9.5 and 11.6, 355 and 384. The error against 64 bits is 0.07 to 0.3 of the
 // chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
@@ -507,7 +514,8 @@ bool moe_f32_pieces_take(int k, const void* a, const void* w) { return k >= 256 
 using namespace kb;
 
 // c [places, n]: a [places, k] (in the lists' order) by the expert's weights w [experts, n, k], tiles of at most FP_CUT_ROWS rows; `order` not null: rows
-// placed by pair number. A block a tile and 128 columns, K in one: the tiles alone fill the GPU. 1,200 pairs of 16 experts of 2,048 x 1,024: see `moe_grouped`.
+// placed by pair number. A block a tile and 128 columns, K in one: the tiles alone fill the GPU. 1,200 pairs of 16 experts of 2,048 x 1,024, both
+// products: 555 us by multiply-adds, 146 so; 16 pairs 316 and 28.
 extern "C" int kb_moe_f32_pieces_takes(const float* a, const float* w, int k) { return moe_f32_pieces_take(k, a, w) ? 1 : 0; }
 extern "C" int kb_moe_f32_pieces(float* c, const float* a, const float* w, int experts, const int* tile_expert, const int* tile_first, const int* tile_rows,
                                  const int* n_tiles, int tile_cap, const int* order, int places, int n, int k, void* stream) {
