@@ -1193,9 +1193,10 @@ def delta_columns_per_warp(n: int = 0) -> None:
 
 
 # The delta rule goes by chunks of 32 rows instead of row by row where some request brings DELTA_CHUNK_LONGEST rows: a row of the scan takes
-# 0.33 us, a chunk 1.65 and the launch ahead of the chain 14 (16 heads of 128: 64 rows 24 us row by row, 21 by chunks; 100 rows 34 and 24, 192 rows 63
-# and 27). Then every request of DELTA_CHUNK_ROWS rows goes that way, side by side with the longest.
-DELTA_CHUNK_ROWS, DELTA_CHUNK_LONGEST = 64, 64
+# 0.33 us, a chunk 1.65 and the launch ahead of the chain 14 (16 heads of 128: 192 rows 63 us row by row, 27 by chunks). From 64 rows on chunks are
+# faster (24 and 21 us; 100 rows 34 and 24), but not as exact: up to 1.08 of the scan's error against 64 bits at 64 to 191 rows. Then every
+# request of DELTA_CHUNK_ROWS rows goes that way, side by side with the longest.
+DELTA_CHUNK_ROWS, DELTA_CHUNK_LONGEST = 64, 192
 
 
 def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: int, conv: torch.Tensor, a_log: torch.Tensor,
