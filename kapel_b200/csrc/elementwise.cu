@@ -309,6 +309,20 @@ __global__ void glu_kernel(T* __restrict__ out, const Src<TI> x, long long rows,
     Elem<T>::store(out + idx, a * u);
 }
 
+// The same for 32-bit values of one slice, n a multiple of four: four values a thread, a row's place without a division. 500 rows of 9,216 took 22 us by a
+// value a thread, whose 64-bit division and remainder were most of it, and take 9 so.
+template <typename T>
+__global__ void __launch_bounds__(256) glu_fours_kernel(T* __restrict__ out, const float* __restrict__ x, int n, int act) {
+    dependent_wait();                                       // returns at once after a plain launch
+    dependent_trigger();
+    const int i = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (i >= n) return;
+    const float* row = x + (size_t)blockIdx.x * 2 * n;
+    const float4 g = load_four(row + i), u = load_four(row + n + i);
+    const auto unit = [&](float v) { return act == 0 ? gelu_tanh(v) : silu(v); };
+    store_four(out + (size_t)blockIdx.x * n + i, make_float4(unit(g.x) * u.x, unit(g.y) * u.y, unit(g.z) * u.z, unit(g.w) * u.w));
+}
+
 // The same for bfloat16 in and out with n a multiple of 8: 16 bytes of gate, 16 of up, 16 out a thread.
 __global__ void glu_bf16x8_kernel(__nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ x, long long rows,
                                   int n, int act) {
@@ -546,6 +560,12 @@ extern "C" int kb_glu(void* out, int out_dt, const void* x, int in_dt, int split
     if (in_dt == KB_DT_BF16 && out_dt == KB_DT_BF16 && splits == 1 && n % 8 == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)out & 15) == 0) {
         const long long vec = rows * (n / 8);
         glu_bf16x8_kernel<<<(unsigned)((vec + 255) / 256), 256, 0, s>>>((bf16*)out, (const bf16*)x, rows, n, act);
+    }
+    else if (in_dt == KB_DT_F32 && (out_dt == KB_DT_F32 || out_dt == KB_DT_BF16) && splits == 1 && n % 4 == 0 && n <= 1024 * 65535 && rows <= 0x7fffffffll &&
+             (((uintptr_t)x | (uintptr_t)out) & 15) == 0) {
+        const dim3 fours((unsigned)rows, (unsigned)((n + 1023) / 1024));
+        if (out_dt == KB_DT_F32) launch_dependent_if(rows <= DEPENDENT_ROWS, glu_fours_kernel<float>, fours, dim3(256), 0, s, (float*)out, (const float*)x, n, act);
+        else launch_dependent_if(rows <= DEPENDENT_ROWS, glu_fours_kernel<bf16>, fours, dim3(256), 0, s, (bf16*)out, (const float*)x, n, act);
     }
     else if (in_dt == KB_DT_F32 && out_dt == KB_DT_F32) KB_GLU(float, float);
     else if (in_dt == KB_DT_F32 && out_dt == KB_DT_BF16) KB_GLU(float, bf16);

@@ -75,3 +75,16 @@ def test_embedding(width, dtype):
         want = torch.stack([table[0].double() * 3 + places[0].double(), table[10].double() * 3 + places[4].double(), table[7].double() * 3])
         assert torch.isnan(got[2:4]).all()
         assert ((got[[0, 1, 4]].double() - want[:, None]).abs() <= 2.0 ** -23 * (want[:, None].abs() + 4.0)).all()
+
+
+@pytest.mark.parametrize("rows,n", [(1, 4), (3, 1020), (65, 1024), (70, 1028), (500, 9216)])
+@pytest.mark.parametrize("act", ["gelu_tanh", "silu"])
+@pytest.mark.parametrize("out", [torch.float32, torch.bfloat16])
+def test_gated_unit_by_fours_and_one_by_one(rows, n, act, out):
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    x = torch.randn(rows, 2 * n, device="cuda", generator=gen) * 4
+    beside = torch.empty(rows * 2 * n + 1, device="cuda")[1:].view(rows, 2 * n)      # begins off a 16-byte boundary: a value a thread
+    beside.copy_(x)
+    assert torch.equal(K.glu(x, act, out_dtype=out), K.glu(beside, act, out_dtype=out))
