@@ -18,6 +18,10 @@
 // have another size than keys (`dv`), and may lie `v_stride` apart: a value table that is the key
 // table itself, whose first `dv` components of a line are the value (attention through a latent).
 // With `sinks`, e^(sinks[head]) joins a row's denominator: a key without a value, not scaled.
+//
+// A chunk's keys and values are waited for, not the arithmetic: a key's place in the tables is divided out once into shared memory (by every thread that
+// read it the 64-bit divisions were most of the time), and eight keys and values are asked for before the first is used. 32-bit, 8 heads over 4 of
+// 256: 4 tokens behind 500 positions 231 -> 46 us, 128 behind 1,024 372 -> 205.
 #pragma once
 #include "common.cuh"
 

@@ -528,7 +528,7 @@ head_linear_mma_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
 // [heads, n_out, n_in] and come straight into registers, 16 bytes a lane, ahead of the wait on the kernel before. A lane's 16 bytes are eight neighbouring
 // inputs of one column, so two MMAs take 32 inputs in the order that gives, and the rows' inputs are read in the same. 32-bit inputs are
 // cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16): nothing is rounded but the sums. 8 rows, 16 heads of
-// 128 -> 512 (20.7 us by a column a warp, its sums by shuffles), 512 -> 128 with the gate (19.2): what is left is a launch's latency.
+// 128 -> 512: 6.4 us (20.7 by a column a warp, its sums by shuffles), 512 -> 128 with the gate: 9.2 (19.2). What is left is a launch's latency.
 constexpr int HF_ROWS = 16, HF_WARPS = 8, HF_COLS = HF_WARPS * 8, HF_HELD = 16;        // HF_HELD: groups of 32 inputs whose weights a lane holds at once
 // Elements between two rows of the inputs: 64 bytes further into the banks from row to row.
 __host__ __device__ constexpr int hf_ld(int n_in) { return (n_in + 31) / 32 * 32 + ((n_in + 31) / 32 % 2 == 0 ? 32 : 0); }

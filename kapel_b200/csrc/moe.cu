@@ -11,7 +11,7 @@
 //  sort      (token, k) pairs listed by expert (identity experts left out), and the row tiles of the grouped products.
 //  product   out[pair] = act(A[row of pair] . W[expert of pair]^T): a block a (row tile of one
 //            expert, column tile); bfloat16 by mma.sync with 32-bit sums, float32 by FMA in
-//            ascending k. What a pair's row computes does not depend on its place in a tile.
+//            ascending k, or in gemm_f32_split.cu. What a pair's row computes does not depend on its place in a tile.
 //  combine   out[token] = sum over k, in order, of weight[token, k] * y[token * top + k]; an identity expert's y is the
 //            token's own input.
 #include "common.cuh"
@@ -551,7 +551,7 @@ moe_combine_kernel(TO* __restrict__ out, const float* __restrict__ y, const floa
 }
 
 // The same, four neighbouring columns a thread and four experts' values asked for before the first is added: a column and an expert at a time, 1,360 rows of 2,048
-// with four experts took 27 us. For widths of a multiple of four and an addend of one slice.
+// with four experts took 27 us, and take 10 so. For widths of a multiple of four and an addend of one slice.
 template <typename TO, typename TA>
 __global__ void __launch_bounds__(256)
 moe_combine_fours_kernel(TO* __restrict__ out, const float* __restrict__ y, const float* __restrict__ weights, long long rows, int width, int top,
