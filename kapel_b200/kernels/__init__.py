@@ -1806,7 +1806,12 @@ def moe_tcgen05_takes(dtype: torch.dtype, rows: int, top: int, n_experts: int, w
 
 def moe_gather(a: torch.Tensor, lists: "ExpertLists") -> torch.Tensor:
     """[pairs, k]: the rows of a [tokens, k] in the lists' order (what lies behind the listed pairs is left as it is)."""
-    _need(a, "moe_gather input")
+    _need(a, "moe_gather input", torch.bfloat16)
+    return _rows_by_lists(a, lists)
+
+
+def _rows_by_lists(a: torch.Tensor, lists: "ExpertLists") -> torch.Tensor:
+    """`moe_gather` of bfloat16 or float32 rows of whole 16-byte pieces."""
     out = _fresh((lists.pairs, a.shape[1]), a.dtype, a.device)
     _check(library().kb_moe_gather(_ptr(out), _ptr(a), _ptr(lists.order), _ptr(lists.offsets[-1:]), lists.pairs, int(a.shape[1]) * a.element_size() // 2,
                                    int(lists.top), _stream()))
@@ -1890,7 +1895,7 @@ def moe_grouped(a: torch.Tensor, w: torch.Tensor, lists: ExpertLists, act: str, 
     if (a.dtype == out_dtype == torch.float32 and act == "none" and lists.tile_rows == 32 and lists.pairs > 0
             and library().kb_moe_f32_pieces_takes(_ptr(a), _ptr(w), k)):
         # 32-bit products on the tensor cores, every value in pieces that hold it; their rows in the lists' order
-        rows = moe_gather(a, lists) if a_by_token else a
+        rows = _rows_by_lists(a, lists) if a_by_token else a
         _check(library().kb_moe_f32_pieces(_ptr(out), _ptr(rows), _ptr(w), int(w.shape[0]), _ptr(t[0]), _ptr(t[1]), _ptr(t[2]), _ptr(t[3]), int(lists.tile_cap),
                                            _ptr(lists.order) if out_by_pair else None, lists.pairs, n, k, _stream()))
         return out
