@@ -22,8 +22,9 @@
 //                 rows are cut here instead, by warps 11-14, which saves that launch
 //   warps 11-18   (15-18) add a finished chunk to the sums they hold in registers, and store them at the end
 //
-// Values that are no finite numbers (and those that round to infinity in bfloat16) have no pieces: infinity less infinity is NaN. A
-// row that holds one is noticed when it is cut, and its elements are computed again by multiply-adds, as the other kernels do.
+// An element that comes out as no finite number is computed again by multiply-adds, as the other kernels do: values that are none (and those that
+// round to infinity in bfloat16) have no pieces, infinity less infinity is NaN, and of a finite product near the largest float or beyond it
+// the small products may be infinities of either sign before the large one is added.
 // Every wait gives up after about a second, raises a flag that `kb_gemm_f32_split_error` reports, and the block still meets at its
 // barriers, frees its TMEM and returns.
 #include "attention_tc.cuh"
@@ -44,7 +45,7 @@ template <int NP> struct Pieces {
     static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
     static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
     static constexpr int STAGES = NP == 128 ? 5 : 8, PLACES = CUTS ? 2 : (NP == 128 ? 3 : 4);      // of the pieces of A
-    static constexpr int SMEM = STAGES * STAGE + PLACES * PIECES + 1024 /* alignment */ + 1536 /* barriers, rows that are not finite */;
+    static constexpr int SMEM = STAGES * STAGE + PLACES * PIECES + 1024 /* alignment */ + 288 /* barriers */;
     static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, TMEM_COLS = COL_W + 192 <= 256 ? 256 : 512;
     static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
     static_assert(SMEM <= 232448, "more shared memory than a block can have");
@@ -58,10 +59,25 @@ __device__ __forceinline__ void fp_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                  : "r"(taddr) : "memory");
 }
 
-// `odd` becomes NaN when one of the two values has no pieces.
-__device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t& two, uint32_t& three, float& odd) {
-    cut_pair(x, y, one, two, three);
-    odd = fmaf(x, y, odd);
+__device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t& two, uint32_t& three) { cut_pair(x, y, one, two, three); }
+
+__device__ __forceinline__ bool fp_finite(float x) { return fabsf(x) < INFINITY; }
+// The product by multiply-adds in ascending k; rows of whole 16-byte pieces.
+__device__ __noinline__ float fp_chain(const float* x, const float* y, int k) {
+    float v = 0.f;
+#pragma unroll 1
+    for (int i = 0; i < k; i += 4) {
+        const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(y + i);
+        v = fmaf(a.x, b.x, v), v = fmaf(a.y, b.y, v), v = fmaf(a.z, b.z, v), v = fmaf(a.w, b.w, v);
+    }
+    return v;
+}
+// A bit for each of a thread's sums that is no finite number.
+template <int COLS> __device__ __forceinline__ uint64_t fp_not_finite(const float (&sum)[COLS]) {
+    uint64_t bits = 0;
+#pragma unroll
+    for (int j = 0; j < COLS; ++j) bits |= fp_finite(sum[j]) ? 0ull : 1ull << j;
+    return bits;
 }
 
 __device__ __forceinline__ void fp_cluster_sync() {
@@ -82,8 +98,8 @@ struct F32Tiles {
 template <int NP, int EPI, bool GROUPED, bool WALK>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ c,
-                       const float* __restrict__ a, const float* __restrict__ w, const int* __restrict__ a_odd, int m, int n, int k, int chunks_a_segment, float cap, const F32Tiles tiles) {
-    // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]; a_odd then says which rows have none
+                       const float* __restrict__ a, const float* __restrict__ w, int m, int n, int k, int chunks_a_segment, float cap, const F32Tiles tiles) {
+    // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]
     using C = Pieces<NP>;
     static_assert(!GROUPED || C::CUTS, "a tile's rows are cut by the blocks that need them");
     static_assert(!WALK || !C::CUTS, "the walk is for many rows");
@@ -98,12 +114,8 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     uint64_t* a_empty = a_full + C::PLACES;                        // [PLACES] and their place is free
     uint64_t* done = a_empty + C::PLACES;                                 // [2] a chunk's products are complete: its pieces' place is free, its sum there
     uint64_t* added = done + 2;                                    // [2] the sum has been read
-    uint64_t* marked = added + 2;                                  // WALK: [2] a tile's rows without pieces are marked, every second tile in one place
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(marked + 2);
-    unsigned char* odd_rows = reinterpret_cast<unsigned char*>(full) + 288;      // [128] of W, [NP] of A; WALK: [2][128 of W by either half's warps, NP]
-    unsigned char* odd_warps = odd_rows + 2 * (2 * FP_M + 128);    // WALK: [2][16] whether a warp marked any
-    int* any_odd = reinterpret_cast<int*>(tmem_slot + 1);
-    static_assert((2 * C::STAGES + 2 * C::PLACES + 8) * 8 + 8 <= 288, "the barriers outgrew their room");
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(added + 2);
+    static_assert((2 * C::STAGES + 2 * C::PLACES + 6) * 8 + 4 <= 288, "the barriers outgrew their room");
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = GROUPED ? tiles.first[blockIdx.x] : blockIdx.x * NP, rows = GROUPED ? min(tiles.rows[blockIdx.x], m - m0) : m - m0;      // what lies behind is not stored
@@ -121,13 +133,10 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             at_mbar_init(cut + b, C::CUTS ? 12 : 8);
             at_mbar_init(done + b, 1);
             at_mbar_init(added + b, C::CUTS ? 4 : 8);
-            at_mbar_init(marked + b, 9);
         }
         for (int b = 0; b < C::PLACES; ++b) { at_mbar_init(a_full + b, 1); at_mbar_init(a_empty + b, 1); }
-        *any_odd = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (tid < FP_M + NP) odd_rows[tid] = 0;
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at_saddr(tmem_slot)), "r"(C::TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
@@ -187,8 +196,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
         const int quarter = warp & 3, half = (warp - FP_WARP_W) >> 2;      // of the TMEM lanes, which are the weight rows; of the chunk
         const int row = quarter * 32 + lane;
-        float odd = 0.f;
-        for (int ch = 0, t = 0, last = chunks - 1; ch < chunks * walk; ++ch) {
+        for (int ch = 0; ch < chunks * walk; ++ch) {
             const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
             const unsigned char* from = smem + s * C::STAGE + row * 128;
@@ -196,8 +204,8 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 const float4 x = *reinterpret_cast<const float4*>(from + ((j ^ (row & 7)) << 4));
-                fp_cut(x.x, x.y, one[2 * j], two[2 * j], three[2 * j], odd);
-                fp_cut(x.z, x.w, one[2 * j + 1], two[2 * j + 1], three[2 * j + 1], odd);
+                fp_cut(x.x, x.y, one[2 * j], two[2 * j], three[2 * j]);
+                fp_cut(x.z, x.w, one[2 * j + 1], two[2 * j + 1], three[2 * j + 1]);
             }
             __syncwarp();
             if (lane == 0) at_mbar_arrive(empty + s);
@@ -212,20 +220,10 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             at_fence_before();
             __syncwarp();
             if (lane == 0) at_mbar_arrive(cut + b);
-            if (WALK && ch == last) {                              // the tile two before this one was stored before its neighbour's last sums were taken
-                odd_rows[(t & 1) * (2 * FP_M + 128) + half * FP_M + row] = odd != odd;
-                const bool any = __any_sync(0xffffffffu, odd != odd);
-                if (lane == 0) odd_warps[(t & 1) * 16 + warp - FP_WARP_W] = any;
-                __syncwarp();
-                if (lane == 0) at_mbar_arrive(marked + (t & 1));
-                ++t, last += chunks, odd = 0.f;
-            }
         }
-        if (!WALK && odd != odd) odd_rows[row] = 1, *any_odd = 1;
     } else if (C::CUTS && warp < C::WARP_SUM) {
         // ---------------------------------------------------------------- cutting a few rows of A, two warps a half of the chunk
         const int half = (warp - FP_WARP_A) >> 1, t = ((warp - FP_WARP_A) & 1) * 32 + lane, row = t % NP;
-        float odd = 0.f;
         for (int ch = 0; ch < chunks; ++ch) {
             const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
@@ -238,10 +236,10 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 const float4 x = *reinterpret_cast<const float4*>(from + (((2 * g) ^ (row & 7)) << 4));
                 const float4 y = *reinterpret_cast<const float4*>(from + (((2 * g + 1) ^ (row & 7)) << 4));
                 uint4 one, two, three;
-                fp_cut(x.x, x.y, one.x, two.x, three.x, odd);
-                fp_cut(x.z, x.w, one.y, two.y, three.y, odd);
-                fp_cut(y.x, y.y, one.z, two.z, three.z, odd);
-                fp_cut(y.z, y.w, one.w, two.w, three.w, odd);
+                fp_cut(x.x, x.y, one.x, two.x, three.x);
+                fp_cut(x.z, x.w, one.y, two.y, three.y);
+                fp_cut(y.x, y.y, one.z, two.z, three.z);
+                fp_cut(y.z, y.w, one.w, two.w, three.w);
                 const int at = ((half * 4 + g) ^ (row & 7)) << 4;
                 *reinterpret_cast<uint4*>(to + at) = one;
                 *reinterpret_cast<uint4*>(to + C::PIECE + at) = two;
@@ -254,14 +252,13 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 at_mbar_arrive(cut + b);
             }
         }
-        if (odd != odd) odd_rows[FP_M + row] = 1, *any_odd = 1;
     } else if (warp == FP_WARP_PIECES) {
         if (!C::CUTS) {
-            // ------------------------------------------------------------ A's pieces, and which of its rows have none
-            int ch = 0;
-            for (int t = 0; t < walk && !failed; ++t) {
-                const int first = tile_m0(t);
-                if (lane == 0) {
+            // ------------------------------------------------------------ A's pieces
+            if (lane == 0) {
+                int ch = 0;
+                for (int t = 0; t < walk && !failed; ++t) {
+                    const int first = tile_m0(t);
                     for (const int begin = ch; ch < begin + chunks; ++ch) {
                         const int b = ch % C::PLACES;
                         if (!at_mbar_wait(a_empty + b, ((uint32_t)(ch / C::PLACES) & 1u) ^ 1u)) { failed = true; break; }
@@ -269,25 +266,9 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         for (int p = 0; p < 3; ++p)
                             at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch - begin) * FP_K, p * m + first, a_full + b);
                     }
-                    if (failed)
-                        for (int i = max(0, ch - C::PLACES); i < ch; ++i) at_mbar_wait(a_full + i % C::PLACES, (uint32_t)(i / C::PLACES) & 1u);
                 }
-                failed = __any_sync(0xffffffffu, failed);
-                if (WALK) {
-                    bool any = false;
-                    for (int j = lane; j < NP; j += 32) {
-                        const bool o = first + j < m && a_odd[first + j] != 0;
-                        odd_rows[(t & 1) * (2 * FP_M + 128) + 2 * FP_M + j] = o;
-                        any = any || o;
-                    }
-                    any = __any_sync(0xffffffffu, any);
-                    if (lane == 0) odd_warps[(t & 1) * 16 + 8] = any;
-                    __syncwarp();
-                    if (lane == 0) at_mbar_arrive(marked + (t & 1));
-                } else {
-                    for (int j = lane; j < NP && m0 + j < m; j += 32)
-                        if (a_odd[m0 + j] != 0) odd_rows[FP_M + j] = 1, *any_odd = 1;
-                }
+                if (failed)                                        // as above
+                    for (int i = max(0, ch - C::PLACES); i < ch; ++i) at_mbar_wait(a_full + i % C::PLACES, (uint32_t)(i / C::PLACES) & 1u);
             }
         }
     } else {
@@ -316,28 +297,24 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 }
             }
             if constexpr (WALK) {
-                if (failed || !__all_sync(0xffffffffu, at_mbar_wait(marked + (t & 1), (uint32_t)(t >> 1) & 1u))) { failed = true; break; }
+                if (failed) break;
                 const int first = tile_m0(t), w_row = tile_w0(t) + quarter * 32 + lane, j0 = half * COLS, many = min(COLS, m - first - j0);
                 if (w_row < n) {
                     float* to = c + (size_t)(first + j0) * n + w_row;
+                    float check = 0.f;                             // NaN once a sum is no finite number
 #pragma unroll
                     for (int j = 0; j < COLS; ++j) {
                         float v = sum[j];
+                        check = fmaf(v, 0.f, check);
                         if (EPI == 1) v = cap * tanhf(v / cap);
                         if (j < many) to[(size_t)j * n] = v;
                     }
-                    bool any = false;
-                    for (int i = 0; i < 9; ++i) any = any || odd_warps[(t & 1) * 16 + i] != 0;
-                    const unsigned char* marks = odd_rows + (t & 1) * (2 * FP_M + 128);
-                    const int r = quarter * 32 + lane;
-                    if (any) {                                     // this thread's elements of rows without pieces again
+                    if (check != check) {
+                        const uint64_t again = fp_not_finite<COLS>(sum);
 #pragma unroll 1
                         for (int j = 0; j < many; ++j) {
-                            if ((marks[r] | marks[FP_M + r] | marks[2 * FP_M + j0 + j]) == 0) continue;
-                            const float *x = a + (size_t)(first + j0 + j) * k, *y = w + (size_t)w_row * k;
-                            float v = 0.f;
-#pragma unroll 1
-                            for (int kk = 0; kk < k; ++kk) v = fmaf(x[kk], y[kk], v);
+                            if ((again >> j & 1) == 0) continue;
+                            const float v = fp_chain(a + (size_t)(first + j0 + j) * k, w + (size_t)w_row * k, k);
                             to[(size_t)j * n] = EPI == 1 ? cap * tanhf(v / cap) : v;
                         }
                     }
@@ -345,34 +322,31 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
         }
     }
-    __syncthreads();                                               // the stages have been read, the rows that are not finite are marked
+    __syncthreads();                                               // the stages have been read
     float* sums = reinterpret_cast<float*>(smem);                  // [NP][128], where K is cut
     auto to = [&](int j) { return (size_t)(GROUPED && tiles.order != nullptr ? tiles.order[m0 + j] : m0 + j) * n + n0; };
     if (!WALK && warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
         const int r = (warp & 3) * 32 + lane, j0 = ((warp - C::WARP_SUM) >> 2) * COLS;
-        if (segments == 1) {
-            if (n0 + r < n)
-#pragma unroll
-                for (int j = 0; j < COLS; ++j) {
-                    float v = sum[j];
-                    if (EPI == 1) v = cap * tanhf(v / cap);
-                    if (j0 + j < rows) c[to(j0 + j) + r] = v;
-                }
-        } else {
+        if (segments > 1) {
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sums[(j0 + j) * FP_M + r] = sum[j];
-        }
-        if (*any_odd != 0 && n0 + r < n) {                         // this thread's elements of rows without pieces again
-            const int k0 = chunk0 * FP_K, k1 = min(k, (chunk0 + chunks) * FP_K);
+        } else if (n0 + r < n) {
+            float check = 0.f;                                     // as above
+#pragma unroll
+            for (int j = 0; j < COLS; ++j) {
+                float v = sum[j];
+                check = fmaf(v, 0.f, check);
+                if (EPI == 1) v = cap * tanhf(v / cap);
+                if (j0 + j < rows) c[to(j0 + j) + r] = v;
+            }
+            if (check != check) {
+                const uint64_t again = fp_not_finite<COLS>(sum);
 #pragma unroll 1
-            for (int j = j0; j < min(j0 + COLS, rows); ++j) {
-                if ((odd_rows[r] | odd_rows[FP_M + j]) == 0) continue;
-                const float *x = a + (size_t)(m0 + j) * k, *y = w + (size_t)(w0 + r) * k;
-                float v = 0.f;
-#pragma unroll 1
-                for (int kk = k0; kk < k1; ++kk) v = fmaf(x[kk], y[kk], v);
-                if (segments > 1) sums[j * FP_M + r] = v;
-                else c[to(j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
+                for (int j = 0; j < min(COLS, rows - j0); ++j) {
+                    if ((again >> j & 1) == 0) continue;
+                    const float v = fp_chain(a + (size_t)(m0 + j0 + j) * k, w + (size_t)(w0 + r) * k, k);
+                    c[to(j0 + j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
+                }
             }
         }
     }
@@ -389,8 +363,10 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                              : "=f"(x) : "r"(at), "r"(s) : "memory");
                 v = s == 0 ? x : v + x;
             }
-            if (EPI == 1) v = cap * tanhf(v / cap);
-            if (j < rows && n0 + r < n) c[to(j) + r] = v;
+            if (j < rows && n0 + r < n) {
+                if (!fp_finite(v)) v = fp_chain(a + (size_t)(m0 + j) * k, w + (size_t)(w0 + r) * k, k);
+                c[to(j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
+            }
         }
         fp_cluster_sync();                                         // nobody leaves while its sums are read
     }
@@ -403,26 +379,23 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
 }
 
-// A's rows cut for a product of more than FP_CUT_ROWS: pieces [3, m, kp], kp the next multiple of 8 (the columns beyond k are zeros), and
-// whether a row has none. A block a row.
+// A's rows cut for a product of more than FP_CUT_ROWS: pieces [3, m, kp], kp the next multiple of 8 (the columns beyond k are zeros).
+// A block a row.
 __global__ void __launch_bounds__(256)
-f32_cut_rows_kernel(const float* __restrict__ a, uint32_t* __restrict__ pieces, int* __restrict__ odd_rows, int m, int k, int kp) {
+f32_cut_rows_kernel(const float* __restrict__ a, uint32_t* __restrict__ pieces, int m, int k, int kp) {
     const int row = blockIdx.x;
     const float* from = a + (size_t)row * k;
     uint32_t* to = pieces + (size_t)row * (kp / 2);
     const size_t piece = (size_t)m * (kp / 2);
-    float odd = 0.f;
     for (int x = threadIdx.x * 4; x < kp; x += 1024) {             // k is a multiple of four
         const float4 v = x < k ? *reinterpret_cast<const float4*>(from + x) : make_float4(0.f, 0.f, 0.f, 0.f);
         uint2 one, two, three;
-        fp_cut(v.x, v.y, one.x, two.x, three.x, odd);
-        fp_cut(v.z, v.w, one.y, two.y, three.y, odd);
+        fp_cut(v.x, v.y, one.x, two.x, three.x);
+        fp_cut(v.z, v.w, one.y, two.y, three.y);
         *reinterpret_cast<uint2*>(to + x / 2) = one;
         *reinterpret_cast<uint2*>(to + piece + x / 2) = two;
         *reinterpret_cast<uint2*>(to + 2 * piece + x / 2) = three;
     }
-    const int any = __syncthreads_or(odd != odd);
-    if (threadIdx.x == 0) odd_rows[row] = any;
 }
 
 template <int NP, int EPI>
@@ -430,12 +403,11 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     using C = Pieces<NP>;
     CUtensorMap map_a, map_w;
     const int kp = (k + 7) & ~7;
-    int* odd_rows = nullptr;
     KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535, "gemm_f32: a weight of %d rows is too much for one launch", n);
-    // More tiles than multiprocessors: blocks walk over them. (The marks of a tile's rows have two places: four chunks a tile keep them apart.)
+    // More tiles than multiprocessors: blocks walk over them.
     const long long all_tiles = (long long)((m + NP - 1) / NP) * ((n + FP_M - 1) / FP_M);
     const int chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
-    const bool walk = !C::CUTS && segments == 1 && all_tiles > sms && all_tiles <= 0x7fffffff - sms && all_tiles / sms * chunks < 0x3fffffff && chunks >= 4;
+    const bool walk = !C::CUTS && segments == 1 && all_tiles > sms && all_tiles <= 0x7fffffff - sms && all_tiles / sms * chunks < 0x3fffffff;
     auto kernel = gemm_f32_pieces_kernel<NP, EPI, false, false>;
     if constexpr (!C::CUTS)
         if (walk) kernel = gemm_f32_pieces_kernel<NP, EPI, false, true>;
@@ -446,9 +418,8 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
         if (int e = encode_map_f32(&map_a, a, m, k, k, NP)) return e;
     } else {
         KB_REQUIRE(scratch != nullptr && ((uintptr_t)scratch & 15) == 0, "gemm_f32: %d rows by pieces without scratch", m);
-        odd_rows = reinterpret_cast<int*>(scratch) + (size_t)3 * m * (kp / 2);
         if (int e = encode_map_bf16(&map_a, scratch, 3ull * m, kp, kp, NP)) return e;
-        f32_cut_rows_kernel<<<m, 256, 0, s>>>(a, reinterpret_cast<uint32_t*>(scratch), odd_rows, m, k, kp);
+        f32_cut_rows_kernel<<<m, 256, 0, s>>>(a, reinterpret_cast<uint32_t*>(scratch), m, k, kp);
         if (int e = check_launch("gemm_f32 cut")) return e;
     }
     cudaLaunchConfig_t cfg = {};
@@ -461,7 +432,7 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
     attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = segments;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, c, a, w, (const int*)odd_rows, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
+    cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, c, a, w, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
     return check_launch("gemm_f32 pieces");
 }
 
@@ -492,7 +463,7 @@ bool gemm_f32_pieces_take(int m, int k, const void* a, const void* w) {
     const bool pays = m > 16 ? k >= 256 : m > 2 && k >= 1024;
     return pays && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
 }
-long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * (3 * ((k + 7) / 8 * 4) + 1); }
+long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * 3 * ((k + 7) / 8 * 4); }
 
 int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, cudaStream_t s) {
     KB_REQUIRE(k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0, "gemm_f32: rows of %d values must begin at 16-byte boundaries", k);
@@ -529,7 +500,7 @@ extern "C" int kb_moe_f32_pieces(float* c, const float* a, const float* w, int e
     CUtensorMap map_a, map_w;
     if (int e = encode_map_f32(&map_a, a, places, k, k, FP_CUT_ROWS)) return e;
     if (int e = encode_map_f32(&map_w, w, (unsigned long long)experts * n, k, k, FP_M)) return e;
-    kernel<<<dim3(tile_cap, (n + FP_M - 1) / FP_M), FP_THREADS, C::SMEM, (cudaStream_t)stream>>>(map_a, map_w, c, a, w, nullptr, places, n, k, (k + FP_K - 1) / FP_K, 0.f,
+    kernel<<<dim3(tile_cap, (n + FP_M - 1) / FP_M), FP_THREADS, C::SMEM, (cudaStream_t)stream>>>(map_a, map_w, c, a, w, places, n, k, (k + FP_K - 1) / FP_K, 0.f,
                                                                                                   F32Tiles{tile_expert, tile_first, tile_rows, n_tiles, order});
     return check_launch("moe_f32 pieces");
 }

@@ -153,3 +153,50 @@ def test_blocks_that_walk_over_tiles(m, more, k):
         if not odd and m != 65:
             want, sizes = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
             assert ((got - want).abs() <= (4 * 2.0 ** -23 + (k // 64 + 2) * 2.0 ** -24) * sizes + 1e-30).all()      # as above
+
+
+def overflowing(m, n, k, gen):
+    """Finite values some of whose products are beyond the largest float, or so near it that the product of their first pieces is."""
+    a, w = torch.randn(m, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    a[3] = 2.0 ** 70 * (1 + torch.rand(k, device="cuda", generator=gen))
+    a[7] = -a[3]
+    w[11] = 2.0 ** 75 * (1 + torch.rand(k, device="cuda", generator=gen))
+    w[n - 1] = -w[11]
+    a[9], w[20] = 0.0, 0.0                                   # one product each that is the largest float less 2^-9 of it
+    a[9, 4], w[20, 4] = 2.0 ** 64 * (1 - 2.0 ** -10), 2.0 ** 64 * (1 - 2.0 ** -10)
+    a[m - 1], w[21] = a[9], w[20]
+    return a, w
+
+
+@pytest.mark.parametrize("m,n", [(20, 600), (50, 600), (200, 600), (200, 9700)])
+@pytest.mark.parametrize("cap", [0.0, 5.0])
+def test_finite_values_whose_products_overflow(m, n, cap):
+    """What is no finite number by pieces is what the multiply-adds make of it: infinities with their signs, under a soft cap the cap, and the
+    finite products next to the largest float."""
+    k = 260
+    a, w = overflowing(m, n, k, torch.Generator(device="cuda").manual_seed(m + n))
+    want = chains(a, w)
+    assert want[3, 11] == float("inf") and want[7, 11] == -float("inf") and torch.isfinite(want[9, 20]) and want[9, 20] > 3.3e38
+    known = torch.isfinite(want)
+    sizes = a.abs().double() @ w.abs().double().T
+    for segments in (1, 4):
+        got = pieces(a, w, segments, cap)
+        if cap:
+            far = want.abs() > 100 * cap                     # tanh is one there
+            assert torch.equal(got[far], cap * torch.sign(want[far])) and not torch.isnan(got).any()
+            continue
+        assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[want.isinf()], want[want.isinf()])
+        assert got[9, 20] == want[9, 20]
+        assert ((got.double() - want.double()).abs() <= k * 2.0 ** -23 * sizes)[known].all()
+
+
+def test_experts_products_that_overflow():
+    from kapel_b200 import kernels as K
+
+    a, flat = overflowing(40, 256, 260, torch.Generator(device="cuda").manual_seed(5))
+    w = flat.view(2, 128, 260)
+    lists = K.moe_sort(torch.arange(2, device="cuda", dtype=torch.int32).repeat(40, 1), 2, torch.float32)       # both experts for every token
+    got = K.moe_grouped(a, w, lists, "none", True, True, torch.float32).view(40, 256)
+    want = chains(a, flat)
+    assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[want.isinf()], want[want.isinf()])
+    assert got[9, 20] == want[9, 20] and torch.isfinite(got[9, 20])
