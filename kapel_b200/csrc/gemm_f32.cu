@@ -313,12 +313,13 @@ extern "C" int kb_gemm_f32(float* c, const float* a, const float* w, int m, int 
 
 // The same by whatever is fastest, the tensor cores included. `scratch`: `kb_gemm_f32_scratch_floats` floats (0: none).
 extern "C" long long kb_gemm_f32_scratch_floats(const float* a, const float* w, int m, int n, int k) {
-    return m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(m, k, a, w) ? gemm_f32_pieces_floats(m, k) : 0;
+    return m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(k, a, w) ? gemm_f32_scratch_floats(m, n, k) : 0;
 }
 extern "C" int kb_gemm_f32_fast(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, float* scratch, void* stream) {
-    if (m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(m, k, a, w)) {
+    if (m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(k, a, w)) {
         KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
-        return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, gemm_f32_segments(m, n, k), scratch, (cudaStream_t)stream);
+        const int groups = gemm_f32_groups(n, k);
+        return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, groups, gemm_f32_way(m, n, k, groups), scratch, (cudaStream_t)stream);
     }
     return kb_gemm_f32_variant(c, a, w, m, n, k, epilogue, cap, -1, stream);
 }

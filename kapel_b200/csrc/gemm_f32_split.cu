@@ -6,12 +6,16 @@
 // nearest.
 //
 // The operands are swapped, 128 weight rows are the MMA's M and 16, 32, 64 or 128 rows of A its N, for a handful of rows and for thousands
-// alike: an element's products and additions are the same in all of them. Where the tiles are too few, K is cut into segments, a block each in a
-// cluster of up to eight, which add up their sums through shared memory in the segments' order. Where they are more than the multiprocessors, a block
-// walks over several, and beginning and ending (some 6 us) are there once: 500 rows by 18,432 x 2,304 204 us by a block a tile, 187 so (now 184).
+// alike. A row's result does not depend on how many others there are: the weight alone says into how many groups of chunks K is cut
+// (`gemm_f32_groups`), a group's chunks are added up in their order, then the groups in theirs, whichever way it is done:
+//   beside   a block a group, in a cluster of up to eight, which add up their sums through shared memory (few rows, narrow weights)
+//   whole    a block has all of a tile's groups one after the other, the sums so far in tensor memory and, of 128 rows, half in shared memory (in the
+//            result's place they took 3.3 us a group), and walks over several tiles where they are more than the multiprocessors: beginning and ending
+//            (some 6 us) are there once
+//   apart    blocks walk over tiles and groups, a group's sums go to scratch, and a second kernel adds them up (tiles that do not fill the GPU)
 //
 // Twenty warps:
-//   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep (five with 128 rows), as 32-bit values (and of up to 32 rows of A)
+//   warp 0        asks TMA for 32 k of the 128 weight rows, eight stages deep (three with 128 rows, as fast as five), as 32-bit values (and of up to 32 rows of A)
 //   warps 3-10    cut the weights, each half of them every second stage: a thread has a row, its pieces go to tensor memory, from where the
 //                 MMA takes its A operand
 //   warps 1, 2    issue the 24 MMAs of a chunk, one the even chunks, the other the odd ones (issuing takes a thread longer than the tensor
@@ -44,12 +48,14 @@ template <int NP> struct Pieces {
     static constexpr bool CUTS = NP <= FP_CUT_ROWS;
     static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
     static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
-    static constexpr int STAGES = NP == 128 ? 5 : 8, PLACES = CUTS ? 2 : (NP == 128 ? 3 : 4);      // of the pieces of A
-    static constexpr int SMEM = STAGES * STAGE + PLACES * PIECES + 1024 /* alignment */ + 288 /* barriers */;
-    static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, TMEM_COLS = COL_W + 192 <= 256 ? 256 : 512;
+    static constexpr int STAGES = NP == 128 ? 3 : 8, PLACES = CUTS ? 2 : (NP == 128 ? 3 : 4);      // of the pieces of A
     static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
-    static_assert(SMEM <= 232448, "more shared memory than a block can have");
-    static_assert(STAGES * STAGE >= NP * FP_M * 4, "the sums take the stages' place");
+    static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, COL_HELD = COL_W + 192, HELD = CUTS ? 0 : 32;      // sums of earlier groups a thread has in tensor memory
+    static constexpr int MORE = CUTS ? 0 : (COLS - HELD) * 2 * FP_M * 4;                           // and what does not fit there
+    static constexpr int SMEM = STAGES * STAGE + PLACES * PIECES + MORE + 1024 /* alignment */ + 288 /* barriers */;
+    static constexpr int TMEM_COLS = COL_HELD + 2 * HELD <= 256 ? 256 : 512;
+    static_assert(SMEM <= 232448 && COL_HELD + 2 * HELD <= 512, "more shared or tensor memory than a block can have");
+    static_assert(STAGES * STAGE + PLACES * PIECES >= NP * FP_M * 4, "the sums take the place of what was multiplied");
 };
 
 __device__ __forceinline__ void fp_ld16(uint32_t taddr, uint32_t (&r)[16]) {
@@ -72,14 +78,6 @@ __device__ __noinline__ float fp_chain(const float* x, const float* y, int k) {
     }
     return v;
 }
-// A bit for each of a thread's sums that is no finite number.
-template <int COLS> __device__ __forceinline__ uint64_t fp_not_finite(const float (&sum)[COLS]) {
-    uint64_t bits = 0;
-#pragma unroll
-    for (int j = 0; j < COLS; ++j) bits |= fp_finite(sum[j]) ? 0ull : 1ull << j;
-    return bits;
-}
-
 __device__ __forceinline__ void fp_cluster_sync() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
@@ -94,11 +92,14 @@ struct F32Tiles {
 };
 
 // epilogue 0: none; 1: cap * tanh(acc / cap). GROUPED: blockIdx.x is a tile of `tiles`, NP rows at most, m the places there are.
-// WALK: a block takes tile after tile, gridDim.x apart; its warps go on to the next one's chunks while the last one's sums are stored.
+// WALK: a block takes item after item, its warps go on to the next one's chunks while the last one's sums are stored. An item is a group of a tile:
+// with `leave_apart` (c is [groups, m, n] then) any of all tiles' groups, gridDim.x apart; else all groups of a tile in turn, the tiles gridDim.x apart.
+// Without WALK a block has the one that its place in the grid says.
 template <int NP, int EPI, bool GROUPED, bool WALK>
 __global__ void __launch_bounds__(FP_THREADS, 1)
 gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_w, float* __restrict__ c,
-                       const float* __restrict__ a, const float* __restrict__ w, int m, int n, int k, int chunks_a_segment, float cap, const F32Tiles tiles) {
+                       const float* __restrict__ a, const float* __restrict__ w, int m, int n, int k, int groups, int chunks_a_group, float cap, int leave_apart,
+                       const F32Tiles tiles) {
     // map_a: of A's 32-bit values where the block cuts them, else of their pieces [3, m, k up to a multiple of 8]
     using C = Pieces<NP>;
     static_assert(!GROUPED || C::CUTS, "a tile's rows are cut by the blocks that need them");
@@ -107,7 +108,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     if (GROUPED && (int)blockIdx.x >= tiles.count[0]) return;
     unsigned char* smem = reinterpret_cast<unsigned char*>(((uintptr_t)fp_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* pieces = smem + C::STAGES * C::STAGE;           // [PLACES][3][NP rows][128 bytes]
-    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::PLACES * C::PIECES);
+    uint64_t* full = reinterpret_cast<uint64_t*>(pieces + C::PLACES * C::PIECES + C::MORE);
     uint64_t* empty = full + C::STAGES;                            // the warps that cut it have read the stage
     uint64_t* cut = empty + C::STAGES;                             // [2] a chunk's pieces are there that are cut here
     uint64_t* a_full = cut + 2;                                    // [PLACES] its pieces of A that are not
@@ -119,13 +120,26 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = GROUPED ? tiles.first[blockIdx.x] : blockIdx.x * NP, rows = GROUPED ? min(tiles.rows[blockIdx.x], m - m0) : m - m0;      // what lies behind is not stored
-    const int n0 = blockIdx.y * FP_M, w0 = GROUPED ? tiles.expert[blockIdx.x] * n + n0 : n0, segment = WALK ? 0 : blockIdx.z, segments = WALK ? 1 : gridDim.z;
-    const int m_tiles = (m + NP - 1) / NP, all_tiles = m_tiles * ((n + FP_M - 1) / FP_M);
-    const int walk = WALK ? (all_tiles - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;      // this block's tiles
-    auto tile_m0 = [&](int t) { return WALK ? ((int)blockIdx.x + t * (int)gridDim.x) % m_tiles * NP : m0; };
-    auto tile_w0 = [&](int t) { return WALK ? ((int)blockIdx.x + t * (int)gridDim.x) / m_tiles * FP_M : w0; };
-    const int chunks_all = (k + FP_K - 1) / FP_K;
-    const int chunk0 = segment * chunks_a_segment, chunks = max(0, min(chunks_a_segment, chunks_all - chunk0));
+    const int n0 = blockIdx.y * FP_M, w0 = GROUPED ? tiles.expert[blockIdx.x] * n + n0 : n0, segment = WALK ? 0 : blockIdx.z;
+    const int m_tiles = (m + NP - 1) / NP, all_tiles = m_tiles * ((n + FP_M - 1) / FP_M), chunks_all = (k + FP_K - 1) / FP_K;
+    const bool apart = WALK && leave_apart != 0;
+    const int units = apart ? all_tiles * groups : all_tiles, mine = WALK ? (units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 1;
+    const int items = WALK && !apart ? mine * groups : mine;       // this block's
+    struct Item { int m0, w0, group, chunk0, chunks; };
+    auto item = [&](int i) {
+        Item r;
+        int tile = 0;
+        if (!WALK) r.group = segment;
+        else if (apart) r.group = ((int)blockIdx.x + i * (int)gridDim.x) / all_tiles, tile = ((int)blockIdx.x + i * (int)gridDim.x) % all_tiles;
+        else r.group = i % groups, tile = (int)blockIdx.x + i / groups * (int)gridDim.x;
+        r.m0 = WALK ? tile % m_tiles * NP : m0, r.w0 = WALK ? tile / m_tiles * FP_M : w0;
+        r.chunk0 = r.group * chunks_a_group, r.chunks = max(0, min(chunks_a_group, chunks_all - r.chunk0));
+        return r;
+    };
+    int chunks = 0;                                                // of all items
+    if (WALK && !apart) chunks = mine * chunks_all;
+    else
+        for (int i = 0; i < items; ++i) chunks += item(i).chunks;
 
     if (tid == 0) {
         for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 6 : 4); }      // the warps that cut the stage
@@ -151,15 +165,17 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
 
     if (warp == 0) {
         if (lane == 0) {
-            int it = 0, t = 0, step = 0, row = tile_w0(0);
-            for (; it < 2 * chunks * walk; ++it, ++step) {
-                if (WALK && step == 2 * chunks) step = 0, row = tile_w0(++t);
-                const int s = it % C::STAGES;
-                if (!at_mbar_wait(empty + s, ((uint32_t)(it / C::STAGES) & 1u) ^ 1u)) { failed = true; break; }
-                const uint32_t dst = at_saddr(smem + s * C::STAGE);
-                at_mbar_expect_tx(full + s, C::STAGE);
-                at_tma_box(dst, &map_w, chunk0 * FP_K + step * FP_STAGE_K, row, full + s);
-                if (C::CUTS) at_tma_box(dst + C::W_BYTES, &map_a, chunk0 * FP_K + it * FP_STAGE_K, m0, full + s);
+            int it = 0;
+            for (int i = 0; i < items && !failed; ++i) {
+                const Item at = item(i);
+                for (int step = 0; step < 2 * at.chunks; ++step, ++it) {
+                    const int s = it % C::STAGES;
+                    if (!at_mbar_wait(empty + s, ((uint32_t)(it / C::STAGES) & 1u) ^ 1u)) { failed = true; break; }
+                    const uint32_t dst = at_saddr(smem + s * C::STAGE);
+                    at_mbar_expect_tx(full + s, C::STAGE);
+                    at_tma_box(dst, &map_w, at.chunk0 * FP_K + step * FP_STAGE_K, at.w0, full + s);
+                    if (C::CUTS) at_tma_box(dst + C::W_BYTES, &map_a, at.chunk0 * FP_K + step * FP_STAGE_K, at.m0, full + s);
+                }
             }
             if (failed)                                            // the copies in flight land before the block goes on
                 for (int i = max(0, it - C::STAGES); i < it; ++i) at_mbar_wait(full + i % C::STAGES, (uint32_t)(i / C::STAGES) & 1u);
@@ -174,7 +190,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         const uint32_t d = tm + (uint32_t)(b * C::ACC), aw = tm + (uint32_t)(C::COL_W + b * 96);
         const uint64_t first = at_desc(at_saddr(pieces), 16, 1024);
         int place = b;
-        for (int ch = b; ch < chunks * walk; ch += 2) {
+        for (int ch = b; ch < chunks; ch += 2) {
             bool there = at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u);
             if (!C::CUTS) there = there && at_mbar_wait(a_full + place, (uint32_t)(ch / C::PLACES) & 1u);
             there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
@@ -196,7 +212,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
         const int quarter = warp & 3, half = (warp - FP_WARP_W) >> 2;      // of the TMEM lanes, which are the weight rows; of the chunk
         const int row = quarter * 32 + lane;
-        for (int ch = 0; ch < chunks * walk; ++ch) {
+        for (int ch = 0; ch < chunks; ++ch) {
             const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
             const unsigned char* from = smem + s * C::STAGE + row * 128;
@@ -257,14 +273,14 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             // ------------------------------------------------------------ A's pieces
             if (lane == 0) {
                 int ch = 0;
-                for (int t = 0; t < walk && !failed; ++t) {
-                    const int first = tile_m0(t);
-                    for (const int begin = ch; ch < begin + chunks; ++ch) {
+                for (int i = 0; i < items && !failed; ++i) {
+                    const Item at = item(i);
+                    for (int j = 0; j < at.chunks; ++j, ++ch) {
                         const int b = ch % C::PLACES;
                         if (!at_mbar_wait(a_empty + b, ((uint32_t)(ch / C::PLACES) & 1u) ^ 1u)) { failed = true; break; }
                         at_mbar_expect_tx(a_full + b, C::PIECES);
                         for (int p = 0; p < 3; ++p)
-                            at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (chunk0 + ch - begin) * FP_K, p * m + first, a_full + b);
+                            at_tma_box(at_saddr(pieces + b * C::PIECES + p * C::PIECE), &map_a, (at.chunk0 + j) * FP_K, p * m + at.m0, a_full + b);
                     }
                 }
                 if (failed)                                        // as above
@@ -275,10 +291,12 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         // ---------------------------------------------------------------- adding up: a weight row and COLS of A's rows a thread
         const int quarter = warp & 3, half = (warp - C::WARP_SUM) >> 2;
         const uint32_t lanes = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * COLS);
-        for (int t = 0; t < walk && !failed; ++t) {
+        int ch = 0;
+        for (int i = 0; i < items && !failed; ++i) {
+            const Item at = item(i);
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sum[j] = 0.f;
-            for (int ch = t * chunks; ch < (t + 1) * chunks; ++ch) {
+            for (const int end = ch + at.chunks; ch < end; ++ch) {
                 const int b = ch & 1;
                 if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, (uint32_t)(ch >> 1) & 1u))) { failed = true; break; }
                 at_fence_after();
@@ -298,23 +316,56 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
             if constexpr (WALK) {
                 if (failed) break;
-                const int first = tile_m0(t), w_row = tile_w0(t) + quarter * 32 + lane, j0 = half * COLS, many = min(COLS, m - first - j0);
+                if (!apart && groups > 1) {                        // the groups so far, half of 128 rows' sums (all of 64) in tensor memory
+                    const uint32_t held = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(C::COL_HELD + half * C::HELD);
+                    float* more = reinterpret_cast<float*>(pieces + C::PLACES * C::PIECES) + half * (COLS - C::HELD) * FP_M + quarter * 32 + lane;
+                    if (at.group > 0) {
+#pragma unroll
+                        for (int c0 = 0; c0 < C::HELD; c0 += 16) {
+                            uint32_t r[16];
+                            fp_ld16(held + (uint32_t)c0, r);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) sum[c0 + j] = __uint_as_float(r[j]) + sum[c0 + j];
+                        }
+#pragma unroll
+                        for (int j = C::HELD; j < COLS; ++j) sum[j] = more[(j - C::HELD) * FP_M] + sum[j];
+                    }
+                    if (at.group < groups - 1) {
+#pragma unroll
+                        for (int c0 = 0; c0 < C::HELD; c0 += 16) {
+                            uint32_t r[16];
+#pragma unroll
+                            for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(sum[c0 + j]);
+                            at_st16(held + (uint32_t)c0, r);
+                        }
+                        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll
+                        for (int j = C::HELD; j < COLS; ++j) more[(j - C::HELD) * FP_M] = sum[j];
+                        continue;
+                    }
+                }
+                const int w_row = at.w0 + quarter * 32 + lane, j0 = half * COLS, many = min(COLS, m - at.m0 - j0);
                 if (w_row < n) {
-                    float* to = c + (size_t)(first + j0) * n + w_row;
+                    float* to = c + (size_t)((apart ? at.group * m : 0) + at.m0 + j0) * n + w_row;
                     float check = 0.f;                             // NaN once a sum is no finite number
 #pragma unroll
                     for (int j = 0; j < COLS; ++j) {
                         float v = sum[j];
                         check = fmaf(v, 0.f, check);
-                        if (EPI == 1) v = cap * tanhf(v / cap);
+                        if (EPI == 1 && !apart) v = cap * tanhf(v / cap);
                         if (j < many) to[(size_t)j * n] = v;
                     }
-                    if (check != check) {
-                        const uint64_t again = fp_not_finite<COLS>(sum);
+                    if (!apart && check != check) {                // as they are, then one after the other
+                        if (EPI == 1) {
+#pragma unroll
+                            for (int j = 0; j < COLS; ++j)
+                                if (j < many) to[(size_t)j * n] = sum[j];
+                        }
 #pragma unroll 1
                         for (int j = 0; j < many; ++j) {
-                            if ((again >> j & 1) == 0) continue;
-                            const float v = fp_chain(a + (size_t)(first + j0 + j) * k, w + (size_t)w_row * k, k);
+                            float v = to[(size_t)j * n];
+                            if (!fp_finite(v)) v = fp_chain(a + (size_t)(at.m0 + j0 + j) * k, w + (size_t)w_row * k, k);
                             to[(size_t)j * n] = EPI == 1 ? cap * tanhf(v / cap) : v;
                         }
                     }
@@ -324,10 +375,11 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
     }
     __syncthreads();                                               // the stages have been read
     float* sums = reinterpret_cast<float*>(smem);                  // [NP][128], where K is cut
+    constexpr bool ONE = C::CUTS;                                  // K may be in one group (many rows walk then)
     auto to = [&](int j) { return (size_t)(GROUPED && tiles.order != nullptr ? tiles.order[m0 + j] : m0 + j) * n + n0; };
     if (!WALK && warp >= C::WARP_SUM && warp != FP_WARP_PIECES) {
         const int r = (warp & 3) * 32 + lane, j0 = ((warp - C::WARP_SUM) >> 2) * COLS;
-        if (segments > 1) {
+        if (!ONE || groups > 1) {
 #pragma unroll
             for (int j = 0; j < COLS; ++j) sums[(j0 + j) * FP_M + r] = sum[j];
         } else if (n0 + r < n) {
@@ -340,24 +392,28 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 if (j0 + j < rows) c[to(j0 + j) + r] = v;
             }
             if (check != check) {
-                const uint64_t again = fp_not_finite<COLS>(sum);
+                if (EPI == 1) {
+#pragma unroll
+                    for (int j = 0; j < COLS; ++j)
+                        if (j0 + j < rows) c[to(j0 + j) + r] = sum[j];
+                }
 #pragma unroll 1
                 for (int j = 0; j < min(COLS, rows - j0); ++j) {
-                    if ((again >> j & 1) == 0) continue;
-                    const float v = fp_chain(a + (size_t)(m0 + j0 + j) * k, w + (size_t)(w0 + r) * k, k);
+                    float v = c[to(j0 + j) + r];
+                    if (!fp_finite(v)) v = fp_chain(a + (size_t)(m0 + j0 + j) * k, w + (size_t)(w0 + r) * k, k);
                     c[to(j0 + j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
                 }
             }
         }
     }
-    if (!WALK && segments > 1) {
+    if (!WALK && (!ONE || groups > 1)) {
         fp_cluster_sync();
-        const int per = NP / segments;                             // rows of A this block adds up
+        const int per = NP / groups;                               // rows of A this block adds up
         for (int i = tid; i < per * FP_M; i += FP_THREADS) {
             const int j = segment * per + i / FP_M, r = i % FP_M;
             const uint32_t at = at_saddr(sums + j * FP_M + r);
             float v = 0.f;
-            for (int s = 0; s < segments; ++s) {
+            for (int s = 0; s < groups; ++s) {
                 float x;
                 asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %1, %2;\n\tld.shared::cluster.f32 %0, [ra];\n\t}"
                              : "=f"(x) : "r"(at), "r"(s) : "memory");
@@ -398,16 +454,39 @@ f32_cut_rows_kernel(const float* __restrict__ a, uint32_t* __restrict__ pieces, 
     }
 }
 
+// c = the groups' sums added up in their order: four elements a thread.
+template <int EPI>
+__global__ void __launch_bounds__(256)
+f32_add_groups_kernel(float* __restrict__ c, const float* __restrict__ partial, const float* __restrict__ a, const float* __restrict__ w, long long all, int n, int k, int groups, float cap) {
+    const long long first = (long long)blockIdx.x * 1024 + threadIdx.x;
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = first + 256 * j < all ? partial[first + 256 * j] : 0.f;
+#pragma unroll 3
+    for (int g = 1; g < groups; ++g)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (first + 256 * j < all) v[j] += partial[(size_t)g * all + first + 256 * j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const long long i = first + 256 * j;
+        if (i >= all) break;
+        if (!fp_finite(v[j])) v[j] = fp_chain(a + (size_t)(i / n) * k, w + (size_t)(i % n) * k, k);
+        c[i] = EPI == 1 ? cap * tanhf(v[j] / cap) : v[j];
+    }
+}
+
 template <int NP, int EPI>
-static int launch_pieces(float* c, const float* a, const float* w, int m, int n, int k, int segments, float cap, float* scratch, cudaStream_t s) {
+static int launch_pieces(float* c, const float* a, const float* w, int m, int n, int k, int groups, int way, float cap, float* scratch, cudaStream_t s) {
     using C = Pieces<NP>;
     CUtensorMap map_a, map_w;
-    const int kp = (k + 7) & ~7;
+    const int kp = (k + 7) & ~7, chunks = (k + FP_K - 1) / FP_K, chunks_a_group = (chunks + groups - 1) / groups, sms = multiprocessors();
     KB_REQUIRE((n + FP_M - 1) / FP_M <= 65535, "gemm_f32: a weight of %d rows is too much for one launch", n);
-    // More tiles than multiprocessors: blocks walk over them.
-    const long long all_tiles = (long long)((m + NP - 1) / NP) * ((n + FP_M - 1) / FP_M);
-    const int chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
-    const bool walk = !C::CUTS && segments == 1 && all_tiles > sms && all_tiles <= 0x7fffffff - sms && all_tiles / sms * chunks < 0x3fffffff;
+    const bool walk = !C::CUTS && (way != FP_BESIDE || groups == 1);
+    if (walk) groups = (chunks + chunks_a_group - 1) / chunks_a_group;       // those that are empty add nothing
+    const long long tiles = (long long)((m + NP - 1) / NP) * ((n + FP_M - 1) / FP_M), units = way == FP_APART ? tiles * groups : tiles;
+    KB_REQUIRE(units <= 0x7fffffff - sms && (units / sms + 1) * chunks < 0x3fffffff, "gemm_f32: %d rows by %d x %d are too much for one launch", m, n, k);
+    float* partial = walk && way == FP_APART ? scratch + gemm_f32_pieces_floats(m, k) : nullptr;
     auto kernel = gemm_f32_pieces_kernel<NP, EPI, false, false>;
     if constexpr (!C::CUTS)
         if (walk) kernel = gemm_f32_pieces_kernel<NP, EPI, false, true>;
@@ -423,53 +502,79 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
         if (int e = check_launch("gemm_f32 cut")) return e;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = walk ? dim3(sms) : dim3((m + NP - 1) / NP, (n + FP_M - 1) / FP_M, segments);
+    cfg.gridDim = walk ? dim3((unsigned)(units < sms ? units : sms)) : dim3((m + NP - 1) / NP, (n + FP_M - 1) / FP_M, groups);
     cfg.blockDim = FP_THREADS;
     cfg.dynamicSmemBytes = C::SMEM;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = segments;
+    attr[0].val.clusterDim.x = 1, attr[0].val.clusterDim.y = 1, attr[0].val.clusterDim.z = walk ? 1 : groups;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, c, a, w, m, n, k, (chunks + segments - 1) / segments, cap, F32Tiles{});
-    return check_launch("gemm_f32 pieces");
+    cudaLaunchKernelEx(&cfg, kernel, map_a, map_w, partial != nullptr ? partial : c, a, w, m, n, k, groups, chunks_a_group, cap, (int)(partial != nullptr), F32Tiles{});
+    if (int e = check_launch("gemm_f32 pieces")) return e;
+    if (partial == nullptr) return 0;
+    const long long all = (long long)m * n;
+    KB_REQUIRE((all + 1023) / 1024 <= 0x7fffffffll, "gemm_f32: %d rows by %d are too much for one launch", m, n);
+    f32_add_groups_kernel<EPI><<<(unsigned)((all + 1023) / 1024), 256, 0, s>>>(c, partial, a, w, all, n, k, groups, cap);
+    return check_launch("gemm_f32 groups");
 }
 
-// Segments of K: the waves of blocks times what a block takes, a chunk 0.65 us with up to 32 rows, 0.7 with 64, 1.2 with 128, and 5 or (in a
-// cluster) 6.5 us to begin and end. A block takes a multiprocessor; clusters of four and eight do not fit every group of them, so that seven
-// eighths and three quarters run at once (144 blocks in clusters of eight: two waves). Of 95 sizes (512 to 18,432 weight rows of 1,024 to 9,216, 1
-// to 500 rows) the choice is the fastest of the four in all, or within 3 % of it.
-int gemm_f32_segments(int m, int n, int k) {
-    const int tiles = ((m + 127) / 128) * ((n + FP_M - 1) / FP_M), chunks = (k + FP_K - 1) / FP_K, sms = multiprocessors();
-    const double chunk_us = m > 64 ? 1.2 : m > 32 ? 0.68 : 0.65;
+// Clusters of four and eight do not fit every group of multiprocessors, so that seven eighths and three quarters run at once (144 blocks in
+// clusters of eight: two waves).
+static int fp_clusters(int groups) {
+    const int sms = multiprocessors();
+    const int at_once = groups <= 2 ? sms : (groups == 4 ? sms * 7 / 8 : sms * 3 / 4) / groups * groups;
+    return at_once > 0 ? at_once : 1;
+}
+// Groups of K: what is fastest for up to 32 rows, whatever the rows there are. The waves of blocks times what a block takes, 0.65 us a chunk, and 5 or (in a
+// cluster) 6.5 us to begin and end.
+int gemm_f32_groups(int n, int k) {
+    const int tiles = (n + FP_M - 1) / FP_M, chunks = (k + FP_K - 1) / FP_K;
     int best = 1;
     double least = 0;
-    for (int s = 1; s <= 8 && s <= chunks; s *= 2) {
-        const int at_once = s <= 2 ? sms : (s == 4 ? sms * 7 / 8 : sms * 3 / 4) / s * s;
-        const int waves = (tiles * s + at_once - 1) / at_once, ends = s == 1 && m > FP_CUT_ROWS ? 1 : waves;      // a block that walks begins and ends once
-        const double us = (double)waves * ((chunks + s - 1) / s * chunk_us) + ends * (s == 1 ? 5.0 : 6.5);
-        if (s == 1 || us < least) least = us, best = s;
+    for (int g = 1; g <= 8 && g <= chunks; g *= 2) {
+        const int at_once = fp_clusters(g), waves = (int)(((long long)tiles * g + at_once - 1) / at_once);
+        const double us = waves * ((chunks + g - 1) / g * 0.65 + (g == 1 ? 5.0 : 6.5));
+        if (g == 1 || us < least) least = us, best = g;
     }
     return best;
 }
-// More than 16 rows of 256 and more, and three to 16 of 1,024 and more: one accumulator an element in ascending k, a kernel for each, is limited by
-// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
-// chains, 184 by pieces; by 2,304 x 9,216 545 and 99, by 2,304 x 2,048 131 and 29, by 64 x 2,048 62 and 16, by 512 x 512 17 and 12, by 1,024 x 256 13 and
-// 12 (64 rows 9.3 and 8.8). Six rows: 54 and 31, 72 and 30, 18 and 11, 18 and 9, 6.3 and 6.6 (of 768: 8.3 and 8.3). Three and four: 44 and 31, 51 and 30, 14 and 12,
-// 13 and 9, by 256,000 x 2,304 440 and 384; one row 37 and 31, 32 and 30, 9.5 and 11.6, 355 and 384. The error against 64 bits is 0.07 to 0.3 of the
-// chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
-bool gemm_f32_pieces_take(int m, int k, const void* a, const void* w) {
-    const bool pays = m > 16 ? k >= 256 : m > 2 && k >= 1024;
-    return pays && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0;
+// How the groups are done: what the three ways take, 0.68 us a chunk with 64 rows a tile and 1.2 with 128, 0.7 us to leave a group's sums and take
+// them up again, 3 us and 4 TB/s to add up what lies apart. In us, beside, whole and apart, by 2,304 x 9,216 in four groups: 128 rows 50, 137, 52; 256 rows
+// 90, 140, 56; 500 rows 140, 155, 101; 2,048 rows 543, 413, 447. By 4,096 x 2,304 in four: 128 rows 25, 44, 27; 500 rows 73, 48, 60; 2,048 rows 266, 176, 200
+// (in one group 165).
+int gemm_f32_way(int m, int n, int k, int groups) {
+    if (m <= FP_CUT_ROWS) return FP_BESIDE;
+    if (groups == 1) return FP_WHOLE;
+    const int np = m <= 64 ? 64 : 128, chunks = (k + FP_K - 1) / FP_K, each = (chunks + groups - 1) / groups, sms = multiprocessors();
+    const long long tiles = (long long)((m + np - 1) / np) * ((n + FP_M - 1) / FP_M);
+    const auto waves = [](long long blocks, int at_once) { return (double)((blocks + at_once - 1) / at_once); };
+    const double chunk_us = np == 64 ? 0.68 : 1.2;
+    const double beside = waves(tiles * groups, fp_clusters(groups)) * (each * chunk_us + 6.5);
+    const double whole = waves(tiles, sms) * (chunks * chunk_us + 0.7 * (groups - 1)) + 5.0;
+    const double apart = waves(tiles * groups, sms) * (each * chunk_us + 0.7) + 5.0 + 3.0 + (groups + 1.0) * m * n * 1e-6;
+    return beside <= whole && beside <= apart ? FP_BESIDE : whole <= apart ? FP_WHOLE : FP_APART;
 }
+// From 256 inputs on, whatever the rows: one accumulator an element in ascending k, a kernel for each, is limited by
+// its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
+// chains, 178 by pieces; by 2,304 x 9,216 545 and 101, by 2,304 x 2,048 131 and 36, by 64 x 2,048 62 and 18, by 512 x 512 17 and 18, by 1,024 x 256 13 and
+// 15 (64 rows 9.3 and 12). Eight rows: 56 and 33, 107 and 45, 27 and 17, 19 and 9, 8.2 and 8.4, 8.3 and 8.3. One and two rows are no
+// faster in all: by 18,432 x 2,304 39 and 33, by 2,304 x 9,216 48 and 45, by 2,304 x 2,048 15 and 17, by 2,048 x 1,024 8.3 and 10.6, by 256,000 x 2,304 369
+// and 416; they go this way so that a row has the same bits alone and beside others. The error against 64 bits is 0.07 to 0.3 of the
+// chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
+bool gemm_f32_pieces_take(int k, const void* a, const void* w) { return k >= 256 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0; }
 long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * 3 * ((k + 7) / 8 * 4); }
+long long gemm_f32_scratch_floats(int m, int n, int k) {
+    const int groups = gemm_f32_groups(n, k);
+    return gemm_f32_pieces_floats(m, k) + (gemm_f32_way(m, n, k, groups) == FP_APART ? (long long)groups * m * n : 0);
+}
 
-int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, cudaStream_t s) {
+int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int groups, int way, float* scratch, cudaStream_t s) {
     KB_REQUIRE(k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0, "gemm_f32: rows of %d values must begin at 16-byte boundaries", k);
-    KB_REQUIRE(segments == 1 || segments == 2 || segments == 4 || segments == 8, "gemm_f32: %d segments", segments);
+    KB_REQUIRE((groups == 1 || groups == 2 || groups == 4 || groups == 8) && way >= FP_BESIDE && way <= FP_APART, "gemm_f32: %d groups by way %d", groups, way);
 #define KB_PIECES(NP) \
-    return epilogue == 0 ? launch_pieces<NP, 0>(c, a, w, m, n, k, segments, cap, scratch, s) : launch_pieces<NP, 1>(c, a, w, m, n, k, segments, cap, scratch, s)
+    return epilogue == 0 ? launch_pieces<NP, 0>(c, a, w, m, n, k, groups, way, cap, scratch, s) : launch_pieces<NP, 1>(c, a, w, m, n, k, groups, way, cap, scratch, s)
     if (m <= 16) KB_PIECES(16);
     if (m <= 32) KB_PIECES(32);
     if (m <= 64) KB_PIECES(64);
@@ -500,7 +605,7 @@ extern "C" int kb_moe_f32_pieces(float* c, const float* a, const float* w, int e
     CUtensorMap map_a, map_w;
     if (int e = encode_map_f32(&map_a, a, places, k, k, FP_CUT_ROWS)) return e;
     if (int e = encode_map_f32(&map_w, w, (unsigned long long)experts * n, k, k, FP_M)) return e;
-    kernel<<<dim3(tile_cap, (n + FP_M - 1) / FP_M), FP_THREADS, C::SMEM, (cudaStream_t)stream>>>(map_a, map_w, c, a, w, places, n, k, (k + FP_K - 1) / FP_K, 0.f,
+    kernel<<<dim3(tile_cap, (n + FP_M - 1) / FP_M), FP_THREADS, C::SMEM, (cudaStream_t)stream>>>(map_a, map_w, c, a, w, places, n, k, 1, (k + FP_K - 1) / FP_K, 0.f, 0,
                                                                                                   F32Tiles{tile_expert, tile_first, tile_rows, n_tiles, order});
     return check_launch("moe_f32 pieces");
 }
@@ -511,10 +616,16 @@ extern "C" int kb_gemm_f32_split_error() {
     if (flag) cudaMemcpyToSymbol(g_gemm_f32_split_error, &zero, sizeof(int));
     return flag;
 }
-// The kernel over pieces whatever the sizes, with `segments` blocks to K (0: as the rule has it).
-extern "C" int kb_gemm_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, void* stream) {
+// The kernels over pieces whatever the sizes, K in `groups` (0: as the rule has it), by `way` (FpWay; -1: as the rule has it).
+extern "C" int kb_gemm_f32_pieces_by(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int groups, int way, float* scratch, void* stream) {
     KB_REQUIRE(m >= 0 && n > 0 && k > 0, "gemm_f32: m %d, n %d, k %d", m, n, k);
     KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
     if (m == 0) return 0;
-    return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, segments > 0 ? segments : gemm_f32_segments(m, n, k), scratch, (cudaStream_t)stream);
+    if (groups <= 0) groups = gemm_f32_groups(n, k);
+    return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, groups, way < 0 ? gemm_f32_way(m, n, k, groups) : way, scratch, (cudaStream_t)stream);
+}
+extern "C" int kb_gemm_f32_groups(int n, int k) { return gemm_f32_groups(n, k); }
+// The same by clusters, or in one group.
+extern "C" int kb_gemm_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, void* stream) {
+    return kb_gemm_f32_pieces_by(c, a, w, m, n, k, epilogue, cap, segments, FP_BESIDE, scratch, stream);
 }

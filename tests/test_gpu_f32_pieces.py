@@ -21,6 +21,23 @@ def pieces(a, w, segments, cap=0.0):
     return guarded[1:-1]
 
 
+BESIDE, WHOLE, APART = 0, 1, 2
+
+
+def by_way(a, w, groups, way, cap=0.0):
+    from kapel_b200 import kernels as K
+
+    m, (n, k) = a.shape[0], w.shape
+    lib, ptr = K.library(), lambda t: ctypes.c_void_p(t.data_ptr())
+    guarded = torch.full((m + 2, n), 7.0, device="cuda")
+    floats = m * 3 * ((k + 7) // 8 * 4) + groups * m * n
+    scratch = torch.full((floats + n,), float("nan"), device="cuda")
+    assert lib.kb_gemm_f32_pieces_by(ptr(guarded[1:]), ptr(a), ptr(w), m, n, k, 1 if cap else 0, ctypes.c_float(cap), groups, way, ptr(scratch),
+                                     ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)) == 0, lib.kb_last_error()
+    assert (guarded[0] == 7.0).all() and (guarded[-1] == 7.0).all() and torch.isnan(scratch[floats:]).all()
+    return guarded[1:-1]
+
+
 def chains(a, w):
     from kapel_b200 import kernels as K
 
@@ -73,12 +90,11 @@ def test_which_products_go_that_way():
     gen = torch.Generator(device="cuda").manual_seed(3)
     flat, w = torch.randn(40 * 1024 + 1, device="cuda", generator=gen), torch.randn(2048, 1024, device="cuda", generator=gen)
     a, shifted = flat[:-1].view(40, 1024), flat[1:].view(40, 1024)
-    by_pieces = [m for m in (1, 2, 3, 8, 33, 40) if not torch.equal(K.gemm(a[:m], w), chains(a[:m], w))]
-    assert by_pieces == [3, 8, 33, 40]
+    assert not any(torch.equal(K.gemm(a[:m], w), chains(a[:m], w)) for m in (1, 2, 3, 8, 33, 40))
     assert torch.equal(K.gemm(shifted, w), chains(shifted, w))                 # rows that do not begin at 16-byte boundaries
     shorter = lambda t, k: t[:, :k].contiguous()
-    by_pieces = [(m, k) for m in (16, 17) for k in (252, 256, 1020, 1024) if not torch.equal(K.gemm(shorter(a[:m], k), shorter(w, k)), chains(shorter(a[:m], k), shorter(w, k)))]
-    assert by_pieces == [(16, 1024), (17, 256), (17, 1020), (17, 1024)]
+    by_pieces = [(m, k) for m in (1, 16, 17) for k in (252, 256, 257, 1024) if not torch.equal(K.gemm(shorter(a[:m], k), shorter(w, k)), chains(shorter(a[:m], k), shorter(w, k)))]
+    assert by_pieces == [(m, k) for m in (1, 16, 17) for k in (256, 1024)]     # by the inner size alone: a row's bits do not depend on the batch
     got, want = K.gemm(a, w, softcap=30.0).double(), 30.0 * torch.tanh(a.double() @ w.double().T / 30.0)
     assert (got - want).abs().max() <= 1e-4
     K.check_async_errors()
@@ -200,3 +216,35 @@ def test_experts_products_that_overflow():
     want = chains(a, flat)
     assert torch.equal(torch.isnan(got), torch.isnan(want)) and torch.equal(got[want.isinf()], want[want.isinf()])
     assert got[9, 20] == want[9, 20] and torch.isfinite(got[9, 20])
+
+
+@pytest.mark.parametrize("n,k", [(1, 256), (130, 260), (512, 1024), (2048, 2304), (2304, 2048), (2304, 9216), (4096, 2304), (19072, 324)])
+def test_a_row_does_not_depend_on_the_batch(n, k):
+    """Bit for bit, through the entry point that models call, for every number of rows."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n + k)
+    a, w = torch.randn(1200, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    want = K.gemm(a[:500].contiguous(), w)
+    for m in (1, 2, 3, 16, 17, 32, 33, 64, 65, 128, 129, 200, 300, 700, 1200):
+        rows = min(m, 500)
+        assert torch.equal(K.gemm(a[:m].contiguous(), w)[:rows], want[:rows]), m
+    assert torch.equal(K.gemm(a[499:500].clone(), w), want[499:])
+    K.check_async_errors()
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 1, 256), (64, 257, 1028), (65, 700, 324), (300, 513, 2304), (129, 9700, 260), (40, 19100, 1100)])
+def test_the_groups_of_k_by_either_way(m, n, k):
+    """Blocks beside each other, one block after another group, and sums that lie apart: the same bits, with what is no finite number, too."""
+    for finite in (True, False):
+        a, w = overflowing(m, max(n, 22), k, torch.Generator(device="cuda").manual_seed(m))
+        w = w[:n].contiguous()
+        if finite:
+            a, w = a.clamp(-4.0, 4.0), w.clamp(-4.0, 4.0)
+        else:
+            a[m - 1, k - 1], w[n // 2, 3] = float("nan"), -float("inf")
+        for groups in (1, 2, 4, 8):
+            for cap in (0.0, 5.0):
+                want = torch.nan_to_num(by_way(a, w, groups, BESIDE, cap), nan=1e30)
+                for way in (WHOLE, APART):
+                    assert torch.equal(torch.nan_to_num(by_way(a, w, groups, way, cap), nan=1e30), want), (groups, way, cap)
