@@ -527,9 +527,12 @@ head_linear_mma_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
 // The same product for a few rows (a decode step): the rows are the 16 of an MMA, a warp has eight columns of M[h], which lie together in mt
 // [heads, n_out, n_in] and come straight into registers, 16 bytes a lane, ahead of the wait on the kernel before. A lane's 16 bytes are eight neighbouring
 // inputs of one column, so two MMAs take 32 inputs in the order that gives, and the rows' inputs are read in the same. 32-bit inputs are
-// cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16): nothing is rounded but the sums. 8 rows, 16 heads of
+// cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16). The tensor cores round towards zero, so they add up 32 inputs,
+// the small pieces first, and those sums are added in registers. What comes out as no finite number is computed again by multiply-adds: infinities have no
+// pieces. 8 rows, 16 heads of
 // 128 -> 512: 6.4 us (20.7 by a column a warp, its sums by shuffles), 512 -> 128 with the gate: 9.2 (19.2). What is left is a launch's latency.
 constexpr int HF_ROWS = 16, HF_WARPS = 8, HF_COLS = HF_WARPS * 8, HF_HELD = 16;        // HF_HELD: groups of 32 inputs whose weights a lane holds at once
+constexpr int HF_PORTION = 2048;                            // inputs that lie in shared memory at once, three pieces of 16 rows 200 KB
 // Elements between two rows of the inputs: 64 bytes further into the banks from row to row.
 __host__ __device__ constexpr int hf_ld(int n_in) { return (n_in + 31) / 32 * 32 + ((n_in + 31) / 32 % 2 == 0 ? 32 : 0); }
 template <typename TX> __host__ __device__ constexpr int hf_pieces() { return sizeof(TX) == 4 ? 3 : 1; }
@@ -551,7 +554,7 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
     uint32_t* xs = reinterpret_cast<uint32_t*>(hf_smem);        // [PIECES][16][ld] bfloat16
     const int h = blockIdx.x;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, row = lane >> 2, quad = lane & 3;
-    const int groups = (n_in + 31) / 32, ld = hf_ld(n_in);
+    const int groups = (n_in + 31) / 32, ld = hf_ld(min(n_in, HF_PORTION));
     const int c0 = blockIdx.y * HF_COLS + warp * 8, mine = c0 + row;      // the column whose weights this lane holds
     const bf16* column = mt + ((size_t)h * n_out + min(mine, n_out - 1)) * n_in;
     auto weights = [&](int group) {
@@ -575,43 +578,54 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
     for (int i = 0; i < HF_HELD; ++i) held[i] = weights(i);     // nobody's output
     dependent_wait();                                       // returns at once after a plain launch
     dependent_trigger();
-    const int pairs = groups * 16;                              // of inputs a row; beyond n_in and the last row zeros
-    for (int idx = tid; idx < 16 * pairs; idx += HF_WARPS * 32) {
-        const int t = idx / pairs, k = (idx - t * pairs) * 2;
-        const size_t at = (size_t)t * x_row + (size_t)h * x_head + x_off + k;
-        float a = t < rows && k < n_in ? x.at(at) : 0.f, b = t < rows && k + 1 < n_in ? x.at(at + 1) : 0.f;
-        uint32_t* to = xs + (t * ld + k) / 2;
-        if (PIECES == 1) {
-            const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-            to[0] = *reinterpret_cast<const uint32_t*>(&v);
-        } else {
-            uint32_t two, three;
-            cut_pair(a, b, to[0], two, three);
-            const uint32_t keep = (a == a ? 0xffffu : 0u) | (b == b ? 0xffff0000u : 0u);      // infinity is its first piece alone
-            to[8 * ld] = two & keep, to[16 * ld] = three & keep;
+    const size_t x0 = (size_t)h * x_head + x_off;
+    float acc[4] = {};
+    for (int g0 = 0; g0 < groups; g0 += HF_PORTION / 32) {
+        const int here = min(groups - g0, HF_PORTION / 32), pairs = here * 16;      // of inputs a row; beyond n_in and the last row zeros
+        if (g0 > 0) __syncthreads();                            // the portion before has been read
+        for (int idx = tid; idx < 16 * pairs; idx += HF_WARPS * 32) {
+            const int t = idx / pairs, j = (idx - t * pairs) * 2, k = g0 * 32 + j;
+            const size_t at = (size_t)t * x_row + x0 + k;
+            float a = t < rows && k < n_in ? x.at(at) : 0.f, b = t < rows && k + 1 < n_in ? x.at(at + 1) : 0.f;
+            uint32_t* to = xs + (t * ld + j) / 2;
+            if (PIECES == 1) {
+                const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+                to[0] = *reinterpret_cast<const uint32_t*>(&v);
+            } else {
+                cut_pair(a, b, to[0], to[8 * ld], to[16 * ld]);
+            }
         }
+        __syncthreads();
+        auto multiply = [&](int group, const uint4& w) {
+            float sum[4] = {};
+#pragma unroll
+            for (int q = PIECES - 1; q >= 0; --q) {
+                const uint32_t* from = xs + (q * 16 + row) * (ld / 2) + group * 16 + quad * 4;
+                const uint4 a = *reinterpret_cast<const uint4*>(from), b = *reinterpret_cast<const uint4*>(from + 4 * ld);      // rows `row` and `row` + 8
+                hf_mma(sum, a.x, b.x, a.y, b.y, w.x, w.y);
+                hf_mma(sum, a.z, b.z, a.w, b.w, w.z, w.w);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) acc[i] += sum[i];
+        };
+        if (g0 == 0) {
+#pragma unroll
+            for (int i = 0; i < HF_HELD; ++i)
+                if (i < here) multiply(i, held[i]);
+        }
+        for (int i = g0 == 0 ? HF_HELD : 0; i < here; ++i) multiply(i, weights(g0 + i));
     }
-    __syncthreads();
-    float acc[PIECES][4] = {};
-    auto multiply = [&](int group, const uint4& w) {
-#pragma unroll
-        for (int q = 0; q < PIECES; ++q) {
-            const uint32_t* from = xs + (q * 16 + row) * (ld / 2) + group * 16 + quad * 4;
-            const uint4 a = *reinterpret_cast<const uint4*>(from), b = *reinterpret_cast<const uint4*>(from + 4 * ld);      // rows `row` and `row` + 8
-            hf_mma(acc[q], a.x, b.x, a.y, b.y, w.x, w.y);
-            hf_mma(acc[q], a.z, b.z, a.w, b.w, w.z, w.w);
-        }
-    };
-#pragma unroll
-    for (int i = 0; i < HF_HELD; ++i)
-        if (i < groups) multiply(i, held[i]);
-    for (int i = HF_HELD; i < groups; ++i) multiply(i, weights(i));
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int t = row + (i >> 1) * 8, c = c0 + quad * 2 + (i & 1);
         if (t >= rows || c >= n_out) continue;
-        float v = acc[0][i];
-        if (PIECES == 3) v = (acc[PIECES - 1][i] + acc[PIECES / 2][i]) + v;
+        float v = acc[i];
+        if (!(fabsf(v) < INFINITY)) {
+            const bf16* m = mt + ((size_t)h * n_out + c) * n_in;
+            v = 0.f;
+#pragma unroll 1
+            for (int k = 0; k < n_in; ++k) v = fmaf(x.at((size_t)t * x_row + x0 + k), __bfloat162float(m[k]), v);
+        }
         if (gate.p != nullptr) {
             const float z = gate.at((size_t)t * g_row + g_off + (size_t)h * n_out + c);
             v *= 1.f / (1.f + expf(-z));
@@ -918,8 +932,8 @@ extern "C" int kb_head_linear_mma(void* y, int y_row, int y_head, const void* x,
     if (rows == 0) return 0;
     cudaStream_t s = (cudaStream_t)stream;
     const Src<float> g{gate, gate ? g_splits : 1, (size_t)g_split_stride};
-    const size_t few_smem = (size_t)(x_dt == KB_DT_F32 ? hf_pieces<float>() : 1) * 16 * hf_ld(n_in) * sizeof(bf16);
-    if (rows <= HF_ROWS && few_smem <= 200 * 1024 && (n_out + HF_COLS - 1) / HF_COLS <= 65535) {     // a decode step
+    const size_t few_smem = (size_t)(x_dt == KB_DT_F32 ? hf_pieces<float>() : 1) * 16 * hf_ld(n_in < HF_PORTION ? n_in : HF_PORTION) * sizeof(bf16);
+    if (rows <= HF_ROWS && (n_out + HF_COLS - 1) / HF_COLS <= 65535) {     // a decode step
         const dim3 few(heads, (n_out + HF_COLS - 1) / HF_COLS);
         const bool vec = n_in % 8 == 0 && ((uintptr_t)mt & 15) == 0;
 #define KB_HF(TX, VEC)                                                                                                                                  \

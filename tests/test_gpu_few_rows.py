@@ -88,3 +88,47 @@ def test_gated_unit_by_fours_and_one_by_one(rows, n, act, out):
     beside = torch.empty(rows * 2 * n + 1, device="cuda")[1:].view(rows, 2 * n)      # begins off a 16-byte boundary: a value a thread
     beside.copy_(x)
     assert torch.equal(K.glu(x, act, out_dtype=out), K.glu(beside, act, out_dtype=out))
+
+
+@pytest.mark.parametrize("rows", [1, 5, 16])
+@pytest.mark.parametrize("n_in", [32, 128, 512, 2040, 2048, 2052, 2100, 4097, 13000])
+def test_per_head_products_keep_32_bits(rows, n_in):
+    """Pairs of inputs that differ by 2^-12 of their size, against each other: whatever the inner size nothing of an input is lost, on both sides of what lies in
+    shared memory at once and of what a lane holds."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(n_in)
+    m = torch.ones(2, 9, n_in, device="cuda").bfloat16()
+    m[:, :, 1::2] = -1.0
+    m[1, 3] *= 2.0
+    big = torch.rand(rows, 2, n_in, device="cuda", generator=gen) + 1.0
+    big[..., 1::2] = big[..., : n_in // 2 * 2 : 2] * (1.0 - 2.0 ** -12)
+    if n_in % 2:
+        big[..., -1] = 0.0
+    want = torch.einsum("rhi,hoi->rho", big.double(), m.double())
+    sizes = torch.einsum("rhi,hoi->rho", big.double(), m.double().abs())
+    got = K.head_linear(big.reshape(rows, -1), 2, n_in, 0, m, transposed=True).view(rows, 2, 9).double()
+    # bfloat16's rounding; of 32 inputs the last two additions are of full size and round towards zero (2^-23 of that sum each), those of the groups to nearest
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + (2.0 ** -22 / max(1, n_in // 32) + 2.0 ** -23 * 3) * sizes).all()
+
+
+@pytest.mark.parametrize("rows", [1, 16])
+@pytest.mark.parametrize("n_in", [33, 520, 2600])
+def test_per_head_products_beyond_what_pieces_hold(rows, n_in):
+    """Finite inputs that round to infinity in bfloat16, products beyond the largest float, infinities."""
+    from kapel_b200 import kernels as K
+
+    x, m = torch.zeros(rows, 3, n_in, device="cuda"), torch.zeros(3, 8, n_in, device="cuda").bfloat16()
+    x[:, 0, 4], m[0, :, 4] = 3.4e38, 0.5
+    x[-1, 1], m[1] = 2.0 ** 70 * 1.01, 2.0 ** 70
+    m[1, 5] = -(2.0 ** 70)
+    x[0, 2, 7], m[2, :, 7], m[2, 2, 7] = float("inf"), 1.0, -1.0
+    y = K.head_linear(x.view(rows, -1), 3, n_in, 0, m, transposed=True).view(rows, 3, 8).float()
+    assert torch.equal(y[:, 0], torch.full_like(y[:, 0], 1.7e38).bfloat16().float())
+    signs = torch.ones(8, device="cuda")
+    signs[5] = -1.0
+    assert torch.equal(y[-1, 1], signs * float("inf"))
+    signs = torch.ones(8, device="cuda")
+    signs[2] = -1.0
+    assert torch.equal(y[0, 2], signs * float("inf"))
+    assert rows == 1 or bool((y[1:, 2] == 0).all() and (y[:-1, 1] == 0).all())
