@@ -533,9 +533,9 @@ extern "C" long long kb_delta_scratch_floats(int rows, int heads, int kv_heads, 
     return (long long)rows * (2ll * kv_heads * d + (long long)heads * e + 2ll * heads + kv_heads);
 }
 
-// Floats of scratch that `rows` rows take on the way by chunks (`kb_delta_scan`'s `chunk_scratch`).
-extern "C" long long kb_delta_chunk_floats(int rows, int entries, int heads, int kv_heads, int d, int e) {
-    return delta_chunk_floats(rows, entries, heads, kv_heads, d, e);
+// Floats of scratch that `rows` rows of `entries` requests take on the way by chunks (`kb_delta_scan`'s `chunk_scratch`).
+extern "C" long long kb_delta_chunk_floats(int rows, int entries, int chunk_rows, int heads, int kv_heads, int d, int e) {
+    return rows > 0 && entries > 0 && chunk_rows > 0 ? delta_chunk_floats(rows, entries, chunk_rows, heads, kv_heads, d, e) : 0;
 }
 
 // Whether long portions of these sizes can go by chunks.

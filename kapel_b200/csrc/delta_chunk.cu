@@ -23,6 +23,16 @@ namespace kb {
 
 constexpr int DCH_THREADS = 128, DCH_E = 16, DCH_MAX_D = 128, DCH_LD = DCH_MAX_D + 4;
 
+// Requests by chunks whose rows lie ahead of row r0; all lanes of a warp call.
+__device__ __forceinline__ int delta_chunks_before(const DeltaChunks& p, int r0) {
+    int before = 0;
+    for (int i = threadIdx.x & 31; i < p.entries; i += 32) {
+        const int start = p.entry_start[i];
+        before += start < r0 && p.entry_end[i] - start >= p.from_rows;
+    }
+    return __reduce_add_sync(0xffffffffu, before);
+}
+
 __global__ void __launch_bounds__(DCH_THREADS, 4)
 delta_chunk_kernel(const DeltaChunks p) {
     __shared__ __align__(16) float sk[DCH_C][DCH_LD], sq[DCH_C][DCH_LD];
@@ -42,7 +52,7 @@ delta_chunk_kernel(const DeltaChunks p) {
         *reinterpret_cast<float4*>(&sq[t][x]) = t < n ? *reinterpret_cast<const float4*>(p.qn + from) : none;
     }
     __syncthreads();
-    const int place = delta_chunk_place(first, entry), ld = delta_piece_row(d);
+    const int place = delta_chunk_place(first, delta_chunks_before(p, r0)), ld = delta_piece_row(d);
     for (int i = h == kvh * per ? tid : DCH_C * d; i < DCH_C * (d >> 1); i += DCH_THREADS) {                  // their pieces, by the kv head's first head
         const int t = i / (d >> 1), x = (i - t * (d >> 1)) * 2;
         uint32_t* q = reinterpret_cast<uint32_t*>(p.qk + (((size_t)place * p.kv_heads + kvh) * 2 * DCH_C + t) * ld + x);
@@ -209,7 +219,7 @@ delta_chain_kernel(const DeltaChunks p) {
     }
     const int kvh = head / (p.heads / p.kv_heads);
     float* st = p.state + (size_t)slot * p.state_floats + p.state_off + ((size_t)head * e + c0) * d;      // [16][d]: a column of the memory lies together
-    const int chunks = (r1 - r0 + DCH_C - 1) / DCH_C, ld = delta_piece_row(d), image = DCH_C * ld;        // an operand's pieces of a chunk
+    const int before = delta_chunks_before(p, r0), chunks = (r1 - r0 + DCH_C - 1) / DCH_C, ld = delta_piece_row(d), image = DCH_C * ld;        // an operand's pieces of a chunk
     __nv_bfloat16* wq = reinterpret_cast<__nv_bfloat16*>(dch_raw + sizeof(DchSmem));                      // [2][W, queries]
     __nv_bfloat16* keys = wq + 4 * image;                                                                 // [2]
     if (tid == 0) {
@@ -219,14 +229,14 @@ delta_chain_kernel(const DeltaChunks p) {
     }
     __syncthreads();
     bool failed = false;                                        // a wait that ran out is not repeated, but the walk goes on: the warps meet in every chunk
-    auto weights = [&](int ch) { return p.within + ((size_t)delta_chunk_place(r0 + ch * DCH_C, entry) * p.heads + head) * DCH_WITHIN; };
+    auto weights = [&](int ch) { return p.within + ((size_t)delta_chunk_place(r0 + ch * DCH_C, before) * p.heads + head) * DCH_WITHIN; };
 
     if (warp >= DCH_WARPS + DCH_WRITERS) {
         // ---------------------------------------------------------------- read-outs: a component of four rows a thread; the copies
         const bool copies = tid == (DCH_WARPS + DCH_WRITERS) * 32;
         auto fetch_wq = [&](int ch) {
             if (ch >= chunks || !copies) return;
-            const size_t place = delta_chunk_place(r0 + ch * DCH_C, entry);
+            const size_t place = delta_chunk_place(r0 + ch * DCH_C, before);
             __nv_bfloat16* to = wq + (ch & 1) * 2 * image;
             dch_expect(&m.wq_full[ch & 1], (uint32_t)image * 4);
             dch_bulk(to, p.w + (place * p.heads + head) * image, (uint32_t)image * 2, &m.wq_full[ch & 1]);
@@ -234,7 +244,7 @@ delta_chain_kernel(const DeltaChunks p) {
         };
         auto fetch_k = [&](int ch) {
             if (ch >= chunks || !copies) return;
-            const size_t place = delta_chunk_place(r0 + ch * DCH_C, entry);
+            const size_t place = delta_chunk_place(r0 + ch * DCH_C, before);
             const int b = ch & 1;
             dch_expect(&m.k_full[b], (uint32_t)image * 2 + sizeof(m.within[0]));
             dch_bulk(keys + b * image, p.qk + ((place * p.kv_heads + kvh) * 2 + 1) * image, (uint32_t)image * 2, &m.k_full[b]);
@@ -291,7 +301,7 @@ delta_chain_kernel(const DeltaChunks p) {
         // ---------------------------------------------------------------- U = U0 - W S: a component of four rows a thread
         const int x = (tid - DCH_WARPS * 32) >> 3, t0 = (tid & 7) * 4;
         auto first_writes = [&](int ch) {
-            return *reinterpret_cast<const float4*>(p.u0 + (((size_t)delta_chunk_place(r0 + ch * DCH_C, entry) * p.heads + head) * e + c0 + x) * DCH_LD_W + t0);
+            return *reinterpret_cast<const float4*>(p.u0 + (((size_t)delta_chunk_place(r0 + ch * DCH_C, before) * p.heads + head) * e + c0 + x) * DCH_LD_W + t0);
         };
         auto fade = [&](int ch) { return *reinterpret_cast<const float4*>(weights(ch) + DCH_F + t0); };
         float4 u = first_writes(0), f = fade(0);
@@ -416,17 +426,17 @@ delta_chain_kernel(const DeltaChunks p) {
 // Keys in whole 32 components, values in whole slices.
 bool delta_chunks_take(int d, int e) { return d > 0 && d <= DCH_MAX_D && d % 32 == 0 && e > 0 && e % DCH_E == 0; }
 
-static size_t dch_places(int rows, int entries) { return (size_t)rows / DCH_C + entries + 1; }
+static size_t dch_places(int rows, int entries, int from_rows) { return (size_t)rows / DCH_C + (entries < rows / from_rows ? entries : rows / from_rows) + 1; }
 static size_t dch_image_floats(int d) { return (size_t)DCH_C * delta_piece_row(d) / 2; }
-long long delta_chunk_floats(int rows, int entries, int heads, int kv_heads, int d, int e) {
-    return (long long)(dch_places(rows, entries) * (heads * (dch_image_floats(d) + DCH_WITHIN + (size_t)e * DCH_LD_W) + (size_t)kv_heads * 2 * dch_image_floats(d)));
+long long delta_chunk_floats(int rows, int entries, int from_rows, int heads, int kv_heads, int d, int e) {
+    return (long long)(dch_places(rows, entries, from_rows) * (heads * (dch_image_floats(d) + DCH_WITHIN + (size_t)e * DCH_LD_W) + (size_t)kv_heads * 2 * dch_image_floats(d)));
 }
 
 int launch_delta_chunks(DeltaChunks p, float* scratch, int rows, int longest, cudaStream_t s) {
     const int chunks = (longest + DCH_C - 1) / DCH_C;
     KB_REQUIRE(p.kv_heads <= 65535 && p.entries <= 65535 && p.heads <= 65535, "delta: too many heads or requests for one launch");
     KB_REQUIRE(((uintptr_t)scratch & 15) == 0, "delta: scratch at %p is not at a multiple of 16 bytes", (void*)scratch);
-    const size_t places = dch_places(rows, p.entries);
+    const size_t places = dch_places(rows, p.entries, p.from_rows);
     p.w = reinterpret_cast<__nv_bfloat16*>(scratch);
     p.qk = reinterpret_cast<__nv_bfloat16*>(scratch += places * p.heads * dch_image_floats(p.d));
     p.within = scratch += places * p.kv_heads * 2 * dch_image_floats(p.d);

@@ -8,9 +8,9 @@ constexpr int DCH_C = 32;              // rows a chunk
 constexpr int DCH_LD_W = DCH_C + 4;    // a row of 32 weights, and four more so that rows begin in different banks
 constexpr int DCH_G = DCH_C * DCH_LD_W, DCH_F = DCH_G + DCH_C, DCH_ALL = DCH_F + DCH_C, DCH_WITHIN = DCH_ALL + 4;      // the decays' places behind them
 
-// Where a chunk's inputs lie: the chunk of request `entry` that begins at row `first`. Requests of a step follow one another, so every
-// chunk has a place of its own below rows / 32 + entries.
-__host__ __device__ inline int delta_chunk_place(int first, int entry) { return first / DCH_C + entry; }
+// Where a chunk's inputs lie: the chunk that begins at row `first` of a request with `before` requests by chunks in the rows ahead of it
+// (`delta_chunks_before`), whatever the order in which the requests are listed. Requests have rows of their own, so every chunk has a place of its own.
+__host__ __device__ inline int delta_chunk_place(int first, int before) { return first / DCH_C + before; }
 __host__ __device__ inline int delta_piece_row(int d) { return 3 * d + 8; }             // 8 more: eight rows begin in different banks
 
 struct DeltaChunks {
@@ -36,8 +36,8 @@ struct DeltaChunks {
 
 // Whether the chunk kernels take these sizes.
 bool delta_chunks_take(int d, int e);
-// Floats of scratch for a step of `rows` rows.
-long long delta_chunk_floats(int rows, int entries, int heads, int kv_heads, int d, int e);
+// Floats of scratch for a step of `rows` rows whose requests of at least `from_rows` go by chunks.
+long long delta_chunk_floats(int rows, int entries, int from_rows, int heads, int kv_heads, int d, int e);
 // Requests that bring at least p.from_rows rows, `longest` being the most any brings.
 // The inputs' places are taken from `scratch`.
 int launch_delta_chunks(DeltaChunks p, float* scratch, int rows, int longest, cudaStream_t s);

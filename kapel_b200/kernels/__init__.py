@@ -1229,7 +1229,7 @@ def delta_scan(stacked, q_off: int, k_off: int, v_off: int, b_off: int, a_off: i
     scratch = _fresh((max(1, int(lib.kb_delta_scratch_floats(rows, heads, kv_heads, d, e))),), torch.float32, src.device)
     chunks = None
     if longest >= DELTA_CHUNK_LONGEST and lib.kb_delta_chunks_take(d, e):
-        chunks = _fresh((int(lib.kb_delta_chunk_floats(rows, int(entries), heads, kv_heads, d, e)),), torch.float32, src.device)
+        chunks = _fresh((int(lib.kb_delta_chunk_floats(rows, int(entries), DELTA_CHUNK_ROWS, heads, kv_heads, d, e)),), torch.float32, src.device)
     _check(lib.kb_delta_scan(
         _ptr(out), _ptr(scratch), _ptr(src), dt, splits, ctypes.c_longlong(stride), width, int(q_off), int(k_off), int(v_off),
         int(b_off), int(a_off), _ptr(conv), _ptr(a_log), _ptr(dt_bias), _ptr(state), int(state.shape[0]), ctypes.c_longlong(per),

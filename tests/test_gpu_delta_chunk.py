@@ -152,3 +152,30 @@ def test_as_near_to_64_bit_as_the_scan(decay):
     # a warp's sums of four components a lane and a tree, against chains of eight to sixteen and pairs: some roundings more, 1.36 to 1.6 with
     # chains over all components
     assert off[1] <= 1.15 * off[0], off
+
+
+def test_requests_in_any_order():
+    """Requests listed in another order than their rows lie in, short ones between them: the same bits."""
+    from kapel_b200 import kernels as K
+
+    H, G, d, e, taps = 4, 2, 64, 32, 4
+    sizes, order = (200, 1, 70, 192, 3, 65, 250), (5, 0, 6, 2, 4, 1, 3)      # `order`: the request that is listed at each place
+    n, nv = G * d, H * e
+    width, rows = 2 * n + nv + 2 * H, sum(sizes)
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)
+    ints = lambda x: torch.tensor(np.asarray(x), dtype=torch.int32, device="cuda")
+    x, conv, a_log, dt_bias, start = rand(rows, width), rand(2 * n + nv, taps), rand(H), rand(H), rand(9, K.delta_state_floats(H, G, d, e, taps)) * 0.1
+    first = np.concatenate([[0], np.cumsum(sizes)[:-1]])
+    out, states = [], []
+    for listed in (tuple(range(7)), order):
+        entry = np.zeros(rows, np.int32)
+        for place, r in enumerate(listed):
+            entry[first[r] : first[r] + sizes[r]] = place
+        state = start.clone()
+        out.append(K.delta_scan(x, 0, n, 2 * n, 2 * n + nv, 2 * n + nv + H, conv, a_log, dt_bias, state, ints(entry),
+                                (ints([first[r] for r in listed]), ints([first[r] + sizes[r] for r in listed])), ints([r + 1 for r in listed]), 7,
+                                H, G, d, e, taps, d ** -0.5, 1e-6, 250, 1))
+        states.append(state)
+    K.check_async_errors()
+    assert torch.equal(out[0], out[1]) and torch.equal(states[0], states[1])

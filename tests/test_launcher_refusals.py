@@ -105,3 +105,13 @@ def test_decode_attention_from_slices_says_what_it_takes(lib):
     refused(lib, call(split=100), "split 100")
     refused(lib, call(scratch=None), "4 slots need scratch memory")
     refused(lib, call(hq=9), "heads 9 over 4")
+
+
+def test_scratch_of_the_delta_rule_by_chunks_is_for_the_requests_that_go_that_way(lib):
+    """64 decoding requests beside a prompt of 1,000 rows take as little more as the rows allow for, not a place of a megabyte each."""
+    lib.kb_delta_chunk_floats.restype = i64
+    lib.kb_delta_chunk_floats.argtypes = [i32] * 7
+    one = lib.kb_delta_chunk_floats(1000, 1, 64, 16, 4, 128, 128)
+    place = one / (1000 // 32 + 2)
+    assert lib.kb_delta_chunk_floats(1064, 65, 64, 16, 4, 128, 128) <= one + place * (1064 // 64 + 2)
+    assert lib.kb_delta_chunk_floats(192, 3, 64, 16, 4, 128, 128) >= place * 6                # three requests of two chunks each
