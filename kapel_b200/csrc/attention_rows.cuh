@@ -330,6 +330,7 @@ rows_kernel(const AttParams p) {
 // out[r, h, :] = sum_z e^(m_z - M) acc_z / sum_z e^(m_z - M) l_z over the slots that held keys of the row.
 // The slots' maxima and sums are read by the block's threads side by side (a slot a thread), the weights
 // e^(m_z - M) left in shared memory; then a thread a component walks the slots with independent loads.
+constexpr int COMBINE_SUMS = 128;      // threads that add up the slots' sums: a block has that many at least
 constexpr int COMBINE_SLOTS = 1024;    // slots whose weights fit shared memory; beyond that they are computed again a component
 template <typename T>
 __global__ void combine_kernel(const AttParams p) {
@@ -352,7 +353,7 @@ __global__ void combine_kernel(const AttParams p) {
     mx = block_max(mx, scratch);
     if (p.sinks != nullptr) mx = fmaxf(mx, p.sinks[h]);
     float denom = 0.f;
-    for (int z = threadIdx.x; z < p.slots; z += blockDim.x) {
+    for (int z = threadIdx.x; z < p.slots && threadIdx.x < COMBINE_SUMS; z += COMBINE_SUMS) {      // the same sums whatever the block's size
         int lo, hi;
         slot_range(p, count, z, lo, hi);
         float w = 0.f;

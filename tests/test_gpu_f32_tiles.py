@@ -125,3 +125,17 @@ def test_on_both_sides_of_two_blocks_a_tile(hq, hkv, d, at_once, more, window):
     by_rows, by_tiles = K.paged_attention_rows(*args), K.paged_attention_rows(*args, tiles=cut([(0, n)], per))
     # sums of up to 600 weights in 32-bit in another order; each side is within 1e-5 of 64 bits (above)
     assert (by_rows - by_tiles).abs().max() <= 2e-5 * by_rows.abs().max()
+
+
+def test_the_merge_of_many_slots_does_not_depend_on_the_batch():
+    """More slots of keys than a merging block of 128 threads has threads: a row alone and among many others, whose blocks have another size."""
+    from kapel_b200 import kernels as K
+
+    T, d = 256 * 140, 256
+    gen = torch.Generator(device="cuda").manual_seed(11)
+    k_table, v_table = (torch.randn(T // 16, 1, 16, d, device="cuda", generator=gen) for _ in range(2))
+    q, rows = torch.randn(1, 1, d, device="cuda", generator=gen), 700
+    table, ints = torch.arange(T // 16, dtype=torch.int32, device="cuda")[None].contiguous(), lambda v, n: torch.full((n,), v, dtype=torch.int32, device="cuda")
+    alone, beside = (K.paged_attention_rows(q.expand(n, 1, d).contiguous(), k_table, v_table, table, ints(0, n), ints(T, n), 16, None, d ** -0.5, None,
+                                            T // K.attention_chunk()) for n in (1, rows))
+    assert torch.equal(beside, alone.expand(rows, 1, d))
