@@ -212,52 +212,48 @@ attention_flash_kernel(const FlashParams p, const __grid_constant__ CUtensorMap 
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- the score products, from one lane
-        {                                                       // the whole warp: see at_elect()
-            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-            constexpr uint32_t IDESC_S = at_idesc(AF_ROWS, AF_KEYS, false);
-            const uint32_t q_addr = at_saddr(q_smem), ring_addr = at_saddr(k_ring);
-            for (int kt = 0; kt < n_tiles; ++kt) {
-                const int s = kt % KS, b = kt % SB;
-                if (!__all_sync(0xffffffffu, at_mbar_wait(k_full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
-                // the buffer still holds tile kt - SB's P until the product that reads it is complete
-                if (kt >= SB && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)(kt / SB - 1) & 1u))) { failed = true; break; }
-                at_fence_after();
-                const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * AF_KEYS);
+        // ---------------------------------------------------------------- the score products: the whole warp walks, see at_elect()
+        const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+        constexpr uint32_t IDESC_S = at_idesc(AF_ROWS, AF_KEYS, false);
+        const uint32_t q_addr = at_saddr(q_smem), ring_addr = at_saddr(k_ring);
+        for (int kt = 0; kt < n_tiles; ++kt) {
+            const int s = kt % KS, b = kt % SB;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(k_full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
+            // the buffer still holds tile kt - SB's P until the product that reads it is complete
+            if (kt >= SB && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)(kt / SB - 1) & 1u))) { failed = true; break; }
+            at_fence_after();
+            const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * AF_KEYS);
 #pragma unroll
-                for (int bx = 0; bx < QB; ++bx) {
-                    const uint64_t adesc = at_desc(q_addr + bx * (AF_ROWS * 128), 16, 1024);
-                    const uint64_t bdesc = at_desc(ring_addr + (uint32_t)s * C::K_BYTES + bx * (AF_KEYS * 128), 16, 1024);
+            for (int bx = 0; bx < QB; ++bx) {
+                const uint64_t adesc = at_desc(q_addr + bx * (AF_ROWS * 128), 16, 1024);
+                const uint64_t bdesc = at_desc(ring_addr + (uint32_t)s * C::K_BYTES + bx * (AF_KEYS * 128), 16, 1024);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk) at_mma_ss_if(one, d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
-                }
-                if (one) at_commit(k_empty + s);
-                if (one) at_commit(s_full + b);
+                for (int kk = 0; kk < 4; ++kk) at_mma_ss_if(one, d_tmem, adesc + (uint64_t)(kk * 2), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
             }
+            if (one) at_commit(k_empty + s);
+            if (one) at_commit(s_full + b);
         }
     } else if (warp == AF_WARP_PV) {
-        // ---------------------------------------------------------------- the P V products, from one lane
-        {                                                       // the whole warp: see at_elect()
-            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-            constexpr uint32_t IDESC_O = at_idesc(AF_ROWS, DV, true);
-            const uint32_t ring_addr = at_saddr(v_ring);
-            for (int kt = 0; kt < n_tiles; ++kt) {
-                const int b = kt % SB, s = kt % VS;
-                if (!__all_sync(0xffffffffu, at_mbar_wait(v_full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
-                if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt / SB) & 1u))) { failed = true; break; }
-                at_fence_after();
-                const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * AF_KEYS);          // P lies over its S
+        // ---------------------------------------------------------------- the P V products, likewise
+        const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+        constexpr uint32_t IDESC_O = at_idesc(AF_ROWS, DV, true);
+        const uint32_t ring_addr = at_saddr(v_ring);
+        for (int kt = 0; kt < n_tiles; ++kt) {
+            const int b = kt % SB, s = kt % VS;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(v_full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
+            if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt / SB) & 1u))) { failed = true; break; }
+            at_fence_after();
+            const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * AF_KEYS);          // P lies over its S
 #pragma unroll
-                for (int kk = 0; kk < AF_KEYS / 16; ++kk) {
-                    // keys 16 kk ..: their two eight-key groups 1 KB apart, chunks of 64 elements 16 KB apart
-                    const uint64_t bdesc = at_desc(ring_addr + (uint32_t)s * C::V_BYTES + (uint32_t)kk * 2048u, AF_KEYS * 128, 1024);
-                    at_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
-                }
-                if (one) at_commit(v_empty + s);
-                if (one) at_commit(s_free + b);
+            for (int kk = 0; kk < AF_KEYS / 16; ++kk) {
+                // keys 16 kk ..: their two eight-key groups 1 KB apart, chunks of 64 elements 16 KB apart
+                const uint64_t bdesc = at_desc(ring_addr + (uint32_t)s * C::V_BYTES + (uint32_t)kk * 2048u, AF_KEYS * 128, 1024);
+                at_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
             }
-            if (!failed && one) at_commit(o_full);
+            if (one) at_commit(v_empty + s);
+            if (one) at_commit(s_free + b);
         }
+        if (!failed && one) at_commit(o_full);
     } else if (warp >= 2 && warp < 10) {
         // ---------------------------------------------------------------- softmax and epilogue, half a row a thread
         const int quarter = warp & 3;

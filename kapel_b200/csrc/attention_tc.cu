@@ -247,57 +247,53 @@ attention_tc_kernel(const AttTcParams p, const __grid_constant__ CUtensorMap map
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- the score products, from one lane
-        {                                                       // the whole warp: see at_elect()
-            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-            constexpr uint32_t IDESC_S = at_idesc(AT_ROWS, AT_KEYS, false);
-            const uint32_t ring_addr = at_saddr(ring);
-            for (int kt = 0; kt < n_tiles; ++kt) {               // S[kt & 1] = Q K(kt)^T
-                const int s = kt % KS, b = kt & 1;
-                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
-                // the buffer still holds tile kt - 2's P until the product that reads it is complete
-                if (kt >= 2 && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)((kt - 2) >> 1) & 1u))) { failed = true; break; }
-                at_fence_after();
-                const uint32_t k_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);
+        // ---------------------------------------------------------------- the score products: the whole warp walks, see at_elect()
+        const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+        constexpr uint32_t IDESC_S = at_idesc(AT_ROWS, AT_KEYS, false);
+        const uint32_t ring_addr = at_saddr(ring);
+        for (int kt = 0; kt < n_tiles; ++kt) {               // S[kt & 1] = Q K(kt)^T
+            const int s = kt % KS, b = kt & 1;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / KS) & 1u))) { failed = true; break; }
+            // the buffer still holds tile kt - 2's P until the product that reads it is complete
+            if (kt >= 2 && !__all_sync(0xffffffffu, at_mbar_wait(s_free + b, (uint32_t)((kt - 2) >> 1) & 1u))) { failed = true; break; }
+            at_fence_after();
+            const uint32_t k_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
+            const uint32_t d_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);
 #pragma unroll
-                for (int bx = 0; bx < NBOX; ++bx) {
-                    const uint32_t a_tmem = tm + (uint32_t)(C::COL_Q + bx * 32);          // 64 elements of Q: 32 columns
-                    const uint64_t bdesc = at_desc(k_addr + bx * (AT_KEYS * 128), 16, 1024);
+            for (int bx = 0; bx < NBOX; ++bx) {
+                const uint32_t a_tmem = tm + (uint32_t)(C::COL_Q + bx * 32);          // 64 elements of Q: 32 columns
+                const uint64_t bdesc = at_desc(k_addr + bx * (AT_KEYS * 128), 16, 1024);
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        at_mma_ts_if(one, d_tmem, a_tmem + (uint32_t)(kk * 8), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
-                }
-                if (one) at_commit(empty + s);                            // the key slot is free when S is complete
-                if (one) at_commit(s_full + b);
+                for (int kk = 0; kk < 4; ++kk)
+                    at_mma_ts_if(one, d_tmem, a_tmem + (uint32_t)(kk * 8), bdesc + (uint64_t)(kk * 2), IDESC_S, (bx | kk) != 0 ? 1u : 0u);
             }
+            if (one) at_commit(empty + s);                            // the key slot is free when S is complete
+            if (one) at_commit(s_full + b);
         }
     } else if (warp == AT_WARP_PV) {
-        // ---------------------------------------------------------------- the P V products, from one lane
-        {                                                       // the whole warp: see at_elect()
-            const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
-            constexpr uint32_t PAGE_BYTES = NBOX * 2048u;
-            constexpr uint32_t IDESC_O = at_idesc(AT_ROWS, HD, true);
-            const uint32_t ring_addr = at_saddr(ring);
-            for (int kt = 0; kt < n_tiles; ++kt) {
-                const int b = kt & 1;
-                const int s = KS + kt % VS;
-                if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
-                if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt >> 1) & 1u))) { failed = true; break; }
-                at_fence_after();
-                const uint32_t v_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
-                const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);          // P lies over its S
+        // ---------------------------------------------------------------- the P V products, likewise
+        const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
+        constexpr uint32_t PAGE_BYTES = NBOX * 2048u;
+        constexpr uint32_t IDESC_O = at_idesc(AT_ROWS, HD, true);
+        const uint32_t ring_addr = at_saddr(ring);
+        for (int kt = 0; kt < n_tiles; ++kt) {
+            const int b = kt & 1;
+            const int s = KS + kt % VS;
+            if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(kt / VS) & 1u))) { failed = true; break; }
+            if (!__all_sync(0xffffffffu, at_mbar_wait(p_full + b, (uint32_t)(kt >> 1) & 1u))) { failed = true; break; }
+            at_fence_after();
+            const uint32_t v_addr = ring_addr + (uint32_t)s * C::SLOT_BYTES;
+            const uint32_t a_tmem = tm + (uint32_t)(C::COL_S + b * AT_KEYS);          // P lies over its S
 #pragma unroll
-                for (int kk = 0; kk < 4; ++kk) {
-                    // keys 16 kk ..: page kk of the tile, its two eight-key groups 1 KB apart, chunks 2 KB apart
-                    const uint64_t bdesc = at_desc(v_addr + (uint32_t)kk * PAGE_BYTES, 2048, 1024);
-                    at_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
-                }
-                if (one) at_commit(empty + s);
-                if (one) at_commit(s_free + b);                           // P has been read: the scores of tile kt + 2 may land
+            for (int kk = 0; kk < 4; ++kk) {
+                // keys 16 kk ..: page kk of the tile, its two eight-key groups 1 KB apart, chunks 2 KB apart
+                const uint64_t bdesc = at_desc(v_addr + (uint32_t)kk * PAGE_BYTES, 2048, 1024);
+                at_mma_ts_if(one, tm + C::COL_O, a_tmem + (uint32_t)(kk * 8), bdesc, IDESC_O, (kt | kk) != 0 ? 1u : 0u);
             }
-            if (!failed && one) at_commit(o_full);
+            if (one) at_commit(empty + s);
+            if (one) at_commit(s_free + b);                           // P has been read: the scores of tile kt + 2 may land
         }
+        if (!failed && one) at_commit(o_full);
     } else if (warp >= 2 && warp < 10) {
         // ---------------------------------------------------------------- softmax and epilogue, half a row a thread
         const int quarter = warp & 3;
@@ -666,8 +662,8 @@ attention_tc_pair_kernel(const AttTcParams p, const __grid_constant__ CUtensorMa
             }
         }
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- the score products of both blocks, from one lane of the first
-        if (rank == 0) {                                        // the whole warp: see at_elect()
+        // ---------------------------------------------------------------- the score products of both blocks: a warp of the first walks, see at_elect()
+        if (rank == 0) {
             const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t IDESC_S = at_idesc(ATP_ROWS, ATP_KEYS, false);
             const uint32_t ring_addr = at_saddr(ring);
@@ -694,7 +690,7 @@ attention_tc_pair_kernel(const AttTcParams p, const __grid_constant__ CUtensorMa
         }
     } else if (warp == AT_WARP_PV) {
         // ---------------------------------------------------------------- the P V products of both blocks
-        if (rank == 0) {                                        // the whole warp: see at_elect()
+        if (rank == 0) {
             const uint32_t one = at_elect(), tm = __shfl_sync(0xffffffffu, tmem, 0);
             constexpr uint32_t IDESC_O = at_idesc(ATP_ROWS, HD, true);
             const uint32_t ring_addr = at_saddr(ring);
