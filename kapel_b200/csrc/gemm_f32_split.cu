@@ -49,6 +49,7 @@ template <int NP> struct Pieces {
     static constexpr int W_BYTES = FP_M * 128, STAGE = W_BYTES + (CUTS ? NP * 128 : 0);            // 32 values of a row are 128 bytes
     static constexpr int PIECE = NP * 128, PIECES = 3 * PIECE;                                     // 64 bfloat16 of a row
     static constexpr int STAGES = NP == 128 ? 3 : 8, PLACES = CUTS ? 2 : (NP == 128 ? 3 : 4);      // of the pieces of A
+    static constexpr bool ALL_STAGES = STAGES % 2 != 0;                                            // see the cutting of the weights
     static constexpr int WARP_SUM = CUTS ? 15 : 11, COLS = CUTS ? NP : NP / 2;                     // rows of A whose sums a thread holds
     static constexpr int ACC = NP < 32 ? 32 : NP, COL_W = 2 * ACC, COL_HELD = COL_W + 192, HELD = CUTS ? 0 : 32;      // sums of earlier groups a thread has in tensor memory
     static constexpr int MORE = CUTS ? 0 : (COLS - HELD) * 2 * FP_M * 4;                           // and what does not fit there
@@ -142,7 +143,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         for (int i = 0; i < items; ++i) chunks += item(i).chunks;
 
     if (tid == 0) {
-        for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 6 : 4); }      // the warps that cut the stage
+        for (int s = 0; s < C::STAGES; ++s) { at_mbar_init(full + s, 1); at_mbar_init(empty + s, C::CUTS ? 6 : C::ALL_STAGES ? 8 : 4); }      // the warps that cut the stage
         for (int b = 0; b < 2; ++b) {
             at_mbar_init(cut + b, C::CUTS ? 12 : 8);
             at_mbar_init(done + b, 1);
@@ -210,10 +211,18 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         }
     } else if (warp < FP_WARP_A) {
         // ---------------------------------------------------------------- cutting the weights: a stage is half a chunk
+        // A wait by parity tells a round of a stage from the one before only. With an even number of stages a half has stages of its own. With an odd one a stage is
+        // the other half's every second time: then both halves' warps wait for each round of each stage, and it is empty when all of them have.
         const int quarter = warp & 3, half = (warp - FP_WARP_W) >> 2;      // of the TMEM lanes, which are the weight rows; of the chunk
         const int row = quarter * 32 + lane;
         for (int ch = 0; ch < chunks; ++ch) {
             const int it = 2 * ch + half, s = it % C::STAGES, b = ch & 1;
+            auto pass_on = [&](int other) {                        // the other half's stage
+                if (!__all_sync(0xffffffffu, at_mbar_wait(full + other % C::STAGES, (uint32_t)(other / C::STAGES) & 1u))) return false;
+                if (lane == 0) at_mbar_arrive(empty + other % C::STAGES);
+                return true;
+            };
+            if (C::ALL_STAGES && half == 1 && !pass_on(it - 1)) { failed = true; break; }
             if (!__all_sync(0xffffffffu, at_mbar_wait(full + s, (uint32_t)(it / C::STAGES) & 1u))) { failed = true; break; }
             const unsigned char* from = smem + s * C::STAGE + row * 128;
             uint32_t one[16], two[16], three[16];
@@ -225,6 +234,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             }
             __syncwarp();
             if (lane == 0) at_mbar_arrive(empty + s);
+            if (C::ALL_STAGES && half == 0 && !pass_on(it + 1)) { failed = true; break; }
             // the chunk two before this one was the last to lie here
             if (!__all_sync(0xffffffffu, at_mbar_wait(done + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u))) { failed = true; break; }
             at_fence_after();
