@@ -66,7 +66,11 @@ __device__ __forceinline__ void fp_ld16(uint32_t taddr, uint32_t (&r)[16]) {
                  : "r"(taddr) : "memory");
 }
 
-__device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t& two, uint32_t& three) { cut_pair(x, y, one, two, three); }
+__device__ __forceinline__ void fp_cut(float x, float y, uint32_t& one, uint32_t& two, uint32_t& three) {
+    x *= PIECE_SCALE, y *= PIECE_SCALE;
+    cut_pair(x, y, one, two, three);
+}
+constexpr float FP_UNSCALE = 1.f / PIECE_SCALE / PIECE_SCALE;       // every sum is too large by the square
 
 __device__ __forceinline__ bool fp_finite(float x) { return fabsf(x) < INFINITY; }
 // The product by multiply-adds in ascending k; rows of whole 16-byte pieces.
@@ -363,6 +367,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                     for (int j = 0; j < COLS; ++j) {
                         float v = sum[j];
                         check = fmaf(v, 0.f, check);
+                        if (!apart) v *= FP_UNSCALE;
                         if (EPI == 1 && !apart) v = cap * tanhf(v / cap);
                         if (j < many) to[(size_t)j * n] = v;
                     }
@@ -370,7 +375,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                         if (EPI == 1) {
 #pragma unroll
                             for (int j = 0; j < COLS; ++j)
-                                if (j < many) to[(size_t)j * n] = sum[j];
+                                if (j < many) to[(size_t)j * n] = sum[j] * FP_UNSCALE;
                         }
 #pragma unroll 1
                         for (int j = 0; j < many; ++j) {
@@ -396,7 +401,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
             float check = 0.f;                                     // as above
 #pragma unroll
             for (int j = 0; j < COLS; ++j) {
-                float v = sum[j];
+                float v = sum[j] * FP_UNSCALE;
                 check = fmaf(v, 0.f, check);
                 if (EPI == 1) v = cap * tanhf(v / cap);
                 if (j0 + j < rows) c[to(j0 + j) + r] = v;
@@ -405,7 +410,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 if (EPI == 1) {
 #pragma unroll
                     for (int j = 0; j < COLS; ++j)
-                        if (j0 + j < rows) c[to(j0 + j) + r] = sum[j];
+                        if (j0 + j < rows) c[to(j0 + j) + r] = sum[j] * FP_UNSCALE;
                 }
 #pragma unroll 1
                 for (int j = 0; j < min(COLS, rows - j0); ++j) {
@@ -430,6 +435,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
                 v = s == 0 ? x : v + x;
             }
             if (j < rows && n0 + r < n) {
+                v *= FP_UNSCALE;
                 if (!fp_finite(v)) v = fp_chain(a + (size_t)(m0 + j) * k, w + (size_t)(w0 + r) * k, k);
                 c[to(j) + r] = EPI == 1 ? cap * tanhf(v / cap) : v;
             }
@@ -481,6 +487,7 @@ f32_add_groups_kernel(float* __restrict__ c, const float* __restrict__ partial, 
     for (int j = 0; j < 4; ++j) {
         const long long i = first + 256 * j;
         if (i >= all) break;
+        v[j] *= FP_UNSCALE;
         if (!fp_finite(v[j])) v[j] = fp_chain(a + (size_t)(i / n) * k, w + (size_t)(i % n) * k, k);
         c[i] = EPI == 1 ? cap * tanhf(v[j] / cap) : v[j];
     }

@@ -592,6 +592,7 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
                 const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
                 to[0] = *reinterpret_cast<const uint32_t*>(&v);
             } else {
+                a *= PIECE_SCALE, b *= PIECE_SCALE;
                 cut_pair(a, b, to[0], to[8 * ld], to[16 * ld]);
             }
         }
@@ -619,7 +620,7 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
     for (int i = 0; i < 4; ++i) {
         const int t = row + (i >> 1) * 8, c = c0 + quad * 2 + (i & 1);
         if (t >= rows || c >= n_out) continue;
-        float v = acc[i];
+        float v = PIECES == 3 ? acc[i] * (1.f / PIECE_SCALE) : acc[i];
         if (!(fabsf(v) < INFINITY)) {
             const bf16* m = mt + ((size_t)h * n_out + c) * n_in;
             v = 0.f;

@@ -248,3 +248,20 @@ def test_the_groups_of_k_by_either_way(m, n, k):
                 want = torch.nan_to_num(by_way(a, w, groups, BESIDE, cap), nan=1e30)
                 for way in (WHOLE, APART):
                     assert torch.equal(torch.nan_to_num(by_way(a, w, groups, way, cap), nan=1e30), want), (groups, way, cap)
+
+
+@pytest.mark.parametrize("m,n", [(5, 130), (50, 130), (200, 700), (200, 9700)])
+def test_the_smallest_values(m, n):
+    """Values down to the subnormal ones: rows of nothing else, against weights of every size, with the error that ordinary values have."""
+    k = 260
+    gen = torch.Generator(device="cuda").manual_seed(m)
+    a, w = torch.randn(m, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    a[1], a[2], a[3], a[4] = a[1] * 2.0 ** -115, a[2] * 2.0 ** -126, a[3] * 2.0 ** -60 * 2.0 ** -74, a[4] * 2.0 ** -60 * 2.0 ** -88
+    w[:50] *= 2.0 ** 100
+    w[60:120] *= 2.0 ** -60
+    want, sizes = a.double() @ w.double().T, a.abs().double() @ w.abs().double().T
+    for groups in (1, 4):
+        for way in (BESIDE, WHOLE, APART) if m > 32 else (BESIDE,):
+            got = by_way(a, w, groups, way)
+            # as in the first test; 2^-150: half of the smallest subnormal
+            assert ((got - want).abs() <= (4 * 2.0 ** -23 + (k // 64 + 2) * 2.0 ** -24) * sizes + 2.0 ** -150).all(), (groups, way)

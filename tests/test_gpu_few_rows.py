@@ -132,3 +132,14 @@ def test_per_head_products_beyond_what_pieces_hold(rows, n_in):
     signs[2] = -1.0
     assert torch.equal(y[0, 2], signs * float("inf"))
     assert rows == 1 or bool((y[1:, 2] == 0).all() and (y[:-1, 1] == 0).all())
+
+
+def test_per_head_products_of_the_smallest_inputs():
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    x = torch.randn(3, 2, 100, device="cuda", generator=gen) * 2.0 ** -60 * torch.tensor([2.0 ** -56, 2.0 ** -68, 2.0 ** -84], device="cuda")[:, None, None]
+    m = (torch.randn(2, 16, 100, device="cuda", generator=gen) * 2.0 ** 100).bfloat16()
+    want = torch.einsum("rhi,hoi->rho", x.double(), m.double())
+    got = K.head_linear(x.view(3, -1), 2, 100, 0, m, transposed=True).view(3, 2, 16).double()
+    assert ((got - want).abs() <= 2.0 ** -8 * want.abs() + 2.0 ** -21 * torch.einsum("rhi,hoi->rho", x.double().abs(), m.double().abs())).all()
