@@ -539,38 +539,37 @@ static int launch_pieces(float* c, const float* a, const float* w, int m, int n,
 
 // Clusters of four and eight do not fit every group of multiprocessors, so that seven eighths and three quarters run at once (144 blocks in
 // clusters of eight: two waves).
-static int fp_clusters(int groups) {
-    const int sms = multiprocessors();
+static int fp_clusters(int groups, int sms) {
     const int at_once = groups <= 2 ? sms : (groups == 4 ? sms * 7 / 8 : sms * 3 / 4) / groups * groups;
     return at_once > 0 ? at_once : 1;
 }
 // Groups of K: what is fastest for up to 32 rows, whatever the rows there are. The waves of blocks times what a block takes, 0.65 us a chunk, and 5 or (in a
 // cluster) 6.5 us to begin and end.
-int gemm_f32_groups(int n, int k) {
+int gemm_f32_groups(int n, int k, int sms) {
     const int tiles = (n + FP_M - 1) / FP_M, chunks = (k + FP_K - 1) / FP_K;
     int best = 1;
     double least = 0;
     for (int g = 1; g <= 8 && g <= chunks; g *= 2) {
-        const int at_once = fp_clusters(g), waves = (int)(((long long)tiles * g + at_once - 1) / at_once);
+        const int at_once = fp_clusters(g, sms), waves = (int)(((long long)tiles * g + at_once - 1) / at_once);
         const double us = waves * ((chunks + g - 1) / g * 0.65 + (g == 1 ? 5.0 : 6.5));
         if (g == 1 || us < least) least = us, best = g;
     }
     return best;
 }
 // How the groups are done: what the three ways take, 0.68 us a chunk with 64 rows a tile and 1.2 with 128, 0.7 us to leave a group's sums and take
-// them up again, 3 us and 4 TB/s to add up what lies apart. In us, beside, whole and apart, by 2,304 x 9,216 in four groups: 128 rows 50, 137, 52; 256 rows
-// 90, 140, 56; 500 rows 140, 155, 101; 2,048 rows 543, 413, 447. By 4,096 x 2,304 in four: 128 rows 25, 44, 27; 500 rows 73, 48, 60; 2,048 rows 266, 176, 200
+// them up again, 1 us and 4 TB/s to add up what lies apart. In us, beside, whole and apart, by 2,304 x 9,216 in four groups: 128 rows 50, 137, 52; 256 rows
+// 90, 140, 56; 500 rows 140, 155, 101; 2,048 rows 543, 413, 447. By 4,096 x 2,304 in four: 128 rows 25, 44, 27; 256 rows 41, 46, 37; 500 rows 73, 48, 60; 2,048 rows 266, 176, 200
 // (in one group 165).
-int gemm_f32_way(int m, int n, int k, int groups) {
+int gemm_f32_way(int m, int n, int k, int groups, int sms) {
     if (m <= FP_CUT_ROWS) return FP_BESIDE;
     if (groups == 1) return FP_WHOLE;
-    const int np = m <= 64 ? 64 : 128, chunks = (k + FP_K - 1) / FP_K, each = (chunks + groups - 1) / groups, sms = multiprocessors();
+    const int np = m <= 64 ? 64 : 128, chunks = (k + FP_K - 1) / FP_K, each = (chunks + groups - 1) / groups;
     const long long tiles = (long long)((m + np - 1) / np) * ((n + FP_M - 1) / FP_M);
     const auto waves = [](long long blocks, int at_once) { return (double)((blocks + at_once - 1) / at_once); };
     const double chunk_us = np == 64 ? 0.68 : 1.2;
-    const double beside = waves(tiles * groups, fp_clusters(groups)) * (each * chunk_us + 6.5);
+    const double beside = waves(tiles * groups, fp_clusters(groups, sms)) * (each * chunk_us + 6.5);
     const double whole = waves(tiles, sms) * (chunks * chunk_us + 0.7 * (groups - 1)) + 5.0;
-    const double apart = waves(tiles * groups, sms) * (each * chunk_us + 0.7) + 5.0 + 3.0 + (groups + 1.0) * m * n * 1e-6;
+    const double apart = waves(tiles * groups, sms) * (each * chunk_us + 0.7) + 5.0 + 1.0 + (groups + 1.0) * m * n * 1e-6;
     return beside <= whole && beside <= apart ? FP_BESIDE : whole <= apart ? FP_WHOLE : FP_APART;
 }
 // From 256 inputs on, whatever the rows: one accumulator an element in ascending k, a kernel for each, is limited by
@@ -583,8 +582,8 @@ int gemm_f32_way(int m, int n, int k, int groups) {
 bool gemm_f32_pieces_take(int k, const void* a, const void* w) { return k >= 256 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0; }
 long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * 3 * ((k + 7) / 8 * 4); }
 long long gemm_f32_scratch_floats(int m, int n, int k) {
-    const int groups = gemm_f32_groups(n, k);
-    return gemm_f32_pieces_floats(m, k) + (gemm_f32_way(m, n, k, groups) == FP_APART ? (long long)groups * m * n : 0);
+    const int sms = multiprocessors(), groups = gemm_f32_groups(n, k, sms);
+    return gemm_f32_pieces_floats(m, k) + (gemm_f32_way(m, n, k, groups, sms) == FP_APART ? (long long)groups * m * n : 0);
 }
 
 int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int groups, int way, float* scratch, cudaStream_t s) {
@@ -638,10 +637,11 @@ extern "C" int kb_gemm_f32_pieces_by(float* c, const float* a, const float* w, i
     KB_REQUIRE(m >= 0 && n > 0 && k > 0, "gemm_f32: m %d, n %d, k %d", m, n, k);
     KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
     if (m == 0) return 0;
-    if (groups <= 0) groups = gemm_f32_groups(n, k);
-    return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, groups, way < 0 ? gemm_f32_way(m, n, k, groups) : way, scratch, (cudaStream_t)stream);
+    const int sms = multiprocessors();
+    if (groups <= 0) groups = gemm_f32_groups(n, k, sms);
+    return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, groups, way < 0 ? gemm_f32_way(m, n, k, groups, sms) : way, scratch, (cudaStream_t)stream);
 }
-extern "C" int kb_gemm_f32_groups(int n, int k) { return gemm_f32_groups(n, k); }
+extern "C" int kb_gemm_f32_groups(int n, int k) { return gemm_f32_groups(n, k, multiprocessors()); }
 // The same by clusters, or in one group.
 extern "C" int kb_gemm_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int segments, float* scratch, void* stream) {
     return kb_gemm_f32_pieces_by(c, a, w, m, n, k, epilogue, cap, segments, FP_BESIDE, scratch, stream);
