@@ -318,8 +318,12 @@ extern "C" long long kb_gemm_f32_scratch_floats(const float* a, const float* w, 
 extern "C" int kb_gemm_f32_fast(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, float* scratch, void* stream) {
     if (m > 0 && n > 0 && k > 0 && gemm_f32_pieces_take(k, a, w)) {
         KB_REQUIRE(epilogue == 0 || (epilogue == 1 && cap > 0.f), "gemm_f32: epilogue %d with cap %g", epilogue, cap);
-        const int sms = multiprocessors(), groups = gemm_f32_groups(n, k, sms);
-        return launch_f32_pieces(c, a, w, m, n, k, epilogue, cap, groups, gemm_f32_way(m, n, k, groups, sms), scratch, (cudaStream_t)stream);
+        const int sms = multiprocessors(), groups = gemm_f32_groups(n, k, sms), at_once = gemm_f32_rows_at_once(k);
+        for (long long r = 0; r < m; r += at_once) {
+            const int rows = m - r < at_once ? (int)(m - r) : at_once;
+            if (int e = launch_f32_pieces(c + r * n, a + r * k, w, rows, n, k, epilogue, cap, groups, gemm_f32_way(rows, n, k, groups, sms), scratch, (cudaStream_t)stream)) return e;
+        }
+        return 0;
     }
     return kb_gemm_f32_variant(c, a, w, m, n, k, epilogue, cap, -1, stream);
 }

@@ -31,6 +31,7 @@
 // the small products may be infinities of either sign before the large one is added.
 // Every wait gives up after about a second, raises a flag that `kb_gemm_f32_split_error` reports, and the block still meets at its
 // barriers, frees its TMEM and returns.
+#include <initializer_list>
 #include "attention_tc.cuh"
 #include "gemm_f32_split.cuh"
 #include "pieces.cuh"
@@ -42,6 +43,7 @@ __device__ int g_gemm_f32_split_error = 0;
 
 constexpr int FP_M = 128, FP_K = 64, FP_STAGE_K = 32, FP_THREADS = 20 * 32;
 constexpr int FP_WARP_W = 3, FP_WARP_A = 11, FP_WARP_PIECES = 19;
+constexpr long long FP_SCRATCH = 256ll << 20;
 constexpr int FP_CUT_ROWS = 32;                                    // up to so many rows of A are cut by the block that needs them
 
 template <int NP> struct Pieces {
@@ -570,7 +572,8 @@ int gemm_f32_way(int m, int n, int k, int groups, int sms) {
     const double beside = waves(tiles * groups, fp_clusters(groups, sms)) * (each * chunk_us + 6.5);
     const double whole = waves(tiles, sms) * (chunks * chunk_us + 0.7 * (groups - 1)) + 5.0;
     const double apart = waves(tiles * groups, sms) * (each * chunk_us + 0.7) + 5.0 + 1.0 + (groups + 1.0) * m * n * 1e-6;
-    return beside <= whole && beside <= apart ? FP_BESIDE : whole <= apart ? FP_WHOLE : FP_APART;
+    const bool room = (long long)groups * m * n * 4 <= FP_SCRATCH;
+    return beside <= whole && (beside <= apart || !room) ? FP_BESIDE : whole <= apart || !room ? FP_WHOLE : FP_APART;
 }
 // From 256 inputs on, whatever the rows: one accumulator an element in ascending k, a kernel for each, is limited by
 // its chain or by the FMA pipe; here a chunk's 24 products take the same time whatever the rows, up to 64. 500 rows by 18,432 x 2,304: 824 us by
@@ -581,9 +584,19 @@ int gemm_f32_way(int m, int n, int k, int groups, int sms) {
 // chains' (500 rows by 2,304 x 9,216: 1.4e-7 and 1.7e-6; by 1,024 x 256: 8.8e-8 and 2.9e-7).
 bool gemm_f32_pieces_take(int k, const void* a, const void* w) { return k >= 256 && k % 4 == 0 && (((uintptr_t)a | (uintptr_t)w) & 15) == 0; }
 long long gemm_f32_pieces_floats(int m, int k) { return m <= FP_CUT_ROWS ? 0 : (long long)m * 3 * ((k + 7) / 8 * 4); }
+// Scratch does not grow with the rows beyond FP_SCRATCH for pieces and as much for groups that lie apart: more rows go by several launches, of at least 1,024.
+int gemm_f32_rows_at_once(int k) {
+    const long long rows = FP_SCRATCH / (6ll * ((k + 7) / 8 * 8)) / 128 * 128;
+    return rows < 1024 ? 1024 : rows > 0x3fffff80 ? 0x3fffff80 : (int)rows;
+}
 long long gemm_f32_scratch_floats(int m, int n, int k) {
-    const int sms = multiprocessors(), groups = gemm_f32_groups(n, k, sms);
-    return gemm_f32_pieces_floats(m, k) + (gemm_f32_way(m, n, k, groups, sms) == FP_APART ? (long long)groups * m * n : 0);
+    const int sms = multiprocessors(), groups = gemm_f32_groups(n, k, sms), at_once = gemm_f32_rows_at_once(k);
+    long long most = 0;
+    for (int rows : {m < at_once ? m : at_once, m % at_once}) {
+        const long long floats = gemm_f32_pieces_floats(rows, k) + (gemm_f32_way(rows, n, k, groups, sms) == FP_APART ? (long long)groups * rows * n : 0);
+        most = floats > most ? floats : most;
+    }
+    return most;
 }
 
 int launch_f32_pieces(float* c, const float* a, const float* w, int m, int n, int k, int epilogue, float cap, int groups, int way, float* scratch, cudaStream_t s) {

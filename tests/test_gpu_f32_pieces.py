@@ -265,3 +265,19 @@ def test_the_smallest_values(m, n):
             got = by_way(a, w, groups, way)
             # as in the first test; 2^-150: half of the smallest subnormal
             assert ((got - want).abs() <= (4 * 2.0 ** -23 + (k // 64 + 2) * 2.0 ** -24) * sizes + 2.0 ** -150).all(), (groups, way)
+
+
+def test_scratch_is_bounded():
+    """More rows than a launch's scratch has room for go by several; the last of one row."""
+    from kapel_b200 import kernels as K
+
+    k, n = 18432, 130
+    at_once = (256 << 20) // (6 * k) // 128 * 128
+    gen = torch.Generator(device="cuda").manual_seed(4)
+    a, w = torch.randn(at_once + 1, k, device="cuda", generator=gen), torch.randn(n, k, device="cuda", generator=gen)
+    lib, ptr = K.library(), lambda t: ctypes.c_void_p(t.data_ptr())
+    for m in (at_once + 1, 1 << 20):
+        assert lib.kb_gemm_f32_scratch_floats(ptr(a), ptr(w), m, n, k) * 4 <= 512 << 20
+    got = K.gemm(a, w)
+    for rows in (slice(0, 40), slice(at_once - 40, at_once), slice(at_once, at_once + 1)):
+        assert torch.equal(got[rows], K.gemm(a[rows].clone(), w))
