@@ -312,17 +312,6 @@ static int launch_f32_tiles_parts(const F32TileParams& p, int tiles, cudaStream_
     return check_launch("attention_f32_tiles");
 }
 
-// Two blocks a tile while the tiles are no more than the GPU takes at once; if a window makes them alike, while the blocks are. In us, one block and two: 16
-// tokens of 8 heads over 4 of 256 behind 1,024 (4 tiles) 291 and 164, 500 tokens behind 0 and 1,024 (128 tiles) 146 and 99, 431 and 373; of 16 over 4 of
-// 128 (252) 121 and 90, 392 and 356. 500 behind 1,024 with a window of 512: 162 and 186, 155 and 177. More tiles: 800 tokens of 256 (200 tiles) 227 and
-// 213, with a window of 512 158 and 197; 1,000 tokens of 128 (500) 246 and 287, of 256 (252) 288 and 304.
-template <int D>
-static int launch_f32_tiles(const F32TileParams& p, int tiles, cudaStream_t s) {
-    const long long at_once = (long long)multiprocessors() * (D == 128 ? 2 : 1), blocks = (long long)p.hkv * tiles;
-    const bool alike = p.window > 0 && p.window < (long long)p.table_width * p.page_size;
-    return (alike ? 2 : 1) * blocks <= at_once ? launch_f32_tiles_parts<D, 2>(p, tiles, s) : launch_f32_tiles_parts<D, 1>(p, tiles, s);
-}
-
 }  // namespace kb
 
 using namespace kb;
@@ -330,15 +319,18 @@ using namespace kb;
 extern "C" int kb_attention_f32_tiles_takes(int hq, int hkv, int d) { return (d == 128 || d == 256) && hkv > 0 && hq % hkv == 0 && hq / hkv <= AFT_ROWS; }
 
 // q and out [rows, hq, d] float32, tables [pages, hkv, page_size, d] float32; tiles of at most 32 / (hq / hkv) tokens of one request at
-// consecutive positions; `window` 0: every key; `cap` 0: no soft cap; `sinks` [hq] or null.
+// consecutive positions; `window` 0: every key; `cap` 0: no soft cap; `sinks` [hq] or null; `blocks` a tile, 1 or 2.
 extern "C" int kb_attention_f32_tiles(float* out, const float* q, const float* k_table, const float* v_table, const int* block_table, const int* row_count,
                                       const int* tile_entry, const int* tile_row0, const int* tile_nq, int tiles, int rows, int hq, int hkv, int d,
-                                      int page_size, int table_width, int n_pages, int window, float scale, float cap, const float* sinks, void* stream) {
+                                      int page_size, int table_width, int n_pages, int window, float scale, float cap, const float* sinks, int blocks, void* stream) {
     KB_REQUIRE(rows >= 0 && tiles >= 0 && tiles <= 65535, "attention_f32_tiles: rows %d, tiles %d", rows, tiles);
+    KB_REQUIRE(blocks == 1 || blocks == 2, "attention_f32_tiles: %d blocks a tile", blocks);
     KB_REQUIRE(kb_attention_f32_tiles_takes(hq, hkv, d), "attention_f32_tiles: %d heads over %d of %d are not taken", hq, hkv, d);
     KB_REQUIRE(page_size > 0 && table_width > 0 && n_pages > 0 && window >= 0, "attention_f32_tiles: pages of %d, table width %d, pages %d, window %d", page_size, table_width, n_pages, window);
     KB_REQUIRE((((uintptr_t)q | (uintptr_t)out | (uintptr_t)k_table | (uintptr_t)v_table) & 15) == 0, "attention_f32_tiles: operands must be 16-byte aligned");
     if (rows == 0 || tiles == 0) return 0;
     F32TileParams p = {q, k_table, v_table, block_table, row_count, tile_entry, tile_row0, tile_nq, sinks, out, hq, hkv, page_size, table_width, n_pages, window, scale, cap};
-    return d == 128 ? launch_f32_tiles<128>(p, tiles, (cudaStream_t)stream) : launch_f32_tiles<256>(p, tiles, (cudaStream_t)stream);
+    cudaStream_t s = (cudaStream_t)stream;
+    if (d == 128) return blocks == 2 ? launch_f32_tiles_parts<128, 2>(p, tiles, s) : launch_f32_tiles_parts<128, 1>(p, tiles, s);
+    return blocks == 2 ? launch_f32_tiles_parts<256, 2>(p, tiles, s) : launch_f32_tiles_parts<256, 1>(p, tiles, s);
 }

@@ -12,6 +12,7 @@ import numpy as np
 import torch
 
 from ..cache import Plan
+from ..kernels import row_tile_blocks, sm_count
 
 
 class GroupBatch:
@@ -69,35 +70,27 @@ ROW_TILE_TOKENS = 16
 
 
 def row_tiles_pay(row_count, tile_row0, tile_nq, kv_heads: int, heads_per_kv: int, head_dim: int, window: Optional[int], sms: int,
-                  ahead: bool = False) -> bool:
-    """Whether the 32-bit attention of these rows is faster by tiles than row by row. A block of the tile kernel walks all the keys of its
-    tile, 64 a step, however few its rows: few tiles behind a long history leave the GPU idle, where the row-wise kernel has a block
-    a row, kv head and 256 keys. Both as measured on a B200 for 16 to 1,024 tokens behind 0 to 16,384, groups of 1 to 16 heads of 128 and 256:
-    a step 17.0 us (heads of 256) or 11.4 (of 128), a block a multiprocessor; a key 0.07 us + 1.45 ns a component + 0.06 us a head of the group,
-    7 (groups of 1) to 4 (of 8) blocks a multiprocessor. 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 146 and 391; 16 tokens
-    behind 256, 1,024 and 4,096 positions 89 and 145, 292 and 149, 1,101 and 219; 128 tokens behind 1,024 and 16,384 311 and 372, 4,374 and 5,685.
-    With `ahead` against the row-wise kernel as it is for what the engine gives it, which asks for several keys before it uses the first: the longest block's
-    keys, 0.08 us (one head of 128) to 0.17 (two of 256, four of 128) each, or all keys, 0.018 to 0.051 us a key and multiprocessor, and a quarter of the
-    shorter; 1 to 500 tokens behind 0 to 4,096, groups of 1 to 4; and with two blocks a tile where the tiles are few, half its steps of 17.2 us (heads of 256) or
-    12.9 (of 128). The same sizes by tiles and row by row: 500 tokens 99 and 215; 16 tokens 60 and 47, 164 and 51, 579 and 110; 128 tokens behind 0, 1,024
-    and 4,096 27 and 27, 166 and 206, 582 and 731; 500 behind 1,024 373 and 895 (the faster one in all of 72)."""
+                  positions: Optional[int] = None) -> bool:
+    """Whether the 32-bit attention of these rows is faster by tiles than row by row; `positions`: what a request's block table holds (None: the longest
+    row's). A block of the tile kernel walks all the keys of its tile, 64 a step, however few its rows: few tiles behind a long history leave
+    the GPU idle, where the row-wise kernel has a block a row, kv head and 256 keys. By tiles a step takes 17.0 us (heads of 256) or 11.4 (of 128), a block a
+    multiprocessor; with two blocks a tile (`kernels.row_tile_blocks`) half the steps of 17.2 or 12.9. Row by row the longest block's keys take 0.08 us (one head of
+    128) to 0.17 (two of 256, four of 128) each, or all keys 0.018 to 0.051 us a key and multiprocessor, and a quarter of the shorter.
+    As measured on a B200, 8 heads over 4 of 256, by tiles and row by row, in us: 500 tokens 99 and 215; 16 tokens behind 256, 1,024 and 4,096 positions
+    60 and 47, 164 and 51, 579 and 110; 128 tokens behind 0, 1,024 and 4,096 27 and 27, 166 and 206, 582 and 731; 500 behind 1,024 373 and 895."""
     count = np.asarray(row_count, np.int64)
     row0 = np.asarray(tile_row0, np.int64)
     first, last = count[row0], count[row0 + np.asarray(tile_nq, np.int64) - 1]
     steps = -(-(last - (np.maximum(0, first - window) if window else 0)) // 64)
-    by_tiles = 6.0 + (5.8 + 0.0438 * head_dim) * max(float(steps.max()), 1.1 * float(steps.sum()) * kv_heads / sms)
+    if row_tile_blocks(len(steps), kv_heads, head_dim, window, int(count.max()) if positions is None else positions, sms) == 2:
+        by_tiles = 3.0 + 0.02 * head_dim + (8.6 + 0.0337 * head_dim) * max(-(-float(steps.max()) // 2), 1.1 * float(steps.sum()) * kv_heads / sms)
+    else:
+        by_tiles = 6.0 + (5.8 + 0.0438 * head_dim) * max(float(steps.max()), 1.1 * float(steps.sum()) * kv_heads / sms)
     seen = np.where(count > window, window + 200, count) if window else count      # a window begins within a block's keys: one more, partly idle
     slices, heads = -(-heads_per_kv // 8), min(heads_per_kv, 8)      # the row-wise kernel's blocks have up to eight heads
-    at_once = (7.5 - 0.42 * heads) * sms
-    by_rows = 3.0 + (0.07 + 0.00145 * head_dim + 0.06 * heads) * max(min(256.0, float(count.max())), float(seen.sum()) * kv_heads * slices / at_once)
-    if ahead:
-        alike = 2 if window and window < float(count.max()) else 1
-        if alike * len(steps) * kv_heads <= sms * (2 if head_dim == 128 else 1):         # as the launcher: two blocks a tile
-            by_tiles = 3.0 + 0.02 * head_dim + (8.6 + 0.0337 * head_dim) * max(-(-float(steps.max()) // 2), 1.1 * float(steps.sum()) * kv_heads / sms)
-        longest = (0.00046 * head_dim + 0.0293 * heads - 0.008) * min(256.0, float(count.max()))
-        every = head_dim * (0.0000794 + 0.000065 * heads) * float(seen.sum()) * kv_heads * slices / sms
-        by_rows = 3.0 + max(longest, every) + 0.25 * min(longest, every)
-    return by_tiles <= by_rows
+    longest = (0.00046 * head_dim + 0.0293 * heads - 0.008) * min(256.0, float(count.max()))
+    every = head_dim * (0.0000794 + 0.000065 * heads) * float(seen.sum()) * kv_heads * slices / sms
+    return by_tiles <= 3.0 + max(longest, every) + 0.25 * min(longest, every)
 
 
 # What a block costs beyond its 64-key steps, what the merge of partial sums costs beyond its traffic
@@ -173,16 +166,6 @@ def pooled_slices(rows: int, longest: int, window: Optional[int], pool: int, sms
     split_keys = -(-(-(-keys // want)) // chunk) * chunk
     slices = -(-keys // split_keys)
     return (slices, split_keys) if slices > 1 else (1, 0)
-
-
-_SMS = {}
-
-
-def sm_count(device) -> int:
-    key = str(device)
-    if key not in _SMS:
-        _SMS[key] = torch.cuda.get_device_properties(device).multi_processor_count if torch.device(device).type == "cuda" else 148
-    return _SMS[key]
 
 
 def cut_tiles(q_start, q_len, tokens_per_tile: int):
@@ -364,17 +347,17 @@ class StepBatch:
         tiles = self.memo[key]
         return tiles[:3] if tiles is not None else None
 
-    def row_tiles(self, heads_per_kv: int, kv_heads: int, head_dim: int, window: Optional[int]):
+    def row_tiles(self, heads_per_kv: int, kv_heads: int, head_dim: int, window: Optional[int], positions: Optional[int] = None):
         """(tile_entry, tile_row0, tile_nq) on the device for the 32-bit attention by tiles of ROW_TILE rows (tokens x query heads of a kv
         head), or None where some request brings fewer than ROW_TILE_TOKENS tokens (its tile would hold a few rows and walk all its keys
         alone) or the tiles take longer than row by row (`row_tiles_pay`)."""
-        key = ("row_tiles", heads_per_kv, kv_heads, head_dim, window)
+        key = ("row_tiles", heads_per_kv, kv_heads, head_dim, window, positions)
         if key not in self.memo:
             plan = self.plan
             arrays = None
             if len(plan.q_len) and self.shortest_portion() >= ROW_TILE_TOKENS and heads_per_kv <= ROW_TILE and self.ids.is_cuda:
                 arrays = cut_tiles(plan.q_start, plan.q_len, ROW_TILE // heads_per_kv)
-                if not row_tiles_pay(plan.row_count, arrays[1], arrays[2], kv_heads, heads_per_kv, head_dim, window, sm_count(self.ids.device), ahead=True):
+                if not row_tiles_pay(plan.row_count, arrays[1], arrays[2], kv_heads, heads_per_kv, head_dim, window, sm_count(self.ids.device), positions):
                     arrays = None
             if arrays is None:
                 self.memo[key] = None

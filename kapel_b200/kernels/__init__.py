@@ -648,6 +648,26 @@ def gemm_glu_fused(a: torch.Tensor, w: torch.Tensor, act: str, limit: float = 0.
     return out
 
 
+_SMS = {}
+
+
+def sm_count(device) -> int:
+    key = str(device)
+    if key not in _SMS:
+        _SMS[key] = torch.cuda.get_device_properties(device).multi_processor_count if torch.device(device).type == "cuda" else 148
+    return _SMS[key]
+
+
+def row_tile_blocks(tiles: int, kv_heads: int, head_dim: int, window: Optional[int], positions: int, sms: int) -> int:
+    """Blocks that take a tile of the 32-bit attention, one or two: two while the tiles are no more than the GPU takes at once; if a window makes them
+    alike (a request's block table holds more `positions`), while the blocks are. In us, one block and two: 16 tokens of 8 heads over 4 of 256 behind 1,024 (4
+    tiles) 291 and 164, 500 tokens behind 0 and 1,024 (128 tiles) 146 and 99, 431 and 373; of 16 over 4 of 128 (252) 121 and 90, 392 and 356. 500 behind 1,024
+    with a window of 512: 162 and 186, 155 and 177. More tiles: 800 tokens of 256 (200 tiles) 227 and 213, with a window of 512 158 and 197; 1,000 tokens of
+    128 (500) 246 and 287, of 256 (252) 288 and 304."""
+    alike = 2 if window and window < positions else 1
+    return 2 if alike * tiles * kv_heads <= sms * (2 if head_dim == 128 else 1) else 1
+
+
 _ATT_CHUNK = None
 
 
@@ -690,9 +710,10 @@ def paged_attention_rows(q, k_table, v_table, block_table, row_entry, row_count,
         n_tiles = tiles[0].numel()
         for t in tiles:
             _need(t, "attention tiles", torch.int32, (n_tiles,))
+        blocks = row_tile_blocks(n_tiles, hkv, d, window, int(block_table.shape[1]) * int(page_size), sm_count(q.device))
         _check(lib.kb_attention_f32_tiles(_ptr(out), _ptr(q), _ptr(k_table), _ptr(v_table), _ptr(block_table), _ptr(row_count), _ptr(tiles[0]), _ptr(tiles[1]),
                                           _ptr(tiles[2]), n_tiles, rows, hq, hkv, d, int(page_size), int(block_table.shape[1]), int(n_pages), int(window or 0),
-                                          _f(scale), _f(softcap or 0.0), _ptr(sinks), _stream()))
+                                          _f(scale), _f(softcap or 0.0), _ptr(sinks), blocks, _stream()))
         return out
     need = lib.kb_paged_attention_scratch_floats(rows, hq, dv, int(slots))
     scratch = _fresh((need,), torch.float32, q.device) if need else None

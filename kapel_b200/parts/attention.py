@@ -316,7 +316,7 @@ class Attention(Part):
             y = K.paged_attention_rows(
                 q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count, self.ctx.page_size, s.window, s.scale,
                 s.softcap, batch.attention_slots(s.window, s.keep_first), s.keep_first, sinks=self.sinks,
-                tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window) if self.ctx.is_f32 else None)
+                tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window, group.block_table.shape[1] * self.ctx.page_size) if self.ctx.is_f32 else None)
         width = product_width(self.ctx, s.num_heads * dv)
         if s.gated:
             y = K.head_gate(y, stacked, nq + nk + own * dv, None, False, 0.0, self.ctx.dtype, pad_to=width)
@@ -353,7 +353,7 @@ class Attention(Part):
         else:
             y = K.paged_attention_rows(q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count, self.ctx.page_size,
                                        s.window, s.scale, s.softcap, batch.attention_slots(s.window), sinks=self.sinks,
-                                       tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window) if self.ctx.is_f32 else None)
+                                       tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window, group.block_table.shape[1] * self.ctx.page_size) if self.ctx.is_f32 else None)
         width = product_width(self.ctx, s.num_heads * dv) if pad_to is None else pad_to
         if s.gated or out is not None:
             return K.head_gate(y, stacked, base + nq + nk + s.num_kv_heads * dv if s.gated else 0, None, False, 0.0, self.ctx.dtype, pad_to=width,
@@ -412,6 +412,6 @@ class Attention(Part):
             y = K.paged_attention_rows(
                 q, k_table, v_table, group.block_table, batch.row_entry, batch.row_count,
                 self.ctx.page_size, s.window, s.scale, s.softcap, batch.attention_slots(s.window),
-                tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window) if self.ctx.is_f32 else None,
+                tiles=batch.row_tiles(heads_per_kv, s.num_kv_heads, s.head_dim, s.window, group.block_table.shape[1] * self.ctx.page_size) if self.ctx.is_f32 else None,
             )
         return linear(self.ctx, y.view(y.shape[0], s.num_heads * s.head_dim), self.w_o, keep_split=True)

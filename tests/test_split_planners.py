@@ -111,14 +111,27 @@ def test_heads_of_a_long_history_are_made_only_where_they_fit():
 
 
 @pytest.mark.parametrize("heads_per_kv,kv_heads,d,window,tokens,before,tiles", [
-    (2, 4, 256, None, 500, 0, 1), (2, 4, 256, None, 16, 256, 1), (2, 4, 256, None, 16, 1024, 0), (2, 4, 256, None, 16, 6144, 0), (2, 4, 256, None, 64, 4096, 0),
+    (2, 4, 256, None, 500, 0, 1), (2, 4, 256, None, 16, 256, 0), (2, 4, 256, None, 16, 1024, 0), (2, 4, 256, None, 16, 6144, 0), (2, 4, 256, None, 64, 4096, 0),
     (2, 4, 256, None, 128, 4096, 1), (2, 4, 256, None, 512, 16384, 1), (2, 8, 256, None, 64, 1024, 1), (2, 8, 256, None, 32, 4096, 0),
     (4, 4, 128, None, 128, 16384, 1), (4, 4, 128, None, 32, 4096, 0), (1, 4, 128, None, 128, 4096, 0), (1, 4, 128, None, 1024, 4096, 1),
-    (8, 1, 256, None, 64, 4096, 0), (16, 1, 128, None, 256, 16384, 1), (16, 2, 128, None, 16, 4096, 0), (2, 4, 256, 512, 128, 16384, 1)])
+    (8, 1, 256, None, 64, 4096, 0), (16, 1, 128, None, 256, 16384, 1), (16, 2, 128, None, 16, 4096, 0), (2, 4, 256, 512, 128, 16384, 1),
+    (8, 1, 256, None, 16, 16384, 0), (8, 1, 256, None, 256, 16384, 1), (8, 2, 128, None, 64, 16384, 0), (16, 2, 256, None, 64, 4096, 1), (16, 1, 128, None, 1000, 4096, 1),
+    (32, 1, 128, None, 16, 4096, 0), (32, 1, 128, None, 64, 4096, 1), (2, 4, 256, 512, 64, 4096, 0), (2, 4, 256, 1024, 1000, 4096, 1)])
 def test_32_bit_attention_goes_by_tiles_where_they_are_faster(heads_per_kv, kv_heads, d, window, tokens, before, tiles):
     """As measured on a B200, one request: a few tiles behind a long history are slower than row by row."""
     from kapel_b200.engine.batch import ROW_TILE, row_tiles_pay
 
     _, row0, nq = cut_tiles(np.asarray([0]), np.asarray([tokens]), ROW_TILE // heads_per_kv)
     count = np.arange(before + 1, before + tokens + 1)
-    assert row_tiles_pay(count, row0, nq, kv_heads, heads_per_kv, d, window, 148) == bool(tiles)
+    for positions in (None, before + tokens):
+        assert row_tiles_pay(count, row0, nq, kv_heads, heads_per_kv, d, window, 148, positions) == bool(tiles)
+
+
+def test_two_blocks_take_a_tile_of_32_bit_attention_while_the_gpu_has_room():
+    """As measured on a B200: alike tiles (a window that the block table goes beyond) only while the blocks fit a wave, others while the tiles do."""
+    from kapel_b200.kernels import row_tile_blocks
+
+    for d, at_once in ((256, 148), (128, 296)):
+        assert [row_tile_blocks(n, 1, d, None, 4096, 148) for n in (1, at_once, at_once + 1)] == [2, 2, 1]
+        assert [row_tile_blocks(n, 1, d, 512, 4096, 148) for n in (1, at_once // 2, at_once // 2 + 1)] == [2, 2, 1]
+        assert [row_tile_blocks(n, 1, d, 512, 512, 148) for n in (at_once, at_once + 1)] == [2, 1]
