@@ -13,8 +13,8 @@
 // What bounds the chain: 144 products of 16 x 8 x 16 a chunk on each quarter of a multiprocessor (1,250 clocks), some 1,900 clocks of shared memory and the
 // hand-overs between its warps: 1.65 us a chunk (3.9 by multiply-adds from shared memory; the scan's 32 steps take 9.7). 2,048 rows, 16 heads of 128 over 4
 // key heads: 49 us for the chunks and 106 us for the chain (54 and 249; the scan: 619 us); 500 rows 18 and 29, 64 rows 14 and 7 (the scan 24).
-// Sums go by short chains, so that the error against 64 bits stays at the scan's: 1.00 to 1.06 of it where memories fade within a row to some twenty
-// rows, 0.87 to 0.98 where they hardly do. (A block a chunk and key head, four heads one after the other, took 61 us.)
+// Sums go by short chains, so that the error against 64 bits stays at the scan's: 1.01 of it where memories fade within a row, 1.08 within some twenty
+// rows, 0.93 to 0.98 where they hardly do (by multiply-adds 0.99, 1.08 and 1.00). (A block a chunk and key head, four heads one after the other, took 61 us.)
 #include <initializer_list>
 #include "delta_chunk.cuh"
 #include "pieces.cuh"

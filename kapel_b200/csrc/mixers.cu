@@ -527,8 +527,9 @@ head_linear_mma_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
 // The same product for a few rows (a decode step): the rows are the 16 of an MMA, a warp has eight columns of M[h], which lie together in mt
 // [heads, n_out, n_in] and come straight into registers, 16 bytes a lane, ahead of the wait on the kernel before. A lane's 16 bytes are eight neighbouring
 // inputs of one column, so two MMAs take 32 inputs in the order that gives, and the rows' inputs are read in the same. 32-bit inputs are
-// cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16). The tensor cores round towards zero, so they add up 32 inputs,
-// the small pieces first, and those sums are added in registers. What comes out as no finite number is computed again by multiply-adds: infinities have no
+// cut into three bfloat16 pieces that hold them (pieces.cuh; the matrices are bfloat16). The tensor cores round towards zero, so they add up 16 inputs,
+// the small pieces first, and those sums are added in registers (one chain over all: two to seven times as many results that are not the
+// exact ones rounded once). What comes out as no finite number is computed again by multiply-adds: infinities have no
 // pieces. 8 rows, 16 heads of
 // 128 -> 512: 6.4 us (20.7 by a column a warp, its sums by shuffles), 512 -> 128 with the gate: 9.2 (19.2). What is left is a launch's latency.
 constexpr int HF_ROWS = 16, HF_WARPS = 8, HF_COLS = HF_WARPS * 8, HF_HELD = 16;        // HF_HELD: groups of 32 inputs whose weights a lane holds at once
@@ -538,7 +539,7 @@ __host__ __device__ constexpr int hf_ld(int n_in) { return (n_in + 31) / 32 * 32
 template <typename TX> __host__ __device__ constexpr int hf_pieces() { return sizeof(TX) == 4 ? 3 : 1; }
 
 __device__ __forceinline__ void hf_mma(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
@@ -598,21 +599,29 @@ head_linear_few_kernel(bf16* __restrict__ y, int y_row, int y_head, const Src<TX
         }
         __syncthreads();
         auto multiply = [&](int group, const uint4& w) {
-            float sum[4] = {};
+            float sum[2][4] = {};                               // of 16 inputs each: two chains side by side
 #pragma unroll
             for (int q = PIECES - 1; q >= 0; --q) {
                 const uint32_t* from = xs + (q * 16 + row) * (ld / 2) + group * 16 + quad * 4;
                 const uint4 a = *reinterpret_cast<const uint4*>(from), b = *reinterpret_cast<const uint4*>(from + 4 * ld);      // rows `row` and `row` + 8
-                hf_mma(sum, a.x, b.x, a.y, b.y, w.x, w.y);
-                hf_mma(sum, a.z, b.z, a.w, b.w, w.z, w.w);
+                hf_mma(sum[0], a.x, b.x, a.y, b.y, w.x, w.y);
+                hf_mma(sum[1], a.z, b.z, a.w, b.w, w.z, w.w);
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[i] += sum[i];
+            for (int i = 0; i < 4; ++i) acc[i] += sum[0][i] + sum[1][i];
         };
         if (g0 == 0) {
 #pragma unroll
-            for (int i = 0; i < HF_HELD; ++i)
-                if (i < here) multiply(i, held[i]);
+            for (int i0 = 0; i0 < HF_HELD; i0 += 4) {
+                if (i0 + 4 <= here) {                           // four groups' products side by side
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) multiply(i0 + i, held[i0 + i]);
+                } else {
+#pragma unroll
+                    for (int i = 0; i < 3; ++i)
+                        if (i0 + i < here) multiply(i0 + i, held[i0 + i]);
+                }
+            }
         }
         for (int i = g0 == 0 ? HF_HELD : 0; i < here; ++i) multiply(i, weights(g0 + i));
     }

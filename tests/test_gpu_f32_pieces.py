@@ -281,3 +281,26 @@ def test_scratch_is_bounded():
     got = K.gemm(a, w)
     for rows in (slice(0, 40), slice(at_once - 40, at_once), slice(at_once, at_once + 1)):
         assert torch.equal(got[rows], K.gemm(a[rows].clone(), w))
+
+
+@pytest.mark.parametrize("k", [256, 260, 512, 1024])
+@pytest.mark.parametrize("kind", ["random", "one sign", "left out", "left out, either sign"])
+def test_no_larger_an_error_than_the_chains(kind, k):
+    """From the shortest inner size on, where chains are short too; sums of one sign; values whose second and third pieces are as large as they can be, so that the
+    three products that are left out are 2^-24 of every product, all of one sign."""
+    from kapel_b200 import kernels as K
+
+    gen = torch.Generator(device="cuda").manual_seed(k)
+
+    def values(rows):
+        if kind == "random":
+            return torch.randn(rows, k, device="cuda", generator=gen)
+        if kind == "one sign":
+            return torch.rand(rows, k, device="cuda", generator=gen) + 0.5
+        x = (1.0 + 2.0 ** -8 - 2.0 ** -17) * torch.exp2(torch.randint(-3, 4, (rows, k), device="cuda", generator=gen).float())
+        return x if kind == "left out" else x * (2.0 * torch.randint(0, 2, (rows, k), device="cuda", generator=gen) - 1.0)
+
+    a, w = values(200), values(600)
+    want = a.double() @ w.double().T
+    off = [float((c.double() - want).norm() / want.norm()) for c in (K.gemm(a, w), chains(a, w))]
+    assert off[0] <= 1.01 * off[1], off                      # 120,000 results: the norms of two errors of one size agree to 1 %
