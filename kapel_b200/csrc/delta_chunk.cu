@@ -23,8 +23,9 @@ namespace kb {
 
 constexpr int DCH_THREADS = 128, DCH_E = 16, DCH_MAX_D = 128, DCH_LD = DCH_MAX_D + 4;
 
-// Requests by chunks whose rows lie ahead of row r0; all lanes of a warp call.
+// Requests by chunks whose rows lie ahead of row r0; all lanes of a warp call (at the kernels' beginning: the loads go beside their first ones).
 __device__ __forceinline__ int delta_chunks_before(const DeltaChunks& p, int r0) {
+    if (p.entries == 1) return 0;
     int before = 0;
     for (int i = threadIdx.x & 31; i < p.entries; i += 32) {
         const int start = p.entry_start[i];
@@ -39,7 +40,7 @@ delta_chunk_kernel(const DeltaChunks p) {
     __shared__ __align__(16) float kk[DCH_C][DCH_C + 4], qk[DCH_C][DCH_C + 4], decay[DCH_C][DCH_C + 4];      // [t][s]
     __shared__ float sg[DCH_C], sbeta[DCH_C];
     const int entry = blockIdx.z, h = blockIdx.y, per = p.heads / p.kv_heads, kvh = h / per;
-    const int r0 = p.entry_start[entry], r1 = p.entry_end[entry];
+    const int r0 = p.entry_start[entry], r1 = p.entry_end[entry], before = delta_chunks_before(p, r0);
     const int first = r0 + blockIdx.x * DCH_C, n = min(DCH_C, r1 - first);
     const int slot = p.slots[entry];
     if (r1 - r0 < p.from_rows || n <= 0 || slot <= 0 || slot >= p.n_slots) return;
@@ -52,7 +53,7 @@ delta_chunk_kernel(const DeltaChunks p) {
         *reinterpret_cast<float4*>(&sq[t][x]) = t < n ? *reinterpret_cast<const float4*>(p.qn + from) : none;
     }
     __syncthreads();
-    const int place = delta_chunk_place(first, delta_chunks_before(p, r0)), ld = delta_piece_row(d);
+    const int place = delta_chunk_place(first, before), ld = delta_piece_row(d);
     for (int i = h == kvh * per ? tid : DCH_C * d; i < DCH_C * (d >> 1); i += DCH_THREADS) {                  // their pieces, by the kv head's first head
         const int t = i / (d >> 1), x = (i - t * (d >> 1)) * 2;
         uint32_t* q = reinterpret_cast<uint32_t*>(p.qk + (((size_t)place * p.kv_heads + kvh) * 2 * DCH_C + t) * ld + x);
@@ -209,7 +210,7 @@ delta_chain_kernel(const DeltaChunks p) {
     extern __shared__ __align__(128) unsigned char dch_raw[];
     DchSmem& m = *reinterpret_cast<DchSmem*>(dch_raw);
     const int entry = blockIdx.z, head = blockIdx.y, c0 = blockIdx.x * DCH_E;
-    const int r0 = p.entry_start[entry], r1 = p.entry_end[entry];
+    const int r0 = p.entry_start[entry], r1 = p.entry_end[entry], before = delta_chunks_before(p, r0);
     const int slot = p.slots[entry];
     if (r1 - r0 < p.from_rows) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, d = p.d, e = p.e;
@@ -219,7 +220,7 @@ delta_chain_kernel(const DeltaChunks p) {
     }
     const int kvh = head / (p.heads / p.kv_heads);
     float* st = p.state + (size_t)slot * p.state_floats + p.state_off + ((size_t)head * e + c0) * d;      // [16][d]: a column of the memory lies together
-    const int before = delta_chunks_before(p, r0), chunks = (r1 - r0 + DCH_C - 1) / DCH_C, ld = delta_piece_row(d), image = DCH_C * ld;        // an operand's pieces of a chunk
+    const int chunks = (r1 - r0 + DCH_C - 1) / DCH_C, ld = delta_piece_row(d), image = DCH_C * ld;        // an operand's pieces of a chunk
     __nv_bfloat16* wq = reinterpret_cast<__nv_bfloat16*>(dch_raw + sizeof(DchSmem));                      // [2][W, queries]
     __nv_bfloat16* keys = wq + 4 * image;                                                                 // [2]
     if (tid == 0) {
