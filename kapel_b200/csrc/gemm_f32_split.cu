@@ -199,6 +199,7 @@ gemm_f32_pieces_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_c
         int place = b;
         for (int ch = b; ch < chunks; ch += 2) {
             bool there = at_mbar_wait(cut + b, (uint32_t)(ch >> 1) & 1u);
+            // With three places this warp meets one every second round; the round between is over: the weights' chunk ch is cut behind the products of ch - 3.
             if (!C::CUTS) there = there && at_mbar_wait(a_full + place, (uint32_t)(ch / C::PLACES) & 1u);
             there = there && at_mbar_wait(added + b, ((uint32_t)(ch >> 1) & 1u) ^ 1u);
             if (!__all_sync(0xffffffffu, there)) { failed = true; break; }
